@@ -2,69 +2,230 @@
 // tensor cores and no TF32.  This is the matrix product of the float32 engine.
 //
 // Each output element is one chain of fmaf over k = 0 .. K-1 in ascending order, so its value does
-// not depend on M, on the tile it falls in or on what else is in the batch.  libmir has no 32-bit
+// not depend on M, on the kernel and tile it falls in or on what else is in the batch.  libmir has no 32-bit
 // model path on CUDA (its ProjectionFormat has no F32 member, cuda/src/backend/linear/mod.rs:80-88);
 // this kernel exists to show faults that bf16 rounding hides.
+//
+// Two kernels, both fed by rings of cp.async stages whose rows keep their k order in shared memory, padded by four
+// floats so that eight neighbouring rows read as 16-byte pieces meet all banks once:
+//   gemm_f32_rows   up to 16 rows of A: bound by reading W once.  A CTA takes 16 rows of W and all of A; a thread owns one
+//                   output and walks down k, so the least a product can take is K dependent multiply-adds (four cycles
+//                   each, 4.2 us for 2,048), which the ring of four stages of 256 k hides behind the reads.
+//   gemm_f32_tile   more rows: bound by the multiply-adds.  A thread owns TM x TN outputs whose rows and columns lie
+//                   (tile / threads) apart, and reads four k of each with one load.
 #include "common.cuh"
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+namespace {
 
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ a, int lda,
-                                                        const float* __restrict__ w, int ldw,
-                                                        const float* __restrict__ bias, float* __restrict__ c, int ldc,
-                                                        int m, int n, int k, float beta) {
-  __shared__ float a_tile[BK][BM + 1];
-  __shared__ float w_tile[BK][BN + 1];
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void copy_async(float* to, const float* from, int bytes) {     // the rest of 16 bytes is zero
+  const unsigned at = (unsigned)__cvta_generic_to_shared(to);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at), "l"(from), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_async_one(float* to, const float* from, bool there) {
+  const unsigned at = (unsigned)__cvta_generic_to_shared(to);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at), "l"(from), "r"(there ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void copy_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory");
+}
+
+// ROWS rows of K-major data from row `row0` and column k0 on into [ROWS][DEPTH + 4]; what lies outside is zero.  WIDE: rows
+// start on 16-byte boundaries and k is a multiple of four.
+template <int ROWS, int DEPTH, int THREADS, bool WIDE>
+__device__ __forceinline__ void load_tile(float* tile, const float* __restrict__ from, int ld, int row0, int rows, int k0, int k) {
+  if (WIDE) {
+    constexpr int PIECES = DEPTH / 4;
+    for (int index = threadIdx.x; index < ROWS * PIECES; index += THREADS) {
+      const int r = index / PIECES, kk = (index % PIECES) * 4;
+      const bool there = row0 + r < rows && k0 + kk < k;
+      copy_async(tile + r * (DEPTH + 4) + kk, there ? from + (size_t)(row0 + r) * ld + k0 + kk : from, there ? 16 : 0);
+    }
+  } else {
+    for (int index = threadIdx.x; index < ROWS * DEPTH; index += THREADS) {
+      const int r = index / DEPTH, kk = index % DEPTH;
+      const bool there = row0 + r < rows && k0 + kk < k;
+      copy_async_one(tile + r * (DEPTH + 4) + kk, there ? from + (size_t)(row0 + r) * ld + k0 + kk : from, there);
+    }
+  }
+}
+
+__device__ __forceinline__ void finish(float* c, int ldc, const float* bias, float beta, int row, int column, float value) {
+  if (bias) value += bias[column];
+  float* dst = c + (size_t)row * ldc + column;
+  *dst = beta != 0.0f ? fmaf(beta, *dst, value) : value;
+}
+
+template <int BM, int BN, int TM, int TN, int DEPTH, int STAGES, bool WIDE>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, const float* __restrict__ bias,
+                     float* __restrict__ c, int ldc, int m, int n, int k, float beta) {
+  constexpr int ACROSS = BN / TN, DOWN = BM / TM, THREADS = ACROSS * DOWN, ROW = DEPTH + 4;
+  extern __shared__ __align__(16) float shared[];
   const int row0 = blockIdx.y * BM, col0 = blockIdx.x * BN;
-  const int ty = tid / (BN / TN), tx = tid % (BN / TN);
+  const int tx = threadIdx.x % ACROSS, ty = threadIdx.x / ACROSS;
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-
-  for (int k0 = 0; k0 < k; k0 += BK) {
-    // 64 x 16 elements of each operand, 256 threads: 4 elements each; consecutive threads read consecutive k.
+  const int steps = (k + DEPTH - 1) / DEPTH;
+  auto fetch = [&](int step) {
+    float* stage = shared + (step % STAGES) * (BM + BN) * ROW;
+    load_tile<BM, DEPTH, THREADS, WIDE>(stage, a, lda, row0, m, step * DEPTH, k);
+    load_tile<BN, DEPTH, THREADS, WIDE>(stage + BM * ROW, w, ldw, col0, n, step * DEPTH, k);
+  };
 #pragma unroll
-    for (int i = 0; i < (BM * BK) / 256; ++i) {
-      const int index = tid + i * 256;
-      const int r = index / BK, kk = index % BK;
-      const int gr = row0 + r, gk = k0 + kk;
-      a_tile[kk][r] = (gr < m && gk < k) ? a[(size_t)gr * lda + gk] : 0.0f;
-      const int gc = col0 + r;
-      w_tile[kk][r] = (gc < n && gk < k) ? w[(size_t)gc * ldw + gk] : 0.0f;
-    }
-    __syncthreads();
+  for (int step = 0; step < STAGES - 1; ++step) {
+    if (step < steps) fetch(step);
+    copy_commit();
+  }
+  for (int step = 0; step < steps; ++step) {
+    copy_wait<STAGES - 2>();
+    __syncthreads();                               // this stage is there for everybody, and the one before has been read
+    if (step + STAGES - 1 < steps) fetch(step + STAGES - 1);
+    copy_commit();
+    const float* at = shared + (step % STAGES) * (BM + BN) * ROW + ty * ROW;
+    const float* wt = shared + (step % STAGES) * (BM + BN) * ROW + (BM + tx) * ROW;
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float av[TM], wv[TN];
+    for (int kk = 0; kk < DEPTH; kk += 4) {
+      float4 av[TM], wv[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) av[i] = a_tile[kk][ty * TM + i];
+      for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const float4*>(at + i * DOWN * ROW + kk);
 #pragma unroll
-      for (int j = 0; j < TN; ++j) wv[j] = w_tile[kk][tx * TN + j];
+      for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const float4*>(wt + j * ACROSS * ROW + kk);
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+        for (int j = 0; j < TN; ++j) {
+          acc[i][j] = fmaf(av[i].x, wv[j].x, acc[i][j]);
+          acc[i][j] = fmaf(av[i].y, wv[j].y, acc[i][j]);
+          acc[i][j] = fmaf(av[i].z, wv[j].z, acc[i][j]);
+          acc[i][j] = fmaf(av[i].w, wv[j].w, acc[i][j]);
+        }
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
-    const int gr = row0 + ty * TM + i;
-    if (gr >= m) continue;
+    const int row = row0 + ty + i * DOWN;
+    if (row >= m) continue;
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
-      const int gc = col0 + tx * TN + j;
-      if (gc >= n) continue;
-      float value = acc[i][j];
-      if (bias) value += bias[gc];
-      float* dst = c + (size_t)gr * ldc + gc;
-      *dst = beta != 0.0f ? fmaf(beta, *dst, value) : value;
+      const int column = col0 + tx + j * ACROSS;
+      if (column < n) finish(c, ldc, bias, beta, row, column, acc[i][j]);
     }
   }
 }
+
+constexpr int kRowsColumns = 16, kRowsDepth = 256, kRowsStages = 4, kRowsThreads = 128;
+
+// MT: rows of A rounded up to a power of two (1 to 16).  With MT = 16 a thread owns two outputs.
+template <int MT, bool WIDE>
+__global__ void __launch_bounds__(kRowsThreads)
+gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, const float* __restrict__ bias,
+                     float* __restrict__ c, int ldc, int m, int n, int k, float beta) {
+  constexpr int ROW = kRowsDepth + 4, STAGE = (kRowsColumns + MT) * ROW;
+  constexpr int EACH = MT * kRowsColumns > kRowsThreads ? MT * kRowsColumns / kRowsThreads : 1;
+  constexpr int DOWN = MT / EACH;
+  extern __shared__ __align__(16) float shared[];
+  const int col0 = blockIdx.x * kRowsColumns;
+  const int tx = threadIdx.x % kRowsColumns, ty = threadIdx.x / kRowsColumns;
+  const bool owner = ty < DOWN;
+  float acc[EACH];
+#pragma unroll
+  for (int e = 0; e < EACH; ++e) acc[e] = 0.0f;
+  const int steps = (k + kRowsDepth - 1) / kRowsDepth;
+  auto fetch = [&](int step) {
+    float* stage = shared + (step % kRowsStages) * STAGE;
+    load_tile<kRowsColumns, kRowsDepth, kRowsThreads, WIDE>(stage, w, ldw, col0, n, step * kRowsDepth, k);
+    load_tile<MT, kRowsDepth, kRowsThreads, WIDE>(stage + kRowsColumns * ROW, a, lda, 0, m, step * kRowsDepth, k);
+  };
+#pragma unroll
+  for (int step = 0; step < kRowsStages - 1; ++step) {
+    if (step < steps) fetch(step);
+    copy_commit();
+  }
+  for (int step = 0; step < steps; ++step) {
+    copy_wait<kRowsStages - 2>();
+    __syncthreads();
+    if (step + kRowsStages - 1 < steps) fetch(step + kRowsStages - 1);
+    copy_commit();
+    if (!owner) continue;
+    const float* wt = shared + (step % kRowsStages) * STAGE + tx * ROW;
+    const float* at = shared + (step % kRowsStages) * STAGE + (kRowsColumns + ty) * ROW;
+#pragma unroll 16
+    for (int kk = 0; kk < kRowsDepth; kk += 4) {
+      const float4 wv = *reinterpret_cast<const float4*>(wt + kk);
+#pragma unroll
+      for (int e = 0; e < EACH; ++e) {
+        const float4 av = *reinterpret_cast<const float4*>(at + e * DOWN * ROW + kk);
+        acc[e] = fmaf(av.x, wv.x, acc[e]);
+        acc[e] = fmaf(av.y, wv.y, acc[e]);
+        acc[e] = fmaf(av.z, wv.z, acc[e]);
+        acc[e] = fmaf(av.w, wv.w, acc[e]);
+      }
+    }
+  }
+  if (!owner || col0 + tx >= n) return;
+#pragma unroll
+  for (int e = 0; e < EACH; ++e)
+    if (ty + e * DOWN < m) finish(c, ldc, bias, beta, ty + e * DOWN, col0 + tx, acc[e]);
+}
+
+struct Product {
+  const float* a; int lda;
+  const float* w; int ldw;
+  const float* bias;
+  float* c; int ldc;
+  int m, n, k;
+  float beta;
+  cudaStream_t stream;
+};
+
+template <typename Kernel>
+int launch(Kernel kernel, dim3 grid, int threads, int smem, const Product& p) {
+  const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) {
+    mir_set_error("gemm_f32: %s", cudaGetErrorString(err));
+    return MIR_CUDA_ERROR;
+  }
+  kernel<<<grid, threads, smem, p.stream>>>(p.a, p.lda, p.w, p.ldw, p.bias, p.c, p.ldc, p.m, p.n, p.k, p.beta);
+  return mir_check_launch("gemm_f32");
+}
+
+template <int MT, bool WIDE>
+int launch_rows(const Product& p) {
+  constexpr int smem = kRowsStages * (kRowsColumns + MT) * (kRowsDepth + 4) * (int)sizeof(float);
+  return launch(gemm_f32_rows_kernel<MT, WIDE>, dim3((p.n + kRowsColumns - 1) / kRowsColumns), kRowsThreads, smem, p);
+}
+
+template <int BM, int BN, int TM, int TN, bool WIDE>
+int launch_tile(const Product& p) {
+  constexpr int DEPTH = 32, STAGES = 3, smem = STAGES * (BM + BN) * (DEPTH + 4) * (int)sizeof(float);
+  const dim3 grid((p.n + BN - 1) / BN, (p.m + BM - 1) / BM);
+  if (grid.y > 65535) {
+    mir_set_error("gemm_f32: %d rows exceed the grid limit", p.m);
+    return MIR_BAD_ARGUMENT;
+  }
+  return launch(gemm_f32_tile_kernel<BM, BN, TM, TN, DEPTH, STAGES, WIDE>, grid, (BM / TM) * (BN / TN), smem, p);
+}
+
+template <bool WIDE>
+int choose(const Product& p) {
+  if (p.m <= 1) return launch_rows<1, WIDE>(p);
+  if (p.m <= 2) return launch_rows<2, WIDE>(p);
+  if (p.m <= 4) return launch_rows<4, WIDE>(p);
+  if (p.m <= 8) return launch_rows<8, WIDE>(p);
+  if (p.m <= 16) return launch_rows<16, WIDE>(p);
+  if (p.m <= 32) return launch_tile<32, 64, 4, 4, WIDE>(p);
+  // A thread of the large tile reads half as much from shared memory for each multiply-add; it is taken once two CTAs of
+  // it for every SM exist (two are resident).
+  const long long large = (long long)((p.m + 127) / 128) * ((p.n + 127) / 128);
+  if (large >= 2LL * mir_sm_count()) return launch_tile<128, 128, 8, 8, WIDE>(p);
+  return launch_tile<64, 64, 8, 4, WIDE>(p);
+}
+
+}  // namespace
 
 MIR_EXPORT int mir_gemm_f32(const float* a, int lda, const float* w, int ldw, const float* bias, float* c, int ldc,
                             int m, int n, int k, float beta, cudaStream_t stream) {
@@ -73,11 +234,7 @@ MIR_EXPORT int mir_gemm_f32(const float* a, int lda, const float* w, int ldw, co
     mir_set_error("gemm_f32: bad sizes m %d n %d k %d lda %d ldw %d ldc %d", m, n, k, lda, ldw, ldc);
     return MIR_BAD_ARGUMENT;
   }
-  const dim3 grid((n + BN - 1) / BN, (m + BM - 1) / BM);
-  if (grid.y > 65535) {
-    mir_set_error("gemm_f32: %d rows exceed the grid limit", m);
-    return MIR_BAD_ARGUMENT;
-  }
-  gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, lda, w, ldw, bias, c, ldc, m, n, k, beta);
-  return mir_check_launch("gemm_f32");
+  const Product p{a, lda, w, ldw, bias, c, ldc, m, n, k, beta, stream};
+  const bool wide = k % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)a | (uintptr_t)w) % 16 == 0;
+  return wide ? choose<true>(p) : choose<false>(p);
 }

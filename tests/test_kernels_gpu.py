@@ -114,6 +114,25 @@ def test_gemm_f32_rows_do_not_depend_on_the_batch():
         assert torch.equal(part, whole[begin:end])
 
 
+@pytest.mark.parametrize("n,k", [(15, 4), (65, 260), (129, 1028), (200, 258), (130, 37)])
+def test_gemm_f32_rows_are_the_same_bits_in_every_kernel(n, k):
+    """The kernels of 1 to 16 rows and the tiles (32, 64 and, with many rows, 128 high), with 16-byte and with single loads."""
+    from libmir_b200 import kernels
+    torch.manual_seed(6)
+    many = 128 * (2 * 148) // max(1, -(-n // 128)) + 5
+    x, w, bias = torch.randn(many, k), torch.randn(n, k), torch.randn(n)
+    base = torch.randn(many, n)
+    whole, gx, gw, gb = cuda(base.clone()), cuda(x), cuda(w), cuda(bias)
+    kernels.linear(gx, gw, whole, gb, accumulate=True)
+    exact = base.double() + plain_impl.linear(x.double(), w, bias)
+    assert float((whole.double().cpu() - exact).abs().max()) <= 2e-7 * k * float(exact.abs().max() + 1)
+    for begin, count in ((0, 1), (3, 2), (1, 3), (5, 5), (2, 8), (7, 9), (4, 16), (9, 17), (0, 32), (11, 33), (6, 64), (3, 65),
+                         (8, 129), (many - 1, 1)):
+        part = cuda(base[begin:begin + count].clone())
+        kernels.linear(gx[begin:begin + count], gw, part, gb, accumulate=True)
+        assert torch.equal(part, whole[begin:begin + count]), (begin, count)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 136, 264), (8, 200, 72), (50, 136, 264), (300, 520, 128)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 def test_gemm_bf16(m, n, k, out_dtype):
