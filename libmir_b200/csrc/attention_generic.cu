@@ -32,7 +32,10 @@ using namespace mir;
 constexpr int kMaxHeadDim = 640;
 constexpr int kWarpsPerBlock = 4;
 
-template <typename T>
+// PIECES: value channels a lane holds (value_dim <= 32 PIECES), so that heads of up to 128 channels walk over four pieces of
+// a key's value instead of twenty that are mostly empty (three prompts of 63 to 130 tokens, 16 heads of 128: 4.3 ms of 51 in
+// a model's pass before).
+template <typename T, int PIECES>
 __global__ void paged_attention_generic_kernel(
     const T* __restrict__ q, size_t q_token_stride, T* __restrict__ out, const T* __restrict__ k_pages,
     const T* __restrict__ v_pages, const int* __restrict__ block_table, int table_width,
@@ -57,9 +60,9 @@ __global__ void paged_attention_generic_kernel(
   for (int d = lane; d < head_dim; d += 32) q_shared[warp][d] = to_float(q_row[d]);
   __syncwarp();
 
-  float acc[kMaxHeadDim / 32];
+  float acc[PIECES];
 #pragma unroll
-  for (int i = 0; i < kMaxHeadDim / 32; ++i) acc[i] = 0.0f;
+  for (int i = 0; i < PIECES; ++i) acc[i] = 0.0f;
   float running_max = -FLT_MAX;
   float denominator = 0.0f;
 
@@ -100,14 +103,14 @@ __global__ void paged_attention_generic_kernel(
     const float weight = valid ? expf(score - next_max) : 0.0f;
     denominator = denominator * correction + warp_sum(weight);
 #pragma unroll
-    for (int i = 0; i < kMaxHeadDim / 32; ++i) acc[i] *= correction;
+    for (int i = 0; i < PIECES; ++i) acc[i] *= correction;
     const int keys_here = min(32, last - base + 1);
     for (int j = 0; j < keys_here; ++j) {
       const float w = __shfl_sync(0xffffffffu, weight, j);
       const size_t offset = __shfl_sync(0xffffffffu, key_offset, j);
       const T* v_row = v_pages + offset * value_row_width;
 #pragma unroll
-      for (int i = 0; i < kMaxHeadDim / 32; ++i) {
+      for (int i = 0; i < PIECES; ++i) {
         const int d = lane + 32 * i;
         if (d < value_dim) acc[i] = fmaf(w, to_float(v_row[d]), acc[i]);
       }
@@ -121,14 +124,14 @@ __global__ void paged_attention_generic_kernel(
     const float correction = expf(running_max - next_max);
     denominator = denominator * correction + expf(sink - next_max);
 #pragma unroll
-    for (int i = 0; i < kMaxHeadDim / 32; ++i) acc[i] *= correction;
+    for (int i = 0; i < PIECES; ++i) acc[i] *= correction;
   }
   T* out_row = out + ((size_t)token * heads + head) * value_dim;
   const T* gate_row = gate != nullptr ? gate + (size_t)token * gate_stride + (size_t)head * (gate_per_head ? 1 : value_dim)
                                       : nullptr;
   const float inverse = denominator > 0.0f ? 1.0f / denominator : 0.0f;   // a padded row has no keys
 #pragma unroll
-  for (int i = 0; i < kMaxHeadDim / 32; ++i) {
+  for (int i = 0; i < PIECES; ++i) {
     const int d = lane + 32 * i;
     if (d < value_dim) {
       float result = acc[i] * inverse;
@@ -166,17 +169,18 @@ MIR_EXPORT int mir_paged_attention_generic(int bf16, const void* q, long long q_
   if (rel_bias != nullptr && rel_rows <= 0) { mir_set_error("paged_attention: a bias by distance needs rows"); return MIR_BAD_ARGUMENT; }
   const dim3 grid(tokens, (heads + kWarpsPerBlock - 1) / kWarpsPerBlock);
   const dim3 block(32, kWarpsPerBlock);
-  if (bf16)
-    paged_attention_generic_kernel<<<grid, block, 0, stream>>>(
-        (const __nv_bfloat16*)q, (size_t)q_token_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)k_pages,
-        (const __nv_bfloat16*)v_pages, block_table, table_width, row_of_token, positions, page_size, heads, kv_heads,
-        head_dim, value_dim, value_row_width, scale, window, keep_first, sinks, (const __nv_bfloat16*)gate,
-        (size_t)gate_stride, gate_per_head, softcap, rel_bias, rel_rows, chunk, slopes);
-  else
-    paged_attention_generic_kernel<<<grid, block, 0, stream>>>(
-        (const float*)q, (size_t)q_token_stride, (float*)out, (const float*)k_pages, (const float*)v_pages,
-        block_table, table_width, row_of_token, positions, page_size, heads, kv_heads, head_dim, value_dim,
-        value_row_width, scale, window, keep_first, sinks, (const float*)gate, (size_t)gate_stride, gate_per_head, softcap,
-        rel_bias, rel_rows, chunk, slopes);
+#define MIR_GENERIC(T, PIECES)                                                                                             \
+  paged_attention_generic_kernel<T, PIECES><<<grid, block, 0, stream>>>(                                                   \
+      (const T*)q, (size_t)q_token_stride, (T*)out, (const T*)k_pages, (const T*)v_pages, block_table, table_width,        \
+      row_of_token, positions, page_size, heads, kv_heads, head_dim, value_dim, value_row_width, scale, window,            \
+      keep_first, sinks, (const T*)gate, (size_t)gate_stride, gate_per_head, softcap, rel_bias, rel_rows, chunk, slopes)
+  if (bf16) {
+    if (value_dim <= 128) MIR_GENERIC(__nv_bfloat16, 4);
+    else MIR_GENERIC(__nv_bfloat16, kMaxHeadDim / 32);
+  } else {
+    if (value_dim <= 128) MIR_GENERIC(float, 4);
+    else MIR_GENERIC(float, kMaxHeadDim / 32);
+  }
+#undef MIR_GENERIC
   return mir_check_launch("paged_attention_generic");
 }
