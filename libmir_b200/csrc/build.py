@@ -51,7 +51,7 @@ LIBRARIES = {
 }
 # the bfloat16 library with time stamps inside its kernels (trace.cuh), for bench.py --phase trace
 LIBRARIES["bf16_trace"] = dict(LIBRARIES["bf16"], defines=LIBRARIES["bf16"]["defines"] + ["-DMIR_TRACE"])
-HEADERS = ["common.cuh", "launchers.h", "trace.cuh", "short_conv.cuh"]
+HEADERS = ["common.cuh", "launchers.h", "trace.cuh", "short_conv.cuh", "scan_pairs.cuh"]
 
 
 def _nvcc() -> str:

@@ -11,12 +11,12 @@
 //   delta_rule_prepare the short convolution (short_conv.cu), then what else the recurrence needs of a token: q and k as unit vectors,
 //                     sigmoid(beta), the decay; all tokens in parallel.
 //   delta_rule_scan   the recurrence: a few lanes per (request, head, value channel) hold one column of S in
-//                     registers, walk over the request's tokens of this step, and write the column back.  No shared
-//                     memory, no block barrier: the two dot products per token are a few shuffles.  The state is
+//                     registers, walk over the request's tokens of this step, and write the column back.  The state is
 //                     stored [head][value channel][key channel], so a column is one contiguous run.
 //   gated_head_norm   out = o / rms(o) * weight * act(gate) per (token, head), act = silu or sigmoid.
 // A row of a captured decode batch whose position is negative is padding: nothing of it is read or written.
 #include "common.cuh"
+#include "scan_pairs.cuh"
 #include "short_conv.cuh"
 
 using namespace mir;
@@ -152,201 +152,211 @@ __global__ void delta_rule_prepare_kernel(const T* __restrict__ x, long long ldx
         expf(-expf(a_log[j / per_head]) * softplus(to_float(decay_raw[(size_t)token * ld_decay + j]) + dt_bias[j]));
 }
 
-__device__ __forceinline__ void copy_async(float* dst, const float* src, bool wide) {
-  const unsigned target = (unsigned)__cvta_generic_to_shared(dst);
-  if (wide) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(target), "l"(src) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(target), "l"(src) : "memory");
-}
-__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-constexpr int kScanWarps = 4;
+constexpr int kScanWarps = 4;           // that walk
+constexpr int kFetchWarps = 4;          // that copy what the others will need
+constexpr int kScanThreads = (kScanWarps + kFetchWarps) * 32;
 constexpr int kScanChunk = 16;          // tokens whose inputs one stage of shared memory holds
+constexpr int kScanStages = 3;
 
-// The recurrence.  LANES lanes share one column of S (one value channel of one head): lane l holds the key channels
-// 4 (m LANES + l) .. + 3 for m < PER / 4 in registers, so a warp works on 32 / LANES columns at once, the two dot
+// The recurrence.  LANES lanes share C columns of S (C value channels of one head): lane l holds the key channels
+// 4 (m LANES + l) .. + 3 for m < PER / 4 in registers, so a warp works on 32 / LANES * C columns at once, the two dot
 // products per token are log2(LANES) shuffle steps, and the state of a column (stored [head][value channel][key
 // channel]) is read and written in 16-byte pieces that lie side by side across the lanes.  The inputs of a token are
-// the same for every column of its head: the CTA (all its warps work on columns of one head) copies them for 16
-// tokens at a time into shared memory with cp.async, two stages, so that the walk over the tokens never waits for
-// global memory.  blockDim (32, kScanWarps), grid (rows, heads, ceil(value_dim / (kScanWarps * 32 / LANES))).
+// the same for every column of its head: the CTA (all its warps work on columns of one head) has kFetchWarps more that copy
+// them for 16 tokens at a time into shared memory with cp.async, three stages.  blockDim (32, kScanWarps + kFetchWarps), grid
+// (rows, heads, ceil(value_dim / (kScanWarps * 32 / LANES * C))).
+//
+// What bounds it: the chain from one token's state to the next (a decay, a dot product of PER channels, the sum over the
+// lanes, the write's factor and a multiply-add) and the instructions of the one walking warp a scheduler has, which can
+// hide little of each other.  So what can be kept away from that warp is: the copies and their addresses belong to the
+// fetching warps, a token's inputs are in registers before the token before it ends, the read-out is summed over the
+// lanes beside the next token's S^T k, a lane has C columns that share a token's inputs, and the arithmetic goes two
+// numbers an instruction.  Every number is formed by the same operations in the same order
+// whatever the step's shape, so a request's 32-bit results do not depend on how it was cut.
 //   qkv    [tokens, 2 G D + H V] 32-bit: unit q | unit k | v (delta_rule_prepare)
 //   beta   [tokens, H]; decay [tokens, H D] (PER_CHANNEL) or [tokens, H]
 //   state  [slots, H, V, D] 32-bit;  out [tokens, H V] 32-bit: o before the head norm
-template <int LANES, int PER, bool PER_CHANNEL>
-__global__ void __launch_bounds__(kScanWarps * 32)
+template <int LANES, int PER, int C, bool PER_CHANNEL>
+__global__ void __launch_bounds__(kScanThreads, 2)
 delta_rule_scan_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
                        float* __restrict__ state, const int* __restrict__ query_starts,
                        const int* __restrict__ state_slots, const int* __restrict__ positions,
                        float* __restrict__ out, int heads, int kv_heads, int key_dim, int value_dim) {
   static_assert(PER % 4 == 0, "a lane holds whole 16-byte pieces");
-  extern __shared__ __align__(16) float staged[];              // [2 stages][kScanChunk tokens][row]
+  extern __shared__ __align__(16) float staged[];              // [kScanStages][kScanChunk tokens][row]
   grid_launch_dependents();
   grid_dependency_wait();
-  constexpr int COLUMNS = 32 / LANES;                           // per warp
+  constexpr int COLUMNS = 32 / LANES * C;                       // per warp
   constexpr int BLOCK_COLUMNS = COLUMNS * kScanWarps;
   constexpr int PADDED = LANES * PER;                           // key channels with padding
   constexpr int DECAYS = PER_CHANNEL ? PADDED : 4;
-  constexpr int ROW = 2 * PADDED + DECAYS + 4 + BLOCK_COLUMNS;  // q | k | decay | beta | v of this CTA's columns
-  const int thread = threadIdx.y * 32 + threadIdx.x;
-  const int l = threadIdx.x % LANES;
+  constexpr int VALUES = 2 * PADDED + DECAYS + 4;               // where a row's values begin
+  constexpr int ROW = VALUES + BLOCK_COLUMNS;                   // q | k | decay | beta | v of this CTA's columns
+  constexpr int STAGE = kScanChunk * ROW;
+  const int lane = threadIdx.x;
   const int row = blockIdx.x, head = blockIdx.y;
   const int first_column = blockIdx.z * BLOCK_COLUMNS;
-  const int local_column = threadIdx.y * COLUMNS + threadIdx.x / LANES;
-  const int column = first_column + local_column;
   const int start = query_starts[row], end = query_starts[row + 1];
   if (end <= start || positions[start] < 0) return;             // the whole CTA: an empty or padding row
-  const bool active = column < value_dim;                        // idle lanes still take part in the shuffles
-  const int kv_head = head / (heads / kv_heads);
   const int width = 2 * kv_heads * key_dim + heads * value_dim;
-  const int g_width = PER_CHANNEL ? heads * key_dim : heads;
   // 16-byte accesses: every piece lies wholly inside or outside the head, and every row starts on a 16-byte boundary
   const bool wide = (key_dim % 4 == 0) && (width % 4 == 0);
-  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + (active ? column : 0)) * key_dim;
-
-  // one stage: the inputs of tokens [from, from + kScanChunk) of this request, zero where a head is narrower than PADDED
-  auto stage_in = [&](int from, float* dst) {
-    const int count = min(kScanChunk, end - from);
-    const int pieces = wide ? 4 : 1;
-    const int per_row = (2 * key_dim + (PER_CHANNEL ? key_dim : 0)) / pieces;
-    for (int index = thread; index < count * per_row; index += kScanWarps * 32) {
-      const int t = index / per_row, e = (index - t * per_row) * pieces;
-      const int which = e / key_dim, i = e - which * key_dim;    // 0 q, 1 k, 2 decay
-      const float* src = which == 2 ? decay + (size_t)(from + t) * g_width + (size_t)head * key_dim + i
-                                    : qkv + (size_t)(from + t) * width + (size_t)(which * kv_heads + kv_head) * key_dim + i;
-      copy_async(dst + t * ROW + which * PADDED + i, src, wide);
-    }
-    for (int index = thread; index < count * (BLOCK_COLUMNS + 2); index += kScanWarps * 32) {
-      const int t = index / (BLOCK_COLUMNS + 2), e = index - t * (BLOCK_COLUMNS + 2);
-      float* target = dst + t * ROW + 2 * PADDED + DECAYS;
-      if (e == 0) copy_async(target, beta + (size_t)(from + t) * heads + head, false);
-      else if (e == 1) { if (!PER_CHANNEL) copy_async(target - DECAYS, decay + (size_t)(from + t) * g_width + head, false); }
-      else if (first_column + e - 2 < value_dim)
-        copy_async(target + 4 + e - 2, qkv + (size_t)(from + t) * width + (size_t)2 * kv_heads * key_dim +
-                                           (size_t)head * value_dim + first_column + e - 2, false);
-    }
-  };
-  // padding channels (key_dim < PADDED) are read as q = k = 0: zero them once in both stages
-  if (key_dim < PADDED)
-    for (int index = thread; index < 2 * kScanChunk * ROW; index += kScanWarps * 32) staged[index] = 0.0f;
-  __syncthreads();
-
-  float s[PER];
-#pragma unroll
-  for (int m = 0; m < PER; m += 4) {
-    const int i = (m / 4 * LANES + l) * 4;
-    if (wide) {
-      const float4 piece = (active && i < key_dim) ? *reinterpret_cast<const float4*>(column_state + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-      s[m] = piece.x; s[m + 1] = piece.y; s[m + 2] = piece.z; s[m + 3] = piece.w;
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) s[m + e] = (active && i + e < key_dim) ? column_state[i + e] : 0.0f;
-    }
-  }
-
-  stage_in(start, staged);
-  copy_commit();
-  int stage = 0;
-  float pending = 0.0f;                                          // the last token's read-out, not yet summed over the lanes
-  bool has_pending = false;
-  __shared__ __align__(16) float exchange[kScanWarps][2][64];   // [warp][token parity][S^T k parts | read-out parts]
-  int parity = 0;
-  auto sum_over_lanes = [&](float& first, float& second) {       // both sums in one fixed order, whichever token it is
-    float* parts = exchange[threadIdx.y][parity];
-    parts[threadIdx.x] = first;
-    parts[32 + threadIdx.x] = second;
-    __syncwarp();
-    const float* mine = parts + (threadIdx.x / LANES) * LANES;
-    float sum_a = 0.0f, sum_b = 0.0f;
-#pragma unroll
-    for (int piece = 0; piece < LANES; piece += 4) {
-      const float4 a = *reinterpret_cast<const float4*>(mine + piece);
-      const float4 b = *reinterpret_cast<const float4*>(mine + 32 + piece);
-      sum_a += (a.x + a.y) + (a.z + a.w);
-      sum_b += (b.x + b.y) + (b.z + b.w);
-    }
-    first = sum_a;
-    second = sum_b;
-    parity ^= 1;
-  };
-  const bool writer = l == 0 && active;
-  const size_t out_step = (size_t)heads * value_dim;
-  float* out_at = out + ((size_t)start * heads + head) * value_dim + (active ? column : 0) - out_step;   // the pending token's place
-  for (int from = start; from < end; from += kScanChunk, stage ^= 1) {
-    if (from + kScanChunk < end) stage_in(from + kScanChunk, staged + (stage ^ 1) * kScanChunk * ROW);
-    copy_commit();
-    copy_wait<1>();
+  // padding channels (key_dim < PADDED) are read as q = k = 0: zero them once in all stages
+  if (key_dim < PADDED) {
+    for (int index = threadIdx.y * 32 + lane; index < kScanStages * STAGE; index += kScanThreads) staged[index] = 0.0f;
     __syncthreads();
-    const int count = min(kScanChunk, end - from);
-    const float* in = staged + stage * kScanChunk * ROW - ROW;
-#pragma unroll 2
-    for (int t = 0; t < count; ++t) {
-      in += ROW;
-      const float b = in[2 * PADDED + DECAYS];
-      const float v = in[2 * PADDED + DECAYS + 4 + local_column];
-      const float head_decay = in[2 * PADDED];
-      float k[PER];
-      float seen[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  }
+  const int chunks = (end - start + kScanChunk - 1) / kScanChunk;
+
+  if (threadIdx.y >= kScanWarps) {                              // the fetching warps: tokens w, w + kFetchWarps, ... of a chunk
+    const int kv_head = head / (heads / kv_heads), mine = threadIdx.y - kScanWarps;
+    const int g_width = PER_CHANNEL ? heads * key_dim : heads;
+    const bool wide_values = wide && value_dim % 4 == 0;
+    const int step = wide ? 4 : 1, value_step = wide_values ? 4 : 1;
+    const size_t key_at = (size_t)kv_heads * key_dim;
+    const float* q0 = qkv + (size_t)kv_head * key_dim;
+    const float* v0 = qkv + 2 * key_at + (size_t)head * value_dim + first_column;
+    const float* b0 = beta + head;
+    const float* g0 = decay + (size_t)head * (PER_CHANNEL ? key_dim : 1);
+    const bool my_value = lane * value_step < BLOCK_COLUMNS && first_column + lane * value_step < value_dim;
+    auto fetch = [&](int chunk) {
+      const int from = start + chunk * kScanChunk;
 #pragma unroll
-      for (int m = 0; m < PER; m += 4) {
-        const int i = (m / 4 * LANES + l) * 4;
-        const float4 key = *reinterpret_cast<const float4*>(in + PADDED + i);
-        float4 g = make_float4(head_decay, head_decay, head_decay, head_decay);
-        if (PER_CHANNEL) g = *reinterpret_cast<const float4*>(in + 2 * PADDED + i);
-        k[m] = key.x; k[m + 1] = key.y; k[m + 2] = key.z; k[m + 3] = key.w;
-        s[m] *= g.x; s[m + 1] *= g.y; s[m + 2] *= g.z; s[m + 3] *= g.w;
-        seen[0] = fmaf(s[m], key.x, seen[0]);
-        seen[1] = fmaf(s[m + 1], key.y, seen[1]);
-        seen[2] = fmaf(s[m + 2], key.z, seen[2]);
-        seen[3] = fmaf(s[m + 3], key.w, seen[3]);
+      for (int tt = 0; tt < kScanChunk / kFetchWarps; ++tt) {
+        const int t = mine + tt * kFetchWarps;
+        const size_t token = from + t;
+        if (from + t >= end) break;
+        float* to = staged + (chunk % kScanStages) * STAGE + t * ROW;
+        const float* q = q0 + token * width;
+        const float* g = g0 + token * g_width;
+        if (wide) {
+          for (int i = lane * 4; i < key_dim; i += 128) {
+            copy_async(to + i, q + i, true);
+            copy_async(to + PADDED + i, q + key_at + i, true);
+            if (PER_CHANNEL) copy_async(to + 2 * PADDED + i, g + i, true);
+          }
+        } else {
+          for (int i = lane * step; i < key_dim; i += 32 * step) {
+            copy_async(to + i, q + i, false);
+            copy_async(to + PADDED + i, q + key_at + i, false);
+            if (PER_CHANNEL) copy_async(to + 2 * PADDED + i, g + i, false);
+          }
+        }
+        if (my_value) copy_async(to + VALUES + lane * value_step, v0 + token * width + lane * value_step, wide_values);
+        // one copy of 4 bytes by two lanes: the write's factor, and (with a decay a head) the decay
+        if (lane >= (PER_CHANNEL ? 31 : 30))
+          copy_async(to + 2 * PADDED + (lane == 31 ? DECAYS : 0), lane == 31 ? b0 + token * heads : g, false);
       }
-      float total = (seen[0] + seen[1]) + (seen[2] + seen[3]);
-      // Two sums over the lanes of a column at once: this token's S^T k and the token before's read-out, which is not
-      // on the path to the next state.  The lanes exchange their parts through shared memory (a store, a warp barrier
-      // and 16-byte loads that every lane of the column adds up in the same order) rather than by shuffles: a chain
-      // of log2(LANES) dependent shuffles costs this lone warp more than the round trip.  Two buffers by the
-      // token's parity: a lane may still read one while the next token's parts are written.
-      sum_over_lanes(total, pending);
-      if (has_pending && writer) *out_at = pending;
+      copy_commit();
+    };
+    fetch(0);
+    if (chunks > 1) fetch(1); else copy_commit();
+    copy_wait<1>();
+    __syncthreads();                                             // the first chunk is there
+    for (int chunk = 0; chunk < chunks; ++chunk) {               // (into the stage of the chunk that was walked last)
+      if (chunk + 2 < chunks) fetch(chunk + 2); else copy_commit();
+      copy_wait<1>();
+      __syncthreads();                                           // this chunk has been walked, and the next one is there
+    }
+    copy_wait<0>();
+    return;
+  }
+
+  const int l = lane % LANES;
+  const int local_column = threadIdx.y * COLUMNS + lane / LANES * C;
+  const int column = first_column + local_column;                // idle lanes (beyond value_dim) still take part in the shuffles
+  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + column) * key_dim;
+  Pair s[C][PER / 2];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    load_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, column + c < value_dim, wide);
+
+  struct Inputs {
+    Pair q[PER / 2], k[PER / 2], g[PER_CHANNEL ? PER / 2 : 1];
+    float beta, value[C];
+  };
+  auto load = [&](Inputs& in, const float* from) {
+#pragma unroll
+    for (int m = 0; m < PER; m += 4) {
+      const int i = (m / 4 * LANES + l) * 4;
+      const ulonglong2 key = *reinterpret_cast<const ulonglong2*>(from + PADDED + i);
+      in.k[m / 2] = key.x; in.k[m / 2 + 1] = key.y;
+      if (PER_CHANNEL) {
+        const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(from + 2 * PADDED + i);
+        in.g[m / 2] = g.x; in.g[m / 2 + 1] = g.y;
+      }
+      const ulonglong2 query = *reinterpret_cast<const ulonglong2*>(from + i);
+      in.q[m / 2] = query.x; in.q[m / 2 + 1] = query.y;
+    }
+    if (!PER_CHANNEL) in.g[0] = pair_from(from[2 * PADDED], from[2 * PADDED]);
+    in.beta = from[2 * PADDED + DECAYS];
+#pragma unroll
+    for (int c = 0; c < C; ++c) in.value[c] = from[VALUES + local_column + c];
+  };
+  float pending[C];                                              // the last token's read-outs, not yet summed over the lanes
+#pragma unroll
+  for (int c = 0; c < C; ++c) pending[c] = 0.0f;
+  const int my_column = lane_sum<C>(l);                          // of the C columns, the one whose read-out this lane writes
+  const bool writer = l < C && column + my_column < value_dim;
+  const size_t out_step = (size_t)heads * value_dim;
+  float* out_at = out + ((size_t)start * heads + head) * value_dim + column + my_column;
+  bool has_pending = false;
+  auto walk = [&](const Inputs& in) {
+    float total[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      Pair seen[2] = {0, 0};
+#pragma unroll
+      for (int m = 0; m < PER / 2; ++m) {
+        s[c][m] = pair_mul(s[c][m], in.g[PER_CHANNEL ? m : 0]);
+        seen[m & 1] = pair_fma(s[c][m], in.k[m], seen[m & 1]);
+      }
+      total[c] = pair_total(seen);
+    }
+#pragma unroll
+    for (int step = 1; step < LANES; step <<= 1)
+#pragma unroll
+      for (int c = 0; c < C; ++c) total[c] += __shfl_xor_sync(0xffffffffu, total[c], step);
+    const float read_out = sum_lanes<LANES, C>(pending, l);
+    if (has_pending) {
+      if (writer) *out_at = read_out;
       out_at += out_step;
-      const float update = b * (v - total);
-      float read[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    }
 #pragma unroll
-      for (int m = 0; m < PER; m += 4) {
-        const int i = (m / 4 * LANES + l) * 4;
-        const float4 query = *reinterpret_cast<const float4*>(in + i);
-        s[m] = fmaf(k[m], update, s[m]);
-        s[m + 1] = fmaf(k[m + 1], update, s[m + 1]);
-        s[m + 2] = fmaf(k[m + 2], update, s[m + 2]);
-        s[m + 3] = fmaf(k[m + 3], update, s[m + 3]);
-        read[0] = fmaf(s[m], query.x, read[0]);
-        read[1] = fmaf(s[m + 1], query.y, read[1]);
-        read[2] = fmaf(s[m + 2], query.z, read[2]);
-        read[3] = fmaf(s[m + 3], query.w, read[3]);
+    for (int c = 0; c < C; ++c) {
+      const float update = in.beta * (in.value[c] - total[c]);
+      const Pair both = pair_from(update, update);
+      Pair read[2] = {0, 0};
+#pragma unroll
+      for (int m = 0; m < PER / 2; ++m) {
+        s[c][m] = pair_fma(in.k[m], both, s[c][m]);
+        read[m & 1] = pair_fma(s[c][m], in.q[m], read[m & 1]);
       }
-      pending = (read[0] + read[1]) + (read[2] + read[3]);
-      has_pending = true;
+      pending[c] = pair_total(read);
     }
-    __syncthreads();                                              // the stage is free for the chunk after next
-  }
-  copy_wait<0>();
-  {
-    float unused = 0.0f;
-    sum_over_lanes(unused, pending);                             // the last token's read-out
-  }
-  if (!active) return;
-  if (l == 0) *out_at = pending;
-#pragma unroll
-  for (int m = 0; m < PER; m += 4) {
-    const int i = (m / 4 * LANES + l) * 4;
-    if (wide) {
-      if (i < key_dim) *reinterpret_cast<float4*>(column_state + i) = make_float4(s[m], s[m + 1], s[m + 2], s[m + 3]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (i + e < key_dim) column_state[i + e] = s[m + e];
+    has_pending = true;
+  };
+  __syncthreads();                                               // the first chunk is there
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int count = min(kScanChunk, end - start - chunk * kScanChunk);
+    const float* in = staged + (chunk % kScanStages) * STAGE;
+    Inputs even, odd;
+    load(even, in);
+    int t = 0;
+    for (; t + 2 <= count; t += 2, in += 2 * ROW) {
+      load(odd, in + ROW);
+      walk(even);
+      if (t + 2 < count) load(even, in + 2 * ROW);
+      walk(odd);
     }
+    if (t < count) walk(even);
+    __syncthreads();                                             // this chunk has been walked, and the next one is there
   }
+  const float read_out = sum_lanes<LANES, C>(pending, l);        // the last token's
+  if (writer) *out_at = read_out;
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, wide);
 }
 
 // One warp per (token, head): out = o / sqrt(mean(o^2) + eps) * weight * act(gate); the weight is [value_dim], the
@@ -480,17 +490,17 @@ constexpr int kWideNormColumns = 512, kWideNormLimit = 16384;   // rows of these
 // How many lanes share a column of the state: 0 lets the launcher choose, 8 / 16 / 32 fix it (for measurements).
 int g_scan_lanes = 0;
 
-template <int LANES, int PER, bool PER_CHANNEL>
+template <int LANES, int PER, int C, bool PER_CHANNEL>
 int launch_scan_as(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
                    const int* query_starts, const int* state_slots, const int* positions, float* out, int rows,
                    int heads, int kv_heads, int key_dim, int value_dim) {
-  constexpr int columns = kScanWarps * (32 / LANES);
+  constexpr int columns = kScanWarps * (32 / LANES) * C;
   constexpr int padded = LANES * PER;
   constexpr int row = 2 * padded + (PER_CHANNEL ? padded : 4) + 4 + columns;
-  constexpr size_t smem = (size_t)2 * kScanChunk * row * sizeof(float);
+  constexpr size_t smem = (size_t)kScanStages * kScanChunk * row * sizeof(float);
   static bool raised = false;                                    // more than 48 KB of shared memory needs the opt-in
   if (smem > 48 * 1024 && !raised) {
-    const cudaError_t err = cudaFuncSetAttribute(delta_rule_scan_kernel<LANES, PER, PER_CHANNEL>,
+    const cudaError_t err = cudaFuncSetAttribute(delta_rule_scan_kernel<LANES, PER, C, PER_CHANNEL>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) {
       mir_set_error("delta_rule_scan: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(err));
@@ -498,8 +508,8 @@ int launch_scan_as(cudaStream_t stream, const float* qkv, const float* beta, con
     }
     raised = true;
   }
-  return mir_launch("delta_rule_scan", delta_rule_scan_kernel<LANES, PER, PER_CHANNEL>,
-                    dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps), smem, stream, 0, qkv,
+  return mir_launch("delta_rule_scan", delta_rule_scan_kernel<LANES, PER, C, PER_CHANNEL>,
+                    dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps + kFetchWarps), smem, stream, 0, qkv,
                     beta, decay, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
 }
 
@@ -508,22 +518,25 @@ int launch_scan(cudaStream_t stream, const float* qkv, const float* beta, const 
                 const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
                 int kv_heads, int key_dim, int value_dim, bool single_tokens) {
 #define MIR_SCAN(L, P)                                                                                              \
-  return launch_scan_as<L, P, PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, \
+  return launch_scan_as<L, P, L / 8, PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, \
                                            out, rows, heads, kv_heads, key_dim, value_dim);
-  // 0: chosen here.  Measured at 16 heads of 128 x 128: a prompt of 2,048 tokens takes 766 / 796 / 935 us with 8 / 16 /
-  // 32 lanes a column; a step of eight single tokens inside a captured graph 8.1 us with 8 lanes, 10.5 with 16.  One
-  // choice for every shape of step, so that a request's 32-bit results do not depend on how it was cut.
+  // 0: chosen here.  Sixteen lanes with two columns each read a token's inputs half as often as eight lanes with one:
+  // a prompt of 2,048 tokens at 16 / 32 heads of 128 x 128 takes 375 / 520 us with a decay per channel (eight lanes: 476 / 707,
+  // thirty-two: 413 / 570; before the fetching warps: 630 / 870) and 345 / 465 with one per head.
+  // One choice for every shape of step, so that a request's 32-bit results do not depend on how it was cut.
   (void)single_tokens;
-  const int lanes = g_scan_lanes ? g_scan_lanes : 8;
+  const int lanes = g_scan_lanes ? g_scan_lanes : 16;
   if (lanes == 8) {
     if (key_dim <= 32) { MIR_SCAN(8, 4) }
     if (key_dim <= 64) { MIR_SCAN(8, 8) }
     if (key_dim <= 96) { MIR_SCAN(8, 12) }
     if (key_dim <= 128) { MIR_SCAN(8, 16) }
   }
-  if (lanes == 16) {
+  if (lanes <= 16) {
     if (key_dim <= 64) { MIR_SCAN(16, 4) }
     if (key_dim <= 128) { MIR_SCAN(16, 8) }
+    if (key_dim <= 192) { MIR_SCAN(16, 12) }
+    if (key_dim <= 256) { MIR_SCAN(16, 16) }
   }
   if (key_dim <= 128) { MIR_SCAN(32, 4) }
   if (key_dim <= 256) { MIR_SCAN(32, 8) }

@@ -11,12 +11,14 @@
 // One lane count and one order of sums for every shape of step: a request's 32-bit results do not depend on how it was
 // cut into steps.  A row of a captured decode batch whose position is negative is padding: nothing is read or written.
 #include "common.cuh"
+#include "scan_pairs.cuh"
 
 using namespace mir;
 
 namespace {
 
 constexpr int kWarps = 4;
+constexpr int kFetchWarps = 4;          // of the walk over prepared rows: they copy what the others will need
 
 // A token's q and k of one head, staged by one warp.  Lane `lane` owns the channels i = lane + 32 e.  A channel of the
 // first half of the rotated ones is rotated together with its partner i + half by the lane that owns it (one sine and
@@ -256,141 +258,182 @@ retention_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, long 
   stage_token(in, frequency, key_scale, lane, half, rotary_dim, activated, prepared + (size_t)unit * (2 * PADDED + 4));
 }
 
-// The walk over prepared rows: as retention_scan_kernel, but a chunk's q, k and q . k arrive by 16-byte asynchronous
-// copies into the other half of the staging buffer while the current chunk is walked.  The same lanes, the same order
-// of sums: the results are those of the kernel above, bit for bit.
-template <typename T, int PER, int kLanes>
-__global__ void __launch_bounds__(kWarps * 32)
+// The walk over prepared rows: the results of retention_scan_kernel, bit for bit (the same lanes, the same order of sums).
+// kWarps warps walk, C columns a lane; kFetchWarps more copy the next chunks' q, k, q . k and v into shared memory (three
+// stages).  Several tokens' inputs are in registers at a time, their read-outs are summed over the lanes together, and the
+// arithmetic goes two numbers an instruction.
+// blockDim (32, kWarps + kFetchWarps), grid (rows, heads, ceil(value_dim / (kWarps * 32 / kLanes * C))).
+// What bounds it: the walking warps' instructions.  One column a lane spends four reads of shared memory on 24 operations of
+// the state; with C columns those reads are shared.
+template <typename T, int PER, int kLanes, int C>
+__global__ void __launch_bounds__((kWarps + kFetchWarps) * 32, 2)
 retention_scan_prepared_kernel(const float* __restrict__ prepared, const T* __restrict__ v, long long ld,
                                const float* __restrict__ decays, float* __restrict__ state,
                                const int* __restrict__ query_starts, const int* __restrict__ state_slots,
                                const int* __restrict__ positions, float* __restrict__ out, int heads, int dim,
                                int value_dim, int activated) {
-  constexpr int COLUMNS = 32 / kLanes;
-  constexpr int BLOCK_COLUMNS = COLUMNS * kWarps;
+  constexpr int BLOCK_COLUMNS = 32 / kLanes * kWarps * C;
   constexpr int PADDED = kLanes * PER;
   constexpr int PREPARED = 2 * PADDED + 4;                        // q | k | q . k
   constexpr int ROW = PREPARED + BLOCK_COLUMNS;                   // and v of this CTA's columns
-  constexpr int CHUNK = PADDED <= 128 ? 16 : 8;
-  constexpr int PIECES = PREPARED / 4;                            // 16-byte pieces of a prepared row
-  constexpr int VALUES_PER_THREAD = (CHUNK * BLOCK_COLUMNS + kWarps * 32 - 1) / (kWarps * 32);
-  __shared__ __align__(16) float staged[2][CHUNK * ROW];
-  __shared__ __align__(16) float partial[CHUNK][kWarps * 32];     // per token: every lane's part of its column's read-out
+  constexpr int CHUNK = PADDED <= 128 ? 16 : 8, STAGES = 3, STAGE = CHUNK * ROW;
+  extern __shared__ __align__(16) float staged[];                 // [STAGES][CHUNK][ROW]
   grid_launch_dependents();
   grid_dependency_wait();
-  const int lane = threadIdx.x, warp = threadIdx.y;
-  const int thread = warp * 32 + lane;
-  const int l = lane % kLanes;
+  const int lane = threadIdx.x;
   const int row = blockIdx.x, head = blockIdx.y;
   const int first_column = blockIdx.z * BLOCK_COLUMNS;
-  const int local_column = warp * COLUMNS + lane / kLanes;
-  const int column = first_column + local_column;
   const int start = query_starts[row], end = query_starts[row + 1];
   if (end <= start || positions[start] < 0) return;
-  const bool active = column < value_dim;
+  const size_t value_at = (size_t)head * value_dim;
+  const int chunks = (end - start + CHUNK - 1) / CHUNK;
+
+  if (threadIdx.y >= kWarps) {                                    // the fetching warps: tokens w, w + kFetchWarps, ... of a chunk
+    constexpr int TOKENS = CHUNK / kFetchWarps, VALUES = (BLOCK_COLUMNS + 31) / 32;
+    const int mine = threadIdx.y - kWarps;
+    T next_v[TOKENS][VALUES];
+    auto fetch = [&](int chunk) {                                 // issues the copies; v passes through registers
+      const int from = start + chunk * CHUNK;
+#pragma unroll
+      for (int tt = 0; tt < TOKENS; ++tt) {
+        const int t = mine + tt * kFetchWarps;
+        const size_t token = from + t;
+        const bool there = from + t < end;
+        float* to = staged + (chunk % STAGES) * STAGE + t * ROW;
+        const float* source = prepared + (token * heads + head) * PREPARED;
+#pragma unroll
+        for (int i = 0; i < PREPARED; i += 128)
+          if (there && i + lane * 4 < PREPARED) copy_async(to + i + lane * 4, source + i + lane * 4, true);
+#pragma unroll
+        for (int e = 0; e < VALUES; ++e) {
+          const int c = e * 32 + lane;
+          next_v[tt][e] = there && c < BLOCK_COLUMNS && first_column + c < value_dim ? v[token * ld + value_at + first_column + c] : T(0.0f);
+        }
+      }
+      copy_commit();
+    };
+    auto commit_values = [&](int chunk) {
+      float* to = staged + (chunk % STAGES) * STAGE + mine * ROW + PREPARED + lane;
+#pragma unroll
+      for (int tt = 0; tt < TOKENS; ++tt)
+#pragma unroll
+        for (int e = 0; e < VALUES; ++e)
+          if (e * 32 + lane < BLOCK_COLUMNS) to[tt * kFetchWarps * ROW + e * 32] = entering(to_float(next_v[tt][e]), activated);
+    };
+    fetch(0);
+    commit_values(0);
+    if (chunks > 1) fetch(1); else copy_commit();
+    copy_wait<1>();
+    __syncthreads();                                              // the first chunk is there
+    for (int chunk = 0; chunk < chunks; ++chunk) {                // (into the stage of the chunk that was walked last)
+      if (chunk + 1 < chunks) commit_values(chunk + 1);
+      if (chunk + 2 < chunks) fetch(chunk + 2); else copy_commit();
+      copy_wait<1>();
+      __syncthreads();                                            // this chunk has been walked, and the next one is there
+    }
+    copy_wait<0>();
+    return;
+  }
+
+  const int l = lane % kLanes;
+  const int local_column = (threadIdx.y * (32 / kLanes) + lane / kLanes) * C;
+  const int column = first_column + local_column;
   const bool wide = dim % 4 == 0;
   const float decay = decays[head];
-  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + (active ? column : 0)) * dim;
-  float s[PER];
+  const Pair both_decays = pair_from(decay, decay);
+  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + column) * dim;
+  Pair s[C][PER / 2];
 #pragma unroll
-  for (int m = 0; m < PER; m += 4) {
-    const int i = (m / 4 * kLanes + l) * 4;
-    if (wide) {
-      const float4 piece = (active && i < dim) ? *reinterpret_cast<const float4*>(column_state + i)
-                                               : make_float4(0.f, 0.f, 0.f, 0.f);
-      s[m] = piece.x; s[m + 1] = piece.y; s[m + 2] = piece.z; s[m + 3] = piece.w;
-    } else {
+  for (int c = 0; c < C; ++c)
+    load_column<kLanes, PER>(s[c], column_state + (size_t)c * dim, l, dim, column + c < value_dim, wide);
+  struct Inputs {
+    Pair q[PER / 2], k[PER / 2];
+    float value[C];
+  };
+  auto load = [&](Inputs& in, const float* from) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[m + e] = (active && i + e < dim) ? column_state[i + e] : 0.0f;
+    for (int m = 0; m < PER; m += 4) {
+      const int i = (m / 4 * kLanes + l) * 4;
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(from + i);
+      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(from + PADDED + i);
+      in.q[m / 2] = a.x; in.q[m / 2 + 1] = a.y;
+      in.k[m / 2] = b.x; in.k[m / 2 + 1] = b.y;
     }
-  }
-  const size_t value_at = (size_t)head * value_dim;
-  T next_v[VALUES_PER_THREAD];
-  auto issue = [&](int from, int stage) {
-    const int count = min(CHUNK, end - from);
-    for (int piece = thread; piece < count * PIECES; piece += kWarps * 32) {
-      const int t = piece / PIECES, c = piece - t * PIECES;
-      const float* source = prepared + ((size_t)(from + t) * heads + head) * PREPARED + 4 * c;
-      const unsigned target = (unsigned)__cvta_generic_to_shared(&staged[stage][t * ROW + 4 * c]);
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(target), "l"(source) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
-    for (int j = 0; j < VALUES_PER_THREAD; ++j) {
-      const int index = thread + j * kWarps * 32;
-      const int t = index / BLOCK_COLUMNS, c = index - t * BLOCK_COLUMNS;
-      next_v[j] = (t < count && first_column + c < value_dim)
-                      ? v[(size_t)(from + t) * ld + value_at + first_column + c] : T(0.0f);
+    for (int c = 0; c < C; ++c) in.value[c] = from[PREPARED + local_column + c];
+  };
+  auto walk = [&](const Inputs& in, float* parts) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const Pair values = pair_from(in.value[c], in.value[c]);
+      Pair read[2] = {0, 0};
+#pragma unroll
+      for (int m = 0; m < PER / 2; ++m) {
+        read[m & 1] = pair_fma(s[c][m], in.q[m], read[m & 1]);
+        s[c][m] = pair_fma(s[c][m], both_decays, pair_mul(in.k[m], values));
+      }
+      parts[c] = pair_total(read);
     }
   };
-  issue(start, 0);
+  // A run of GROUP tokens: their inputs, their walk, then the sums of all their columns at once, each of which ends in a lane of
+  // its own that writes it.
+  constexpr int GROUP = kLanes / C < 4 ? kLanes / C : 4, SUMS = GROUP * C;
   const size_t out_width = (size_t)heads * value_dim;
-  int stage = 0;
-  for (int from = start; from < end; from += CHUNK, stage ^= 1) {
-    const int count = min(CHUNK, end - from);
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+  float* const out_of = out + (size_t)start * out_width + value_at + column;
+  auto finish = [&](float total, int number, const float* from, int token) {
+    const int t = number / C, c = number % C;
+    if (column + c < value_dim)
+      out_of[(size_t)(token + t) * out_width + c] =
+          fmaf(from[t * ROW + 2 * PADDED], from[t * ROW + PREPARED + local_column + c], decay * total);
+  };
+  __syncthreads();                                                // the first chunk is there
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int count = min(CHUNK, end - start - chunk * CHUNK);
+    const float* in = staged + (chunk % STAGES) * STAGE;
+    int t = 0;
+#pragma unroll 1
+    for (; t + GROUP <= count; t += GROUP, in += GROUP * ROW) {
+      Inputs inputs[GROUP];
 #pragma unroll
-    for (int j = 0; j < VALUES_PER_THREAD; ++j) {
-      const int index = thread + j * kWarps * 32;
-      const int t = index / BLOCK_COLUMNS, c = index - t * BLOCK_COLUMNS;
-      if (t < CHUNK) staged[stage][t * ROW + PREPARED + c] = entering(to_float(next_v[j]), activated);
+      for (int g = 0; g < GROUP; ++g) load(inputs[g], in + g * ROW);
+      float parts[SUMS];
+#pragma unroll
+      for (int g = 0; g < GROUP; ++g) walk(inputs[g], parts + g * C);
+      const float total = sum_lanes<kLanes, SUMS>(parts, l);
+      if (l < SUMS) finish(total, lane_sum<SUMS>(l), in, chunk * CHUNK + t);
     }
-    __syncthreads();                   // this chunk is whole, and every thread has left the chunk before
-    if (from + CHUNK < end) issue(from + CHUNK, stage ^ 1);
-#pragma unroll 4
-    for (int t = 0; t < count; ++t) {
-      const float* in = staged[stage] + t * ROW;
-      const float value = in[PREPARED + local_column];
-      float read[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int m = 0; m < PER; m += 4) {
-        const int i = (m / 4 * kLanes + l) * 4;
-        const float4 query = *reinterpret_cast<const float4*>(in + i);
-        const float4 key = *reinterpret_cast<const float4*>(in + PADDED + i);
-        read[0] = fmaf(s[m], query.x, read[0]);
-        read[1] = fmaf(s[m + 1], query.y, read[1]);
-        read[2] = fmaf(s[m + 2], query.z, read[2]);
-        read[3] = fmaf(s[m + 3], query.w, read[3]);
-        s[m] = fmaf(s[m], decay, key.x * value);
-        s[m + 1] = fmaf(s[m + 1], decay, key.y * value);
-        s[m + 2] = fmaf(s[m + 2], decay, key.z * value);
-        s[m + 3] = fmaf(s[m + 3], decay, key.w * value);
-      }
-      partial[t][thread] = (read[0] + read[1]) + (read[2] + read[3]);
+#pragma unroll 1
+    for (; t < count; ++t, in += ROW) {
+      Inputs inputs;
+      load(inputs, in);
+      float parts[C];
+      walk(inputs, parts);
+      const float total = sum_lanes<kLanes, C>(parts, l);
+      if (l < C) finish(total, lane_sum<C>(l), in, chunk * CHUNK + t);
     }
-    __syncthreads();
-    // the lanes' parts of a column are summed as the butterfly of shuffles in the kernel above sums them (neighbours
-    // first, then pairs of pairs, ...), so that the bits are the same; one (token, column) a thread and pass
-    for (int index = thread; index < count * BLOCK_COLUMNS; index += kWarps * 32) {
-      const int t = index / BLOCK_COLUMNS, c = index - t * BLOCK_COLUMNS;
-      float parts[kLanes];
-#pragma unroll
-      for (int i = 0; i < kLanes; i += 4) {
-        const float4 four = *reinterpret_cast<const float4*>(&partial[t][c * kLanes + i]);
-        parts[i] = four.x; parts[i + 1] = four.y; parts[i + 2] = four.z; parts[i + 3] = four.w;
-      }
-#pragma unroll
-      for (int width = 1; width < kLanes; width <<= 1)
-#pragma unroll
-        for (int i = 0; i < kLanes; i += 2 * width) parts[i] += parts[i + width];
-      const float* in = staged[stage] + t * ROW;
-      if (first_column + c < value_dim)
-        out[(size_t)(from + t) * out_width + value_at + first_column + c] =
-            fmaf(in[2 * PADDED], in[PREPARED + c], decay * parts[0]);
-    }
+    __syncthreads();                                              // this chunk has been walked, and the next one is there
   }
-  if (!active) return;
 #pragma unroll
-  for (int m = 0; m < PER; m += 4) {
-    const int i = (m / 4 * kLanes + l) * 4;
-    if (wide) {
-      if (i < dim) *reinterpret_cast<float4*>(column_state + i) = make_float4(s[m], s[m + 1], s[m + 2], s[m + 3]);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (i + e < dim) column_state[i + e] = s[m + e];
-    }
+  for (int c = 0; c < C; ++c)
+    if (column + c < value_dim) store_column<kLanes, PER>(s[c], column_state + (size_t)c * dim, l, dim, wide);
+}
+
+template <typename T, int PER, int kLanes, int C>
+int launch_walk(cudaStream_t stream, const float* prepared, const void* v, long long ld, const float* decays, float* state,
+                const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
+                int dim, int value_dim, int activated) {
+  constexpr int columns = kWarps * (32 / kLanes) * C;
+  constexpr int smem = 3 * (kLanes * PER <= 128 ? 16 : 8) * (2 * kLanes * PER + 4 + columns) * (int)sizeof(float);
+  const cudaError_t err = cudaFuncSetAttribute(retention_scan_prepared_kernel<T, PER, kLanes, C>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) {
+    mir_set_error("retention_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
+    return MIR_CUDA_ERROR;
   }
+  return mir_launch("retention_scan", retention_scan_prepared_kernel<T, PER, kLanes, C>,
+                    dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kWarps + kFetchWarps), smem, stream, 0,
+                    prepared, (const T*)v, ld, decays, state, query_starts, state_slots, positions, out, heads, dim,
+                    value_dim, activated);
 }
 
 template <typename T, int PER, int kLanes>
@@ -398,17 +441,21 @@ int launch_prepared(cudaStream_t stream, const void* q, const void* k, const voi
                     int rotary_dim, const float* decays, float key_scale, float* state, const int* query_starts,
                     const int* state_slots, const int* positions, float* out, float* prepared, int tokens, int rows,
                     int heads, int dim, int value_dim, int activated) {
-  constexpr int columns = kWarps * (32 / kLanes);
   const long long units = (long long)tokens * heads;
   int status = mir_launch("retention_prepare", retention_prepare_kernel<T, kLanes * PER / 32>,
                           dim3((unsigned)((units + kWarps - 1) / kWarps)), dim3(32, kWarps), 0, stream, 0, (const T*)q,
                           (const T*)k, ld, inv_freq, rotary_dim, key_scale, positions, prepared, tokens, heads, dim,
                           activated);
   if (status != MIR_OK) return status;
-  return mir_launch("retention_scan", retention_scan_prepared_kernel<T, PER, kLanes>,
-                    dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kWarps), 0, stream, 0,
-                    (const float*)prepared, (const T*)v, ld, decays, state, query_starts, state_slots, positions, out,
-                    heads, dim, value_dim, activated);
+#define MIR_WALK(C)                                                                                                    \
+  return launch_walk<T, PER, kLanes, C>(stream, prepared, v, ld, decays, state, query_starts, state_slots, positions, \
+                                        out, rows, heads, dim, value_dim, activated)
+  // More columns a lane share a token's reads of shared memory; fewer fill the GPU with the heads of few requests.
+  const int narrow = kWarps * (32 / kLanes) * 2;                  // columns of a CTA with two a lane
+  if constexpr (PER <= 8)
+    if ((long long)rows * heads * ((value_dim + narrow - 1) / narrow) > mir_sm_count()) MIR_WALK(4);
+  MIR_WALK(2);
+#undef MIR_WALK
 }
 
 template <typename T, int PER, int kLanes, bool SHORT>

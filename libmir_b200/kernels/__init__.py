@@ -89,7 +89,7 @@ _SIGNATURES = {
                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                c_int, c_int, c_void_p],
         "mir_wkv_scan": [c_int, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                         c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
+                         c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],
         "mir_moe_route": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_int, c_float, c_int, c_int, c_void_p],
         "mir_moe_tile_slots": [c_int, c_int, c_int],
@@ -892,17 +892,33 @@ def wkv_mix(h: torch.Tensor, tail: torch.Tensor, mu: torch.Tensor, row_of_token:
                                 _stream()))
 
 
+def wkv_prepared_floats(tokens: int, heads: int, dim: int) -> int:
+    """How many 32-bit numbers wkv_scan's `prepared` scratch holds: per token and head r, k, the decays and v, padded to the
+    kernel's width for heads of `dim` channels, and the bonus term."""
+    padded = next((width for width in (32, 64, 96, 128, 192, 256) if dim <= width), dim)
+    return tokens * heads * (4 * padded + 4)
+
+
 def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_raw: torch.Tensor, decay_bias: torch.Tensor,
              bonus: torch.Tensor, state: torch.Tensor, query_starts: torch.Tensor, state_slots: torch.Tensor,
-             positions: torch.Tensor, out: torch.Tensor, heads: int, dim: int) -> None:
+             positions: torch.Tensor, out: torch.Tensor, heads: int, dim: int,
+             prepared: Optional[torch.Tensor] = None) -> None:
     """The wkv recurrence over the tokens of each request row, from and into state [slots, heads, dim (value channel),
     dim (key channel)] (32-bit): per head o = S^T r + (sum_i r_i u_i k_i) v; S <- diag(w) S + k v^T with
     w = exp(-exp(decay_raw + decay_bias)).  r, k, v [tokens, heads * dim] (one row stride, the activations' dtype);
-    decay_raw 32-bit [tokens, heads * dim]; decay_bias, bonus (u) 32-bit [heads * dim]; out 32-bit [tokens, heads * dim]."""
-    _cuda(r, k, v, decay_raw, decay_bias, bonus, state, query_starts, state_slots, positions, out)
+    decay_raw 32-bit [tokens, heads * dim]; decay_bias, bonus (u) 32-bit [heads * dim]; out 32-bit [tokens, heads * dim].
+    A step that brings more than single tokens first writes what its walk needs of every token into `prepared` (32-bit
+    scratch of wkv_prepared_floats numbers, allocated here if it is not given)."""
+    _cuda(r, k, v, decay_raw, decay_bias, bonus, state, query_starts, state_slots, positions, out, prepared)
     tokens = r.shape[0]
     rows = query_starts.numel() - 1
     width = heads * dim
+    if prepared is None and tokens != rows:
+        prepared = torch.empty(wkv_prepared_floats(tokens, heads, dim), dtype=torch.float32, device=r.device)
+    _require(prepared is None or (prepared.dtype == torch.float32 and prepared.is_contiguous()
+                                  and prepared.numel() >= wkv_prepared_floats(tokens, heads, dim)
+                                  and prepared.data_ptr() % 16 == 0),
+             "wkv_scan: prepared is float32 scratch of wkv_prepared_floats numbers on a 16-byte boundary")
     _require(all(t.shape == (tokens, width) and t.stride(1) == 1 and t.stride(0) == r.stride(0) and t.dtype == r.dtype
                  for t in (r, k, v)), "wkv_scan: r, k, v are [tokens, heads * dim] with one row stride and dtype")
     _require(decay_raw.dtype == torch.float32 and decay_raw.is_contiguous() and decay_raw.shape == (tokens, width)
@@ -913,8 +929,8 @@ def wkv_scan(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay_raw: torch
     lib = library("core")
     _check(lib, lib.mir_wkv_scan(_is_bf16(r), r.data_ptr(), k.data_ptr(), v.data_ptr(), r.stride(0), decay_raw.data_ptr(),
                                  decay_bias.data_ptr(), bonus.data_ptr(), state.data_ptr(), query_starts.data_ptr(),
-                                 state_slots.data_ptr(), positions.data_ptr(), out.data_ptr(), tokens, rows, heads, dim,
-                                 _stream()))
+                                 state_slots.data_ptr(), positions.data_ptr(), out.data_ptr(), _ptr(prepared), tokens, rows,
+                                 heads, dim, _stream()))
 
 
 # --------------------------------------------------------------------------- retention
