@@ -23,6 +23,28 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
   for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = ok ? to_float(src[c]) * scale : 0.0f;
 }
 
+// The same, eight neighbouring columns a thread (hidden a multiple of 8, rows on 16-byte boundaries): one load a thread for rows
+// of up to 4,096 (2 rows of 4,096: 8.5 us column by column).
+template <typename T>
+__global__ void __launch_bounds__(512) embed_wide_kernel(const T* __restrict__ table, const int* __restrict__ ids,
+                                                         float* __restrict__ out, int hidden, int vocab, float scale) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int row = blockIdx.x;
+  const int id = ids[row];
+  const bool ok = id >= 0 && id < vocab;
+  const T* src = table + (size_t)(ok ? id : 0) * hidden;
+  float* dst = out + (size_t)row * hidden;
+  for (int c = threadIdx.x * 8; c < hidden; c += blockDim.x * 8) {
+    float v[8];
+    load8(src + c, v);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = ok ? v[i] * scale : 0.0f;
+    reinterpret_cast<float4*>(dst + c)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(dst + c)[1] = make_float4(v[4], v[5], v[6], v[7]);
+  }
+}
+
 // out[r, :] = float(table[ids[r], :]) * scale + float(pairs[bucket(r), :]): a second table indexed by a hash of the
 // token and the token before it in its request, bucket = (previous * mul_previous + id * mul_current) mod buckets;
 // a request's first token (previous < 0) takes row `buckets`, the table's last.
@@ -54,6 +76,22 @@ __global__ void gelu_tanh_kernel(T* __restrict__ x, size_t total) {
   const float inner = 0.7978845608028654f * fmaf(0.044715f * z * z, z, z);
   x[index] = from_float<T>(0.5f * z * (1.0f + tanhf(inner)));
 }
+
+// Kernels that keep a row in registers: four columns a thread in a few places.  The threads follow from the row's
+// width alone, so that a row's result does not depend on how many rows there are.
+constexpr int kRowThreads = 512;
+inline int row_pieces(int quads) { return (quads + kRowThreads - 1) / kRowThreads; }
+inline int row_threads(int quads) {
+  const int pieces = row_pieces(quads), each = (quads + pieces - 1) / pieces;
+  return (each + 31) / 32 * 32;
+}
+__device__ __forceinline__ void store_rounded(__nv_bfloat16* row, int quad, float4 v) {
+  uint2 packed;
+  *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(v.x, v.y);
+  *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(v.z, v.w);
+  reinterpret_cast<uint2*>(row)[quad] = packed;
+}
+__device__ __forceinline__ void store_rounded(float* row, int quad, float4 v) { reinterpret_cast<float4*>(row)[quad] = v; }
 
 // residual[r, :] += scale * sum over branches b of branch_b[r, :] * rsqrt(mean(branch_b[r, :]^2) + eps) * weight_b:
 // several branch outputs (32-bit rows), each normalised over the model width with a weight of its own, added to the
@@ -89,44 +127,62 @@ __global__ void add_normed_branches_kernel(NormedBranches branches, float* __res
   }
 }
 
-// The same with 16-byte accesses (hidden a multiple of 4, every pointer 16-byte aligned); the second pass finds the
-// rows in L1.
-__global__ void add_normed_branches_vec4_kernel(NormedBranches branches, float* __restrict__ residual,
-                                                __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
-  __shared__ float scratch[32];
+// The same with 16-byte accesses (hidden a multiple of 4, every pointer 16-byte aligned): a CTA keeps its row of every branch
+// in registers, four columns a thread in PIECES places, asks for the residual with them and for the weights before it waits
+// for the kernel before, and sums all branches behind one barrier.  Few rows are bound by these latencies (2 rows of
+// 4,096: 8.7 us when the row was read twice and the weights behind the sum), many by their bytes.
+template <int BRANCHES, int PIECES>
+__global__ void __launch_bounds__(kRowThreads) add_normed_branches_vec4_kernel(
+    NormedBranches branches, float* __restrict__ residual, __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
+  __shared__ float scratch[BRANCHES][32];
   grid_launch_dependents();
-  grid_dependency_wait();
-  const int row = blockIdx.x;
   const int quads = hidden >> 2;
-  float inverse[4];
-  for (int b = 0; b < branches.count; ++b) {
-    const float4* src = reinterpret_cast<const float4*>(branches.rows[b] + (size_t)row * hidden);
-    float sum = 0.0f;
-    for (int c = threadIdx.x; c < quads; c += blockDim.x) {
-      const float4 v = src[c];
-      sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sum))));
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  float4 w[BRANCHES][PIECES], v[BRANCHES][PIECES], old[PIECES];
+#pragma unroll
+  for (int b = 0; b < BRANCHES; ++b)
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      const int c = p * blockDim.x + threadIdx.x;
+      if (c < quads) w[b][p] = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
     }
-    sum = block_sum(sum, scratch);
-    inverse[b] = rsqrtf(sum / (float)hidden + eps);
+  grid_dependency_wait();
+  const size_t base = (size_t)blockIdx.x * hidden;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = p * blockDim.x + threadIdx.x;
+#pragma unroll
+    for (int b = 0; b < BRANCHES; ++b)
+      v[b][p] = c < quads ? reinterpret_cast<const float4*>(branches.rows[b] + base)[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (c < quads) old[p] = reinterpret_cast<const float4*>(residual + base)[c];
   }
-  float4* dst = reinterpret_cast<float4*>(residual + (size_t)row * hidden);
-  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
+  float inverse[BRANCHES];
+#pragma unroll
+  for (int b = 0; b < BRANCHES; ++b) {
+    float sum = 0.0f;
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p)
+      sum = fmaf(v[b][p].x, v[b][p].x, fmaf(v[b][p].y, v[b][p].y, fmaf(v[b][p].z, v[b][p].z, fmaf(v[b][p].w, v[b][p].w, sum))));
+    sum = warp_sum(sum);
+    if (lane == 0) scratch[b][warp] = sum;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int b = 0; b < BRANCHES; ++b) inverse[b] = rsqrtf(warp_sum(lane < warps ? scratch[b][lane] : 0.0f) / (float)hidden + eps);
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = p * blockDim.x + threadIdx.x;
+    if (c >= quads) continue;
     float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int b = 0; b < branches.count; ++b) {
-      const float4 v = reinterpret_cast<const float4*>(branches.rows[b] + (size_t)row * hidden)[c];
-      const float4 w = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
-      total.x += v.x * inverse[b] * w.x; total.y += v.y * inverse[b] * w.y;
-      total.z += v.z * inverse[b] * w.z; total.w += v.w * inverse[b] * w.w;
+#pragma unroll
+    for (int b = 0; b < BRANCHES; ++b) {
+      total.x += v[b][p].x * inverse[b] * w[b][p].x; total.y += v[b][p].y * inverse[b] * w[b][p].y;
+      total.z += v[b][p].z * inverse[b] * w[b][p].z; total.w += v[b][p].w * inverse[b] * w[b][p].w;
     }
-    float4 r = dst[c];
+    float4 r = old[p];
     r.x += scale * total.x; r.y += scale * total.y; r.z += scale * total.z; r.w += scale * total.w;
-    dst[c] = r;
-    if (rounded) {
-      uint2 packed;
-      *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(r.x, r.y);
-      *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(r.z, r.w);
-      reinterpret_cast<uint2*>(rounded + (size_t)row * hidden)[c] = packed;
-    }
+    reinterpret_cast<float4*>(residual + base)[c] = r;
+    if (rounded) store_rounded(rounded + base, c, r);
   }
 }
 
@@ -264,39 +320,64 @@ __global__ void rms_norm_kernel(const float* __restrict__ x, const float* __rest
   for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = from_float<Tout>(src[c] * inverse * weight[c]);
 }
 
-// The same with 16-byte loads (hidden a multiple of 4); the second pass finds the row in L1.
-template <typename Tout>
-__global__ void rms_norm_vec4_kernel(const float* __restrict__ x, const float* __restrict__ weight,
-                                     Tout* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
+// The same with 16-byte accesses (hidden a multiple of 4) and the row in registers; with PAIR a second norm of the same rows,
+// out_b = x * s * weight_b with the same s.  The weights are asked for before the wait for the kernel before.
+template <typename Tout, bool PAIR, int PIECES>
+__global__ void __launch_bounds__(kRowThreads) rms_norm_vec4_kernel(const float* __restrict__ x, const float* __restrict__ weight,
+                                                                    const float* __restrict__ weight_b, Tout* __restrict__ out,
+                                                                    Tout* __restrict__ out_b, const int* __restrict__ rows,
+                                                                    int hidden, float eps) {
   __shared__ float scratch[32];
   grid_launch_dependents();
+  const int quads = hidden >> 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  float4 w[PIECES], second[PAIR ? PIECES : 1], v[PIECES];
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = p * blockDim.x + threadIdx.x;
+    if (c >= quads) continue;
+    w[p] = __ldg(reinterpret_cast<const float4*>(weight) + c);
+    if (PAIR) second[p] = __ldg(reinterpret_cast<const float4*>(weight_b) + c);
+  }
   grid_dependency_wait();
   const int row = blockIdx.x;
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[row] : row) * hidden);
-  const float4* w4 = reinterpret_cast<const float4*>(weight);
-  const int quads = hidden >> 2;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = p * blockDim.x + threadIdx.x;
+    v[p] = c < quads ? src[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  }
   float sum = 0.0f;
-  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
-    const float4 v = src[c];
-    sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sum))));
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) sum = fmaf(v[p].x, v[p].x, fmaf(v[p].y, v[p].y, fmaf(v[p].z, v[p].z, fmaf(v[p].w, v[p].w, sum))));
+  sum = warp_sum(sum);
+  if (lane == 0) scratch[warp] = sum;
+  __syncthreads();
+  const float inverse = rsqrtf(warp_sum(lane < warps ? scratch[lane] : 0.0f) / (float)hidden + eps);
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = p * blockDim.x + threadIdx.x;
+    if (c >= quads) continue;
+    const float4 n = make_float4(v[p].x * inverse, v[p].y * inverse, v[p].z * inverse, v[p].w * inverse);
+    store_rounded(out + (size_t)row * hidden, c, make_float4(n.x * w[p].x, n.y * w[p].y, n.z * w[p].z, n.w * w[p].w));
+    if (PAIR)
+      store_rounded(out_b + (size_t)row * hidden, c,
+                    make_float4(n.x * second[p].x, n.y * second[p].y, n.z * second[p].z, n.w * second[p].w));
   }
-  sum = block_sum(sum, scratch);
-  const float inverse = rsqrtf(sum / (float)hidden + eps);
-  Tout* dst = out + (size_t)row * hidden;
-  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
-    const float4 v = src[c];
-    const float4 w = __ldg(w4 + c);
-    const float a = v.x * inverse * w.x, b = v.y * inverse * w.y, d = v.z * inverse * w.z, e = v.w * inverse * w.w;
-    if (sizeof(Tout) == 4) {
-      reinterpret_cast<float4*>(dst)[c] = make_float4(a, b, d, e);
-    } else {
-      const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(d, e);
-      uint2 packed;
-      packed.x = *reinterpret_cast<const uint32_t*>(&lo);
-      packed.y = *reinterpret_cast<const uint32_t*>(&hi);
-      reinterpret_cast<uint2*>(dst)[c] = packed;
-    }
-  }
+}
+constexpr int kRowLimit = 8 * 4 * kRowThreads;                   // the widest row that the register form takes
+template <typename Tout, bool PAIR>
+int launch_rms_norm(const float* x, const float* weight, const float* weight_b, Tout* out, Tout* out_b, const int* rows,
+                    int n_rows, int hidden, float eps, cudaStream_t stream) {
+  const int quads = hidden >> 2, pieces = row_pieces(quads);
+#define MIR_RMS(P)                                                                                                        \
+  return mir_launch(PAIR ? "rms_norm_pair" : "rms_norm", rms_norm_vec4_kernel<Tout, PAIR, P>, dim3(n_rows),              \
+                    dim3(row_threads(quads)), 0, stream, 0, x, weight, weight_b, out, out_b, rows, hidden, eps)
+  if (pieces == 1) MIR_RMS(1);
+  if (pieces == 2) MIR_RMS(2);
+  if (pieces <= 4) MIR_RMS(4);
+  MIR_RMS(8);
+#undef MIR_RMS
 }
 
 // out[r, c] = silu(gu[r, c]) * gu[r, inter + c]; gu rows are [gate | up].
@@ -357,6 +438,14 @@ MIR_EXPORT int mir_embed(int bf16, const void* table, const int* ids, float* out
                          float scale, cudaStream_t stream) {
   if (rows == 0) return MIR_OK;
   if (rows < 0 || hidden <= 0 || vocab <= 0) { mir_set_error("embed: bad sizes"); return MIR_BAD_ARGUMENT; }
+  if (hidden % 8 == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {
+    const int threads = hidden >= 4096 ? 512 : (hidden / 8 + 31) / 32 * 32;
+    if (bf16)
+      return mir_launch("embed", embed_wide_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), 0, stream, 0,
+                        (const __nv_bfloat16*)table, ids, out, hidden, vocab, scale);
+    return mir_launch("embed", embed_wide_kernel<float>, dim3(rows), dim3(threads), 0, stream, 0, (const float*)table, ids, out,
+                      hidden, vocab, scale);
+  }
   if (bf16)
     return mir_launch("embed", embed_kernel<__nv_bfloat16>, dim3(rows), dim3(256), 0, stream, 0,
                       (const __nv_bfloat16*)table, ids, out, hidden, vocab, scale);
@@ -450,9 +539,25 @@ MIR_EXPORT int mir_add_normed_branches(const float* const* branch_rows, const fl
   bool aligned = (hidden & 3) == 0 && ((uintptr_t)residual & 15) == 0 && ((uintptr_t)rounded & 7) == 0;
   for (int b = 0; b < count; ++b)
     aligned = aligned && ((uintptr_t)branch_rows[b] & 15) == 0 && ((uintptr_t)branch_weights[b] & 15) == 0;
-  if (aligned)
-    return mir_launch("add_normed_branches", add_normed_branches_vec4_kernel, dim3(rows), dim3(hidden >= 4096 ? 256 : 128),
-                      0, stream, 0, branches, residual, (__nv_bfloat16*)rounded, hidden, eps, scale);
+  const int quads = hidden >> 2, pieces = row_pieces(quads);
+#define MIR_NORMED(B, P)                                                                                             \
+  return mir_launch("add_normed_branches", add_normed_branches_vec4_kernel<B, P>, dim3(rows), dim3(row_threads(quads)), 0, \
+                    stream, 0, branches, residual, (__nv_bfloat16*)rounded, hidden, eps, scale)
+  if (aligned && count == 1) {
+    if (pieces == 1) MIR_NORMED(1, 1);
+    if (pieces == 2) MIR_NORMED(1, 2);
+    if (pieces <= 4) MIR_NORMED(1, 4);
+  }
+  if (aligned && count == 2) {
+    if (pieces == 1) MIR_NORMED(2, 1);
+    if (pieces == 2) MIR_NORMED(2, 2);
+    if (pieces <= 4) MIR_NORMED(2, 4);
+  }
+  if (aligned && pieces <= 4) {
+    if (count == 3) MIR_NORMED(3, 4);
+    MIR_NORMED(4, 4);
+  }
+#undef MIR_NORMED
   const int threads = hidden >= 2048 ? 512 : 256;
   return mir_launch("add_normed_branches", add_normed_branches_kernel, dim3(rows), dim3(threads), 0, stream, 0, branches,
                     residual, (__nv_bfloat16*)rounded, hidden, eps, scale);
@@ -512,13 +617,11 @@ MIR_EXPORT int mir_rms_norm(int bf16, const float* x, const float* weight, void*
                             int hidden, float eps, cudaStream_t stream) {
   if (n_rows == 0) return MIR_OK;
   if (n_rows < 0 || hidden <= 0) { mir_set_error("rms_norm: bad sizes"); return MIR_BAD_ARGUMENT; }
-  if ((hidden & 3) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)weight & 15) == 0 && ((uintptr_t)out & 15) == 0) {
-    const int vec_threads = hidden >= 1024 ? 256 : 128;
+  if ((hidden & 3) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)weight & 15) == 0 && ((uintptr_t)out & 15) == 0 &&
+      hidden <= kRowLimit) {
     if (bf16)
-      return mir_launch("rms_norm", rms_norm_vec4_kernel<__nv_bfloat16>, dim3(n_rows), dim3(vec_threads), 0, stream, 0,
-                        x, weight, (__nv_bfloat16*)out, rows, hidden, eps);
-    return mir_launch("rms_norm", rms_norm_vec4_kernel<float>, dim3(n_rows), dim3(vec_threads), 0, stream, 0, x, weight,
-                      (float*)out, rows, hidden, eps);
+      return launch_rms_norm<__nv_bfloat16, false>(x, weight, nullptr, (__nv_bfloat16*)out, nullptr, rows, n_rows, hidden, eps, stream);
+    return launch_rms_norm<float, false>(x, weight, nullptr, (float*)out, nullptr, rows, n_rows, hidden, eps, stream);
   }
   const int threads = hidden >= 2048 ? 512 : 256;
   if (bf16)
@@ -553,6 +656,13 @@ MIR_EXPORT int mir_rms_norm_pair(int bf16, const float* x, const float* weight_a
                                  void* out_b, int n_rows, int hidden, float eps, cudaStream_t stream) {
   if (n_rows == 0) return MIR_OK;
   if (n_rows < 0 || hidden <= 0) { mir_set_error("rms_norm_pair: bad sizes"); return MIR_BAD_ARGUMENT; }
+  if ((hidden & 3) == 0 && (((uintptr_t)x | (uintptr_t)weight_a | (uintptr_t)weight_b | (uintptr_t)out_a | (uintptr_t)out_b) & 15) == 0 &&
+      hidden <= kRowLimit) {
+    if (bf16)
+      return launch_rms_norm<__nv_bfloat16, true>(x, weight_a, weight_b, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, nullptr,
+                                                  n_rows, hidden, eps, stream);
+    return launch_rms_norm<float, true>(x, weight_a, weight_b, (float*)out_a, (float*)out_b, nullptr, n_rows, hidden, eps, stream);
+  }
   const int threads = hidden >= 2048 ? 512 : 256;
   if (bf16)
     return mir_launch("rms_norm_pair", rms_norm_pair_kernel<__nv_bfloat16>, dim3(n_rows), dim3(threads), 0, stream, 0, x,
