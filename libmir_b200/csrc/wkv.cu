@@ -32,7 +32,8 @@ __global__ void wkv_mix_kernel(const T* __restrict__ h, long long ld, float* __r
   const T* before = token > start ? h + (size_t)(token - 1) * ld : nullptr;
   float* kept = tail + (size_t)state_slots[row] * width;
   const bool alone = end - start == 1;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
+  // the CTAs of a token (gridDim.y of them, more where a step has few tokens) share its columns out
+  for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
     const float x = to_float(mine[c]);
     const float previous = before != nullptr ? to_float(before[c]) : kept[c];
     const float step = previous - x;
@@ -436,13 +437,16 @@ MIR_EXPORT int mir_wkv_mix(int bf16, const void* h, long long ld, float* tail, c
     return MIR_BAD_ARGUMENT;
   }
   const int threads = width >= 1024 ? 256 : 128;
+  // three tokens of 2,048 columns: 9.1 us with one CTA each, a column's loads behind the other's
+  const int most = (width + threads - 1) / threads, wanted = (4 * mir_sm_count() + tokens - 1) / tokens;
+  const int parts = wanted < 1 ? 1 : (wanted > most ? most : wanted);
   int status;
   if (bf16)
-    status = mir_launch("wkv_mix", wkv_mix_kernel<__nv_bfloat16>, dim3(tokens), dim3(threads), 0, stream, 0,
+    status = mir_launch("wkv_mix", wkv_mix_kernel<__nv_bfloat16>, dim3(tokens, parts), dim3(threads), 0, stream, 0,
                         (const __nv_bfloat16*)h, ld, tail, mu, row_of_token, query_starts, state_slots, positions,
                         (__nv_bfloat16*)out, tokens, width);
   else
-    status = mir_launch("wkv_mix", wkv_mix_kernel<float>, dim3(tokens), dim3(threads), 0, stream, 0, (const float*)h, ld,
+    status = mir_launch("wkv_mix", wkv_mix_kernel<float>, dim3(tokens, parts), dim3(threads), 0, stream, 0, (const float*)h, ld,
                         tail, mu, row_of_token, query_starts, state_slots, positions, (float*)out, tokens, width);
   if (status != MIR_OK || single_tokens_only) return status;
   if (bf16)
