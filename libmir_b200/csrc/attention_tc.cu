@@ -71,9 +71,16 @@ constexpr int kKeys = 128;                  // keys per tile
 constexpr int kDim = 128;                   // head_dim
 constexpr int kHalf = 128 * 128;            // bytes of a 128-row x 64-element half tile
 constexpr int kTile = 2 * kHalf;            // 32 KB
-constexpr int kKeyStages = 3;              // the key ring: a tile is asked for when the product with the one three back is over
-constexpr int kOffQ = 0, kOffK = kTile, kOffV = (1 + kKeyStages) * kTile;
-constexpr int kSmemBytes = (3 + kKeyStages) * kTile + 1024;
+constexpr int kWideDim = 192;               // key heads of the attention whose keys and values come out of cached latents
+constexpr int kKeyStages = 3;              // most stages of the key ring: a tile is asked for when the product with the one that many back is over
+// Shared memory for key heads of KEY_DIM: queries, the key ring, two value tiles.  Tiles of 192-wide keys take 48 KB: two stages.
+template <int KEY_DIM> struct Layout {
+  static constexpr int kHalves = KEY_DIM / 64;
+  static constexpr int kKeyTile = kHalves * kHalf;
+  static constexpr int kStages = KEY_DIM <= 128 ? kKeyStages : 2;
+  static constexpr int kOffQ = 0, kOffK = kKeyTile, kOffV = (1 + kStages) * kKeyTile;
+  static constexpr int kSmemBytes = kOffV + 2 * kTile + 1024;
+};
 constexpr int kParts = 2;                   // softmax threads per query row and stream (each takes 64 columns)
 constexpr int kCols = kKeys / kParts;       // columns of a tile that one softmax thread handles
 constexpr int kStreamThreads = kRows * kParts;
@@ -364,8 +371,9 @@ __device__ __forceinline__ int item_of(int k, int cta, int ctas, int items) {
 }
 
 // kValueDim: width of a value head, 128 or 64 (then one 64-wide half of the value tiles is loaded and the products with V
-// and the output accumulator are 64 columns wide).
-template <int kStreams, bool kShared, bool kScored = false, int kValueDim = kDim>
+// and the output accumulator are 64 columns wide).  kKeyDim: width of a key head, 128 or 192 (three 64-wide parts of a tile,
+// pages of 128 keys only, so that a tile always is one box for each part).
+template <int kStreams, bool kShared, bool kScored = false, int kValueDim = kDim, int kKeyDim = kDim>
 __global__ void __launch_bounds__(threads_for(kStreams), 1)
 tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__ CUtensorMap k_map,
                             const __grid_constant__ CUtensorMap v_map, const __grid_constant__ CUtensorMap k_tile_map,
@@ -374,6 +382,8 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                             const int* __restrict__ context_lens, int num_rows, int page_size, int heads, int kv_heads,
                             float scale_log2, int window, int tile_slots, int keep_first, AttentionExtras extras) {
   constexpr int kThreads = threads_for(kStreams);
+  using L = Layout<kKeyDim>;
+  constexpr int kOffQ = L::kOffQ, kOffK = L::kOffK, kOffV = L::kOffV, kRing = L::kStages;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long barriers[BARRIERS];
   __shared__ uint32_t tmem_base_slot;
@@ -447,14 +457,15 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     const uint32_t box_bytes = (uint32_t)page_size * 128u;
     // lane l loads half (l & 1) of page slot (l >> 1): at most 16 pages of 8 keys, so one round of 32 lanes
     const int slot = lane >> 1, half = lane & 1;
-    const int halves = which ? kValueDim / 64 : 2, width = which ? kValueDim : kDim;
+    const int halves = which ? kValueDim / 64 : L::kHalves, width = which ? kValueDim : kKeyDim;
+    const uint32_t stage_bytes = which ? (uint32_t)kTile : (uint32_t)L::kKeyTile;
     const bool loads = lane < 2 * pages_per_tile && half < halves;
     const uint32_t lane_dst = smem_base + (which ? kOffV : kOffK) + (uint32_t)half * kHalf +
                               (uint32_t)(slot * page_size) * 128u;
     const CUtensorMap* map = which ? &v_map : &k_map;
     const CUtensorMap* tile_map = which ? &v_tile_map : &k_tile_map;     // boxes of 128 keys
     const uint32_t tile_dst = smem_base + (which ? kOffV : kOffK);
-    const int stages = which ? 2 : kKeyStages;
+    const int stages = which ? 2 : kRing;
     const uint32_t full0 = bar(which ? V_FULL : K_FULL), free0 = bar(which ? V_FREE : K_FREE);
     int stage = 0;                                            // of the CTA's tile g = g0 + t: g % stages,
     uint32_t parity = 0;                                      // (g / stages) & 1
@@ -467,9 +478,10 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         // the queries, once the products with the last item's are over
         if (n > 0 && !wait_barrier(bar(Q_FREE), (uint32_t)(n - 1) & 1u)) { g_tc_attention_error = 1; break; }
         if (lane == 0) {
-          barrier_expect_bytes(bar(Q_FULL), kTile);
-          tma_load_2d(smem_base + kOffQ, &q_map, bar(Q_FULL), w.head * kDim, w.q_row0);
-          tma_load_2d(smem_base + kOffQ + kHalf, &q_map, bar(Q_FULL), w.head * kDim + 64, w.q_row0);
+          barrier_expect_bytes(bar(Q_FULL), L::kKeyTile);
+#pragma unroll
+          for (int part = 0; part < L::kHalves; ++part)
+            tma_load_2d(smem_base + kOffQ + (uint32_t)part * kHalf, &q_map, bar(Q_FULL), w.head * kKeyDim + part * 64, w.q_row0);
         }
       }
       const int x = w.kv_head * width + half * 64;
@@ -502,13 +514,13 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
           if (lane == 0) barrier_expect_bytes(full, (uint32_t)(halves * kHalf));
           __syncwarp();
           if (lane < halves)
-            tma_load_2d(tile_dst + (uint32_t)lane * kHalf + (uint32_t)stage * kTile, tile_map, full,
+            tma_load_2d(tile_dst + (uint32_t)lane * kHalf + (uint32_t)stage * stage_bytes, tile_map, full,
                         w.kv_head * width + lane * 64, first_page << page_shift);
         } else {
           const unsigned valid = __ballot_sync(0xffffffffu, page >= 0);
           if (lane == 0) barrier_expect_bytes(full, (uint32_t)__popc(valid) * box_bytes);
           __syncwarp();
-          if (page >= 0) tma_load_2d(lane_dst + (uint32_t)stage * kTile, map, full, x, page << page_shift);
+          if (page >= 0) tma_load_2d(lane_dst + (uint32_t)stage * stage_bytes, map, full, x, page << page_shift);
         }
         if (lane == 0 && which == 0) ATT_STAMP(g0 + t, 15);
         if (++stage == stages) { stage = 0; parity ^= 1u; }
@@ -529,9 +541,9 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     const uint32_t v_low = operand_low_mn_major(smem_base + kOffV, kHalf);
     bool alive = true;
     int g0 = 0, n = 0;
-    uint32_t key_stage = 0, key_parity = 0;                   // of the next tile of scores: g % kKeyStages, (g / kKeyStages) & 1
+    uint32_t key_stage = 0, key_parity = 0;                   // of the next tile of scores: g % kRing, (g / kRing) & 1
+    uint32_t score_turn = 0;                                  // kShared: its accumulator, g % 3
     uint32_t p_stage = 0, p_parity = 0;                       // kShared: of the next product with V: g % 3, (g / 3) & 1
-    static_assert(!kShared || kKeyStages == 3, "the score accumulators go round with the key ring");
     for (int k = 0; more(k); ++k) {
       const Work w = work(k);
       if (!w.valid) continue;
@@ -544,12 +556,12 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         if (alive && !wait_barrier(bar(K_FULL + key_stage), key_parity)) { g_tc_attention_error = 2; alive = false; }
         if (elected) ATT_STAMP(g, 12);
         tensor_fence_after_sync();
-        // (with the shared reference the scores have three buffers and go round with the key ring)
-        const uint32_t score_stage = kShared ? key_stage : stage;
-        const uint32_t b_low = k_low + key_stage * (uint32_t)(kTile >> 4), d = tmem_base + score_stage * 128u;
+        // (with the shared reference the scores have three buffers)
+        const uint32_t score_stage = kShared ? score_turn : stage;
+        const uint32_t b_low = k_low + key_stage * (uint32_t)(L::kKeyTile >> 4), d = tmem_base + score_stage * 128u;
         mma_bf16_ss_halves<false>(d, q_low, b_low, idesc_qk, elected);
 #pragma unroll
-        for (int kk = 1; kk < kDim / 16; ++kk) {
+        for (int kk = 1; kk < kKeyDim / 16; ++kk) {
           constexpr uint32_t kHalfStep = (uint32_t)(kHalf >> 4);
           const uint32_t offset = (uint32_t)(kk >> 2) * kHalfStep + (uint32_t)(kk & 3) * 2u;
           mma_bf16_ss_halves<true>(d, q_low + offset, b_low + offset, idesc_qk, elected);
@@ -558,7 +570,8 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         mma_commit_elected(bar(K_FREE + key_stage), elected);
         if (elected) ATT_STAMP(g, 2);
         if (t == tiles - 1) mma_commit_elected(bar(Q_FREE), elected);   // the item's last product with its queries
-        if (++key_stage == (uint32_t)kKeyStages) { key_stage = 0; key_parity ^= 1u; }   // (scores are issued in order)
+        if (++key_stage == (uint32_t)kRing) { key_stage = 0; key_parity ^= 1u; }   // (scores are issued in order)
+        if (kShared && ++score_turn == 3u) score_turn = 0;
       };
       // P(t) is written over S(t) in tensor memory, so S(t + 2), which takes the same accumulator, is issued
       // behind the product with P(t): the tensor cores run products in the order of issue, and while they work
@@ -858,9 +871,10 @@ static int prefill_attention_tc_with(const void* q, long long q_stride, void* ou
     return MIR_BAD_ARGUMENT;
   }
   if (keep_first < 0) { mir_set_error("prefill_attention_tc: keep_first is negative"); return MIR_BAD_ARGUMENT; }
-  if (!mir_prefill_attention_tc_takes(head_dim, page_size) || heads <= 0 || kv_heads <= 0 || heads % kv_heads ||
+  const bool wide = head_dim == kWideDim && page_size == kKeys && window == 0 && !scores_modified(extras) && extras.value_dim == kDim;
+  if ((!wide && !mir_prefill_attention_tc_takes(head_dim, page_size)) || heads <= 0 || kv_heads <= 0 || heads % kv_heads ||
       table_width <= 0 || window < 0 || num_rows < 0 || tokens < 0 || scale <= 0.0f ||
-      (q_stride % 8) || q_stride < (long long)heads * kDim || ((uintptr_t)q & 15) || ((uintptr_t)k_pages & 15) ||
+      (q_stride % 8) || q_stride < (long long)heads * head_dim || ((uintptr_t)q & 15) || ((uintptr_t)k_pages & 15) ||
       ((uintptr_t)v_pages & 15) || ((uintptr_t)out & 15) || cache_rows <= 0 || cache_rows > 0x7fffffffll ||
       q_stride > 0x7fffffffll) {
     mir_set_error("prefill_attention_tc: takes head_dim 128, pages of 8..128 keys that divide 128, a positive scale "
@@ -870,7 +884,7 @@ static int prefill_attention_tc_with(const void* q, long long q_stride, void* ou
   }
   const int value_dim = extras.value_dim > 0 ? extras.value_dim : head_dim;
   const bool scored = scores_modified(extras);
-  if (!mir_prefill_attention_tc_takes_values(value_dim) || (value_dim != kDim && !scored) ||
+  if ((!wide && !mir_prefill_attention_tc_takes_values(value_dim)) || (value_dim != kDim && !scored) ||
       (extras.slopes != nullptr && (extras.rel_bias != nullptr || (keep_first > 0 && window > 0)))) {
     mir_set_error("prefill_attention_tc: value heads of %d (64 goes with modified scores), one kind of bias at a time, no kept keys beside slopes",
                   value_dim);
@@ -879,33 +893,29 @@ static int prefill_attention_tc_with(const void* q, long long q_stride, void* ou
   CUtensorMap q_map, k_map, v_map, k_tile_map, v_tile_map;
   int status = tensor_map_for(q, tokens, (int)q_stride, (int)q_stride, kRows, &q_map);
   if (status != MIR_OK) return status;
-  status = tensor_map_for(k_pages, (int)cache_rows, kv_heads * kDim, kv_heads * kDim, page_size, &k_map);
+  status = tensor_map_for(k_pages, (int)cache_rows, kv_heads * head_dim, kv_heads * head_dim, page_size, &k_map);
   if (status != MIR_OK) return status;
   status = tensor_map_for(v_pages, (int)cache_rows, kv_heads * value_dim, kv_heads * value_dim, page_size, &v_map);
   if (status != MIR_OK) return status;
-  status = tensor_map_for(k_pages, (int)cache_rows, kv_heads * kDim, kv_heads * kDim, kKeys, &k_tile_map);
+  status = tensor_map_for(k_pages, (int)cache_rows, kv_heads * head_dim, kv_heads * head_dim, kKeys, &k_tile_map);
   if (status != MIR_OK) return status;
   status = tensor_map_for(v_pages, (int)cache_rows, kv_heads * value_dim, kv_heads * value_dim, kKeys, &v_tile_map);
   if (status != MIR_OK) return status;
+  constexpr int kSmemBytes = Layout<kDim>::kSmemBytes, kWideBytes = Layout<kWideDim>::kSmemBytes;
   static bool configured = false;
   if (!configured) {
-    cudaError_t err = cudaFuncSetAttribute(tc_prefill_attention_kernel<2, false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(tc_prefill_attention_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(tc_prefill_attention_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(tc_prefill_attention_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmemBytes);
-    if (err == cudaSuccess)
-      err = cudaFuncSetAttribute(tc_prefill_attention_kernel<2, true, true, 64>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    cudaError_t err = cudaSuccess;
+    auto reserve = [&](auto kernel, int bytes) {
+      if (err == cudaSuccess) err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    reserve(tc_prefill_attention_kernel<2, false>, kSmemBytes);
+    reserve(tc_prefill_attention_kernel<2, true>, kSmemBytes);
+    reserve(tc_prefill_attention_kernel<1, false>, kSmemBytes);
+    reserve(tc_prefill_attention_kernel<2, true, true>, kSmemBytes);
+    reserve(tc_prefill_attention_kernel<2, true, true, 64>, kSmemBytes);
+    reserve(tc_prefill_attention_kernel<2, true, false, kDim, kWideDim>, kWideBytes);
     if (err != cudaSuccess) {
-      mir_set_error("prefill_attention_tc: cannot reserve %d bytes of shared memory: %s", kSmemBytes,
-                    cudaGetErrorString(err));
+      mir_set_error("prefill_attention_tc: cannot reserve %d bytes of shared memory: %s", kWideBytes, cudaGetErrorString(err));
       return MIR_CUDA_ERROR;
     }
     configured = true;
@@ -923,6 +933,11 @@ static int prefill_attention_tc_with(const void* q, long long q_stride, void* ou
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms <= 0) sms = 148;
   }
   const int ctas = (int)std::min<long long>(items, g_ctas > 0 ? g_ctas : sms);
+  if (wide)
+    return mir_launch("prefill_attention_tc", tc_prefill_attention_kernel<2, true, false, kDim, kWideDim>, dim3(ctas),
+                      dim3(threads_for(2)), (size_t)kWideBytes, stream, 0, q_map, k_map, v_map, k_tile_map, v_tile_map,
+                      (bf16*)out, block_table, table_width, query_starts, context_lens, num_rows, page_size, heads, kv_heads,
+                      scale * 1.4426950408889634f, 0, tile_slots, 0, extras);
   if (value_dim == 64)
     return mir_launch("prefill_attention_tc", tc_prefill_attention_kernel<2, true, true, 64>, dim3(ctas), dim3(threads_for(2)),
                       (size_t)kSmemBytes, stream, 0, q_map, k_map, v_map, k_tile_map, v_tile_map, (bf16*)out, block_table, table_width,
@@ -977,6 +992,19 @@ MIR_EXPORT int mir_prefill_attention_tc_scored_bf16(const void* q, long long q_s
   return prefill_attention_tc_with(q, q_stride, out, k_pages, v_pages, cache_rows, block_table, table_width, query_starts,
                                    context_lens, num_rows, tokens, page_size, heads, kv_heads, head_dim, scale, window, 0,
                                    stream, extras);
+}
+
+// Key heads of 192 and value heads of 128 beside them, rows in pages of 128 (keys and values that were formed from cached
+// latents for this step): k [rows, heads, 192], v [rows, heads, 128].  gate: one number for each result column, or null.
+MIR_EXPORT int mir_prefill_attention_tc_wide_bf16(const void* q, long long q_stride, void* out, const void* k, const void* v,
+                                                  long long rows, const int* block_table, int table_width,
+                                                  const int* query_starts, const int* context_lens, int num_rows, int tokens,
+                                                  int heads, float scale, const void* gate, long long gate_stride,
+                                                  cudaStream_t stream) {
+  AttentionExtras extras{nullptr, (const bf16*)gate, gate_stride};
+  extras.value_dim = kDim;
+  return prefill_attention_tc_with(q, q_stride, out, k, v, rows, block_table, table_width, query_starts, context_lens,
+                                   num_rows, tokens, kKeys, heads, heads, kWideDim, scale, 0, 0, stream, extras);
 }
 
 MIR_EXPORT int mir_prefill_attention_tc_kept_bf16(const void* q, long long q_stride, void* out, const void* k_pages,

@@ -93,6 +93,34 @@ __global__ void latent_prepare_kernel(const T* __restrict__ packed, long long ld
   }
 }
 
+// The cached rows of every request in one run of tiles of 128 rows each, for products over all of them: request r's tile p is
+// tile number first(r) + p, first(r) counting the tiles of the requests before it; rows beyond the request's context are
+// zeros.  tile_table [rows, tile_width] receives those numbers: a block table over pages of 128 rows.  A CTA copies a tile in
+// 16-byte pieces (one read and one write of the context, behind which the products run).
+constexpr int kGatherRows = 128;
+template <typename T>
+__global__ void __launch_bounds__(256)
+latent_gather_kernel(const T* __restrict__ pages, int width, const int* __restrict__ block_table, int table_width,
+                     const int* __restrict__ context_lens, int page_size, T* __restrict__ gathered,
+                     int* __restrict__ tile_table, int tile_width) {
+  const int row = blockIdx.y, tile = blockIdx.x;
+  const int context = context_lens[row], first_key = tile * kGatherRows;
+  if (first_key >= context) return;
+  int number = tile;
+  for (int r = 0; r < row; ++r) number += (context_lens[r] + kGatherRows - 1) / kGatherRows;
+  if (threadIdx.x == 0) tile_table[(size_t)row * tile_width + tile] = number;
+  constexpr int PIECE = 16 / sizeof(T);
+  const int pieces = width / PIECE;
+  T* to = gathered + (size_t)number * kGatherRows * width;
+  for (int index = threadIdx.x; index < kGatherRows * pieces; index += blockDim.x) {
+    const int r = index / pieces, c = (index - r * pieces) * PIECE, key = first_key + r;
+    uint4 value = make_uint4(0u, 0u, 0u, 0u);
+    const int page = key < context ? block_table[(size_t)row * table_width + key / page_size] : -1;
+    if (page >= 0) value = *reinterpret_cast<const uint4*>(pages + ((size_t)page * page_size + key % page_size) * width + c);
+    *reinterpret_cast<uint4*>(to + (size_t)r * width + c) = value;
+  }
+}
+
 // One thread per (token, head, pair).  src and dst may be the same buffer.
 template <typename T>
 __global__ void rope_rows_kernel(const T* __restrict__ src, long long src_token, long long src_head, T* dst,
@@ -204,6 +232,28 @@ MIR_EXPORT int mir_latent_prepare(int bf16, const void* packed, long long ld, in
                     (const float*)packed, ld, q_offset, q_rank, kv_offset, kv_rank, rotary, q_norm, kv_norm, eps, positions,
                     slot_mapping, inv_freq, magnitude, interleaved, (float*)latent_q, (float*)pages, (const float*)turn_src,
                     src_token, src_head, (float*)turn_dst, dst_token, dst_head, turn_heads);
+}
+
+// pages [cache rows, width] in rows of whole 16-byte pieces; tiles: the most tiles of 128 rows a request has; gathered has room
+// for every request's tiles, tile_table for `tiles` numbers a request.
+MIR_EXPORT int mir_latent_gather(int bf16, const void* pages, int width, const int* block_table, int table_width,
+                                 const int* context_lens, int rows, int tiles, int page_size, void* gathered, int* tile_table,
+                                 cudaStream_t stream) {
+  if (rows == 0 || tiles == 0) return MIR_OK;
+  if (rows < 0 || rows > 65535 || tiles < 0 || width <= 0 || page_size <= 0 || table_width <= 0 || width % (bf16 ? 8 : 4) ||
+      (((uintptr_t)pages | (uintptr_t)gathered) & 15)) {
+    mir_set_error("latent_gather: bad sizes (rows %d, tiles %d, width %d, page %d) or rows that are not 16-byte pieces", rows,
+                  tiles, width, page_size);
+    return MIR_BAD_ARGUMENT;
+  }
+  const dim3 grid(tiles, rows);
+  if (bf16)
+    latent_gather_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pages, width, block_table, table_width, context_lens,
+                                                   page_size, (__nv_bfloat16*)gathered, tile_table, tiles);
+  else
+    latent_gather_kernel<<<grid, 256, 0, stream>>>((const float*)pages, width, block_table, table_width, context_lens, page_size,
+                                                   (float*)gathered, tile_table, tiles);
+  return mir_check_launch("latent_gather");
 }
 
 MIR_EXPORT int mir_rope_rows(int bf16, const void* src, long long src_token, long long src_head, void* dst,

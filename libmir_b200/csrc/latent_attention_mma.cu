@@ -297,25 +297,49 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
   }
 }
 
-// One CTA per (token, head): the partitions' partial results into the normalised output.
-__global__ void latent_attention_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
-                                              __nv_bfloat16* __restrict__ out, int rank, int partitions) {
+// One CTA per (token, head): the partitions' partial results into the normalised output.  The partitions' maxima and sums are
+// read side by side, and a thread takes four columns whose loads do not wait for one another (a column at a time, each
+// partition's numbers behind the other's: 8.5 us for 48 rows of 512 columns).
+constexpr int kMergeThreads = 128, kMergePartitions = 256;
+__global__ void __launch_bounds__(kMergeThreads)
+latent_attention_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
+                              __nv_bfloat16* __restrict__ out, int rank, int partitions) {
+  __shared__ float factor_s[kMergePartitions], sum_s[kMergePartitions];
   const size_t unit = blockIdx.x;
-  float top = -INFINITY;
-  for (int p = 0; p < partitions; ++p) top = fmaxf(top, partial_ml[(unit * partitions + p) * 2]);
+  const int lane = threadIdx.x & 31;
+  const float2* ml = reinterpret_cast<const float2*>(partial_ml) + unit * partitions;
+  float top = -INFINITY;                                         // (every warp for itself)
+  for (int p = lane; p < partitions; p += 32) top = fmaxf(top, ml[p].x);
+  top = warp_max(top);
+  for (int p = threadIdx.x; p < min(partitions, kMergePartitions); p += kMergeThreads) {
+    const float2 both = ml[p];
+    factor_s[p] = both.x != -INFINITY ? exp2f(both.x - top) : 0.0f;
+    sum_s[p] = both.x != -INFINITY ? both.y : 0.0f;
+  }
+  __syncthreads();
+  auto factor_of = [&](int p) {                                  // (more partitions than are kept: formed again)
+    return p < kMergePartitions ? factor_s[p] : (ml[p].x != -INFINITY ? exp2f(ml[p].x - top) : 0.0f);
+  };
   float total = 0.0f;
   for (int p = 0; p < partitions; ++p) {
-    const float m = partial_ml[(unit * partitions + p) * 2];
-    if (m != -INFINITY) total += partial_ml[(unit * partitions + p) * 2 + 1] * exp2f(m - top);
+    const float factor = factor_of(p);
+    if (factor != 0.0f) total += (p < kMergePartitions ? sum_s[p] : ml[p].y) * factor;
   }
   const float inverse = total > 0.0f ? 1.0f / total : 0.0f;
-  for (int c = threadIdx.x; c < rank; c += blockDim.x) {
-    float sum = 0.0f;
+  for (int c = threadIdx.x * 4; c < rank; c += kMergeThreads * 4) {          // (rank is a multiple of 8)
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float* from = partial_o + unit * partitions * rank + c;
+#pragma unroll 4
     for (int p = 0; p < partitions; ++p) {
-      const float m = partial_ml[(unit * partitions + p) * 2];
-      if (m != -INFINITY) sum = fmaf(partial_o[(unit * partitions + p) * rank + c], exp2f(m - top), sum);
+      const float factor = factor_of(p);
+      if (factor == 0.0f) continue;                              // (a partition without keys)
+      const float4 v = *reinterpret_cast<const float4*>(from + (size_t)p * rank);
+      sum.x = fmaf(v.x, factor, sum.x); sum.y = fmaf(v.y, factor, sum.y);
+      sum.z = fmaf(v.z, factor, sum.z); sum.w = fmaf(v.w, factor, sum.w);
     }
-    out[unit * rank + c] = __float2bfloat16_rn(sum * inverse);
+    __nv_bfloat162* to = reinterpret_cast<__nv_bfloat162*>(out + unit * rank + c);
+    to[0] = __floats2bfloat162_rn(sum.x * inverse, sum.y * inverse);
+    to[1] = __floats2bfloat162_rn(sum.z * inverse, sum.w * inverse);
   }
 }
 
@@ -388,7 +412,7 @@ MIR_EXPORT int mir_latent_attention_bf16(const void* q, long long q_stride, void
   else MIR_LATENT(8);
 #undef MIR_LATENT
   if (status != MIR_OK || partitions == 1) return status;
-  latent_attention_merge_kernel<<<dim3(tokens * heads), dim3(128), 0, stream>>>(partial_o, partial_ml,
+  latent_attention_merge_kernel<<<dim3(tokens * heads), dim3(kMergeThreads), 0, stream>>>(partial_o, partial_ml,
                                                                                (__nv_bfloat16*)out, rank, partitions);
   return mir_check_launch("latent_attention_merge");
 }

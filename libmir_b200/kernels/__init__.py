@@ -11,7 +11,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 from ctypes import c_double, c_float, c_int, c_longlong, c_size_t, c_void_p
-from typing import Optional
+from typing import Sequence, Optional
 
 import numpy as np
 import torch
@@ -78,6 +78,8 @@ _SIGNATURES = {
         "mir_latent_prepare": [c_int, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_float,
                                c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p, c_longlong,
                                c_longlong, c_void_p, c_longlong, c_longlong, c_int, c_int, c_void_p],
+        "mir_latent_gather": [c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                              c_void_p],
         "mir_rope_rows": [c_int, c_void_p, c_longlong, c_longlong, c_void_p, c_longlong, c_longlong, c_void_p, c_void_p,
                           c_float, c_int, c_int, c_int, c_int, c_void_p],
         "mir_sigmoid_gate": [c_int, c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p],
@@ -152,6 +154,9 @@ _SIGNATURES = {
         "mir_decode_attention_tc_takes": [c_int, c_int, c_int],
         "mir_decode_attention_tc_takes_values": [c_int],
         "mir_prefill_attention_tc_takes_values": [c_int],
+        "mir_prefill_attention_tc_wide_bf16": [c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p,
+                                               c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p,
+                                               c_longlong, c_void_p],
         "mir_head_logits_bf16": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                  c_int, c_void_p, c_size_t, c_void_p, c_void_p],
         "mir_gemm_tc_stream_head_candidates": [c_int],
@@ -777,6 +782,52 @@ def rope_rows(src: torch.Tensor, dst: torch.Tensor, positions: torch.Tensor, inv
     _check(lib, lib.mir_rope_rows(_is_bf16(src), src.data_ptr(), src.stride(0), src.stride(1), dst.data_ptr(),
                                   dst.stride(0), dst.stride(1), positions.data_ptr(), inv_freq.data_ptr(),
                                   float(magnitude), int(interleaved), tokens, heads, rotary, _stream()))
+
+
+GATHER_ROWS = 128               # rows of a tile that latent_gather lays out
+
+
+def latent_gather(pages: torch.Tensor, block_table: torch.Tensor, context_lens: torch.Tensor, page_size: int,
+                  contexts: Sequence[int], gathered: torch.Tensor, tile_table: torch.Tensor) -> None:
+    """Every request's cached rows (pages [cache rows, 1, width]) behind one another in tiles of GATHER_ROWS rows, zeros
+    beyond a request's context; tile_table [rows, most tiles of a request] receives the tiles' numbers.  `contexts`: the
+    context lengths as the host knows them; gathered is [all tiles * GATHER_ROWS, width]."""
+    _cuda(pages, block_table, context_lens, gathered, tile_table)
+    rows, width = len(contexts), pages.shape[-1]
+    tiles = [-(-n // GATHER_ROWS) for n in contexts]
+    _require(pages.is_contiguous() and gathered.is_contiguous() and gathered.dtype == pages.dtype
+             and gathered.shape == (sum(tiles) * GATHER_ROWS, width) and block_table.dtype == torch.int32
+             and block_table.is_contiguous() and block_table.shape[0] >= rows and context_lens.dtype == torch.int32
+             and context_lens.numel() >= rows and tile_table.dtype == torch.int32 and tile_table.is_contiguous()
+             and tile_table.shape == (rows, max(tiles)), "latent_gather: the cached rows, tiles or tables do not fit")
+    lib = library("core")
+    _check(lib, lib.mir_latent_gather(_is_bf16(pages), pages.data_ptr(), width, block_table.data_ptr(), block_table.shape[1],
+                                      context_lens.data_ptr(), rows, max(tiles), page_size, gathered.data_ptr(),
+                                      tile_table.data_ptr(), _stream()))
+
+
+def prefill_attention_wide(q: torch.Tensor, out: torch.Tensor, keys: torch.Tensor, values: torch.Tensor,
+                           tile_table: torch.Tensor, query_starts: torch.Tensor, context_lens: torch.Tensor, heads: int,
+                           scale: float, gate: Optional[torch.Tensor] = None) -> None:
+    """Causal attention of portions on the tcgen05 kernel with key heads of 192 and value heads of 128: q [tokens, >= heads *
+    192] rows, keys [n, heads * 192] and values [n, heads * 128] in pages of 128 rows (tile_table [rows, pages of a request]),
+    out [tokens, heads * 128], multiplied by the sigmoid of `gate` (rows of heads * 128) where there is one."""
+    _cuda(q, out, keys, values, tile_table, query_starts, context_lens, gate)
+    rows = context_lens.numel()
+    _require(all(t.dtype == torch.bfloat16 for t in (q, out, keys, values)) and q.stride(1) == 1 and out.is_contiguous()
+             and keys.is_contiguous() and values.is_contiguous() and out.shape[1] == heads * 128
+             and keys.shape[1] == heads * 192 and values.shape == (keys.shape[0], heads * 128)
+             and q.shape == (out.shape[0], heads * 192), "prefill_attention_wide: shapes do not fit")
+    _require(tile_table.dtype == torch.int32 and tile_table.is_contiguous() and tile_table.shape[0] == rows
+             and query_starts.dtype == torch.int32 and query_starts.numel() == rows + 1
+             and context_lens.dtype == torch.int32, "prefill_attention_wide: bad metadata")
+    _require(gate is None or (gate.dtype == torch.bfloat16 and gate.shape == out.shape and gate.stride(1) == 1),
+             "prefill_attention_wide: the gate is one number for each result")
+    lib = library("bf16")
+    _check(lib, lib.mir_prefill_attention_tc_wide_bf16(
+        q.data_ptr(), q.stride(0), out.data_ptr(), keys.data_ptr(), values.data_ptr(), keys.shape[0], tile_table.data_ptr(),
+        tile_table.shape[1], query_starts.data_ptr(), context_lens.data_ptr(), rows, out.shape[0], heads, scale, _ptr(gate),
+        gate.stride(0) if gate is not None else 0, _stream()))
 
 
 HEAD_LINEAR_LIBRARY = True       # False: the products per head always run the 32-bit multiply-add kernel

@@ -25,6 +25,8 @@ from ..config.spec import PagedKv, ParamSpec
 from ..registry import build_part
 from .base import Mixer
 
+PORTION_QUERIES = 48        # queries of a portion for each key of context from which on keys and values are formed for it
+
 
 def _pad8(n: int) -> int:
     return -(-n // 8) * 8
@@ -90,6 +92,17 @@ class LatentAttention(Mixer):
         self.w_uv = tensors["uv"].view(s.heads, s.value_dim, s.kv_rank).transpose(1, 2).contiguous()
         self.w_o = tensors["o"].contiguous()
         self.kv_norm = tensors["dkv.norm"].contiguous()
+        # For portions of prompts: keys [latent's key | rotated part] of every head and values out of whole cached rows, by two
+        # products (the rotated part passes through rows of the identity).
+        self.w_keys = self.w_values = None
+        if (self.env.dtype == torch.bfloat16 and (s.head_dim, s.rotary_dim, s.value_dim) == (128, 64, 128)
+                and self.position is not None and self.key_width % 8 == 0 and self.packed_width % 8 == 0 and (self.segments["g"] % 8 == 0 if s.gate else True)):
+            w_keys = torch.zeros((s.heads, s.head_dim + s.rotary_dim, self.key_width), dtype=tensors["uk"].dtype,
+                                 device=tensors["uk"].device)
+            w_keys[:, :s.head_dim, :s.kv_rank] = tensors["uk"].view(s.heads, s.head_dim, s.kv_rank)
+            w_keys[:, s.head_dim:, s.kv_rank:] = torch.eye(s.rotary_dim, dtype=w_keys.dtype, device=w_keys.device)
+            self.w_keys = w_keys.view(s.heads * (s.head_dim + s.rotary_dim), self.key_width)
+            self.w_values = tensors["uv"].contiguous()
 
     def weight_bytes(self):
         return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_uq, self.w_uk, self.w_uv, self.w_o)
@@ -107,6 +120,14 @@ class LatentAttention(Mixer):
         packed = ctx.alloc((tokens, self.packed_width), dtype)
         kernels.linear(x, self.w_in, packed, alloc=ctx.alloc)
         per_head = s.head_dim + s.rotary_dim
+        gate = packed[:, self.segments["g"]:self.segments["g"] + self.out_width] if s.gate else None
+        if self._takes_portions(ctx):
+            mixed = self._portions(ctx, group, cache, packed, gate, table, magnitude, interleaved)
+            if overwrite:
+                kernels.linear(mixed, self.w_o, residual, alloc=ctx.alloc)
+            else:
+                ctx.accumulate(mixed, self.w_o, residual)
+            return
         folded = ctx.alloc((tokens, s.heads, self.key_width), dtype)
         latent_q, turn = None, None
         if s.q_rank:
@@ -129,13 +150,62 @@ class LatentAttention(Mixer):
         attended = ctx.alloc((tokens, s.heads * s.kv_rank), dtype)
         self.attend(ctx, group, cache, folded.view(tokens, s.heads * self.key_width), attended)
         mixed = ctx.alloc((tokens, self.out_width), dtype)
-        gate = packed[:, self.segments["g"]:self.segments["g"] + self.out_width] if s.gate else None
         kernels.head_linear(attended.view(tokens, s.heads, s.kv_rank), self.w_uv, mixed.view(tokens, s.heads, s.value_dim),
                             gate)
         if overwrite:
             kernels.linear(mixed, self.w_o, residual, alloc=ctx.alloc)
         else:
             ctx.accumulate(mixed, self.w_o, residual)
+
+    def _takes_portions(self, ctx) -> bool:
+        """Whether the step's rows attend over keys and values formed from the cached latents (`_portions`) instead of over
+        the latents themselves.  Forming them costs a pass over every request's whole context, and saves 768 of 1,088
+        multiply-adds for each query and key and the products that fold queries and unfold results, on a kernel that runs
+        at several times the rate: from about 48 queries for each key of context on it is less."""
+        if self.w_keys is None or ctx.decode_only or ctx.single_rows:
+            return False
+        starts, before = ctx.host_query_starts, ctx.host_start_positions
+        portions = [b - a for a, b in zip(starts, starts[1:])]
+        contexts = [n + k for n, k in zip(before, portions)]
+        return min(portions, default=0) > 0 and sum(p * c for p, c in zip(portions, contexts)) >= PORTION_QUERIES * sum(contexts)
+
+    def _portions(self, ctx, group, cache, packed, gate, table, magnitude, interleaved):
+        """The mixer's result before its output projection, for portions of prompts: queries of head_dim + rotary numbers
+        against keys and values of every head."""
+        s = self.spec
+        tokens, dtype = packed.shape[0], self.env.dtype
+        per_head = s.head_dim + s.rotary_dim
+        latent_q, turn = None, None
+        if s.q_rank:
+            latent_q = ctx.alloc((tokens, s.q_rank), dtype)
+        else:
+            q = packed[:, self.segments["q"]:self.segments["q"] + self.q_width]
+            turned = q.unflatten(1, (s.heads, per_head))[:, :, s.head_dim:]
+            turn = (turned, turned)
+        kernels.latent_prepare(packed, self.segments.get("dq", 0), s.q_rank, self.segments["dkv"], s.kv_rank, s.rotary_dim,
+                               self.q_norm, self.kv_norm, s.norm_eps, ctx.positions,
+                               group.slot_mapping if cache.writes else None, table, magnitude, interleaved, latent_q,
+                               cache.k_pages, turn)
+        if s.q_rank:
+            q = ctx.alloc((tokens, self.q_width), dtype)
+            kernels.linear(latent_q, self.w_uq, q, alloc=ctx.alloc)
+            turned = q.view(tokens, s.heads, per_head)[:, :, s.head_dim:]
+            kernels.rope_rows(turned, turned, ctx.positions, table, magnitude, interleaved)
+        starts, before = ctx.host_query_starts, ctx.host_start_positions
+        contexts = [n + b - a for n, a, b in zip(before, starts, starts[1:])]
+        tiles = [-(-n // kernels.GATHER_ROWS) for n in contexts]
+        rows = sum(tiles) * kernels.GATHER_ROWS
+        gathered = ctx.alloc((rows, self.key_width), dtype)
+        tile_table = ctx.alloc((len(contexts), max(tiles)), torch.int32)
+        kernels.latent_gather(cache.k_pages, group.block_table, ctx.context_lens, cache.page_size, contexts, gathered, tile_table)
+        keys = ctx.alloc((rows, s.heads * per_head), dtype)
+        kernels.linear(gathered, self.w_keys, keys, alloc=ctx.alloc)
+        values = ctx.alloc((rows, self.out_width), dtype)
+        kernels.linear(gathered[:, :s.kv_rank], self.w_values, values, alloc=ctx.alloc)
+        mixed = ctx.alloc((tokens, self.out_width), dtype)
+        kernels.prefill_attention_wide(q, mixed, keys, values, tile_table, ctx.query_starts, ctx.context_lens, s.heads, s.scale,
+                                       gate)
+        return mixed
 
     def attend(self, ctx, group, cache, folded, out):
         """Every packed row's folded query heads over its request's cached rows: one key head of kv_rank + rotary

@@ -297,6 +297,75 @@ def test_tensor_core_attention_over_cached_latents(heads, page_size, rank, rotar
         at += n
 
 
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("heads,portions,contexts", [(1, [1], [1]), (3, [130, 7, 257], [130, 300, 257]), (2, [128, 129], [128, 385]),
+                                                     (5, [700], [1000])])
+def test_tcgen05_attention_with_key_heads_of_192(heads, portions, contexts, gated):
+    """Keys and values in pages of 128 rows that lie in any order, NaN in the pages nobody names; edges of query and key tiles."""
+    from libmir_b200 import kernels
+    generator = torch.Generator().manual_seed(sum(portions) + heads)
+    normal = lambda *shape, scale=1.0: (torch.randn(*shape, generator=generator) * scale).to(torch.bfloat16)
+    tiles = [-(-n // 128) for n in contexts]
+    order = torch.randperm(sum(tiles) + 3, generator=generator)[:sum(tiles)]
+    keys, values = (torch.full(((sum(tiles) + 3) * 128, heads * d), float("nan")).to(torch.bfloat16) for d in (192, 128))
+    table = torch.full((len(tiles), max(tiles)), -1, dtype=torch.int32)
+    tokens = sum(portions)
+    q = normal(tokens, heads * 192 + 64)
+    gate = normal(tokens, heads * 128 + 8)
+    want = torch.zeros(tokens, heads, 128, dtype=F64)
+    cursor = begin = 0
+    for r, (count, context, n) in enumerate(zip(portions, contexts, tiles)):
+        k, v = normal(n * 128, heads * 192), normal(n * 128, heads * 128)
+        k[context:], v[context:] = 0, 0
+        for t in range(n):
+            page = int(order[cursor + t])
+            table[r, t] = page
+            keys[page * 128:(page + 1) * 128], values[page * 128:(page + 1) * 128] = k[t * 128:(t + 1) * 128], v[t * 128:(t + 1) * 128]
+        hidden = torch.arange(context)[None, :] > torch.arange(context - count, context)[:, None]
+        for h in range(heads):
+            rows = q[begin:begin + count, h * 192:(h + 1) * 192].double()
+            scores = rows @ k[:context, h * 192:(h + 1) * 192].double().T * 0.07
+            want[begin:begin + count, h] = torch.softmax(scores.masked_fill(hidden, -math.inf), -1) @ v[:context, h * 128:(h + 1) * 128].double()
+        cursor, begin = cursor + n, begin + count
+    if gated:
+        want = want * torch.sigmoid(gate[:, :heads * 128].double()).view(tokens, heads, 128)
+    starts = torch.tensor(np.concatenate([[0], np.cumsum(portions)]), dtype=torch.int32)
+    out = torch.full((tokens, heads * 128), float("nan"), dtype=torch.bfloat16, device=device())
+    kernels.prefill_attention_wide(on_device(q)[:, :heads * 192], out, on_device(keys), on_device(values), on_device(table),
+                                   on_device(starts), on_device(torch.tensor(contexts, dtype=torch.int32)), heads, 0.07,
+                                   on_device(gate)[:, :heads * 128] if gated else None)
+    # weights and results are rounded to 8 bits; the weights' roundings average over the keys
+    close(out.view(tokens, heads, 128), want, 1.2e-2)
+    assert kernels.prefill_attention_error() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("page_size,width,contexts", [(16, 64, [1, 129, 300]), (8, 24, [128]), (100, 40, [256, 5])])
+def test_cached_rows_gathered_into_tiles(dtype, page_size, width, contexts):
+    from libmir_b200 import kernels
+    torch.manual_seed(3)
+    pages = [-(-n // page_size) for n in contexts]
+    order = torch.randperm(sum(pages) + 2)
+    pool = torch.randn((sum(pages) + 2) * page_size, 1, width).to(dtype)
+    table = torch.full((len(pages), max(pages) + 1), -1, dtype=torch.int32)
+    tiles = [-(-n // 128) for n in contexts]
+    want, cursor = [], 0
+    for r, (n, count) in enumerate(zip(contexts, pages)):
+        table[r, :count] = order[cursor:cursor + count].int()
+        rows = torch.cat([pool[int(p) * page_size:(int(p) + 1) * page_size, 0] for p in order[cursor:cursor + count]])[:n]
+        want.append(torch.cat([rows, torch.zeros(tiles[r] * 128 - n, width, dtype=dtype)]))
+        cursor += count
+    got = torch.full((sum(tiles) * 128, width), float("nan"), dtype=dtype, device=device())
+    numbers = torch.full((len(tiles), max(tiles)), -7, dtype=torch.int32, device=device())
+    kernels.latent_gather(on_device(pool), on_device(table), on_device(torch.tensor(contexts, dtype=torch.int32)), page_size,
+                          contexts, got, numbers)
+    assert torch.equal(got.cpu(), torch.cat(want))
+    first = 0
+    for r, n in enumerate(tiles):
+        assert numbers[r, :n].tolist() == list(range(first, first + n))
+        first += n
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_blends_with_the_token_before_carry_over_portions(dtype):
     """wkv_mix: the token before a portion's first token is the request's state (zeros at its start); slots of other
@@ -575,6 +644,36 @@ def test_whole_prompts_token_by_token_and_portions(tmp_path, name, dtype):
         assert np.array_equal(whole, single) and np.array_equal(whole, portions) and np.array_equal(whole, late)
     for group in model.cache_stats()["groups"]:
         assert group["free"] == group["pages"]
+
+
+def test_portions_attend_over_keys_and_values_formed_from_latents(tmp_path):
+    """Heads of 128 + 64 rotated and values of 128: prompts and long portions form keys and values, short portions and single
+    tokens attend over the latents, and all of them continue one another's requests."""
+    from libmir_b200 import StepEntry, kernels
+    config = {"architecture": "Zufotar", "vocab": 101, "width": 128, "norm": {"eps": 1e-6}, "embedding": {"scale": 1.0},
+              "layers": [{"type": "latent_attention", "mlp": {"kind": "dense", "ff": 64}, "mixer": {
+                  "heads": h, "dim": 128, "rot_dim": 64, "vdim": 128, "q_rank": 40, "kv_rank": 72, "scale": 0.07,
+                  "rot": {"dims": 64, "base": 1000.0}}} for h in (2, 3)]}
+    folder = make_folder(tmp_path, config, seed=5, dtype="bfloat16")
+    rng = np.random.default_rng(9)
+    ids = random_ids(rng, config["vocab"], 420)
+    want = reference(folder, ids)
+    model = load(folder, "bfloat16", 16, 120)
+    assert all(block.mixer.w_keys is not None for block in model.decoder.blocks)
+    for what, cuts in (("whole", [420]), ("long portions", [130, 100, 190]), ("a short one between", [200, 9, 1, 210]),
+                       ("single tokens behind", [400, 1])):
+        before = kernels.launch_counts().get("latent_gather", 0)
+        close_logits(feed(model, what, ids, cuts), want, "bfloat16", what)
+        assert kernels.launch_counts().get("latent_gather", 0) - before == 2 * sum(c >= 100 for c in cuts)
+    # two requests of unequal length, then more of both
+    other = random_ids(rng, config["vocab"], 300)
+    for name in ("a", "b"):
+        model.admit(name)
+    first = model.step([StepEntry("a", ids[:150], range(150)), StepEntry("b", other[:77], range(77))]).logits.cpu().numpy().copy()
+    second = model.step([StepEntry("a", ids[150:], range(270)), StepEntry("b", other[77:], range(223))]).logits.cpu().numpy()
+    close_logits(np.concatenate([first[:150], second[:270]]), want, "bfloat16", "beside another request")
+    close_logits(np.concatenate([first[150:], second[270:]]), reference(folder, other), "bfloat16", "the other request")
+    assert kernels.prefill_attention_error() == 0
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
