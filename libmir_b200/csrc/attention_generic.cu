@@ -84,6 +84,7 @@ __global__ void paged_attention_generic_kernel(
       const T* k_row = k_pages + key_offset * head_dim;
       float dot = 0.0f;
       if (head_dim % 8 == 0) {                                // (then every key row starts on a 16-byte boundary)
+#pragma unroll 4
         for (int d = 0; d < head_dim; d += 8) {
           float k8[8];
           load8(k_row + d, k8);
@@ -105,7 +106,25 @@ __global__ void paged_attention_generic_kernel(
 #pragma unroll
     for (int i = 0; i < PIECES; ++i) acc[i] *= correction;
     const int keys_here = min(32, last - base + 1);
-    for (int j = 0; j < keys_here; ++j) {
+    // Several keys' values are asked for before the first is used: with one warp a query and head the loop is otherwise bound
+    // by the latency of a load per key (a decoded token at 136 keys 63 us).  The sum still goes key by key.
+    constexpr int RUN = PIECES <= 4 ? 8 : 1;
+    int j = 0;
+    for (; j + RUN <= keys_here; j += RUN) {
+      float values[RUN][PIECES], w[RUN];
+#pragma unroll
+      for (int r = 0; r < RUN; ++r) {
+        w[r] = __shfl_sync(0xffffffffu, weight, j + r);
+        const T* v_row = v_pages + __shfl_sync(0xffffffffu, key_offset, j + r) * value_row_width;
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) values[r][i] = lane + 32 * i < value_dim ? to_float(v_row[lane + 32 * i]) : 0.0f;
+      }
+#pragma unroll
+      for (int r = 0; r < RUN; ++r)
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) acc[i] = fmaf(w[r], values[r][i], acc[i]);
+    }
+    for (; j < keys_here; ++j) {
       const float w = __shfl_sync(0xffffffffu, weight, j);
       const size_t offset = __shfl_sync(0xffffffffu, key_offset, j);
       const T* v_row = v_pages + offset * value_row_width;

@@ -152,6 +152,140 @@ __global__ void delta_rule_prepare_kernel(const T* __restrict__ x, long long ldx
         expf(-expf(a_log[j / per_head]) * softplus(to_float(decay_raw[(size_t)token * ld_decay + j]) + dt_bias[j]));
 }
 
+// The same for up to four taps and key heads of up to 128 channels in multiples of four (value channels likewise): a warp takes
+// 128 neighbouring channels (a key head, or value channels, or decays, four channels a lane) and a run of RUN tokens.  The
+// taps' weights and the decays' constants are read once for the run, an input once for all taps, and all inputs of the run
+// are on their way before the first is used.  Bound by latency: 2,274 tokens of 4,096 channels 38 us (one token a CTA with every
+// tap read anew: 58), 2 tokens of 6,144 channels and 2,048 decays 4.8 us (8.8).
+__device__ __forceinline__ float4 quad_of(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 quad_of(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename T> struct Quad;
+template <> struct Quad<float> { using Raw = uint4; };
+template <> struct Quad<__nv_bfloat16> { using Raw = uint2; };
+
+constexpr int kRunWarps = 4, kRunTaps = 4;
+template <typename T, typename TD, int RUN>
+__global__ void __launch_bounds__(kRunWarps * 32)
+delta_rule_prepare_run_kernel(const T* __restrict__ x, long long ldx, const T* __restrict__ w, float* __restrict__ tail,
+                              const T* __restrict__ beta_raw, long long ld_beta, const TD* __restrict__ decay_raw,
+                              long long ld_decay, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
+                              const int* __restrict__ row_of_token, const int* __restrict__ query_starts,
+                              const int* __restrict__ state_slots, const int* __restrict__ positions,
+                              float* __restrict__ qkv, float* __restrict__ beta, float* __restrict__ decay, int tokens,
+                              int heads, int kv_heads, int key_dim, int value_dim, int decay_width, int taps) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int lane = threadIdx.x;
+  const int first = blockIdx.x * RUN, last = min(first + RUN, tokens);
+  const int keys = 2 * kv_heads, values = heads * value_dim;
+  const int value_units = (values + 127) / 128, decay_units = (decay_width + 127) / 128;
+  const int channels = keys * key_dim + values;
+  int unit = blockIdx.y * kRunWarps + threadIdx.y;
+  if (unit >= keys + value_units) {
+    unit -= keys + value_units;
+    if (unit < decay_units) {                                    // decays
+      const int per_head = decay_width / heads;
+      float rate[4], bias[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int j = unit * 128 + lane + 32 * e;
+        rate[e] = j < decay_width ? -expf(a_log[j / per_head]) : 0.0f;
+        bias[e] = j < decay_width ? dt_bias[j] : 0.0f;
+      }
+#pragma unroll 2
+      for (int t = first; t < last; ++t) {
+        if (positions[t] < 0) continue;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int j = unit * 128 + lane + 32 * e;
+          if (j < decay_width)
+            decay[(size_t)t * decay_width + j] = expf(rate[e] * softplus(to_float(decay_raw[(size_t)t * ld_decay + j]) + bias[e]));
+        }
+      }
+    } else if (unit == decay_units) {                            // the writes' factors
+      for (int t = first; t < last; ++t) {
+        if (positions[t] < 0) continue;
+        for (int h = lane; h < heads; h += 32) beta[(size_t)t * heads + h] = sigmoid(to_float(beta_raw[(size_t)t * ld_beta + h]));
+      }
+    }
+    return;
+  }
+  const bool key_head = unit < keys;
+  const int base = key_head ? unit * key_dim : keys * key_dim + (unit - keys) * 128;
+  const int count = key_head ? key_dim : min(128, values - (unit - keys) * 128);
+  const bool active = lane * 4 < count;
+  const int c = base + (active ? lane * 4 : 0);
+  // the run's inputs, and which request each token belongs to
+  using Raw = typename Quad<T>::Raw;
+  Raw inputs[RUN];
+#pragma unroll
+  for (int i = 0; i < RUN; ++i)
+    if (first + i < last) inputs[i] = *reinterpret_cast<const Raw*>(x + (size_t)(first + i) * ldx + c);
+  const int mine = min(first + lane, last - 1);
+  const int my_row = row_of_token[mine];
+  const int my_start = query_starts[my_row], my_end = query_starts[my_row + 1], my_position = positions[mine];
+  float taps_of[4][kRunTaps];                                    // [channel][tap], right-aligned: the last is the token's own
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < kRunTaps; ++j) {
+      const int tap = j - (kRunTaps - taps);
+      taps_of[i][j] = tap >= 0 ? to_float(w[(size_t)(c + i) * taps + tap]) : 0.0f;
+    }
+  const float q_scale = rsqrtf((float)key_dim);
+  float4 before[kRunTaps - 1] = {};                              // the inputs before the token, right-aligned
+  int row = -1;
+#pragma unroll
+  for (int i = 0; i < RUN; ++i) {
+    const int t = first + i;
+    if (t >= last) break;
+    const int here = __shfl_sync(0xffffffffu, my_row, i), start = __shfl_sync(0xffffffffu, my_start, i);
+    const int end = __shfl_sync(0xffffffffu, my_end, i), position = __shfl_sync(0xffffffffu, my_position, i);
+    if (position < 0) { row = -1; continue; }                    // padding
+    if (here != row) {                                           // the run's first token of a request
+      row = here;
+      const float* old = tail + (size_t)state_slots[row] * (taps - 1) * channels;
+#pragma unroll
+      for (int j = 0; j < kRunTaps - 1; ++j) {
+        const int tap = j - (kRunTaps - taps);                   // of the tail's taps - 1 inputs
+        if (tap < 0) continue;
+        const int src = t - start - (taps - 1) + tap;
+        before[j] = src >= 0 ? quad_of(x + (size_t)(start + src) * ldx + c) : quad_of(old + (size_t)(taps - 1 + src) * channels + c);
+      }
+    }
+    const float4 now = quad_of(reinterpret_cast<const T*>(&inputs[i]));
+    float4 y = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int j = 0; j < kRunTaps; ++j) {
+      if (j < kRunTaps - taps) continue;
+      const float4 in = j < kRunTaps - 1 ? before[j < kRunTaps - 1 ? j : 0] : now;
+      y.x = fmaf(taps_of[0][j], in.x, y.x); y.y = fmaf(taps_of[1][j], in.y, y.y);
+      y.z = fmaf(taps_of[2][j], in.z, y.z); y.w = fmaf(taps_of[3][j], in.w, y.w);
+    }
+    if (end - start == 1 && active) {                            // a request that brings one token: its tail moves on
+      float* old = tail + (size_t)state_slots[row] * (taps - 1) * channels;
+#pragma unroll
+      for (int j = 0; j < kRunTaps - 1; ++j) {
+        const int tap = j - (kRunTaps - taps);
+        if (tap >= 0) *reinterpret_cast<float4*>(old + (size_t)tap * channels + c) = j + 1 < kRunTaps - 1 ? before[j + 1 < kRunTaps - 1 ? j + 1 : 0] : now;
+      }
+    }
+    before[0] = before[1]; before[1] = before[2]; before[2] = now;
+    y = make_float4(silu(y.x), silu(y.y), silu(y.z), silu(y.w));
+    if (key_head) {                                              // a unit vector, the query's scaled
+      const float square = active ? fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w))) : 0.0f;
+      const float factor = rsqrtf(warp_sum(square) + 1e-6f) * (unit < kv_heads ? q_scale : 1.0f);
+      y.x *= factor; y.y *= factor; y.z *= factor; y.w *= factor;
+    }
+    if (active) *reinterpret_cast<float4*>(qkv + (size_t)t * channels + c) = y;
+  }
+}
+
 constexpr int kScanWarps = 4;           // that walk
 constexpr int kFetchWarps = 4;          // that copy what the others will need
 constexpr int kScanThreads = (kScanWarps + kFetchWarps) * 32;
@@ -574,6 +708,18 @@ MIR_EXPORT int mir_delta_rule_prepare(int bf16, int decay_f32, const void* x, lo
   const size_t element = bf16 ? 2 : 4;
   const bool paired = key_dim % 2 == 0 && (heads * value_dim) % 2 == 0 && ldx % 2 == 0 &&
                       (uintptr_t)x % (2 * element) == 0 && (uintptr_t)qkv % 8 == 0 && (uintptr_t)tail % 8 == 0;
+  const int values = heads * value_dim;
+  const bool runs = taps <= kRunTaps && key_dim <= 128 && key_dim % 4 == 0 && values % 4 == 0 && ldx % 4 == 0 &&
+                    (uintptr_t)x % (4 * element) == 0 && ((uintptr_t)qkv | (uintptr_t)tail) % 16 == 0;
+  const int units = 2 * kv_heads + (values + 127) / 128 + (decay_width + 127) / 128 + 1;
+  // eight tokens a warp once that still makes several warps for every SM's schedulers
+  const bool long_runs = (long long)tokens * units >= 8LL * 16 * mir_sm_count();
+#define MIR_PREPARE_RUN(T, TD, RUN)                                                                                    \
+  status = mir_launch("delta_rule_prepare", delta_rule_prepare_run_kernel<T, TD, RUN>,                                 \
+                      dim3((tokens + RUN - 1) / RUN, (units + kRunWarps - 1) / kRunWarps), dim3(32, kRunWarps), 0,     \
+                      stream, 0, (const T*)x, ldx, (const T*)w, tail, (const T*)beta_raw, ld_beta,                     \
+                      (const TD*)decay_raw, ld_decay, dt_bias, a_log, row_of_token, query_starts, state_slots,         \
+                      positions, qkv, beta, decay, tokens, heads, kv_heads, key_dim, value_dim, decay_width, taps)
 #define MIR_PREPARE_AS(T, TD, P)                                                                                       \
   status = mir_launch("delta_rule_prepare", delta_rule_prepare_kernel<T, TD, P>, dim3(tokens, parts), dim3(256), 0,    \
                       stream, 0, (const T*)x, ldx, (const T*)w, tail, (const T*)beta_raw, ld_beta,       \
@@ -581,7 +727,9 @@ MIR_EXPORT int mir_delta_rule_prepare(int bf16, int decay_f32, const void* x, lo
                       positions, qkv, beta, decay, heads, kv_heads, key_dim, value_dim, decay_width, taps)
 #define MIR_PREPARE(T, TD)                                                                                             \
   do {                                                                                                                 \
-    if (paired) MIR_PREPARE_AS(T, TD, true);                                                                           \
+    if (runs && long_runs) MIR_PREPARE_RUN(T, TD, 8);                                                                  \
+    else if (runs) MIR_PREPARE_RUN(T, TD, 1);                                                                          \
+    else if (paired) MIR_PREPARE_AS(T, TD, true);                                                                      \
     else MIR_PREPARE_AS(T, TD, false);                                                                                 \
   } while (0)
   if (bf16 && decay_f32) MIR_PREPARE(__nv_bfloat16, float);
@@ -589,6 +737,7 @@ MIR_EXPORT int mir_delta_rule_prepare(int bf16, int decay_f32, const void* x, lo
   else MIR_PREPARE(float, float);
 #undef MIR_PREPARE
 #undef MIR_PREPARE_AS
+#undef MIR_PREPARE_RUN
   // rows of one token have moved their tails on themselves; a step of single tokens needs nothing more
   if (status != MIR_OK || taps == 1 || tokens == rows) return status;
   const int threads = channels >= 256 ? 256 : ((channels + 31) / 32) * 32;

@@ -10,7 +10,8 @@
 // floats so that eight neighbouring rows read as 16-byte pieces meet all banks once:
 //   gemm_f32_rows   up to 16 rows of A: bound by reading W once.  A CTA takes 16 rows of W and all of A; a thread owns one
 //                   output and walks down k, so the least a product can take is K dependent multiply-adds (four cycles
-//                   each, 4.2 us for 2,048), which the ring of four stages of 256 k hides behind the reads.
+//                   each, 4.2 us for 2,048), which several CTAs on an SM, each with a ring of four
+//                   stages of 128 k, hide behind the reads.
 //   gemm_f32_tile   more rows: bound by the multiply-adds.  A thread owns TM x TN outputs whose rows and columns lie
 //                   (tile / threads) apart, and reads four k of each with one load.
 #include "common.cuh"
@@ -57,7 +58,7 @@ __device__ __forceinline__ void finish(float* c, int ldc, const float* bias, flo
 }
 
 template <int BM, int BN, int TM, int TN, int DEPTH, int STAGES, bool WIDE>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN > 32 ? 1 : 3)
 gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, const float* __restrict__ bias,
                      float* __restrict__ c, int ldc, int m, int n, int k, float beta) {
   constexpr int ACROSS = BN / TN, DOWN = BM / TM, THREADS = ACROSS * DOWN, ROW = DEPTH + 4;
@@ -87,21 +88,26 @@ gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restri
     copy_commit();
     const float* at = shared + (step % STAGES) * (BM + BN) * ROW + ty * ROW;
     const float* wt = shared + (step % STAGES) * (BM + BN) * ROW + (BM + tx) * ROW;
+    float4 av[2][TM], wv[2][TN];                   // the next four k are read while these four are multiplied
+    auto read = [&](int buffer, int kk) {
+#pragma unroll
+      for (int i = 0; i < TM; ++i) av[buffer][i] = *reinterpret_cast<const float4*>(at + i * DOWN * ROW + kk);
+#pragma unroll
+      for (int j = 0; j < TN; ++j) wv[buffer][j] = *reinterpret_cast<const float4*>(wt + j * ACROSS * ROW + kk);
+    };
+    read(0, 0);
 #pragma unroll
     for (int kk = 0; kk < DEPTH; kk += 4) {
-      float4 av[TM], wv[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) av[i] = *reinterpret_cast<const float4*>(at + i * DOWN * ROW + kk);
-#pragma unroll
-      for (int j = 0; j < TN; ++j) wv[j] = *reinterpret_cast<const float4*>(wt + j * ACROSS * ROW + kk);
+      const int buffer = kk / 4 & 1;
+      if (kk + 4 < DEPTH) read(buffer ^ 1, kk + 4);
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
-          acc[i][j] = fmaf(av[i].x, wv[j].x, acc[i][j]);
-          acc[i][j] = fmaf(av[i].y, wv[j].y, acc[i][j]);
-          acc[i][j] = fmaf(av[i].z, wv[j].z, acc[i][j]);
-          acc[i][j] = fmaf(av[i].w, wv[j].w, acc[i][j]);
+          acc[i][j] = fmaf(av[buffer][i].x, wv[buffer][j].x, acc[i][j]);
+          acc[i][j] = fmaf(av[buffer][i].y, wv[buffer][j].y, acc[i][j]);
+          acc[i][j] = fmaf(av[buffer][i].z, wv[buffer][j].z, acc[i][j]);
+          acc[i][j] = fmaf(av[buffer][i].w, wv[buffer][j].w, acc[i][j]);
         }
     }
   }
@@ -117,11 +123,11 @@ gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restri
   }
 }
 
-constexpr int kRowsColumns = 16, kRowsDepth = 256, kRowsStages = 4, kRowsThreads = 128;
+constexpr int kRowsColumns = 16, kRowsDepth = 128, kRowsStages = 4, kRowsThreads = 128, kRun = 4;
 
 // MT: rows of A rounded up to a power of two (1 to 16).  With MT = 16 a thread owns two outputs.
 template <int MT, bool WIDE>
-__global__ void __launch_bounds__(kRowsThreads)
+__global__ void __launch_bounds__(kRowsThreads, 4)
 gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, const float* __restrict__ bias,
                      float* __restrict__ c, int ldc, int m, int n, int k, float beta) {
   constexpr int ROW = kRowsDepth + 4, STAGE = (kRowsColumns + MT) * ROW;
@@ -153,17 +159,34 @@ gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restri
     if (!owner) continue;
     const float* wt = shared + (step % kRowsStages) * STAGE + tx * ROW;
     const float* at = shared + (step % kRowsStages) * STAGE + (kRowsColumns + ty) * ROW;
-#pragma unroll 16
-    for (int kk = 0; kk < kRowsDepth; kk += 4) {
-      const float4 wv = *reinterpret_cast<const float4*>(wt + kk);
+    // Runs of kRun pieces of four k, the next run's reads on their way while this one's chain of multiply-adds goes on.
+    float4 wv[2][kRun], av[2][EACH][kRun];
+    auto read = [&](int buffer, int kk) {
 #pragma unroll
-      for (int e = 0; e < EACH; ++e) {
-        const float4 av = *reinterpret_cast<const float4*>(at + e * DOWN * ROW + kk);
-        acc[e] = fmaf(av.x, wv.x, acc[e]);
-        acc[e] = fmaf(av.y, wv.y, acc[e]);
-        acc[e] = fmaf(av.z, wv.z, acc[e]);
-        acc[e] = fmaf(av.w, wv.w, acc[e]);
+      for (int i = 0; i < kRun; ++i) {
+        wv[buffer][i] = *reinterpret_cast<const float4*>(wt + kk + 4 * i);
+#pragma unroll
+        for (int e = 0; e < EACH; ++e) av[buffer][e][i] = *reinterpret_cast<const float4*>(at + e * DOWN * ROW + kk + 4 * i);
       }
+    };
+    auto multiply = [&](int buffer) {
+#pragma unroll
+      for (int i = 0; i < kRun; ++i)
+#pragma unroll
+        for (int e = 0; e < EACH; ++e) {
+          acc[e] = fmaf(av[buffer][e][i].x, wv[buffer][i].x, acc[e]);
+          acc[e] = fmaf(av[buffer][e][i].y, wv[buffer][i].y, acc[e]);
+          acc[e] = fmaf(av[buffer][e][i].z, wv[buffer][i].z, acc[e]);
+          acc[e] = fmaf(av[buffer][e][i].w, wv[buffer][i].w, acc[e]);
+        }
+    };
+    read(0, 0);
+#pragma unroll 1
+    for (int kk = 0; kk < kRowsDepth; kk += 8 * kRun) {
+      read(1, kk + 4 * kRun);
+      multiply(0);
+      if (kk + 8 * kRun < kRowsDepth) read(0, kk + 8 * kRun);
+      multiply(1);
     }
   }
   if (!owner || col0 + tx >= n) return;
@@ -218,11 +241,17 @@ int choose(const Product& p) {
   if (p.m <= 8) return launch_rows<8, WIDE>(p);
   if (p.m <= 16) return launch_rows<16, WIDE>(p);
   if (p.m <= 32) return launch_tile<32, 64, 4, 4, WIDE>(p);
-  // A thread of the large tile reads half as much from shared memory for each multiply-add; it is taken once two CTAs of
-  // it for every SM exist (two are resident).
-  const long long large = (long long)((p.m + 127) / 128) * ((p.n + 127) / 128);
-  if (large >= 2LL * mir_sm_count()) return launch_tile<128, 128, 8, 8, WIDE>(p);
-  return launch_tile<64, 64, 8, 4, WIDE>(p);
+  // The tile whose busiest SM has the least to do: multiply-adds of its tiles, a thread of a smaller tile reading more of
+  // shared memory for each (by the weights below).
+  const int sms = mir_sm_count();
+  auto cost = [&](int rows, int columns, int weight) {
+    const long long tiles = (long long)((p.m + rows - 1) / rows) * ((p.n + columns - 1) / columns);
+    return (tiles + sms - 1) / sms * rows * columns * weight;
+  };
+  const long long small = cost(32, 64, 6), middle = cost(64, 64, 5), large = cost(128, 128, 4);
+  if (large <= middle && large <= small) return launch_tile<128, 128, 8, 8, WIDE>(p);
+  if (middle <= small) return launch_tile<64, 64, 8, 4, WIDE>(p);
+  return launch_tile<32, 64, 4, 4, WIDE>(p);
 }
 
 }  // namespace

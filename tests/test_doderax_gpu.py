@@ -182,6 +182,45 @@ def test_delta_rule_against_the_plain_recurrence(per_channel, heads, kv_heads, k
         assert torch.all(state[2] == 7.0) and torch.all(state[0] == 0.0) and torch.all(tail[0] == 0.0)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("taps,key_dim,value_dim,per_channel", [(4, 128, 64, True), (2, 100, 24, False), (1, 64, 128, True), (3, 4, 200, False)])
+def test_what_the_recurrence_needs_is_the_same_in_long_steps_and_short_ones(dtype, taps, key_dim, value_dim, per_channel):
+    """Runs of eight tokens a warp (long steps) against one token a warp: the same bits, and the same inputs kept."""
+    from libmir_b200 import kernels
+    torch.manual_seed(taps)
+    heads, kv_heads = 4, 2
+    portions = [1, 2003, 3, 1, 1300, 9]
+    tokens, rows = sum(portions), len(portions)
+    channels, width = 2 * kv_heads * key_dim + heads * value_dim, heads * key_dim if per_channel else heads
+    cuda = lambda t, kind=None: t.to(device="cuda", dtype=kind or t.dtype).contiguous()
+    x = cuda(torch.randn(tokens, channels + 8), dtype)
+    weight, beta_raw = cuda(torch.randn(channels, taps), dtype), cuda(torch.randn(tokens, heads), dtype)
+    decay_raw, bias, a_log = cuda(torch.randn(tokens, width)), cuda(torch.randn(width)), cuda(torch.randn(heads))
+    tail0 = torch.randn(rows, taps - 1, channels)
+    slots = cuda(torch.randperm(rows).int())
+
+    def prepare(first, counts, rows_here, tail):
+        total = sum(counts)
+        starts = cuda(torch.tensor([0] + list(np.cumsum(counts)), dtype=torch.int32))
+        row_of = cuda(torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts)).int())
+        made = [torch.full((total, w), float("nan"), device="cuda") for w in (channels, heads, width)]
+        kernels.delta_rule_prepare(x[first:first + total, :channels], weight, tail, beta_raw[first:first + total],
+                                   decay_raw[first:first + total], bias, a_log, row_of, starts, slots[rows_here].contiguous(),
+                                   torch.zeros(total, dtype=torch.int32, device="cuda"), *made, heads, kv_heads, key_dim, value_dim)
+        return made
+    tail = cuda(tail0.clone())
+    whole = prepare(0, portions, slice(0, rows), tail)
+    pieces_tail, pieces, first = cuda(tail0.clone()), [], 0
+    for r, count in enumerate(portions):
+        for begin in range(0, count, 50):
+            n = min(50, count - begin)
+            pieces.append(prepare(first + begin, [n], slice(r, r + 1), pieces_tail))
+        first += count
+    for got, parts in zip(whole, zip(*pieces)):
+        assert torch.equal(got, torch.cat(parts)) and bool(torch.isfinite(got).all())
+    assert torch.equal(tail, pieces_tail)
+
+
 @pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-6), (torch.bfloat16, 8e-3)])
 @pytest.mark.parametrize("sigmoid_gate", [False, True])
 def test_gated_head_norm(dtype, tol, sigmoid_gate):
