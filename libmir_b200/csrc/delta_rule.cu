@@ -493,6 +493,309 @@ delta_rule_scan_kernel(const float* __restrict__ qkv, const float* __restrict__ 
     if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, wide);
 }
 
+// The recurrence four tokens at a time, for prompts whose results may be grouped by where the step begins (the bfloat16 engine;
+// the 32-bit engine's results must not depend on the cut and run the kernel above).  With S the state before a group,
+// G_t the product of the decays up to token t of it, G_ts the product of those behind token s up to t:
+//     P_t = S^T (G_t k_t),  R_t = S^T (G_t q_t)                            eight dot products that need only S
+//     u_t = beta_t (v_t - P_t - sum_{s<t} (k_t . G_ts k_s) u_s)            four short sums
+//     o_t = R_t + sum_{s<=t} (q_t . G_ts k_s) u_s;   S <- G_4 S + sum_t (G_4t k_t) u_t^T
+// Every factor is a product of decays, at most one: nothing is divided, nothing can overflow.  The vectors and the scalars
+// do not depend on the column: delta_rule_group forms them once for a head, one warp a (group, head).
+//   grouped [group, head, 13 PADDED + 28]: G_t k_t (4), G_t q_t (4), G_4t k_t (4), G_4 | the k products [1][0], [2][0..1],
+//   [3][0..2] and two zeros | beta (4) | the q products [4][4], zero above the diagonal.  A request's groups begin at
+//   start / 4 + its number; tokens a last group lacks have no key, no query, no decay (1) and no write.
+constexpr int kGroup = 4, kGroupScalars = 28;
+__host__ __device__ constexpr int group_floats(int padded) { return 13 * padded + kGroupScalars; }
+
+template <int PADDED, bool PER_CHANNEL>
+__global__ void __launch_bounds__(128)
+delta_rule_group_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
+                        const int* __restrict__ query_starts, const int* __restrict__ positions, float* __restrict__ grouped,
+                        int rows, int heads, int kv_heads, int key_dim, int value_dim) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int lane = threadIdx.x, group = blockIdx.x, head = blockIdx.y * 4 + threadIdx.y;
+  if (head >= heads) return;
+  int start = -1, end = 0, begin = 0;
+  for (int base = 0; base < rows && start < 0; base += 32) {     // whose group it is
+    const int r = base + lane;
+    const int a = r < rows ? query_starts[r] : 0, b = r < rows ? query_starts[r + 1] : 0, first = a / kGroup + r;
+    const unsigned found = __ballot_sync(0xffffffffu, r < rows && group >= first && group < first + (b - a + kGroup - 1) / kGroup);
+    if (found == 0) continue;
+    const int source = __ffs(found) - 1;
+    start = __shfl_sync(0xffffffffu, a, source);
+    end = __shfl_sync(0xffffffffu, b, source);
+    begin = start + (group - __shfl_sync(0xffffffffu, first, source)) * kGroup;
+  }
+  if (start < 0 || positions[start] < 0) return;
+  const int kv_head = head / (heads / kv_heads);
+  const int width = 2 * kv_heads * key_dim + heads * value_dim;
+  const int g_width = PER_CHANNEL ? heads * key_dim : heads;
+  const bool wide = key_dim % 4 == 0 && width % 4 == 0;
+  auto read = [&](const float* from, int i) {                    // channels i .. i + 3 of a head, zeros beyond it
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (wide) {
+      if (i < key_dim) v = *reinterpret_cast<const float4*>(from + i);
+    } else {
+      if (i < key_dim) v.x = from[i];
+      if (i + 1 < key_dim) v.y = from[i + 1];
+      if (i + 2 < key_dim) v.z = from[i + 2];
+      if (i + 3 < key_dim) v.w = from[i + 3];
+    }
+    return v;
+  };
+  auto times = [](float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); };
+  auto dot = [](float4 a, float4 b, float sum) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, sum)))); };
+  float* to = grouped + ((size_t)group * heads + head) * group_floats(PADDED);
+  float sums[16];                                                // k products (6), q products (10)
+#pragma unroll
+  for (int i = 0; i < 16; ++i) sums[i] = 0.0f;
+#pragma unroll
+  for (int piece = 0; piece < (PADDED + 127) / 128; ++piece) {
+    const int i = piece * 128 + lane * 4;
+    if (i >= PADDED) continue;                                   // (no shuffles inside)
+    float4 k[kGroup], q[kGroup], g[kGroup];
+#pragma unroll
+    for (int t = 0; t < kGroup; ++t) {
+      k[t] = q[t] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      g[t] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+      if (begin + t >= end) continue;
+      const float* row = qkv + (size_t)(begin + t) * width + (size_t)kv_head * key_dim;
+      q[t] = read(row, i);
+      k[t] = read(row + (size_t)kv_heads * key_dim, i);
+      const float* d = decay + (size_t)(begin + t) * g_width + (size_t)head * (PER_CHANNEL ? key_dim : 1);
+      if (PER_CHANNEL) {
+        if (g_width % 4 == 0 && key_dim % 4 == 0) g[t] = i < key_dim ? *reinterpret_cast<const float4*>(d + i) : g[t];
+        else g[t] = read(d, i);
+      } else {
+        g[t] = make_float4(d[0], d[0], d[0], d[0]);
+      }
+    }
+    float4 so_far = g[0];
+#pragma unroll
+    for (int t = 0; t < kGroup; ++t) {
+      if (t > 0) so_far = times(so_far, g[t]);
+      *reinterpret_cast<float4*>(to + t * PADDED + i) = times(k[t], so_far);
+      *reinterpret_cast<float4*>(to + (kGroup + t) * PADDED + i) = times(q[t], so_far);
+    }
+    *reinterpret_cast<float4*>(to + 3 * kGroup * PADDED + i) = so_far;
+#pragma unroll
+    for (int s = 0; s < kGroup; ++s) {
+      float4 reach = k[s];                                       // key s as token t sees it
+      sums[6 + s * (s + 1) / 2 + s] = dot(q[s], reach, sums[6 + s * (s + 1) / 2 + s]);
+#pragma unroll
+      for (int t = s + 1; t < kGroup; ++t) {
+        reach = times(reach, g[t]);
+        sums[t * (t - 1) / 2 + s] = dot(k[t], reach, sums[t * (t - 1) / 2 + s]);
+        sums[6 + t * (t + 1) / 2 + s] = dot(q[t], reach, sums[6 + t * (t + 1) / 2 + s]);
+      }
+      *reinterpret_cast<float4*>(to + (2 * kGroup + s) * PADDED + i) = reach;
+    }
+  }
+  const float total = sum_lanes<32, 16>(sums, lane);
+  float* scalars = to + 13 * PADDED;
+  if (lane < 16) {
+    const int number = lane_sum<16>(lane);
+    if (number < 6) {
+      scalars[number] = total;
+    } else {
+      int t = 0;
+      while ((t + 1) * (t + 2) / 2 <= number - 6) ++t;
+      scalars[12 + t * 4 + (number - 6 - t * (t + 1) / 2)] = total;
+    }
+  } else if (lane < 24) {                                        // what is never reached
+    const int above[8] = {6, 7, 13, 14, 15, 18, 19, 23};
+    scalars[above[lane - 16]] = 0.0f;
+  } else if (lane < 28) {
+    const int t = begin + lane - 24;
+    scalars[8 + lane - 24] = t < end ? beta[(size_t)t * heads + head] : 0.0f;
+  }
+}
+
+// The walk over groups: lanes, columns, roles and stages as in delta_rule_scan_kernel, LANES = 16.  A group costs its chain one
+// sum over the lanes (4 C sums together, each in a lane of its own), one exchange and the four short sums, where four
+// tokens one after the other cost four of each.
+// What bounds it: shared memory.  A lane reads PER numbers of thirteen vectors a group whatever the columns it has, and a
+// warp's 16-byte read takes four cycles though its halves read the same: so C columns a lane cost 52 / C cycles a column.
+// 2,048 tokens with the group kernel, decay per channel / head: 16 heads 268 / 266 us (a token at a time 377 / 345), 32 heads
+// 392 / 388 (521 / 466); 1,400 and 874 tokens, 16 heads 267 / 264 (360 / 321), 32 heads 448 / 442 (598 / 537).
+template <int PER, int C>
+__global__ void __launch_bounds__(kScanThreads, 2)
+delta_rule_grouped_scan_kernel(const float* __restrict__ grouped, const float* __restrict__ qkv, float* __restrict__ state,
+                               const int* __restrict__ query_starts, const int* __restrict__ state_slots,
+                               const int* __restrict__ positions, float* __restrict__ out, int heads, int kv_heads,
+                               int key_dim, int value_dim) {
+  constexpr int LANES = 16, PADDED = LANES * PER, SUMS = kGroup * C;
+  constexpr int COLUMNS = 32 / LANES * C, BLOCK_COLUMNS = COLUMNS * kScanWarps;
+  constexpr int GROUPED = group_floats(PADDED), ROW = GROUPED + kGroup * BLOCK_COLUMNS, CHUNK = kFetchWarps;   // groups of a stage
+  constexpr int STAGE = CHUNK * ROW;
+  constexpr int STAGES = 3;
+  extern __shared__ __align__(16) float staged[];                // [STAGES][CHUNK groups][row]
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int lane = threadIdx.x;
+  const int row = blockIdx.x, head = blockIdx.y;
+  const int first_column = blockIdx.z * BLOCK_COLUMNS;
+  const int start = query_starts[row], end = query_starts[row + 1];
+  if (end <= start || positions[start] < 0) return;             // the whole CTA: an empty or padding row
+  const int width = 2 * kv_heads * key_dim + heads * value_dim;
+  const int groups = (end - start + kGroup - 1) / kGroup, first_group = start / kGroup + row;
+  const int chunks = (groups + CHUNK - 1) / CHUNK;
+
+  if (threadIdx.y >= kScanWarps) {                              // the fetching warps: a group of the stage each
+    const int mine = threadIdx.y - kScanWarps;
+    const float* v0 = qkv + (size_t)2 * kv_heads * key_dim + (size_t)head * value_dim + first_column;
+    const bool wide = width % 4 == 0 && key_dim % 4 == 0 && value_dim % 4 == 0;
+    auto fetch = [&](int chunk) {
+      const int group = chunk * CHUNK + mine;
+      if (group < groups) {
+        float* to = staged + (chunk % STAGES) * STAGE + mine * ROW;
+        const float* from = grouped + ((size_t)(first_group + group) * heads + head) * GROUPED;
+#pragma unroll
+        for (int i = 0; i < GROUPED; i += 128)
+          if (GROUPED - i >= 128 || i + lane * 4 < GROUPED) copy_async(to + i + lane * 4, from + i + lane * 4, true);
+        float* values = to + GROUPED;
+        const int token = start + group * kGroup;
+        if (wide) {
+          constexpr int PIECES = BLOCK_COLUMNS / 4;              // 4 or 8: the lanes take all of them once
+          static_assert(kGroup * PIECES <= 32, "a lane copies at most one piece of the values");
+          const int t = lane / PIECES, c = lane % PIECES * 4;
+          if (t < kGroup) {
+            if (token + t < end && first_column + c < value_dim)
+              copy_async(values + t * BLOCK_COLUMNS + c, v0 + (size_t)(token + t) * width + c, true);
+            else
+              *reinterpret_cast<float4*>(values + t * BLOCK_COLUMNS + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          }
+        } else {
+          for (int index = lane; index < kGroup * BLOCK_COLUMNS; index += 32) {
+            const int t = index / BLOCK_COLUMNS, c = index % BLOCK_COLUMNS;
+            if (token + t < end && first_column + c < value_dim) copy_async(values + index, v0 + (size_t)(token + t) * width + c, false);
+            else values[index] = 0.0f;
+          }
+        }
+      }
+      copy_commit();
+    };
+    fetch(0);
+    if (chunks > 1) fetch(1); else copy_commit();
+    copy_wait<1>();
+    __syncthreads();                                             // the first stage is there
+    for (int chunk = 0; chunk < chunks; ++chunk) {               // (into the stage that was walked last)
+      if (chunk + 2 < chunks) fetch(chunk + 2); else copy_commit();
+      copy_wait<1>();
+      __syncthreads();                                           // this stage has been walked, and the next one is there
+    }
+    copy_wait<0>();
+    return;
+  }
+
+  const int l = lane % LANES, base_lane = lane & 16;
+  const int local_column = threadIdx.y * COLUMNS + lane / LANES * C;
+  const int column = first_column + local_column;                // idle lanes (beyond value_dim) still take part in the shuffles
+  const bool wide = key_dim % 4 == 0;
+  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + column) * key_dim;
+  Pair s[C][PER / 2];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    load_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, column + c < value_dim, wide);
+  auto pairs_at = [&](const float* vector, Pair (&to)[PER / 2]) {
+#pragma unroll
+    for (int m = 0; m < PER; m += 4) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(vector + (m / 4 * LANES + l) * 4);
+      to[m / 2] = a.x;
+      to[m / 2 + 1] = a.y;
+    }
+  };
+  // sums of S^T (G_t k_t), and likewise of S^T (G_t q_t): token t = number / C, column number % C
+  const int number = lane_sum<SUMS>(l);
+  const int my_token = number / C, my_column = number % C;
+  const bool writes = l < SUMS && column + my_column < value_dim;
+  const size_t out_step = (size_t)heads * value_dim;
+  float* out_of = out + ((size_t)start * heads + head) * value_dim + column + my_column;
+  __syncthreads();                                               // the first stage is there
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int count = min(CHUNK, groups - chunk * CHUNK);
+    const float* in = staged + (chunk % STAGES) * STAGE;
+#pragma unroll 1
+    for (int g = 0; g < count; ++g, in += ROW) {
+      const float* scalars = in + 13 * PADDED;
+      float seen_parts[SUMS], read_parts[SUMS];
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t) {
+        Pair key[PER / 2], query[PER / 2];
+        pairs_at(in + t * PADDED, key);
+        pairs_at(in + (kGroup + t) * PADDED, query);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          Pair seen[2] = {0, 0}, read[2] = {0, 0};
+#pragma unroll
+          for (int m = 0; m < PER / 2; ++m) {
+            seen[m & 1] = pair_fma(s[c][m], key[m], seen[m & 1]);
+            read[m & 1] = pair_fma(s[c][m], query[m], read[m & 1]);
+          }
+          seen_parts[t * C + c] = pair_total(seen);
+          read_parts[t * C + c] = pair_total(read);
+        }
+      }
+      const float4 k_low = *reinterpret_cast<const float4*>(scalars), k_high = *reinterpret_cast<const float4*>(scalars + 4);
+      const float4 b = *reinterpret_cast<const float4*>(scalars + 8);
+      const float4 reach = *reinterpret_cast<const float4*>(scalars + 12 + (my_token & 3) * 4);
+      float v[kGroup][C];
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t)
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[t][c] = in[GROUPED + t * BLOCK_COLUMNS + local_column + c];
+      const float seen_sum = sum_lanes<LANES, SUMS>(seen_parts, l);
+      const float read_sum = sum_lanes<LANES, SUMS>(read_parts, l);
+      float u[C][kGroup];
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t)
+#pragma unroll
+        for (int c = 0; c < C; ++c) v[t][c] -= __shfl_sync(0xffffffffu, seen_sum, base_lane | lane_with<SUMS>(t * C + c));
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        u[c][0] = b.x * v[0][c];
+        u[c][1] = b.y * fmaf(-k_low.x, u[c][0], v[1][c]);
+        u[c][2] = b.z * fmaf(-k_low.z, u[c][1], fmaf(-k_low.y, u[c][0], v[2][c]));
+        u[c][3] = b.w * fmaf(-k_high.y, u[c][2], fmaf(-k_high.x, u[c][1], fmaf(-k_low.w, u[c][0], v[3][c])));
+      }
+      const int token = (chunk * CHUNK + g) * kGroup + my_token;
+      if (writes && token < end - start) {
+        float mine[kGroup];
+#pragma unroll
+        for (int t = 0; t < kGroup; ++t) {
+          mine[t] = u[0][t];
+#pragma unroll
+          for (int c = 1; c < C; ++c) mine[t] = my_column == c ? u[c][t] : mine[t];
+        }
+        out_of[(size_t)token * out_step] =
+            fmaf(reach.w, mine[3], fmaf(reach.z, mine[2], fmaf(reach.y, mine[1], fmaf(reach.x, mine[0], read_sum))));
+      }
+      Pair decay[PER / 2];
+      pairs_at(in + 3 * kGroup * PADDED, decay);
+#pragma unroll
+      for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int m = 0; m < PER / 2; ++m) s[c][m] = pair_mul(s[c][m], decay[m]);
+#pragma unroll
+      for (int t = 0; t < kGroup; ++t) {
+        Pair key[PER / 2];
+        pairs_at(in + (2 * kGroup + t) * PADDED, key);
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const Pair both = pair_from(u[c][t], u[c][t]);
+#pragma unroll
+          for (int m = 0; m < PER / 2; ++m) s[c][m] = pair_fma(key[m], both, s[c][m]);
+        }
+      }
+    }
+    __syncthreads();                                             // this stage has been walked, and the next one is there
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, wide);
+}
+
 // One warp per (token, head): out = o / sqrt(mean(o^2) + eps) * weight * act(gate); the weight is [value_dim], the
 // same for every head, or (weight_per_head) [heads, value_dim].
 template <typename T, typename TG>
@@ -679,6 +982,54 @@ int launch_scan(cudaStream_t stream, const float* qkv, const float* beta, const 
   return MIR_BAD_ARGUMENT;
 }
 
+template <int PER, int C>
+int launch_grouped_walk(cudaStream_t stream, const float* grouped, const float* qkv, float* state, const int* query_starts,
+                        const int* state_slots, const int* positions, float* out, int rows, int heads, int kv_heads, int key_dim,
+                        int value_dim) {
+  constexpr int columns = kScanWarps * 2 * C;
+  constexpr int smem = 3 * kFetchWarps * (group_floats(16 * PER) + kGroup * columns) * (int)sizeof(float);
+  const cudaError_t err = cudaFuncSetAttribute(delta_rule_grouped_scan_kernel<PER, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (err != cudaSuccess) {
+    mir_set_error("delta_rule_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
+    return MIR_CUDA_ERROR;
+  }
+  return mir_launch("delta_rule_scan", delta_rule_grouped_scan_kernel<PER, C>,
+                    dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps + kFetchWarps), smem, stream, 0,
+                    grouped, qkv, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
+}
+
+template <int PER, bool PER_CHANNEL>
+int launch_grouped_as(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
+                      const int* query_starts, const int* state_slots, const int* positions, float* out, float* grouped,
+                      int tokens, int rows, int heads, int kv_heads, int key_dim, int value_dim) {
+  constexpr int padded = 16 * PER;
+  int status = mir_launch("delta_rule_group", delta_rule_group_kernel<padded, PER_CHANNEL>,
+                          dim3(tokens / kGroup + rows, (heads + 3) / 4), dim3(32, 4), 0, stream, 0, qkv, beta, decay,
+                          query_starts, positions, grouped, rows, heads, kv_heads, key_dim, value_dim);
+  if (status != MIR_OK) return status;
+  // Four columns a lane once their CTAs are enough for most SMs (1,400 and 874 tokens, 16 heads: 267 us, 310 with two), else
+  // two (2,048 tokens, 16 heads: 64 CTAs of four columns would leave most of the chip idle).
+  const long long ctas = (long long)rows * heads * ((value_dim + kScanWarps * 8 - 1) / (kScanWarps * 8));
+  if (ctas * 3 >= 2LL * mir_sm_count())
+    return launch_grouped_walk<PER, 4>(stream, grouped, qkv, state, query_starts, state_slots, positions, out, rows, heads, kv_heads,
+                                       key_dim, value_dim);
+  return launch_grouped_walk<PER, 2>(stream, grouped, qkv, state, query_starts, state_slots, positions, out, rows, heads, kv_heads,
+                                     key_dim, value_dim);
+}
+
+template <bool PER_CHANNEL>
+int launch_grouped(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
+                   const int* query_starts, const int* state_slots, const int* positions, float* out, float* grouped,
+                   int tokens, int rows, int heads, int kv_heads, int key_dim, int value_dim) {
+#define MIR_GROUPED(P)                                                                                                    \
+  return launch_grouped_as<P, PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out,   \
+                                           grouped, tokens, rows, heads, kv_heads, key_dim, value_dim)
+  if (key_dim <= 64) MIR_GROUPED(4);
+  MIR_GROUPED(8);
+#undef MIR_GROUPED
+}
+constexpr int kGroupedKeys = 128;                                // the widest key head that is walked in groups
+
 }  // namespace
 
 // bf16: the type of x, w and beta_raw (and of decay_raw unless decay_f32).  decay_width: heads, or heads * key_dim for
@@ -712,7 +1063,7 @@ MIR_EXPORT int mir_delta_rule_prepare(int bf16, int decay_f32, const void* x, lo
   const bool runs = taps <= kRunTaps && key_dim <= 128 && key_dim % 4 == 0 && values % 4 == 0 && ldx % 4 == 0 &&
                     (uintptr_t)x % (4 * element) == 0 && ((uintptr_t)qkv | (uintptr_t)tail) % 16 == 0;
   const int units = 2 * kv_heads + (values + 127) / 128 + (decay_width + 127) / 128 + 1;
-  // eight tokens a warp once that still makes several warps for every SM's schedulers
+  // eight tokens a warp (sixteen: 59 us where eight take 38) once that still makes several warps for every SM's schedulers
   const bool long_runs = (long long)tokens * units >= 8LL * 16 * mir_sm_count();
 #define MIR_PREPARE_RUN(T, TD, RUN)                                                                                    \
   status = mir_launch("delta_rule_prepare", delta_rule_prepare_run_kernel<T, TD, RUN>,                                 \
@@ -755,16 +1106,26 @@ MIR_EXPORT int mir_delta_rule_set_lanes(int lanes) {
   return MIR_OK;
 }
 
-// qkv, beta, decay as delta_rule_prepare leaves them; per_channel: decay is [tokens, heads * key_dim].
+// qkv, beta, decay as delta_rule_prepare leaves them; per_channel: decay is [tokens, heads * key_dim].  grouped: null, or
+// 32-bit scratch (16-byte aligned) of (tokens / 4 + rows) * heads * (13 padded + 28) numbers, padded = the key width rounded
+// up to 64 or 128: a step that brings more than single tokens then walks four tokens at a time (results then depend, in the
+// last places, on where a request's portions begin); not used for key heads wider than 128.
 MIR_EXPORT int mir_delta_rule_scan(int per_channel, const float* qkv, const float* beta, const float* decay, float* state,
                                    const int* query_starts, const int* state_slots, const int* positions, float* out,
-                                   int tokens, int rows, int heads, int kv_heads, int key_dim, int value_dim,
+                                   float* grouped, int tokens, int rows, int heads, int kv_heads, int key_dim, int value_dim,
                                    cudaStream_t stream) {
   if (rows == 0) return MIR_OK;
   if (rows < 0 || heads <= 0 || kv_heads <= 0 || heads % kv_heads || key_dim <= 0 || value_dim <= 0) {
     mir_set_error("delta_rule_scan: bad sizes (rows %d, heads %d, kv heads %d, key_dim %d, value_dim %d)", rows, heads,
                   kv_heads, key_dim, value_dim);
     return MIR_BAD_ARGUMENT;
+  }
+  if (grouped != nullptr && tokens != rows && key_dim <= kGroupedKeys && ((uintptr_t)grouped & 15) == 0 && heads <= 4 * 65535) {
+    if (per_channel)
+      return launch_grouped<true>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, grouped, tokens,
+                                  rows, heads, kv_heads, key_dim, value_dim);
+    return launch_grouped<false>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, grouped, tokens,
+                                 rows, heads, kv_heads, key_dim, value_dim);
   }
   if (per_channel)
     return launch_scan<true>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, rows, heads,

@@ -81,6 +81,12 @@ template <int N> __device__ __forceinline__ int lane_sum(int l) {
   for (int bit = 1, half = N / 2; half > 0; bit <<= 1, half >>= 1) index += (l & bit) ? half : 0;
   return index;
 }
+// The lane that has sum `index`: lane_sum<N>(lane_with<N>(index)) == index.
+template <int N> __host__ __device__ constexpr int lane_with(int index) {
+  int lane = 0;
+  for (int bit = 1, half = N / 2; half > 0; bit <<= 1, half >>= 1) lane += (index & half) ? bit : 0;
+  return lane;
+}
 template <int LANES, int N, int STEP = 1>
 __device__ __forceinline__ float sum_lanes(const float (&parts)[N], int l) {
   if constexpr (N == 1) {

@@ -67,7 +67,7 @@ _SIGNATURES = {
                                    c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "mir_delta_rule_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                                c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "mir_delta_rule_set_lanes": [c_int],
         "mir_gated_head_norm": [c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_float, c_int, c_int, c_void_p],
@@ -607,16 +607,32 @@ def delta_rule_prepare(x: torch.Tensor, weight: torch.Tensor, tail: torch.Tensor
         taps, _stream()))
 
 
+DELTA_GROUPED_KEYS = 128         # the widest key heads that delta_rule_scan walks in groups
+
+
+def delta_rule_grouped_floats(tokens: int, rows: int, heads: int, key_dim: int) -> int:
+    """How many 32-bit numbers delta_rule_scan's `grouped` scratch holds: per group of four tokens and head thirteen vectors of
+    the padded key width and 28 numbers; a request's last group may lack tokens."""
+    return (tokens // 4 + rows) * heads * (13 * (64 if key_dim <= 64 else 128) + 28)
+
+
 def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, state: torch.Tensor,
                     query_starts: torch.Tensor, state_slots: torch.Tensor, positions: torch.Tensor, out: torch.Tensor,
-                    heads: int, kv_heads: int, key_dim: int, value_dim: int) -> None:
+                    heads: int, kv_heads: int, key_dim: int, value_dim: int,
+                    grouped: Optional[torch.Tensor] = None) -> None:
     """The gated delta rule over the tokens of each request row, from and into state [slots, heads, value_dim,
     key_dim] (32-bit): per head S <- diag(decay) S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q.  qkv, beta and
     decay as delta_rule_prepare leaves them (decay [tokens, heads * key_dim] means one decay per key channel); out
-    [tokens, heads * value_dim] 32-bit."""
-    _cuda(qkv, beta, decay, state, query_starts, state_slots, positions, out)
+    [tokens, heads * value_dim] 32-bit.  With `grouped` (32-bit scratch of delta_rule_grouped_floats numbers) a step that brings
+    more than single tokens walks four tokens at a time, for key heads of up to DELTA_GROUPED_KEYS: the same sums in another
+    order, which depends on where a request's portions begin."""
+    _cuda(qkv, beta, decay, state, query_starts, state_slots, positions, out, grouped)
     tokens = qkv.shape[0]
     rows = query_starts.numel() - 1
+    _require(grouped is None or (grouped.dtype == torch.float32 and grouped.is_contiguous() and grouped.data_ptr() % 16 == 0
+                                 and key_dim <= DELTA_GROUPED_KEYS
+                                 and grouped.numel() >= delta_rule_grouped_floats(tokens, rows, heads, key_dim)),
+             "delta_rule_scan: grouped is float32 scratch of delta_rule_grouped_floats numbers on a 16-byte boundary")
     per_channel = decay.shape[1] != heads
     for tensor, shape in ((qkv, (tokens, 2 * kv_heads * key_dim + heads * value_dim)), (beta, (tokens, heads)),
                           (decay, (tokens, heads * key_dim if per_channel else heads)),
@@ -628,8 +644,8 @@ def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, 
     lib = library("core")
     _check(lib, lib.mir_delta_rule_scan(int(per_channel), qkv.data_ptr(), beta.data_ptr(), decay.data_ptr(),
                                         state.data_ptr(), query_starts.data_ptr(), state_slots.data_ptr(),
-                                        positions.data_ptr(), out.data_ptr(), tokens, rows, heads, kv_heads, key_dim,
-                                        value_dim, _stream()))
+                                        positions.data_ptr(), out.data_ptr(), _ptr(grouped), tokens, rows, heads, kv_heads,
+                                        key_dim, value_dim, _stream()))
 
 
 def set_delta_rule_lanes(lanes: int) -> None:

@@ -182,6 +182,56 @@ def test_delta_rule_against_the_plain_recurrence(per_channel, heads, kv_heads, k
         assert torch.all(state[2] == 7.0) and torch.all(state[0] == 0.0) and torch.all(tail[0] == 0.0)
 
 
+@pytest.mark.parametrize("per_channel", [True, False])
+@pytest.mark.parametrize("heads,kv_heads,key_dim,value_dim", [(2, 1, 128, 128), (4, 4, 64, 40), (3, 3, 100, 16), (5, 5, 21, 9), (1, 1, 4, 1),
+                                                              (16, 8, 128, 40), (24, 24, 36, 9)])   # (four columns a lane)
+def test_delta_rule_four_tokens_at_a_time(per_channel, heads, kv_heads, key_dim, value_dim):
+    """Portions of every remainder, a padding row among them, decays of exactly zero and one: as near to 64 bits as one token
+    at a time, and slots that no row names stay as they were."""
+    from libmir_b200 import kernels
+    torch.manual_seed(key_dim + value_dim)
+    portions = [1, 4, 5, 130, 3, 2, 66]
+    tokens, rows, slots_held = sum(portions), len(portions), len(portions) + 2
+    starts = [0] + np.cumsum(portions).tolist()
+    slots = torch.randperm(slots_held)[:rows]
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    q, k = unit(torch.randn(tokens, kv_heads, key_dim)) * key_dim ** -0.5, unit(torch.randn(tokens, kv_heads, key_dim))
+    v, beta = torch.randn(tokens, heads, value_dim), torch.rand(tokens, heads)
+    decay = torch.rand(tokens, heads, key_dim if per_channel else 1) ** 0.2
+    decay[torch.rand(decay.shape) < 0.02], decay[torch.rand(decay.shape) < 0.02] = 0.0, 1.0
+    state = torch.randn(slots_held, heads, value_dim, key_dim)
+    positions = torch.zeros(tokens, dtype=torch.int32)
+    skipped = 5                                                   # this row is padding
+    positions[starts[skipped]:starts[skipped + 1]] = -1
+    want, want_state = torch.zeros(tokens, heads, value_dim, dtype=torch.float64), state.double().clone()
+    for r in range(rows):
+        if r == skipped:
+            continue
+        for h in range(heads):
+            s, g = want_state[slots[r], h].T.clone(), h // (heads // kv_heads)           # [key, value]
+            for t in range(starts[r], starts[r + 1]):
+                s = decay[t, h].double()[:, None] * s
+                u = beta[t, h].double() * (v[t, h].double() - s.T @ k[t, g].double())
+                s = s + torch.outer(k[t, g].double(), u)
+                want[t, h] = s.T @ q[t, g].double()
+            want_state[slots[r], h] = s.T
+    cuda = lambda t, kind=None: t.to(device="cuda", dtype=kind or t.dtype).contiguous()
+    qkv = cuda(torch.cat([q.flatten(1), k.flatten(1), v.flatten(1)], 1))
+    live = [t for r in range(rows) if r != skipped for t in range(starts[r], starts[r + 1])]
+    errors = []
+    for grouped in (True, False):
+        held, out = cuda(state.clone()), torch.full((tokens, heads * value_dim), float("nan"), device="cuda")
+        scratch = torch.full((kernels.delta_rule_grouped_floats(tokens, rows, heads, key_dim),), float("nan"), device="cuda") if grouped else None
+        kernels.delta_rule_scan(qkv, cuda(beta), cuda(decay.flatten(1)), held, cuda(torch.tensor(starts), torch.int32),
+                                cuda(slots, torch.int32), cuda(positions), out, heads, kv_heads, key_dim, value_dim, grouped=scratch)
+        got = out.view(tokens, heads, value_dim).double().cpu()
+        assert bool(torch.isnan(got[starts[skipped]:starts[skipped + 1]]).all())
+        errors.append((float((got[live] - want[live]).norm() / want[live].norm()),
+                       float((held.double().cpu() - want_state).norm() / want_state.norm())))
+    # 32-bit sums of up to 128 + 3 terms, 130 tokens deep
+    assert max(errors[0]) <= 1e-5 and all(a <= 1.5 * b + 2e-8 for a, b in zip(*errors)), errors
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps,key_dim,value_dim,per_channel", [(4, 128, 64, True), (2, 100, 24, False), (1, 64, 128, True), (3, 4, 200, False)])
 def test_what_the_recurrence_needs_is_the_same_in_long_steps_and_short_ones(dtype, taps, key_dim, value_dim, per_channel):
