@@ -677,3 +677,24 @@ def test_configurations_drawn_at_random(tmp_path, seed):
         if dtype == "float32":
             assert all(np.array_equal(outputs[0], other) for other in outputs[1:]), json.dumps(config)
         model.unload()
+
+
+@pytest.mark.parametrize("value_dim,offset", [(4, 4), (60, 8), (64, 4), (68, 8), (124, 4), (128, 8), (128, 1), (132, 8)])
+@pytest.mark.parametrize("dtype,gate_dtype,tol", [(torch.float32, torch.float32, 1e-6), (torch.bfloat16, torch.float32, 2 ** -8),
+                                                  (torch.bfloat16, torch.bfloat16, 2 ** -8)])
+def test_gated_head_norm_of_every_width(dtype, gate_dtype, tol, value_dim, offset):
+    """Heads of one to 32 lanes of four channels, the general kernel's beside them (wider heads, gates off the boundary), to
+    the output's own rounding; a count of heads that fills no CTA."""
+    from libmir_b200 import kernels
+    torch.manual_seed(value_dim)
+    tokens, heads = 5, 3
+    read = torch.randn(tokens, heads * value_dim)
+    packed = torch.randn(tokens, offset + heads * value_dim).to(gate_dtype)
+    gate = packed[:, offset:].double().view(tokens, heads, value_dim)
+    weight = torch.rand(value_dim) + 0.5
+    x = read.double().view(tokens, heads, value_dim)
+    want = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-5) * weight.double() * torch.nn.functional.silu(gate)
+    out = torch.empty(tokens, heads * value_dim, dtype=dtype, device=device())
+    kernels.gated_head_norm(read.to(device()), packed.to(device())[:, offset:], weight.to(device()), out, heads, value_dim, 1e-5, False)
+    error = (out.double().cpu().view_as(want) - want).abs()
+    assert bool((error <= tol * want.abs() + 4e-6 * want.abs().max()).all())
