@@ -884,3 +884,23 @@ def test_configurations_drawn_at_random(tmp_path, seed):
         if dtype == "float32":
             assert all(np.array_equal(outputs[0], other) for other in outputs[1:]), json.dumps(config)
         model.unload()
+
+
+@pytest.mark.parametrize("tokens,top,experts", [(1, 1, 1), (32, 1, 1024), (64, 8, 5), (512, 1, 64), (513, 1, 64), (171, 3, 40)])
+def test_pairs_in_the_order_of_their_experts(tokens, top, experts):
+    """The sort of one CTA (512 pairs at most) and the one over many: whole numbers, so exact.  Every tenth pair chose an
+    identity expert (an id beyond the experts) and is in no list."""
+    from libmir_b200 import kernels
+    generator = torch.Generator().manual_seed(tokens)
+    ids = torch.randint(0, experts, (tokens, top), generator=generator)
+    ids.view(-1)[9::10] = experts + 2
+    alloc = lambda shape, kind: torch.full(shape, -7, dtype=kind, device=device())
+    found = kernels.moe_sort(on_device(ids.to(torch.int32)), experts, alloc, 8)
+    flat = ids.view(-1)
+    want = [pair for expert in range(experts) for pair in (flat == expert).nonzero().view(-1).tolist()]
+    counts = torch.bincount(flat, minlength=experts)[:experts].tolist()
+    offsets = [sum(counts[:e]) for e in range(experts + 1)]
+    tiles = [(e, offsets[e] + first) for e in range(experts) for first in range(0, counts[e], 8)]
+    assert found.order.cpu().tolist()[:len(want)] == want and found.offsets.cpu().tolist() == offsets
+    assert int(found.tile_count.cpu()) == len(tiles)
+    assert found.tiles.cpu().view(-1, 2).tolist()[:len(tiles)] == [list(t) for t in tiles]
