@@ -237,7 +237,25 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
         }
         if (c0 + 64 >= out_width) release();                 // the last columns are in registers
         const int limit = min(n, n0 + out_width);            // columns of this tile that exist
-        if (source_row < row_end) {
+        if (MODE == F32 && n0 + c0 + 32 <= limit && (ldo % 4) == 0 && bias == nullptr) {
+          // 32-bit rows: through shared memory, so that a store writes four rows of 128 bytes instead of sixteen bytes of
+          // each of 32 rows (19,800 sorted rows of 2,048 columns, K 1,024: 86 us, 106 the other way)
+          float4* block = reinterpret_cast<float4*>(smem + (size_t)kStages * kStageStride) + (warp - 2) * 256;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            block[lane * 8 + (i ^ (lane & 7))] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          __syncwarp();
+          const int place = source_row < row_end ? row : -1;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = i * 4 + (lane >> 3);
+            const int to = __shfl_sync(0xffffffffu, place, r);
+            if (to >= 0)
+              reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + (size_t)to * ldo + n0 + c0)[lane & 7] =
+                  block[r * 8 + ((lane & 7) ^ (r & 7))];
+          }
+          __syncwarp();                                      // (the block is written again for the next columns)
+        } else if (source_row < row_end) {
           if (MODE == STORE || MODE == SWIGLU || MODE == GELU || MODE == GELU_ERF || MODE == RELU2) {
             bf16* dst = reinterpret_cast<bf16*>(out) + (size_t)row * ldo + n0 + c0;
             if (n0 + c0 + 32 <= limit && (ldo % 8) == 0) {
@@ -335,7 +353,7 @@ int launch(const void* x, int ldx, const void* w, const void* bias, void* out, i
   if (status != MIR_OK) return status;
   status = tensor_map_for(w, MODE == SWIGLU ? up_offset + n : n, k, k, out_width, &w_map);
   if (status != MIR_OK) return status;
-  const size_t smem = (size_t)kStages * kStageStride + 1024;
+  const size_t smem = (size_t)kStages * kStageStride + 1024 + (MODE == F32 ? kEpilogueWarps * 4096 : 0);
   static bool configured = false;
   if (!configured) {
     const cudaError_t err = cudaFuncSetAttribute(tc_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -364,7 +382,7 @@ int launch_grouped(const void* x, int ldx, int rows, const void* w, int weight_r
   if (status != MIR_OK) return status;
   status = tensor_map_for(w, weight_rows, k, k, out_width, &w_map);
   if (status != MIR_OK) return status;
-  const size_t smem = (size_t)kStages * kStageStride + 1024;
+  const size_t smem = (size_t)kStages * kStageStride + 1024 + (MODE == F32 ? kEpilogueWarps * 4096 : 0);
   static bool configured = false;
   if (!configured) {
     const cudaError_t err = cudaFuncSetAttribute(tc_gemm_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
