@@ -84,7 +84,7 @@ __global__ void paged_attention_generic_kernel(
       const T* k_row = k_pages + key_offset * head_dim;
       float dot = 0.0f;
       if (head_dim % 8 == 0) {                                // (then every key row starts on a 16-byte boundary)
-#pragma unroll 4
+#pragma unroll 8
         for (int d = 0; d < head_dim; d += 8) {
           float k8[8];
           load8(k_row + d, k8);
@@ -107,8 +107,8 @@ __global__ void paged_attention_generic_kernel(
     for (int i = 0; i < PIECES; ++i) acc[i] *= correction;
     const int keys_here = min(32, last - base + 1);
     // Several keys' values are asked for before the first is used: with one warp a query and head the loop is otherwise bound
-    // by the latency of a load per key (a decoded token at 136 keys 63 us).  The sum still goes key by key.
-    constexpr int RUN = PIECES <= 4 ? 8 : 1;
+    // by the latency of a load per key (a decoded token at 136 keys 63 us; eight at a time 37, sixteen and twice as many pieces of the keys 29).  The sum still goes key by key.
+    constexpr int RUN = PIECES <= 4 ? 16 : 1;
     int j = 0;
     for (; j + RUN <= keys_here; j += RUN) {
       float values[RUN][PIECES], w[RUN];

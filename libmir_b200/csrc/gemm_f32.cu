@@ -11,7 +11,8 @@
 //   gemm_f32_rows   up to 16 rows of A: bound by reading W once.  A CTA takes 16 rows of W and all of A; a thread owns one
 //                   output and walks down k, so the least a product can take is K dependent multiply-adds (four cycles
 //                   each, 4.2 us for 2,048), which several CTAs on an SM, each with a ring of four
-//                   stages of 128 k, hide behind the reads.
+//                   stages of 128 k that two warps of its own fill, hide behind the reads (3 rows, the products of
+//                   a layer of 2,048 with 5,504 inside: 27.6 us on average; all warps filling the ring: 29.5).
 //   gemm_f32_tile   more rows: bound by the multiply-adds.  A thread owns TM x TN outputs whose rows and columns lie
 //                   (tile / threads) apart, and reads four k of each with one load.
 #include "common.cuh"
@@ -34,16 +35,17 @@ template <int LEFT> __device__ __forceinline__ void copy_wait() {
 // ROWS rows of K-major data from row `row0` and column k0 on into [ROWS][DEPTH + 4]; what lies outside is zero.  WIDE: rows
 // start on 16-byte boundaries and k is a multiple of four.
 template <int ROWS, int DEPTH, int THREADS, bool WIDE>
-__device__ __forceinline__ void load_tile(float* tile, const float* __restrict__ from, int ld, int row0, int rows, int k0, int k) {
+__device__ __forceinline__ void load_tile(float* tile, const float* __restrict__ from, int ld, int row0, int rows, int k0, int k,
+                                          int thread) {
   if (WIDE) {
     constexpr int PIECES = DEPTH / 4;
-    for (int index = threadIdx.x; index < ROWS * PIECES; index += THREADS) {
+    for (int index = thread; index < ROWS * PIECES; index += THREADS) {
       const int r = index / PIECES, kk = (index % PIECES) * 4;
       const bool there = row0 + r < rows && k0 + kk < k;
       copy_async(tile + r * (DEPTH + 4) + kk, there ? from + (size_t)(row0 + r) * ld + k0 + kk : from, there ? 16 : 0);
     }
   } else {
-    for (int index = threadIdx.x; index < ROWS * DEPTH; index += THREADS) {
+    for (int index = thread; index < ROWS * DEPTH; index += THREADS) {
       const int r = index / DEPTH, kk = index % DEPTH;
       const bool there = row0 + r < rows && k0 + kk < k;
       copy_async_one(tile + r * (DEPTH + 4) + kk, there ? from + (size_t)(row0 + r) * ld + k0 + kk : from, there);
@@ -58,7 +60,7 @@ __device__ __forceinline__ void finish(float* c, int ldc, const float* bias, flo
 }
 
 template <int BM, int BN, int TM, int TN, int DEPTH, int STAGES, bool WIDE>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN > 32 ? 1 : 3)
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), 3)
 gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, const float* __restrict__ bias,
                      float* __restrict__ c, int ldc, int m, int n, int k, float beta) {
   constexpr int ACROSS = BN / TN, DOWN = BM / TM, THREADS = ACROSS * DOWN, ROW = DEPTH + 4;
@@ -73,8 +75,8 @@ gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restri
   const int steps = (k + DEPTH - 1) / DEPTH;
   auto fetch = [&](int step) {
     float* stage = shared + (step % STAGES) * (BM + BN) * ROW;
-    load_tile<BM, DEPTH, THREADS, WIDE>(stage, a, lda, row0, m, step * DEPTH, k);
-    load_tile<BN, DEPTH, THREADS, WIDE>(stage + BM * ROW, w, ldw, col0, n, step * DEPTH, k);
+    load_tile<BM, DEPTH, THREADS, WIDE>(stage, a, lda, row0, m, step * DEPTH, k, threadIdx.x);
+    load_tile<BN, DEPTH, THREADS, WIDE>(stage + BM * ROW, w, ldw, col0, n, step * DEPTH, k, threadIdx.x);
   };
 #pragma unroll
   for (int step = 0; step < STAGES - 1; ++step) {
@@ -123,11 +125,11 @@ gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restri
   }
 }
 
-constexpr int kRowsColumns = 16, kRowsDepth = 128, kRowsStages = 4, kRowsThreads = 128, kRun = 4;
+constexpr int kRowsColumns = 16, kRowsDepth = 128, kRowsStages = 4, kRowsThreads = 128, kRowsLoaders = 64, kRun = 4;
 
 // MT: rows of A rounded up to a power of two (1 to 16).  With MT = 16 a thread owns two outputs.
 template <int MT, bool WIDE>
-__global__ void __launch_bounds__(kRowsThreads, 4)
+__global__ void __launch_bounds__(kRowsThreads + kRowsLoaders, 3)
 gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restrict__ w, int ldw, const float* __restrict__ bias,
                      float* __restrict__ c, int ldc, int m, int n, int k, float beta) {
   constexpr int ROW = kRowsDepth + 4, STAGE = (kRowsColumns + MT) * ROW;
@@ -141,22 +143,30 @@ gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restri
 #pragma unroll
   for (int e = 0; e < EACH; ++e) acc[e] = 0.0f;
   const int steps = (k + kRowsDepth - 1) / kRowsDepth;
-  auto fetch = [&](int step) {
-    float* stage = shared + (step % kRowsStages) * STAGE;
-    load_tile<kRowsColumns, kRowsDepth, kRowsThreads, WIDE>(stage, w, ldw, col0, n, step * kRowsDepth, k);
-    load_tile<MT, kRowsDepth, kRowsThreads, WIDE>(stage + kRowsColumns * ROW, a, lda, 0, m, step * kRowsDepth, k);
-  };
+  if (threadIdx.x >= kRowsThreads) {               // two warps fetch: the others' chain of multiply-adds is not interrupted
+    const int thread = threadIdx.x - kRowsThreads;
+    auto fetch = [&](int step) {
+      if (step < steps) {
+        float* stage = shared + (step % kRowsStages) * STAGE;
+        load_tile<kRowsColumns, kRowsDepth, kRowsLoaders, WIDE>(stage, w, ldw, col0, n, step * kRowsDepth, k, thread);
+        load_tile<MT, kRowsDepth, kRowsLoaders, WIDE>(stage + kRowsColumns * ROW, a, lda, 0, m, step * kRowsDepth, k, thread);
+      }
+      copy_commit();
+    };
 #pragma unroll
-  for (int step = 0; step < kRowsStages - 1; ++step) {
-    if (step < steps) fetch(step);
-    copy_commit();
-  }
-  for (int step = 0; step < steps; ++step) {
+    for (int step = 0; step < kRowsStages - 1; ++step) fetch(step);
     copy_wait<kRowsStages - 2>();
-    __syncthreads();
-    if (step + kRowsStages - 1 < steps) fetch(step + kRowsStages - 1);
-    copy_commit();
-    if (!owner) continue;
+    __syncthreads();                               // the first stage is there
+    for (int step = 0; step < steps; ++step) {     // (into the stage that was multiplied last)
+      fetch(step + kRowsStages - 1);
+      copy_wait<kRowsStages - 2>();
+      __syncthreads();                             // this stage has been read, and the next one is there
+    }
+    copy_wait<0>();
+    return;
+  }
+  __syncthreads();
+  for (int step = 0; step < steps; ++step) {
     const float* wt = shared + (step % kRowsStages) * STAGE + tx * ROW;
     const float* at = shared + (step % kRowsStages) * STAGE + (kRowsColumns + ty) * ROW;
     // Runs of kRun pieces of four k, the next run's reads on their way while this one's chain of multiply-adds goes on.
@@ -180,14 +190,17 @@ gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restri
           acc[e] = fmaf(av[buffer][e][i].w, wv[buffer][i].w, acc[e]);
         }
     };
-    read(0, 0);
+    if (owner) {
+      read(0, 0);
 #pragma unroll 1
-    for (int kk = 0; kk < kRowsDepth; kk += 8 * kRun) {
-      read(1, kk + 4 * kRun);
-      multiply(0);
-      if (kk + 8 * kRun < kRowsDepth) read(0, kk + 8 * kRun);
-      multiply(1);
+      for (int kk = 0; kk < kRowsDepth; kk += 8 * kRun) {
+        read(1, kk + 4 * kRun);
+        multiply(0);
+        if (kk + 8 * kRun < kRowsDepth) read(0, kk + 8 * kRun);
+        multiply(1);
+      }
     }
+    __syncthreads();
   }
   if (!owner || col0 + tx >= n) return;
 #pragma unroll
@@ -219,7 +232,8 @@ int launch(Kernel kernel, dim3 grid, int threads, int smem, const Product& p) {
 template <int MT, bool WIDE>
 int launch_rows(const Product& p) {
   constexpr int smem = kRowsStages * (kRowsColumns + MT) * (kRowsDepth + 4) * (int)sizeof(float);
-  return launch(gemm_f32_rows_kernel<MT, WIDE>, dim3((p.n + kRowsColumns - 1) / kRowsColumns), kRowsThreads, smem, p);
+  return launch(gemm_f32_rows_kernel<MT, WIDE>, dim3((p.n + kRowsColumns - 1) / kRowsColumns),
+                kRowsThreads + kRowsLoaders, smem, p);
 }
 
 template <int BM, int BN, int TM, int TN, bool WIDE>
@@ -241,16 +255,17 @@ int choose(const Product& p) {
   if (p.m <= 8) return launch_rows<8, WIDE>(p);
   if (p.m <= 16) return launch_rows<16, WIDE>(p);
   if (p.m <= 32) return launch_tile<32, 64, 4, 4, WIDE>(p);
-  // The tile whose busiest SM has the least to do: multiply-adds of its tiles, a thread of a smaller tile reading more of
-  // shared memory for each (by the weights below).
+  // The tile whose busiest SM has the least to do: multiply-adds of its tiles, a thread of the smaller tile reading more of
+  // shared memory for each (by the weights below).  290 rows: N 11,008, K 2,048 by 64 x 64 364 us, the average of a layer's
+  // products by 64 x 64 249 us and by 32 x 64 212 (each where it is taken); 2,048 rows, N 2,048, K 5,504: 1,107 us (41.7 TF).
+  // Larger tiles are no better: 64 x 128 with 64 outputs a thread 373 us for what these two do in 230, 128 x 128 1,173 us
+  // for the last product and the same to 1 % for N 11,008.
   const int sms = mir_sm_count();
   auto cost = [&](int rows, int columns, int weight) {
     const long long tiles = (long long)((p.m + rows - 1) / rows) * ((p.n + columns - 1) / columns);
     return (tiles + sms - 1) / sms * rows * columns * weight;
   };
-  const long long small = cost(32, 64, 6), middle = cost(64, 64, 5), large = cost(128, 128, 4);
-  if (large <= middle && large <= small) return launch_tile<128, 128, 8, 8, WIDE>(p);
-  if (middle <= small) return launch_tile<64, 64, 8, 4, WIDE>(p);
+  if (cost(64, 64, 5) <= cost(32, 64, 6)) return launch_tile<64, 64, 8, 4, WIDE>(p);
   return launch_tile<32, 64, 4, 4, WIDE>(p);
 }
 

@@ -116,7 +116,7 @@ def test_gemm_f32_rows_do_not_depend_on_the_batch():
 
 @pytest.mark.parametrize("n,k", [(15, 4), (65, 260), (129, 1028), (200, 258), (130, 37)])
 def test_gemm_f32_rows_are_the_same_bits_in_every_kernel(n, k):
-    """The kernels of 1 to 16 rows and the tiles (32, 64 and, with many rows, 128 high), with 16-byte and with single loads."""
+    """The kernels of 1 to 16 rows and the tiles (32 and 64 high), with 16-byte and with single loads."""
     from libmir_b200 import kernels
     torch.manual_seed(6)
     many = 128 * (2 * 148) // max(1, -(-n // 128)) + 5
