@@ -14,6 +14,7 @@ from typing import Dict, Optional, Tuple
 
 import torch
 
+from .. import kernels
 from .manager import CacheManager
 
 _DTYPES = {"float32": torch.float32, "bfloat16": torch.bfloat16, "int32": torch.int32}
@@ -57,6 +58,11 @@ class CacheStorage:
                                                dtype=_DTYPES[requirement.dtype], device=device)
         for entry, requirement in manager.state_entries.items():
             self.states[entry] = tuple(make(r) for r in requirement) if isinstance(requirement, tuple) else make(requirement)
+        tensors = self._state_tensors()
+        if tensors and tensors[0].device.type == "cuda":       # where each state's records are, for the kernel that zeroes them
+            record = [t[0].numel() * t.element_size() for t in tensors]
+            self._regions = torch.tensor([[t.data_ptr(), size] for t, size in zip(tensors, record)], device=device)
+            self._largest = max(record)
         self.views: Dict[int, CacheView] = {}
         for item in plan:
             view = CacheView(writes=item.source == item.entry)
@@ -77,12 +83,20 @@ class CacheStorage:
         """Fixed-size state of newly admitted requests starts at zero."""
         if not slots or not self.states:
             return
-        tensors = [t for held in self.states.values() for t in (held if isinstance(held, tuple) else (held,))]
-        index = torch.tensor(slots, dtype=torch.long, device=tensors[0].device)
-        for state in tensors:
-            state.index_fill_(0, index, 0)
+        tensors = self._state_tensors()
+        if tensors[0].device.type != "cuda":
+            index = torch.tensor(slots, dtype=torch.long)
+            for state in tensors:
+                state.index_fill_(0, index, 0)
+            return
+        limit = self.manager.max_requests
+        if any(not 0 <= slot < limit for slot in slots):
+            raise IndexError(f"state slots {list(slots)} are not all within 0 .. {limit - 1}")
+        kernels.zero_slots(self._regions, self._largest, slots)
+
+    def _state_tensors(self):
+        return [t for held in self.states.values() for t in (held if isinstance(held, tuple) else (held,))]
 
     def bytes(self) -> int:
         return sum(b.numel() * b.element_size() for b in self.buffers) + \
-            sum(t.numel() * t.element_size() for held in self.states.values()
-                for t in (held if isinstance(held, tuple) else (held,)))
+            sum(t.numel() * t.element_size() for t in self._state_tensors())

@@ -724,6 +724,26 @@ MIR_EXPORT int mir_random_normal(int bf16, void* out, size_t total, unsigned lon
   return mir_check_launch("random_normal");
 }
 
+// The fixed-size states of newly admitted requests: zero.  regions[2 n], [2 n + 1]: where the n-th state tensor starts and the
+// bytes one request's record takes in it.  One launch for all tensors and up to kSlotsAtOnce requests, whose slots travel in the
+// launch: 24 tensors filled one by one cost a prompt 24 launches and a copy before its first kernel.
+constexpr int kSlotsAtOnce = 64, kZeroPiece = 64 * 1024;
+struct ZeroSlots { int slot[kSlotsAtOnce]; };
+
+__global__ void __launch_bounds__(256) zero_slots_kernel(const long long* __restrict__ regions, ZeroSlots slots) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  char* base = reinterpret_cast<char*>(regions[2 * blockIdx.y]);
+  const long long bytes = regions[2 * blockIdx.y + 1];
+  char* record = base + (long long)slots.slot[blockIdx.z] * bytes;
+  const long long first = (long long)blockIdx.x * kZeroPiece, last = min(bytes, first + kZeroPiece);
+  if (((reinterpret_cast<uintptr_t>(record) | (uintptr_t)bytes) & 15) == 0) {
+    for (long long i = first + threadIdx.x * 16; i < last; i += 256 * 16) *reinterpret_cast<uint4*>(record + i) = make_uint4(0, 0, 0, 0);
+  } else {
+    for (long long i = first + threadIdx.x; i < last; i += 256) record[i] = 0;
+  }
+}
+
 // ---- decode batches that run as a captured graph -------------------------------------------------
 // Before the layers: where each row's new key/value goes, from its position and block table.  A row
 // with a negative position is padding (the batch is smaller than the captured size): no cache write.
@@ -762,6 +782,25 @@ __global__ void decode_advance_kernel(const int* __restrict__ sampled, int* __re
     if (step < log_steps) token_log[(size_t)step * rows + row] = token;
   }
   if (threadIdx.x == 0) *step_counter = step + 1;
+}
+
+// regions [states][2] on the device as above, largest: the most bytes a record takes; slots on the host.
+MIR_EXPORT int mir_zero_slots(const long long* regions, int states, long long largest, const int* slots, int count,
+                              cudaStream_t stream) {
+  if (states < 0 || states > 65535 || largest < 0 || count < 0) {
+    mir_set_error("zero_slots: bad sizes (states %d, largest %lld, count %d)", states, largest, count);
+    return MIR_BAD_ARGUMENT;
+  }
+  if (states == 0 || largest == 0) return MIR_OK;
+  for (int done = 0; done < count; done += kSlotsAtOnce) {
+    const int now = min(kSlotsAtOnce, count - done);
+    ZeroSlots these = {};
+    for (int i = 0; i < now; ++i) these.slot[i] = slots[done + i];
+    const int status = mir_launch("zero_slots", zero_slots_kernel, dim3((unsigned)((largest + kZeroPiece - 1) / kZeroPiece), states, now),
+                                  dim3(256), 0, stream, 0, regions, these);
+    if (status != MIR_OK) return status;
+  }
+  return MIR_OK;
 }
 
 MIR_EXPORT int mir_decode_prepare(const int* positions, const int* block_table, int table_width, int page_size,

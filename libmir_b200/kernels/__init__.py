@@ -109,6 +109,7 @@ _SIGNATURES = {
         "mir_sample": [c_void_p, c_longlong, c_int, c_int, c_void_p, c_void_p, c_longlong, c_int, c_void_p, c_void_p,
                        c_void_p, c_int, c_void_p],
         "mir_repetition_penalty": [c_void_p, c_longlong, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
+        "mir_zero_slots": [c_void_p, c_int, c_longlong, c_void_p, c_int, c_void_p],
         "mir_decode_prepare": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_void_p],
         "mir_decode_advance": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p],
     },
@@ -1360,6 +1361,16 @@ def random_normal(out: torch.Tensor, seed: int, deviation: float) -> None:
     lib.mir_random_normal.restype = c_int
     _check(lib, lib.mir_random_normal(int(out.dtype == torch.bfloat16), out.data_ptr(), out.numel(),
                                       seed & ((1 << 64) - 1), float(deviation), _stream()))
+
+
+def zero_slots(regions: torch.Tensor, largest: int, slots) -> None:
+    """Zero the records `slots` (host numbers) of every state tensor; regions [states, 2] int64 on the device: address and
+    bytes a record, `largest` the most of those bytes."""
+    _require(regions.dtype == torch.int64 and regions.is_contiguous() and regions.dim() == 2 and regions.shape[1] == 2,
+             "zero_slots: contiguous int64 [states, 2] is needed")
+    held = (c_int * len(slots))(*slots)
+    lib = library("core")
+    _check(lib, lib.mir_zero_slots(regions.data_ptr(), regions.shape[0], largest, held, len(slots), _stream()))
 
 
 def decode_prepare(positions, block_table, page_size, slot_mapping, context_lens) -> None:

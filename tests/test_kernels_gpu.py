@@ -647,3 +647,23 @@ def test_random_weights_from_the_device_generator():
     half = torch.empty(4096, device="cuda", dtype=torch.bfloat16)
     kernels.random_normal(half, 12345, 0.02)
     assert torch.equal(half, a[:4096].bfloat16())
+
+
+@pytest.mark.parametrize("slots", [[0], [3, 1], [69, 2] + list(range(5, 68))])
+def test_states_of_new_requests_are_zeroed_and_no_others(slots):
+    """Records of 2 bytes to several pieces of 64 KB, on and off the 16-byte boundary, one and several launches of slots."""
+    from types import SimpleNamespace
+    from libmir_b200.cache import CacheStorage
+    made = lambda dtype, *shape: SimpleNamespace(shape=shape, dtype=dtype)
+    entries = {0: made("float32", 3, 7), 1: (made("bfloat16", 1), made("float32", 4, 128, 129), made("bfloat16", 3, 11)), 4: made("int32", 4)}
+    manager = SimpleNamespace(groups=[], state_entries=entries, entry_group={}, max_requests=70)
+    storage = CacheStorage(manager, [], torch.bfloat16, torch.device("cuda"))
+    tensors = [storage.states[0], *storage.states[1], storage.states[4]]
+    for t in tensors:
+        t.fill_(7)
+    storage.zero_slots(slots)
+    others = [s for s in range(70) if s not in slots]
+    for t in tensors:
+        assert bool((t[slots] == 0).all()) and bool((t[others] == 7).all())
+    with pytest.raises(IndexError):
+        storage.zero_slots([70])
