@@ -9,6 +9,7 @@ graph.rs:112-121).
 
 from __future__ import annotations
 
+import contextlib
 from dataclasses import dataclass, field
 from typing import Dict, List, Optional, Sequence
 
@@ -73,6 +74,13 @@ class Arena:
             self.chunk += 1
             self.offset = 0
 
+    def mark(self) -> tuple:
+        """Where the next allocation goes: `rewind` to it gives back everything asked for since."""
+        return self.chunk, self.offset
+
+    def rewind(self, mark: tuple) -> None:
+        self.chunk, self.offset = mark
+
     def bytes(self) -> int:
         return sum(chunk.numel() for chunk in self.chunks)
 
@@ -130,6 +138,12 @@ class StepContext(PartContext):
 
     def alloc(self, shape, dtype: torch.dtype) -> torch.Tensor:
         return self.arena.alloc(shape, dtype)
+
+    @contextlib.contextmanager
+    def temporary(self):
+        mark = self.arena.mark()
+        yield
+        self.arena.rewind(mark)
 
     def note_residual_stats(self, residual: torch.Tensor, sumsq: Optional[torch.Tensor], tiles: int,
                             weighted: Optional[torch.Tensor] = None, norm_weight: Optional[torch.Tensor] = None) -> None:

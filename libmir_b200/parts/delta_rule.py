@@ -161,10 +161,11 @@ class GatedDeltaRule(Mixer):
         read = ctx.alloc((tokens, self.v_width), torch.float32)
         # portions of prompts walk four tokens at a time, but for the 32-bit engine, whose results do not depend on the cut
         grouped = None
-        if self.env.dtype == torch.bfloat16 and not ctx.decode_only and s.key_dim <= kernels.DELTA_GROUPED_KEYS:
-            grouped = ctx.alloc((kernels.delta_rule_grouped_floats(tokens, ctx.num_rows, s.heads, s.key_dim),), torch.float32)
-        kernels.delta_rule_scan(prepared, beta, decays, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,
-                                s.heads, s.kv_heads, s.key_dim, s.value_dim, grouped=grouped)
+        with ctx.temporary():
+            if self.env.dtype == torch.bfloat16 and not ctx.decode_only and s.key_dim <= kernels.DELTA_GROUPED_KEYS:
+                grouped = ctx.alloc((kernels.delta_rule_grouped_floats(tokens, ctx.num_rows, s.heads, s.key_dim),), torch.float32)
+            kernels.delta_rule_scan(prepared, beta, decays, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,
+                                    s.heads, s.kv_heads, s.key_dim, s.value_dim, grouped=grouped)
         mixed = ctx.alloc((tokens, self.v_width), self.env.dtype)
         kernels.gated_head_norm(read, gate, self.norm, mixed, s.heads, s.value_dim, s.norm_eps, s.gate == "sigmoid")
         if overwrite:

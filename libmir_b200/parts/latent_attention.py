@@ -26,6 +26,7 @@ from ..registry import build_part
 from .base import Mixer
 
 PORTION_QUERIES = 48        # queries of a portion for each key of context from which on keys and values are formed for it
+PORTION_SCRATCH = 512 << 20  # the most bytes that may take: 47,000 rows of 16 heads of 192 + 128, 24,800 of 32
 
 
 def _pad8(n: int) -> int:
@@ -167,7 +168,11 @@ class LatentAttention(Mixer):
         starts, before = ctx.host_query_starts, ctx.host_start_positions
         portions = [b - a for a, b in zip(starts, starts[1:])]
         contexts = [n + k for n, k in zip(before, portions)]
-        return min(portions, default=0) > 0 and sum(p * c for p, c in zip(portions, contexts)) >= PORTION_QUERIES * sum(contexts)
+        s = self.spec
+        rows = sum(-(-n // kernels.GATHER_ROWS) for n in contexts) * kernels.GATHER_ROWS
+        scratch = rows * (self.key_width + s.heads * (s.head_dim + s.rotary_dim) + self.out_width) * 2
+        return (min(portions, default=0) > 0 and scratch <= PORTION_SCRATCH
+                and sum(p * c for p, c in zip(portions, contexts)) >= PORTION_QUERIES * sum(contexts))
 
     def _portions(self, ctx, group, cache, packed, gate, table, magnitude, interleaved):
         """The mixer's result before its output projection, for portions of prompts: queries of head_dim + rotary numbers
@@ -195,16 +200,17 @@ class LatentAttention(Mixer):
         contexts = [n + b - a for n, a, b in zip(before, starts, starts[1:])]
         tiles = [-(-n // kernels.GATHER_ROWS) for n in contexts]
         rows = sum(tiles) * kernels.GATHER_ROWS
-        gathered = ctx.alloc((rows, self.key_width), dtype)
-        tile_table = ctx.alloc((len(contexts), max(tiles)), torch.int32)
-        kernels.latent_gather(cache.k_pages, group.block_table, ctx.context_lens, cache.page_size, contexts, gathered, tile_table)
-        keys = ctx.alloc((rows, s.heads * per_head), dtype)
-        kernels.linear(gathered, self.w_keys, keys, alloc=ctx.alloc)
-        values = ctx.alloc((rows, self.out_width), dtype)
-        kernels.linear(gathered[:, :s.kv_rank], self.w_values, values, alloc=ctx.alloc)
         mixed = ctx.alloc((tokens, self.out_width), dtype)
-        kernels.prefill_attention_wide(q, mixed, keys, values, tile_table, ctx.query_starts, ctx.context_lens, s.heads, s.scale,
-                                       gate)
+        with ctx.temporary():
+            gathered = ctx.alloc((rows, self.key_width), dtype)
+            tile_table = ctx.alloc((len(contexts), max(tiles)), torch.int32)
+            kernels.latent_gather(cache.k_pages, group.block_table, ctx.context_lens, cache.page_size, contexts, gathered, tile_table)
+            keys = ctx.alloc((rows, s.heads * per_head), dtype)
+            kernels.linear(gathered, self.w_keys, keys, alloc=ctx.alloc)
+            values = ctx.alloc((rows, self.out_width), dtype)
+            kernels.linear(gathered[:, :s.kv_rank], self.w_values, values, alloc=ctx.alloc)
+            kernels.prefill_attention_wide(q, mixed, keys, values, tile_table, ctx.query_starts, ctx.context_lens, s.heads,
+                                           s.scale, gate)
         return mixed
 
     def attend(self, ctx, group, cache, folded, out):

@@ -101,12 +101,13 @@ class Retention(Mixer):
         view = lambda name, width: packed[:, self.offsets[name]:self.offsets[name] + width]
         read = ctx.alloc((tokens, self.v_width), torch.float32)
         # a step with portions of prompts rotates once per token and head in a kernel of its own
-        prepared = None if ctx.decode_only else ctx.alloc(
-            (kernels.retention_prepared_floats(tokens, s.heads, s.key_dim),), torch.float32)
-        kernels.retention_scan(view("q", self.qk_width), view("k", self.qk_width), view("v", self.v_width),
-                               self.position.table if self.position is not None else None, self.decays,
-                               self.key_scale, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,
-                               s.heads, s.key_dim, s.value_dim, prepared=prepared, activated=s.activated)
+        with ctx.temporary():
+            prepared = None if ctx.decode_only else ctx.alloc(
+                (kernels.retention_prepared_floats(tokens, s.heads, s.key_dim),), torch.float32)
+            kernels.retention_scan(view("q", self.qk_width), view("k", self.qk_width), view("v", self.v_width),
+                                   self.position.table if self.position is not None else None, self.decays,
+                                   self.key_scale, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,
+                                   s.heads, s.key_dim, s.value_dim, prepared=prepared, activated=s.activated)
         mixed = ctx.alloc((tokens, self.v_width), self.env.dtype)
         kernels.gated_head_norm(read, view("g", self.v_width), self.norm, mixed, self.norm_units, self.norm_width,
                                 s.norm_eps, s.gate == "sigmoid")

@@ -101,10 +101,11 @@ class Wkv(Mixer):
         kernels.linear(low, self.w_2, decay_raw, alloc=ctx.alloc)
         read = ctx.alloc((tokens, self.width), torch.float32)
         # a step with portions of prompts forms the decays once per token and head in a kernel of its own
-        prepared = None if ctx.decode_only else ctx.alloc(
-            (kernels.wkv_prepared_floats(tokens, s.heads, s.head_dim),), torch.float32)
-        kernels.wkv_scan(projected[0], projected[1], projected[2], decay_raw, self.decay_bias, self.bonus, state,
-                         ctx.query_starts, ctx.state_slots, ctx.positions, read, s.heads, s.head_dim, prepared=prepared)
+        with ctx.temporary():
+            prepared = None if ctx.decode_only else ctx.alloc(
+                (kernels.wkv_prepared_floats(tokens, s.heads, s.head_dim),), torch.float32)
+            kernels.wkv_scan(projected[0], projected[1], projected[2], decay_raw, self.decay_bias, self.bonus, state,
+                             ctx.query_starts, ctx.state_slots, ctx.positions, read, s.heads, s.head_dim, prepared=prepared)
         mixed = ctx.alloc((tokens, self.width), dtype)
         kernels.gated_head_norm(read, projected[3], self.norm, mixed, s.heads, s.head_dim, s.norm_eps, False)
         if overwrite:

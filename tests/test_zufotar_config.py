@@ -149,3 +149,29 @@ def test_plain_implementation_fixed_points():
     o = torch.tensor([2.0 * 1.0, 2.0 * 3.0])                                 # (r . (u * k)) v = 2 * v
     want = o / torch.sqrt((o * o).mean()) * plain.silu(h[0])
     assert torch.allclose(out[0], want.double())
+
+
+def test_scratch_of_a_with_block_is_given_back():
+    from libmir_b200.engine.context import Arena
+    arena = Arena(torch.device("cpu"), chunk_bytes=4096)
+    arena.alloc((256,), torch.float32)
+    mark = arena.mark()
+    first = arena.alloc((3000,), torch.float32)                   # does not fit: a buffer of its own
+    arena.rewind(mark)
+    kept = arena.alloc((16,), torch.float32)                      # behind the first, as if nothing had been asked for
+    again = arena.alloc((3000,), torch.float32)
+    assert again.data_ptr() == first.data_ptr() and kept.data_ptr() == arena.chunks[0].data_ptr() + 1024
+    assert len(arena.chunks) == 2
+
+
+@pytest.mark.parametrize("portion,before,expected", [(47, 0, False), (48, 0, True), (100, 150, True), (24000, 0, True), (30, 3000, False), (25000, 0, False)])
+def test_when_keys_of_a_portion_are_formed(portion, before, expected):
+    """From 48 queries for each key of context on, and while the keys and values take 512 MB at most."""
+    from types import SimpleNamespace
+    from libmir_b200.parts.latent_attention import LatentAttention
+    part = SimpleNamespace(w_keys=object(), key_width=576, out_width=32 * 128,
+                           spec=SimpleNamespace(heads=32, head_dim=128, rotary_dim=64))
+    ctx = SimpleNamespace(decode_only=False, single_rows=0, host_query_starts=[0, portion], host_start_positions=[before])
+    assert LatentAttention._takes_portions(part, ctx) is expected
+    ctx.decode_only = True
+    assert LatentAttention._takes_portions(part, ctx) is False
