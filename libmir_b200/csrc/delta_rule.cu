@@ -13,6 +13,7 @@
 //   delta_rule_scan   the recurrence: a few lanes per (request, head, value channel) hold one column of S in
 //                     registers, walk over the request's tokens of this step, and write the column back.  The state is
 //                     stored [head][value channel][key channel], so a column is one contiguous run.
+//   delta_rule_group  and the walk over its groups: the recurrence four tokens a step, for prompts of the bfloat16 engine.
 //   gated_head_norm   out = o / rms(o) * weight * act(gate) per (token, head), act = silu or sigmoid.
 // A row of a captured decode batch whose position is negative is padding: nothing of it is read or written.
 #include "common.cuh"
