@@ -13,6 +13,7 @@
 //   delta_rule_scan   the recurrence: a few lanes per (request, head, value channel) hold one column of S in
 //                     registers, walk over the request's tokens of this step, and write the column back.  The state is
 //                     stored [head][value channel][key channel], so a column is one contiguous run.
+//   delta_rule_step   the same for a step of single tokens, with nothing staged.
 //   delta_rule_group  and the walk over its groups: the recurrence four tokens a step, for prompts of the bfloat16 engine.
 //   gated_head_norm   out = o / rms(o) * weight * act(gate) per (token, head), act = silu or sigmoid.
 // A row of a captured decode batch whose position is negative is padding: nothing of it is read or written.
@@ -489,6 +490,81 @@ delta_rule_scan_kernel(const float* __restrict__ qkv, const float* __restrict__ 
   }
   const float read_out = sum_lanes<LANES, C>(pending, l);        // the last token's
   if (writer) *out_at = read_out;
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, wide);
+}
+
+// A step of single tokens: the same operations on every number in the same order as delta_rule_scan_kernel (sixteen lanes a
+// column; C columns a lane, whose number changes no result), but a token's inputs go from global memory to registers and
+// nothing is staged: a step reads and writes the state once and has no next token to fetch for.
+// What bounds it: the bytes of the state.  64 rows of 32 heads of 128 x 128 61 us with a decay per channel (the walk's kernel 108), 49 with
+// one a head (105), 268 MB either way; eight rows of 16 heads 4.9 us (7.6), two rows 3.6 (3.3).
+// blockDim (32, kScanWarps), grid (rows, heads, ceil(value_dim / (kScanWarps * 2 C))).
+template <int PER, int C, bool PER_CHANNEL>
+__global__ void __launch_bounds__(kScanWarps * 32)
+delta_rule_step_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
+                       float* __restrict__ state, const int* __restrict__ query_starts, const int* __restrict__ state_slots,
+                       const int* __restrict__ positions, float* __restrict__ out, int heads, int kv_heads, int key_dim,
+                       int value_dim) {
+  constexpr int LANES = 16, COLUMNS = 32 / LANES * C;            // of a warp
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int lane = threadIdx.x, l = lane % LANES;
+  const int row = blockIdx.x, head = blockIdx.y;
+  const int start = query_starts[row], end = query_starts[row + 1];
+  if (end <= start || positions[start] < 0) return;             // the whole CTA: an empty or padding row
+  const int column = blockIdx.z * (COLUMNS * kScanWarps) + threadIdx.y * COLUMNS + lane / LANES * C;
+  const int width = 2 * kv_heads * key_dim + heads * value_dim, kv_head = head / (heads / kv_heads);
+  const bool wide = key_dim % 4 == 0 && width % 4 == 0;
+  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + column) * key_dim;
+  Pair s[C][PER / 2];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    load_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, column + c < value_dim, wide);
+  const int my_column = lane_sum<C>(l);                          // of the C columns, the one whose read-out this lane writes
+  for (int at = start; at < end; ++at) {                         // (one token, but for steps whose other rows are empty)
+    const float* from = qkv + (size_t)at * width + (size_t)kv_head * key_dim;
+    const float* value_of = qkv + (size_t)at * width + (size_t)2 * kv_heads * key_dim + (size_t)head * value_dim;
+    const float* g_of = decay + ((size_t)at * heads + head) * (PER_CHANNEL ? key_dim : 1);
+    Pair q[PER / 2], k[PER / 2], g[PER_CHANNEL ? PER / 2 : 1];
+    load_column<LANES, PER>(k, from + (size_t)kv_heads * key_dim, l, key_dim, true, wide);
+    if constexpr (PER_CHANNEL) load_column<LANES, PER>(g, g_of, l, key_dim, true, wide);
+    else g[0] = pair_from(*g_of, *g_of);
+    load_column<LANES, PER>(q, from, l, key_dim, true, wide);
+    const float factor = beta[(size_t)at * heads + head];
+    float value[C], total[C], parts[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) value[c] = column + c < value_dim ? value_of[column + c] : 0.0f;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      Pair seen[2] = {0, 0};
+#pragma unroll
+      for (int m = 0; m < PER / 2; ++m) {
+        s[c][m] = pair_mul(s[c][m], g[PER_CHANNEL ? m : 0]);
+        seen[m & 1] = pair_fma(s[c][m], k[m], seen[m & 1]);
+      }
+      total[c] = pair_total(seen);
+    }
+#pragma unroll
+    for (int step = 1; step < LANES; step <<= 1)
+#pragma unroll
+      for (int c = 0; c < C; ++c) total[c] += __shfl_xor_sync(0xffffffffu, total[c], step);
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const float update = factor * (value[c] - total[c]);
+      const Pair both = pair_from(update, update);
+      Pair read[2] = {0, 0};
+#pragma unroll
+      for (int m = 0; m < PER / 2; ++m) {
+        s[c][m] = pair_fma(k[m], both, s[c][m]);
+        read[m & 1] = pair_fma(s[c][m], q[m], read[m & 1]);
+      }
+      parts[c] = pair_total(read);
+    }
+    const float read_out = sum_lanes<LANES, C>(parts, l);
+    if (l < C && column + my_column < value_dim) out[((size_t)at * heads + head) * value_dim + column + my_column] = read_out;
+  }
 #pragma unroll
   for (int c = 0; c < C; ++c)
     if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, wide);
@@ -1000,6 +1076,32 @@ int launch_scan_as(cudaStream_t stream, const float* qkv, const float* beta, con
                     beta, decay, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
 }
 
+template <int PER, int C, bool PER_CHANNEL>
+int launch_step_as(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
+                   const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
+                   int kv_heads, int key_dim, int value_dim) {
+  constexpr int columns = kScanWarps * 2 * C;
+  return mir_launch("delta_rule_step", delta_rule_step_kernel<PER, C, PER_CHANNEL>,
+                    dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps), 0, stream, 0, qkv, beta,
+                    decay, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
+}
+
+template <bool PER_CHANNEL>
+int launch_step(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
+                const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
+                int kv_heads, int key_dim, int value_dim) {
+#define MIR_STEP(P, C)                                                                                               \
+  return launch_step_as<P, C, PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, rows, \
+                                           heads, kv_heads, key_dim, value_dim)
+  // Four columns a lane share a token's inputs; two make twice as many CTAs of a few rows.
+  const bool many = (long long)rows * heads * ((value_dim + 31) / 32) >= 2LL * mir_sm_count();
+  if (key_dim <= 64) { if (many) MIR_STEP(4, 4); MIR_STEP(4, 2); }
+  if (key_dim <= 128) { if (many) MIR_STEP(8, 4); MIR_STEP(8, 2); }
+  if (key_dim <= 192) MIR_STEP(12, 2);
+  MIR_STEP(16, 2);
+#undef MIR_STEP
+}
+
 template <bool PER_CHANNEL>
 int launch_scan(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
                 const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
@@ -1011,8 +1113,10 @@ int launch_scan(cudaStream_t stream, const float* qkv, const float* beta, const 
   // a prompt of 2,048 tokens at 16 / 32 heads of 128 x 128 takes 375 / 520 us with a decay per channel (eight lanes: 476 / 707,
   // thirty-two: 413 / 570; before the fetching warps: 630 / 870) and 345 / 465 with one per head.
   // One choice for every shape of step, so that a request's 32-bit results do not depend on how it was cut.
-  (void)single_tokens;
   const int lanes = g_scan_lanes ? g_scan_lanes : 16;
+  if (single_tokens && lanes == 16 && key_dim <= 256)
+    return launch_step<PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, rows, heads,
+                                    kv_heads, key_dim, value_dim);
   if (lanes == 8) {
     if (key_dim <= 32) { MIR_SCAN(8, 4) }
     if (key_dim <= 64) { MIR_SCAN(8, 8) }

@@ -232,6 +232,45 @@ def test_delta_rule_four_tokens_at_a_time(per_channel, heads, kv_heads, key_dim,
     assert max(errors[0]) <= 1e-5 and all(a <= 1.5 * b + 2e-8 for a, b in zip(*errors)), errors
 
 
+@pytest.mark.parametrize("per_channel", [True, False])
+@pytest.mark.parametrize("rows,heads,kv_heads,key_dim,value_dim", [(2, 2, 1, 128, 128), (40, 16, 8, 128, 40), (3, 3, 3, 30, 5), (70, 12, 12, 64, 9),
+                                                                   (1, 1, 1, 1, 1), (2, 2, 2, 192, 33), (2, 1, 1, 250, 7), (80, 5, 5, 100, 16)])
+def test_single_tokens_are_the_bits_of_a_walk(per_channel, rows, heads, kv_heads, key_dim, value_dim):
+    """A step of single tokens (two and four columns a lane, empty and padding rows) against the same tokens in a step that
+    also brings a portion; slots that no row names stay as they were."""
+    from libmir_b200 import kernels
+    torch.manual_seed(rows + key_dim)
+    tokens = rows + 2
+    qkv = torch.randn(tokens, 2 * kv_heads * key_dim + heads * value_dim, device="cuda") * 0.3
+    beta = torch.rand(tokens, heads, device="cuda")
+    decay = torch.rand(tokens, heads * key_dim if per_channel else heads, device="cuda")
+    state = torch.randn(rows + 3, heads, value_dim, key_dim, device="cuda")
+    slots = torch.randperm(rows + 3, device="cuda")[:rows + 1].int()
+    starts = torch.arange(rows + 2, dtype=torch.int32, device="cuda")
+    starts[-1] = tokens                                           # the last row of the longer step brings two tokens
+    positions = torch.ones(tokens, dtype=torch.int32, device="cuda")
+    if rows > 2:
+        positions[1] = -1                                         # padding
+    walked, stepped = state.clone(), state.clone()
+    want, got = (torch.full((n, heads * value_dim), float("nan"), device="cuda") for n in (tokens, rows))
+    kernels.delta_rule_scan(qkv, beta, decay, walked, starts, slots, positions, want, heads, kv_heads, key_dim, value_dim)
+    before = kernels.launch_counts().get("delta_rule_step", 0)
+    kernels.delta_rule_scan(qkv[:rows], beta[:rows], decay[:rows], stepped, starts[:rows + 1], slots[:rows], positions[:rows],
+                            got, heads, kv_heads, key_dim, value_dim)
+    assert kernels.launch_counts()["delta_rule_step"] == before + 1
+    walked[slots[-1].long()] = state[slots[-1].long()]
+    assert torch.equal(torch.nan_to_num(got, 7.0), torch.nan_to_num(want[:rows], 7.0)) and torch.equal(stepped, walked)
+    # as many tokens as rows, but two of them in one row
+    if rows > 2:
+        positions[:], starts[1] = 1, 2
+        walked, stepped = state.clone(), state.clone()
+        kernels.delta_rule_scan(qkv, beta, decay, walked, starts, slots, positions, want, heads, kv_heads, key_dim, value_dim)
+        kernels.delta_rule_scan(qkv[:rows], beta[:rows], decay[:rows], stepped, starts[:rows + 1], slots[:rows],
+                                positions[:rows], got, heads, kv_heads, key_dim, value_dim)
+        walked[slots[-1].long()] = state[slots[-1].long()]
+        assert torch.equal(got, want[:rows]) and torch.equal(stepped, walked)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("taps,key_dim,value_dim,per_channel", [(4, 128, 64, True), (2, 100, 24, False), (1, 64, 128, True), (3, 4, 200, False)])
 def test_what_the_recurrence_needs_is_the_same_in_long_steps_and_short_ones(dtype, taps, key_dim, value_dim, per_channel):
