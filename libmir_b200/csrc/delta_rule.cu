@@ -199,14 +199,27 @@ delta_rule_prepare_run_kernel(const T* __restrict__ x, long long ldx, const T* _
         rate[e] = j < decay_width ? -expf(a_log[j / per_head]) : 0.0f;
         bias[e] = j < decay_width ? dt_bias[j] : 0.0f;
       }
-#pragma unroll 2
-      for (int t = first; t < last; ++t) {
-        if (positions[t] < 0) continue;
+      const int my_position = positions[min(first + lane, last - 1)];
+      constexpr int AHEAD = RUN < 4 ? RUN : 4;                   // tokens whose inputs are asked for together
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = unit * 128 + lane + 32 * e;
-          if (j < decay_width)
-            decay[(size_t)t * decay_width + j] = expf(rate[e] * softplus(to_float(decay_raw[(size_t)t * ld_decay + j]) + bias[e]));
+      for (int i = 0; i < RUN; i += AHEAD) {
+        float raw[AHEAD][4];
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int j = unit * 128 + lane + 32 * e;
+            raw[a][e] = first + i + a < last && j < decay_width ? to_float(decay_raw[(size_t)(first + i + a) * ld_decay + j]) : 0.0f;
+          }
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+          const int t = first + i + a;
+          if (__shfl_sync(0xffffffffu, my_position, i + a) < 0 || t >= last) continue;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int j = unit * 128 + lane + 32 * e;
+            if (j < decay_width) decay[(size_t)t * decay_width + j] = expf(rate[e] * softplus(raw[a][e] + bias[e]));
+          }
         }
       }
     } else if (unit == decay_units) {                            // the writes' factors
@@ -1218,7 +1231,9 @@ MIR_EXPORT int mir_delta_rule_prepare(int bf16, int decay_f32, const void* x, lo
                     (uintptr_t)x % (4 * element) == 0 && ((uintptr_t)qkv | (uintptr_t)tail) % 16 == 0;
   const int units = 2 * kv_heads + (values + 127) / 128 + (decay_width + 127) / 128 + 1;
   // eight tokens a warp (sixteen: 59 us where eight take 38) once that still makes several warps for every SM's schedulers
-  const bool long_runs = (long long)tokens * units >= 8LL * 16 * mir_sm_count();
+  // - but single tokens have no neighbour to share inputs with, and eight of them behind one another in a warp wait for eight
+  // tails (200 rows of 32 heads of 64, decays per channel: 23 us)
+  const bool long_runs = tokens != rows && (long long)tokens * units >= 8LL * 16 * mir_sm_count();
 #define MIR_PREPARE_RUN(T, TD, RUN)                                                                                    \
   status = mir_launch("delta_rule_prepare", delta_rule_prepare_run_kernel<T, TD, RUN>,                                 \
                       dim3((tokens + RUN - 1) / RUN, (units + kRunWarps - 1) / kRunWarps), dim3(32, kRunWarps), 0,     \

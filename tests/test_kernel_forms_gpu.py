@@ -1,0 +1,50 @@
+"""Kernels that have several forms, one of which is taken by the sizes of the call: both sides of every rule against plain torch
+in 64 bits, exactly where the numbers are whole or only moved."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def ints(values):
+    return torch.as_tensor(values, dtype=torch.int32).to("cuda")
+
+
+def batch(counts, slots=None):
+    """(row_of_token, query_starts, state_slots, positions) of portions that start their requests."""
+    counts = list(counts)
+    starts = np.concatenate([[0], np.cumsum(counts)])
+    return (ints(np.repeat(np.arange(len(counts)), counts)), ints(starts), ints(range(len(counts)) if slots is None else slots),
+            ints(np.concatenate([np.arange(n) for n in counts])))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim,rows", [(32, 64, 210), (16, 128, 230), (5, 20, 7)])
+def test_what_the_delta_rule_needs_of_many_single_tokens(dtype, heads, dim, rows):
+    """A step of many decoded tokens (one token a warp, however many there are) against the same tokens a few at a time and in a
+    step that also brings a portion (eight tokens a warp): the same bits, and the same inputs kept."""
+    from libmir_b200 import kernels
+    torch.manual_seed(rows)
+    width, decays = 3 * heads * dim, heads * dim
+    make = lambda *shape: torch.randn(*shape, device="cuda")
+    tokens = rows + 2500
+    x, weight, beta_raw = make(tokens, width).to(dtype), make(width, 4).to(dtype), make(tokens, heads).to(dtype)
+    decay_raw, bias, a_log = make(tokens, decays).to(dtype), make(decays), make(heads)
+    tail0 = make(rows + 1, 3, width)
+
+    def prepare(first, counts, slots, tail):
+        n = sum(counts)
+        row_of, starts, slots, positions = batch(counts, slots)
+        made = [torch.full((n, w), float("nan"), device="cuda") for w in (width, heads, decays)]
+        kernels.delta_rule_prepare(x[first:first + n], weight, tail, beta_raw[first:first + n], decay_raw[first:first + n], bias, a_log,
+                                   row_of, starts, slots, positions, *made, heads, heads, dim, dim)
+        return made
+    tails = [tail0.clone() for _ in range(3)]
+    whole = prepare(0, [1] * rows, range(rows), tails[0])
+    pieces = [prepare(first, [1] * min(3, rows - first), range(first, min(first + 3, rows)), tails[1]) for first in range(0, rows, 3)]
+    beside = prepare(0, [1] * rows + [2500], range(rows + 1), tails[2])
+    for got, parts, other in zip(whole, zip(*pieces), beside):
+        assert bool(torch.isfinite(got).all()) and torch.equal(got, torch.cat(parts)) and torch.equal(got, other[:rows])
+    assert torch.equal(tails[0], tails[1]) and torch.equal(tails[0][:rows], tails[2][:rows])
