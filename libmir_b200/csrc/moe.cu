@@ -30,10 +30,16 @@ __device__ __forceinline__ float sigmoid_of(float z) { return 1.0f / (1.0f + exp
 
 // One warp per token, four tokens a CTA.  logits [tokens, >= experts (+ 1)] 32-bit: the router's logits and, behind
 // them, the shared expert's gate logit (has_gate).  Shared memory per warp: score[E] | choice[E] | group score[groups] |
-// the chosen scores[top].
+// the chosen scores[top] (RANKED).
 // Among equal scores the expert (or group) with the lower index wins.
 constexpr int kRouteWarps = 4;
-constexpr int kRankedExperts = 256;   // up to so many are ranked by counting; more are searched, slot by slot
+// Whether a token's experts are ranked by counting, every expert against every other (a lane's own ones at a time), or searched
+// for slot by slot.  The first takes experts / 32 rounds of `experts` comparisons, a slot of the second about as long as 32 of
+// them: three tokens, 64 experts 4.1 us ranked and 2.8 / 3.4 / 5.3 / 6.3 searched for 1 / 2 / 6 / 8 slots, 32 experts 2.7 and 2.7 to
+// 5.7.  More than 64 are never ranked: 2,000 tokens, 96 experts 9.7 us ranked and 5.2 to 7.9 searched, 256 experts 47 and 6.7 to 9.3.
+__host__ __device__ constexpr bool route_by_rank(int experts, int top) {
+  return experts <= 64 && (experts + 31) / 32 * experts <= 32 * top;
+}
 
 __device__ __forceinline__ void warp_best(float& value, int& index, bool want_max) {
 #pragma unroll
@@ -46,6 +52,7 @@ __device__ __forceinline__ void warp_best(float& value, int& index, bool want_ma
   }
 }
 
+template <bool RANKED>
 __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ correction,
                                  int has_gate, int* __restrict__ ids, float* __restrict__ weights,
                                  float* __restrict__ shared_gate, int tokens, int experts, int top, int groups, int keep,
@@ -56,7 +63,7 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int token = blockIdx.x * kRouteWarps + warp;
   if (token >= tokens) return;
-  float* score = route_shared + (size_t)warp * (2 * experts + groups + (experts <= kRankedExperts ? top : 0));
+  float* score = route_shared + (size_t)warp * (2 * experts + groups + (RANKED ? top : 0));
   float* choice = score + experts;
   float* group_score = choice + experts;
   float* chosen = group_score + groups;
@@ -119,7 +126,7 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
     }
   }
   float total = 0.0f;
-  if (experts <= kRankedExperts) {
+  if constexpr (RANKED) {
     // An expert's rank among those that can be chosen is its slot: every lane counts for its own experts at once, instead
     // of one search over the warp for each slot (three tokens, 64 experts in 8 groups, 6 chosen: 9.2 us by searches).
     int choosable = 0;
@@ -146,28 +153,28 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
     for (int slot = 0; slot < top; ++slot) total += chosen[slot];
     const float factor = scale / (total + 1e-20f);
     for (int slot = lane; slot < top; slot += 32) weights[(size_t)token * top + slot] = chosen[slot] * factor;
-    return;
-  }
-  for (int slot = 0; slot < top; ++slot) {
-    float high = -FLT_MAX;
-    int best = -1;
-    for (int e = lane; e < experts; e += 32) {
-      const float c = choice[e];
-      if (c > high) { high = c; best = e; }
+  } else {
+    for (int slot = 0; slot < top; ++slot) {
+      float high = -FLT_MAX;
+      int best = -1;
+      for (int e = lane; e < experts; e += 32) {
+        const float c = choice[e];
+        if (c > high) { high = c; best = e; }
+      }
+      if (best >= 0 && high == -FLT_MAX) best = -1;
+      warp_best(high, best, true);
+      if (best < 0) best = 0;                                      // (fewer choosable experts than top: not a valid model)
+      if (lane == 0) {
+        choice[best] = -FLT_MAX;
+        ids[(size_t)token * top + slot] = best;
+        weights[(size_t)token * top + slot] = score[best];
+      }
+      total += score[best];
+      __syncwarp();
     }
-    if (best >= 0 && high == -FLT_MAX) best = -1;
-    warp_best(high, best, true);
-    if (best < 0) best = 0;                                      // (fewer choosable experts than top: not a valid model)
-    if (lane == 0) {
-      choice[best] = -FLT_MAX;
-      ids[(size_t)token * top + slot] = best;
-      weights[(size_t)token * top + slot] = score[best];
-    }
-    total += score[best];
-    __syncwarp();
+    const float factor = scale / (total + 1e-20f);
+    for (int slot = lane; slot < top; slot += 32) weights[(size_t)token * top + slot] *= factor;
   }
-  const float factor = scale / (total + 1e-20f);
-  for (int slot = lane; slot < top; slot += 32) weights[(size_t)token * top + slot] *= factor;
 }
 
 // The pairs ordered by expert, in three small kernels.  order[i] = the i-th pair when the pairs are sorted by expert
@@ -491,10 +498,12 @@ MIR_EXPORT int mir_moe_route(const float* logits, long long ld, const float* cor
                   top, groups, keep);
     return MIR_BAD_ARGUMENT;
   }
-  const size_t smem = (size_t)kRouteWarps * (2 * experts + groups + (experts <= kRankedExperts ? top : 0)) * sizeof(float);
-  return mir_launch("moe_route", moe_route_kernel, dim3((tokens + kRouteWarps - 1) / kRouteWarps), dim3(32, kRouteWarps),
-                    smem, stream, 0, logits, ld, correction, has_gate, ids, weights, shared_gate, tokens, experts, top,
-                    groups, keep, scale, softmax_scores, group_by_max);
+  const bool ranked = route_by_rank(experts, top);
+  const size_t smem = (size_t)kRouteWarps * (2 * experts + groups + (ranked ? top : 0)) * sizeof(float);
+  return mir_launch("moe_route", ranked ? moe_route_kernel<true> : moe_route_kernel<false>,
+                    dim3((tokens + kRouteWarps - 1) / kRouteWarps), dim3(32, kRouteWarps), smem, stream, 0, logits, ld,
+                    correction, has_gate, ids, weights, shared_gate, tokens, experts, top, groups, keep, scale,
+                    softmax_scores, group_by_max);
 }
 
 // How many tiles of tile_pairs pairs there can be at most for `pairs` pairs over `experts` experts (`tiles` holds two

@@ -48,3 +48,34 @@ def test_what_the_delta_rule_needs_of_many_single_tokens(dtype, heads, dim, rows
     for got, parts, other in zip(whole, zip(*pieces), beside):
         assert bool(torch.isfinite(got).all()) and torch.equal(got, torch.cat(parts)) and torch.equal(got, other[:rows])
     assert torch.equal(tails[0], tails[1]) and torch.equal(tails[0][:rows], tails[2][:rows])
+
+
+@pytest.mark.parametrize("groups,keep", [(1, 1), (4, 2), (36, 5)])
+@pytest.mark.parametrize("top", [1, 2, 4, 6, 8])
+@pytest.mark.parametrize("experts", [8, 32, 36, 64, 72, 96, 128, 200, 256, 288])
+def test_experts_that_are_ranked_and_experts_that_are_searched(experts, top, groups, keep):
+    """Scores with many equal ones (the lower expert comes first), masked experts among them; whole numbers are exact."""
+    from libmir_b200 import kernels
+    if experts % groups or top > keep * (experts // groups) - experts // 16:
+        pytest.skip("no such router")
+    generator = torch.Generator().manual_seed(experts + top)
+    tokens = 9
+    logits = (torch.randint(-3, 4, (tokens, experts + 1), generator=generator) * 0.5).float()
+    logits[:, :experts][torch.rand(tokens, experts, generator=generator) < 1 / 32] = -float("inf")
+    ids, weights = torch.full((tokens, top), -1, dtype=torch.int32, device="cuda"), torch.empty(tokens, top, device="cuda")
+    gate = torch.empty(tokens, device="cuda")
+    kernels.moe_route(logits.cuda(), None, True, ids, weights, gate, experts, top, groups, keep, 1.5)
+    score = torch.sigmoid(logits[:, :experts].double())
+    for t in range(tokens):
+        choice = score[t].clone()
+        if keep < groups:
+            per = choice.view(groups, -1)
+            best = per.topk(min(2, per.shape[1]), dim=1).values.sum(1)
+            kept = sorted(range(groups), key=lambda g: (-float(best[g].float()), g))[:keep]
+            dropped = [g for g in range(groups) if g not in kept]
+            choice.view(groups, -1)[dropped] = -1.0
+        want = sorted(range(experts), key=lambda e: (-float(choice[e].float()), e))[:top]
+        assert ids[t].tolist() == want, (t, ids[t].tolist(), want)
+        chosen = score[t][want]
+        assert torch.allclose(weights[t].double().cpu(), chosen / chosen.sum() * 1.5, rtol=1e-5)
+    assert torch.allclose(gate.double().cpu(), torch.sigmoid(logits[:, experts].double()), rtol=1e-5)
