@@ -180,12 +180,11 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
 // The pairs ordered by expert, in three small kernels.  order[i] = the i-th pair when the pairs are sorted by expert
 // (pairs of one expert stay in their own order); offsets[e] .. offsets[e + 1] is expert e's range in it; tiles[2 n],
 // tiles[2 n + 1] = expert and first sorted pair of the n-th tile of tile_pairs pairs, tile_count[0] = how many there are.
-constexpr int kSortThreads = 1024;
 
 // All of the sort in one CTA, for the pairs of decoded tokens (up to kFewPairs): three launches' work in one
-// (18 pairs of 64 experts 3.0 us, the three 6).  A pair's place is counted over the pairs before it, which is why more go to
-// the kernels below.
-constexpr int kFewPairs = 512;
+// (18 pairs of 64 experts 3.0 us, the three 5.5; 256 pairs 4.8 and 5.3).  A pair's place is counted over the pairs before it,
+// which is why more go to the kernels below (384 pairs 5.9 us and 6.3; 510 pairs 7.1 and 6.3).
+constexpr int kFewPairs = 416;
 __global__ void __launch_bounds__(kMaxExperts)
 moe_sort_few_kernel(const int* __restrict__ ids, int pairs, int experts, int tile_pairs, int* __restrict__ order,
                     int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ tile_count) {
@@ -233,14 +232,15 @@ moe_sort_few_kernel(const int* __restrict__ ids, int pairs, int experts, int til
 }
 
 // One CTA per expert: how many pairs chose it.  (A prompt's 15,000 pairs are a few trips over the L2 for 1,024 threads.)
-__global__ void __launch_bounds__(kSortThreads) moe_count_kernel(const int* __restrict__ ids, int pairs, int* __restrict__ counts) {
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) moe_count_kernel(const int* __restrict__ ids, int pairs, int* __restrict__ counts) {
   __shared__ float scratch[32];
   grid_launch_dependents();
   grid_dependency_wait();
   const int expert = blockIdx.x;
   int n = 0;
 #pragma unroll 4
-  for (int p = threadIdx.x; p < pairs; p += kSortThreads) n += ids[p] == expert;
+  for (int p = threadIdx.x; p < pairs; p += THREADS) n += ids[p] == expert;
   const float total = block_sum((float)n, scratch);              // (exact: fewer than 2^24 pairs)
   if (threadIdx.x == 0) counts[expert] = (int)(total + 0.5f);
 }
@@ -288,10 +288,11 @@ __global__ void moe_offsets_kernel(const int* __restrict__ counts, int experts, 
 
 // One CTA per expert: its pairs into their places, in their own order, and its tiles.  A warp counts a run of the pairs, and
 // behind one barrier places them (15,000 pairs, 64 experts: 19.5 us when every 256 pairs met at two barriers).
-__global__ void __launch_bounds__(kSortThreads)
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS)
 moe_place_kernel(const int* __restrict__ ids, int pairs, int tile_pairs, const int* __restrict__ offsets,
                  const int* __restrict__ first_tile, int* __restrict__ order, int* __restrict__ tiles) {
-  constexpr int WARPS = kSortThreads / 32;
+  constexpr int WARPS = THREADS / 32;
   __shared__ int warp_counts[WARPS];
   grid_launch_dependents();
   grid_dependency_wait();
@@ -299,7 +300,7 @@ moe_place_kernel(const int* __restrict__ ids, int pairs, int tile_pairs, const i
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int begin = offsets[expert], total = offsets[expert + 1] - begin;
   const int n = (total + tile_pairs - 1) / tile_pairs;
-  for (int t = threadIdx.x; t < n; t += kSortThreads) {
+  for (int t = threadIdx.x; t < n; t += THREADS) {
     tiles[2 * (first_tile[expert] + t)] = expert;
     tiles[2 * (first_tile[expert] + t) + 1] = begin + t * tile_pairs;
   }
@@ -523,12 +524,17 @@ MIR_EXPORT int mir_moe_sort(const int* ids, int pairs, int experts, int tile_pai
   if (pairs <= kFewPairs)
     return mir_launch("moe_sort_few", moe_sort_few_kernel, dim3(1), dim3(kMaxExperts), 0, stream, 0, ids, pairs, experts,
                       tile_pairs, order, offsets, tiles, tile_count);
-  int status = mir_launch("moe_count", moe_count_kernel, dim3(experts), dim3(kSortThreads), 0, stream, 0, ids, pairs, counts);
+  // 1,024 threads an expert, but 256 where more CTAs of that size than an SM each holds have few pairs to go over: 768 pairs of
+  // 300 experts 6.8 us (1,024 threads: 7.9), 1,536 of 300 7.8 (8.7), 4,096 of 300 10.0 (9.1); 768 of 200 6.8 (7.0), 1,536 of
+  // 200 the same, 4,096 of 200 10.0 (7.8); 768 of 64 6.5 (6.3).
+  const int sms = mir_sm_count();
+  const bool many = experts <= sms || pairs >= (experts <= 2 * sms ? 1024 : 4096);
+  int status = mir_launch("moe_count", many ? moe_count_kernel<1024> : moe_count_kernel<256>, dim3(experts), dim3(many ? 1024 : 256), 0, stream, 0, ids, pairs, counts);
   if (status != MIR_OK) return status;
   status = mir_launch("moe_offsets", moe_offsets_kernel, dim3(1), dim3(kMaxExperts), 0, stream, 0, counts, experts,
                       tile_pairs, offsets, first_tile, tile_count);
   if (status != MIR_OK) return status;
-  return mir_launch("moe_place", moe_place_kernel, dim3(experts), dim3(kSortThreads), 0, stream, 0, ids, pairs, tile_pairs,
+  return mir_launch("moe_place", many ? moe_place_kernel<1024> : moe_place_kernel<256>, dim3(experts), dim3(many ? 1024 : 256), 0, stream, 0, ids, pairs, tile_pairs,
                     offsets, first_tile, order, tiles);
 }
 

@@ -79,3 +79,22 @@ def test_experts_that_are_ranked_and_experts_that_are_searched(experts, top, gro
         chosen = score[t][want]
         assert torch.allclose(weights[t].double().cpu(), chosen / chosen.sum() * 1.5, rtol=1e-5)
     assert torch.allclose(gate.double().cpu(), torch.sigmoid(logits[:, experts].double()), rtol=1e-5)
+
+
+@pytest.mark.parametrize("pairs,experts", [(416, 64), (417, 64), (1023, 200), (1024, 200), (1023, 300), (4095, 300), (4096, 300),
+                                           (700, 1024), (20000, 1), (3001, 3), (900, 148), (900, 149), (17, 1024)])
+def test_pairs_by_expert_on_both_sides_of_the_rules(pairs, experts):
+    """One CTA (416 pairs at most), 256 and 1,024 threads an expert; every ninth pair is in no list; more than 1,024 tiles of one expert."""
+    from libmir_b200 import kernels
+    generator = torch.Generator().manual_seed(pairs)
+    ids = torch.randint(0, experts, (pairs,), generator=generator)
+    ids[8::9] = experts + 1
+    alloc = lambda shape, kind: torch.full(shape, -7, dtype=kind, device="cuda")
+    found = kernels.moe_sort(ids.view(pairs, 1).int().cuda(), experts, alloc, 8)
+    held = ids < experts
+    want = torch.argsort(torch.where(held, ids, experts), stable=True)[:int(held.sum())].tolist()
+    counts = torch.bincount(ids[held], minlength=experts).tolist()
+    offsets = np.concatenate([[0], np.cumsum(counts)]).tolist()
+    tiles = [[e, offsets[e] + first] for e in range(experts) for first in range(0, counts[e], 8)]
+    assert found.order.cpu().tolist()[:len(want)] == want and found.offsets.cpu().tolist() == offsets
+    assert int(found.tile_count.cpu()) == len(tiles) and found.tiles.cpu().view(-1, 2).tolist()[:len(tiles)] == tiles
