@@ -107,22 +107,25 @@ __global__ void paged_attention_generic_kernel(
     for (int i = 0; i < PIECES; ++i) acc[i] *= correction;
     const int keys_here = min(32, last - base + 1);
     // Several keys' values are asked for before the first is used: with one warp a query and head the loop is otherwise bound
-    // by the latency of a load per key (a decoded token at 136 keys 63 us; eight at a time 37, sixteen and twice as many pieces of the keys 29).  The sum still goes key by key.
-    constexpr int RUN = PIECES <= 4 ? 16 : 1;
+    // by the latency of a load per key (a decoded token at 136 keys 63 us; eight keys at a time 37, sixteen 29).  They are
+    // kept as they are stored until all have been asked for: a conversion beside its load waits for it (64 tokens at 1,000
+    // keys, 16 heads of 256 bfloat16: 1.9 ms).  The sum goes key by key.
+    constexpr int RUN = PIECES <= 4 ? 16 : 2;
     int j = 0;
     for (; j + RUN <= keys_here; j += RUN) {
-      float values[RUN][PIECES], w[RUN];
+      T values[RUN][PIECES];
+      float w[RUN];
 #pragma unroll
       for (int r = 0; r < RUN; ++r) {
         w[r] = __shfl_sync(0xffffffffu, weight, j + r);
         const T* v_row = v_pages + __shfl_sync(0xffffffffu, key_offset, j + r) * value_row_width;
 #pragma unroll
-        for (int i = 0; i < PIECES; ++i) values[r][i] = lane + 32 * i < value_dim ? to_float(v_row[lane + 32 * i]) : 0.0f;
+        for (int i = 0; i < PIECES; ++i) values[r][i] = lane + 32 * i < value_dim ? v_row[lane + 32 * i] : from_float<T>(0.0f);
       }
 #pragma unroll
       for (int r = 0; r < RUN; ++r)
 #pragma unroll
-        for (int i = 0; i < PIECES; ++i) acc[i] = fmaf(w[r], values[r][i], acc[i]);
+        for (int i = 0; i < PIECES; ++i) acc[i] = fmaf(w[r], to_float(values[r][i]), acc[i]);
     }
     for (; j < keys_here; ++j) {
       const float w = __shfl_sync(0xffffffffu, weight, j);

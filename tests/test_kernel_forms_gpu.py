@@ -98,3 +98,37 @@ def test_pairs_by_expert_on_both_sides_of_the_rules(pairs, experts):
     tiles = [[e, offsets[e] + first] for e in range(experts) for first in range(0, counts[e], 8)]
     assert found.order.cpu().tolist()[:len(want)] == want and found.offsets.cpu().tolist() == offsets
     assert int(found.tile_count.cpu()) == len(tiles) and found.tiles.cpu().view(-1, 2).tolist()[:len(tiles)] == tiles
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.bfloat16, 1e-2)])
+@pytest.mark.parametrize("dim,value_dim", [(64, 128), (64, 129), (192, 192), (256, 250), (576, 640), (24, 320)])
+def test_reference_attention_of_every_value_width(dtype, tol, dim, value_dim):
+    """Value heads that a lane holds in four places or in twenty; keys that fill no run of them."""
+    from libmir_b200 import kernels
+    generator = torch.Generator().manual_seed(value_dim)
+    lengths, heads, kv_heads, page = [1, 2, 17, 33, 71], 4, 2, 8
+    pages = [-(-n // page) for n in lengths]
+    order = torch.randperm(sum(pages) + 1, generator=generator).tolist()
+    k_pool = torch.full(((sum(pages) + 1) * page, kv_heads, dim), 50.0, dtype=dtype)
+    v_pool = torch.full(((sum(pages) + 1) * page, kv_heads, value_dim), float("nan"), dtype=dtype)
+    table = torch.full((len(lengths), max(pages)), -1, dtype=torch.int32)
+    q = (torch.randn(len(lengths), heads, dim, generator=generator)).to(dtype)
+    want, cursor = [], 0
+    for r, n in enumerate(lengths):
+        k = (torch.randn(n, kv_heads, dim, generator=generator) * 0.3).to(dtype)
+        v = torch.randn(n, kv_heads, value_dim, generator=generator).to(dtype)
+        for block in range(pages[r]):
+            at = order[cursor] * page
+            cursor += 1
+            piece = slice(block * page, min((block + 1) * page, n))
+            k_pool[at:at + piece.stop - piece.start], v_pool[at:at + piece.stop - piece.start] = k[piece], v[piece]
+            table[r, block] = at // page
+        for h in range(heads):
+            weights = torch.softmax(q[r, h].double() @ k[:, h // 2].double().T * 0.2, -1)
+            want.append(weights @ v[:, h // 2].double())
+    out = torch.full((len(lengths), heads * value_dim), float("nan"), dtype=dtype, device="cuda")
+    kernels.paged_attention_generic(q.flatten(1).cuda(), out, k_pool.cuda(), v_pool.cuda(), table.cuda(), ints(range(len(lengths))),
+                                    ints([n - 1 for n in lengths]), page, heads, kv_heads, dim, 0.2, None, value_dim=value_dim)
+    want = torch.stack(want).view(len(lengths), -1)
+    error = (out.double().cpu() - want).abs().max()
+    assert float(error) <= tol * float(want.abs().max()), float(error)
