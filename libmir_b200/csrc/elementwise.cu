@@ -320,13 +320,39 @@ __global__ void rms_norm_kernel(const float* __restrict__ x, const float* __rest
   for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = from_float<Tout>(src[c] * inverse * weight[c]);
 }
 
-// The same with 16-byte accesses (hidden a multiple of 4) and the row in registers; with PAIR a second norm of the same rows,
-// out_b = x * s * weight_b with the same s.  The weights are asked for before the wait for the kernel before.
-template <typename Tout, bool PAIR, int PIECES>
-__global__ void __launch_bounds__(kRowThreads) rms_norm_vec4_kernel(const float* __restrict__ x, const float* __restrict__ weight,
-                                                                    const float* __restrict__ weight_b, Tout* __restrict__ out,
-                                                                    Tout* __restrict__ out_b, const int* __restrict__ rows,
-                                                                    int hidden, float eps) {
+// The same with 16-byte loads (hidden a multiple of 4), for rows wider than the registers of a CTA take: the second pass finds
+// the row in L1 (2,000 rows of 20,480: 54 us, column by column 119).
+template <typename Tout>
+__global__ void rms_norm_vec4_kernel(const float* __restrict__ x, const float* __restrict__ weight,
+                                     Tout* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
+  __shared__ float scratch[32];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int row = blockIdx.x;
+  const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[row] : row) * hidden);
+  const float4* w4 = reinterpret_cast<const float4*>(weight);
+  const int quads = hidden >> 2;
+  float sum = 0.0f;
+  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
+    const float4 v = src[c];
+    sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sum))));
+  }
+  sum = block_sum(sum, scratch);
+  const float inverse = rsqrtf(sum / (float)hidden + eps);
+  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
+    const float4 v = src[c], w = __ldg(w4 + c);
+    store_rounded(out + (size_t)row * hidden, c,
+                  make_float4(v.x * inverse * w.x, v.y * inverse * w.y, v.z * inverse * w.z, v.w * inverse * w.w));
+  }
+}
+
+// The same with the row in registers, read once, and the weights (EARLY) asked for with it; with PAIR a second norm of the same
+// rows, out_b = x * s * weight_b with the same s.
+template <typename Tout, bool PAIR, int PIECES, int THREADS, bool EARLY = true>
+__global__ void __launch_bounds__(THREADS) rms_norm_row_kernel(const float* __restrict__ x, const float* __restrict__ weight,
+                                                               const float* __restrict__ weight_b, Tout* __restrict__ out,
+                                                               Tout* __restrict__ out_b, const int* __restrict__ rows,
+                                                               int hidden, float eps) {
   __shared__ float scratch[32];
   grid_launch_dependents();
   const int quads = hidden >> 2;
@@ -335,7 +361,7 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_vec4_kernel(const float*
 #pragma unroll
   for (int p = 0; p < PIECES; ++p) {
     const int c = p * blockDim.x + threadIdx.x;
-    if (c >= quads) continue;
+    if (!EARLY || c >= quads) continue;
     w[p] = __ldg(reinterpret_cast<const float4*>(weight) + c);
     if (PAIR) second[p] = __ldg(reinterpret_cast<const float4*>(weight_b) + c);
   }
@@ -358,6 +384,7 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_vec4_kernel(const float*
   for (int p = 0; p < PIECES; ++p) {
     const int c = p * blockDim.x + threadIdx.x;
     if (c >= quads) continue;
+    if (!EARLY) w[p] = __ldg(reinterpret_cast<const float4*>(weight) + c);
     const float4 n = make_float4(v[p].x * inverse, v[p].y * inverse, v[p].z * inverse, v[p].w * inverse);
     store_rounded(out + (size_t)row * hidden, c, make_float4(n.x * w[p].x, n.y * w[p].y, n.z * w[p].z, n.w * w[p].w));
     if (PAIR)
@@ -365,14 +392,37 @@ __global__ void __launch_bounds__(kRowThreads) rms_norm_vec4_kernel(const float*
                     make_float4(n.x * second[p].x, n.y * second[p].y, n.z * second[p].z, n.w * second[p].w));
   }
 }
-constexpr int kRowLimit = 8 * 4 * kRowThreads;                   // the widest row that the register form takes
-template <typename Tout, bool PAIR>
-int launch_rms_norm(const float* x, const float* weight, const float* weight_b, Tout* out, Tout* out_b, const int* rows,
-                    int n_rows, int hidden, float eps, cudaStream_t stream) {
+// 256 threads a row (128 below 1,024 columns): more are no faster (2,000 rows of 8,192 15 us, with 512 threads 18; two rows the
+// same), and the order of the sum is one for rows in registers and rows that are read twice.  The weights are asked for with a
+// row of up to 5,120, and with a wider one where no SM has a second row (two rows of 8,192: 2.5 us, 3.1 behind the sum; 2,000 rows
+// 17 and 15).
+template <typename Tout>
+int launch_rms_norm(const float* x, const float* weight, Tout* out, const int* rows, int n_rows, int hidden, float eps,
+                    cudaStream_t stream) {
+  const int threads = hidden >= 1024 ? 256 : 128, pieces = ((hidden >> 2) + threads - 1) / threads;
+#define MIR_RMS(P)                                                                                                        \
+  return mir_launch("rms_norm", P <= 5 || n_rows <= mir_sm_count() ? rms_norm_row_kernel<Tout, false, P, 256, true> \
+                                                                   : rms_norm_row_kernel<Tout, false, P, 256, P <= 5>, dim3(n_rows), dim3(threads), 0, stream, 0, x,  \
+                    weight, nullptr, out, nullptr, rows, hidden, eps)
+  if (pieces == 1) MIR_RMS(1);
+  if (pieces == 2) MIR_RMS(2);
+  if (pieces == 3) MIR_RMS(3);
+  if (pieces == 4) MIR_RMS(4);
+  if (pieces == 5) MIR_RMS(5);
+  if (pieces <= 8) MIR_RMS(8);
+  if (pieces <= 16) MIR_RMS(16);
+#undef MIR_RMS
+  return mir_launch("rms_norm", rms_norm_vec4_kernel<Tout>, dim3(n_rows), dim3(threads), 0, stream, 0, x, weight, out, rows,
+                    hidden, eps);
+}
+constexpr int kPairLimit = 8 * 4 * kRowThreads;                  // the widest row that the register form of the pair takes
+template <typename Tout>
+int launch_rms_norm_pair(const float* x, const float* weight, const float* weight_b, Tout* out, Tout* out_b, int n_rows,
+                         int hidden, float eps, cudaStream_t stream) {
   const int quads = hidden >> 2, pieces = row_pieces(quads);
 #define MIR_RMS(P)                                                                                                        \
-  return mir_launch(PAIR ? "rms_norm_pair" : "rms_norm", rms_norm_vec4_kernel<Tout, PAIR, P>, dim3(n_rows),              \
-                    dim3(row_threads(quads)), 0, stream, 0, x, weight, weight_b, out, out_b, rows, hidden, eps)
+  return mir_launch("rms_norm_pair", rms_norm_row_kernel<Tout, true, P, kRowThreads>, dim3(n_rows), dim3(row_threads(quads)), \
+                    0, stream, 0, x, weight, weight_b, out, out_b, nullptr, hidden, eps)
   if (pieces == 1) MIR_RMS(1);
   if (pieces == 2) MIR_RMS(2);
   if (pieces <= 4) MIR_RMS(4);
@@ -617,11 +667,9 @@ MIR_EXPORT int mir_rms_norm(int bf16, const float* x, const float* weight, void*
                             int hidden, float eps, cudaStream_t stream) {
   if (n_rows == 0) return MIR_OK;
   if (n_rows < 0 || hidden <= 0) { mir_set_error("rms_norm: bad sizes"); return MIR_BAD_ARGUMENT; }
-  if ((hidden & 3) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)weight & 15) == 0 && ((uintptr_t)out & 15) == 0 &&
-      hidden <= kRowLimit) {
-    if (bf16)
-      return launch_rms_norm<__nv_bfloat16, false>(x, weight, nullptr, (__nv_bfloat16*)out, nullptr, rows, n_rows, hidden, eps, stream);
-    return launch_rms_norm<float, false>(x, weight, nullptr, (float*)out, nullptr, rows, n_rows, hidden, eps, stream);
+  if ((hidden & 3) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)weight & 15) == 0 && ((uintptr_t)out & 15) == 0) {
+    if (bf16) return launch_rms_norm(x, weight, (__nv_bfloat16*)out, rows, n_rows, hidden, eps, stream);
+    return launch_rms_norm(x, weight, (float*)out, rows, n_rows, hidden, eps, stream);
   }
   const int threads = hidden >= 2048 ? 512 : 256;
   if (bf16)
@@ -657,11 +705,10 @@ MIR_EXPORT int mir_rms_norm_pair(int bf16, const float* x, const float* weight_a
   if (n_rows == 0) return MIR_OK;
   if (n_rows < 0 || hidden <= 0) { mir_set_error("rms_norm_pair: bad sizes"); return MIR_BAD_ARGUMENT; }
   if ((hidden & 3) == 0 && (((uintptr_t)x | (uintptr_t)weight_a | (uintptr_t)weight_b | (uintptr_t)out_a | (uintptr_t)out_b) & 15) == 0 &&
-      hidden <= kRowLimit) {
+      hidden <= kPairLimit) {
     if (bf16)
-      return launch_rms_norm<__nv_bfloat16, true>(x, weight_a, weight_b, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, nullptr,
-                                                  n_rows, hidden, eps, stream);
-    return launch_rms_norm<float, true>(x, weight_a, weight_b, (float*)out_a, (float*)out_b, nullptr, n_rows, hidden, eps, stream);
+      return launch_rms_norm_pair(x, weight_a, weight_b, (__nv_bfloat16*)out_a, (__nv_bfloat16*)out_b, n_rows, hidden, eps, stream);
+    return launch_rms_norm_pair(x, weight_a, weight_b, (float*)out_a, (float*)out_b, n_rows, hidden, eps, stream);
   }
   const int threads = hidden >= 2048 ? 512 : 256;
   if (bf16)

@@ -132,3 +132,57 @@ def test_reference_attention_of_every_value_width(dtype, tol, dim, value_dim):
     want = torch.stack(want).view(len(lengths), -1)
     error = (out.double().cpu() - want).abs().max()
     assert float(error) <= tol * float(want.abs().max()), float(error)
+
+
+def rounded(x):
+    return x.astype(np.float32).astype(np.float64)
+
+
+def sum_of_squares(row, threads):
+    """A row's sum of squares as the norms form it: quads dealt out to `threads` threads, a thread's chain of multiply-adds, then
+    neighbours' sums by halves of a warp and of the warps (each step rounded to 32 bits)."""
+    quads = np.zeros((-(-len(row) // 4 // threads) * threads, 4))
+    quads.reshape(-1)[:len(row)] = row
+    total = np.zeros(threads)
+    for quad in quads.reshape(-1, threads, 4):
+        for i in (3, 2, 1, 0):
+            total = rounded(quad[:, i] * quad[:, i] + total)
+    sums = total.reshape(-1, 32)
+    for _ in range(2):
+        for step in (16, 8, 4, 2, 1):
+            sums = rounded(sums + sums[:, np.arange(32) ^ step])
+        sums = np.concatenate([sums[:, 0], np.zeros(32 - len(sums))])[None, :] if _ == 0 else sums
+    return sums[0, 0]
+
+
+@pytest.mark.parametrize("hidden", [100, 1020, 1024, 2560, 4096, 4100, 5120, 8192, 8196, 16384, 16388, 20480])
+def test_rms_norm_sums_in_one_order_whatever_holds_the_row(hidden):
+    """Rows in registers and rows read twice: bit for bit the sums of 256 threads (128 below 1,024 columns)."""
+    from libmir_b200 import kernels
+    torch.manual_seed(hidden)
+    x, weight = torch.randn(5, hidden), torch.rand(hidden) + 0.5
+    sums = torch.tensor([sum_of_squares(row.double().numpy(), 256 if hidden >= 1024 else 128) for row in x], dtype=torch.float32)
+    mean = sums.numpy() / np.float32(hidden) + np.float32(1e-5)
+    inverse = torch.rsqrt(torch.from_numpy(mean).cuda())
+    for dtype in (torch.float32, torch.bfloat16):
+        out = torch.empty(5, hidden, dtype=dtype, device="cuda")
+        kernels.rms_norm(x.cuda(), weight.cuda(), 1e-5, out)
+        assert torch.equal(out, (x.cuda() * inverse[:, None] * weight.cuda()).to(dtype))
+    rows = ints([4, 0])
+    out = torch.empty(2, hidden, device="cuda")
+    kernels.rms_norm(x.cuda(), weight.cuda(), 1e-5, out, rows)
+    assert torch.equal(out, (x.cuda() * inverse[:, None] * weight.cuda())[rows.long()])
+
+
+@pytest.mark.parametrize("hidden", [100, 2048, 2052, 4100, 8192, 16384, 16388])
+def test_two_norms_of_the_same_rows(hidden):
+    from libmir_b200 import kernels
+    torch.manual_seed(hidden)
+    x, a, b = torch.randn(3, hidden), torch.rand(hidden) + 0.5, torch.rand(hidden) + 0.5
+    normed = x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5)
+    for dtype, tol in ((torch.float32, 2e-6), (torch.bfloat16, 2 ** -8)):
+        out_a, out_b = (torch.empty(3, hidden, dtype=dtype, device="cuda") for _ in range(2))
+        kernels.rms_norm_pair(x.cuda(), a.cuda(), b.cuda(), 1e-5, out_a, out_b)
+        for out, weight in ((out_a, a), (out_b, b)):
+            want = normed * weight.double()
+            assert bool(((out.double().cpu() - want).abs() <= tol * want.abs() + 1e-7).all())
