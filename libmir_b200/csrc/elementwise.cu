@@ -127,12 +127,46 @@ __global__ void add_normed_branches_kernel(NormedBranches branches, float* __res
   }
 }
 
-// The same with 16-byte accesses (hidden a multiple of 4, every pointer 16-byte aligned): a CTA keeps its row of every branch
-// in registers, four columns a thread in PIECES places, asks for the residual with them and for the weights before it waits
-// for the kernel before, and sums all branches behind one barrier.  Few rows are bound by these latencies (2 rows of
+// The same with 16-byte accesses (hidden a multiple of 4, every pointer 16-byte aligned), for rows wider than the registers of a
+// CTA take; the second pass finds the rows in L1 (2,000 rows of 12,288, one branch: 66 us, column by column 170).
+__global__ void add_normed_branches_vec4_kernel(NormedBranches branches, float* __restrict__ residual,
+                                                __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
+  __shared__ float scratch[32];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const size_t base = (size_t)blockIdx.x * hidden;
+  const int quads = hidden >> 2;
+  float inverse[4];
+  for (int b = 0; b < branches.count; ++b) {
+    const float4* src = reinterpret_cast<const float4*>(branches.rows[b] + base);
+    float sum = 0.0f;
+    for (int c = threadIdx.x; c < quads; c += blockDim.x) {
+      const float4 v = src[c];
+      sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sum))));
+    }
+    sum = block_sum(sum, scratch);
+    inverse[b] = rsqrtf(sum / (float)hidden + eps);
+  }
+  for (int c = threadIdx.x; c < quads; c += blockDim.x) {
+    float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int b = 0; b < branches.count; ++b) {
+      const float4 v = reinterpret_cast<const float4*>(branches.rows[b] + base)[c];
+      const float4 w = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
+      total.x += v.x * inverse[b] * w.x; total.y += v.y * inverse[b] * w.y;
+      total.z += v.z * inverse[b] * w.z; total.w += v.w * inverse[b] * w.w;
+    }
+    float4 r = reinterpret_cast<float4*>(residual + base)[c];
+    r.x += scale * total.x; r.y += scale * total.y; r.z += scale * total.z; r.w += scale * total.w;
+    reinterpret_cast<float4*>(residual + base)[c] = r;
+    if (rounded) store_rounded(rounded + base, c, r);
+  }
+}
+
+// The same with the row of every branch in registers, read once, four columns a thread in PIECES places; the residual and the
+// weights are asked for with them, and all branches are summed behind one barrier.  Few rows are bound by these latencies (2 rows of
 // 4,096: 8.7 us when the row was read twice and the weights behind the sum), many by their bytes.
-template <int BRANCHES, int PIECES>
-__global__ void __launch_bounds__(kRowThreads) add_normed_branches_vec4_kernel(
+template <int BRANCHES, int PIECES, bool EARLY>
+__global__ void __launch_bounds__(256) add_normed_branches_row_kernel(
     NormedBranches branches, float* __restrict__ residual, __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
   __shared__ float scratch[BRANCHES][32];
   grid_launch_dependents();
@@ -144,7 +178,7 @@ __global__ void __launch_bounds__(kRowThreads) add_normed_branches_vec4_kernel(
 #pragma unroll
     for (int p = 0; p < PIECES; ++p) {
       const int c = p * blockDim.x + threadIdx.x;
-      if (c < quads) w[b][p] = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
+      if (EARLY && c < quads) w[b][p] = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
     }
   grid_dependency_wait();
   const size_t base = (size_t)blockIdx.x * hidden;
@@ -176,6 +210,7 @@ __global__ void __launch_bounds__(kRowThreads) add_normed_branches_vec4_kernel(
     float4 total = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int b = 0; b < BRANCHES; ++b) {
+      if (!EARLY) w[b][p] = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
       total.x += v[b][p].x * inverse[b] * w[b][p].x; total.y += v[b][p].y * inverse[b] * w[b][p].y;
       total.z += v[b][p].z * inverse[b] * w[b][p].z; total.w += v[b][p].w * inverse[b] * w[b][p].w;
     }
@@ -589,24 +624,36 @@ MIR_EXPORT int mir_add_normed_branches(const float* const* branch_rows, const fl
   bool aligned = (hidden & 3) == 0 && ((uintptr_t)residual & 15) == 0 && ((uintptr_t)rounded & 7) == 0;
   for (int b = 0; b < count; ++b)
     aligned = aligned && ((uintptr_t)branch_rows[b] & 15) == 0 && ((uintptr_t)branch_weights[b] & 15) == 0;
-  const int quads = hidden >> 2, pieces = row_pieces(quads);
+  // 256 threads a row (128 below 4,096 columns), so that two CTAs and more share an SM and three or four branches do not spill
+  // (2,000 rows of 2,048, four branches, with 512 threads: 65 us); the order of the sums is the same in both forms.  The
+  // weights are asked for with the rows while both take 100 registers at most, and 224 where no SM has a second row (two rows
+  // of 8,192, two branches: 3.4 us, 4.5 behind the sums; 2,000 rows 53 and 46).
+  const int threads_of_row = hidden >= 4096 ? 256 : 128, pieces = ((hidden >> 2) + threads_of_row - 1) / threads_of_row;
 #define MIR_NORMED(B, P)                                                                                             \
-  return mir_launch("add_normed_branches", add_normed_branches_vec4_kernel<B, P>, dim3(rows), dim3(row_threads(quads)), 0, \
-                    stream, 0, branches, residual, (__nv_bfloat16*)rounded, hidden, eps, scale)
+  return mir_launch("add_normed_branches", rows <= mir_sm_count() ? add_normed_branches_row_kernel<B, P, (2 * B + 1) * P * 4 <= 224> \
+                                                                  : add_normed_branches_row_kernel<B, P, (2 * B + 1) * P * 4 <= 100>, \
+                    dim3(rows), dim3(threads_of_row), 0, stream, 0, branches, residual, (__nv_bfloat16*)rounded, hidden, eps, scale)
   if (aligned && count == 1) {
     if (pieces == 1) MIR_NORMED(1, 1);
     if (pieces == 2) MIR_NORMED(1, 2);
     if (pieces <= 4) MIR_NORMED(1, 4);
+    if (pieces <= 5) MIR_NORMED(1, 5);
+    if (pieces <= 8) MIR_NORMED(1, 8);
+    if (pieces <= 16) MIR_NORMED(1, 16);
   }
   if (aligned && count == 2) {
-    if (pieces == 1) MIR_NORMED(2, 1);
-    if (pieces == 2) MIR_NORMED(2, 2);
+    if (pieces <= 2) MIR_NORMED(2, 2);
     if (pieces <= 4) MIR_NORMED(2, 4);
+    if (pieces <= 5) MIR_NORMED(2, 5);
+    if (pieces <= 8) MIR_NORMED(2, 8);
   }
-  if (aligned && pieces <= 4) {
-    if (count == 3) MIR_NORMED(3, 4);
-    MIR_NORMED(4, 4);
-  }
+  if (aligned && count == 3 && pieces <= 5) MIR_NORMED(3, 5);
+  if (aligned && count == 3 && pieces <= 8) MIR_NORMED(3, 8);
+  if (aligned && count == 4 && pieces <= 5) MIR_NORMED(4, 5);
+  if (aligned && count == 4 && pieces <= 8) MIR_NORMED(4, 8);
+  if (aligned)
+    return mir_launch("add_normed_branches", add_normed_branches_vec4_kernel, dim3(rows), dim3(threads_of_row), 0, stream, 0,
+                      branches, residual, (__nv_bfloat16*)rounded, hidden, eps, scale);
 #undef MIR_NORMED
   const int threads = hidden >= 2048 ? 512 : 256;
   return mir_launch("add_normed_branches", add_normed_branches_kernel, dim3(rows), dim3(threads), 0, stream, 0, branches,

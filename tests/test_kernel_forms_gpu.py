@@ -186,3 +186,22 @@ def test_two_norms_of_the_same_rows(hidden):
         for out, weight in ((out_a, a), (out_b, b)):
             want = normed * weight.double()
             assert bool(((out.double().cpu() - want).abs() <= tol * want.abs() + 1e-7).all())
+
+
+@pytest.mark.parametrize("hidden", [36, 512, 2048, 2052, 2560, 4096, 4100, 5124, 8192, 8196, 16384, 16388])
+@pytest.mark.parametrize("count", [1, 2, 3, 4])
+def test_normed_branches_of_every_count_and_width(count, hidden):
+    """Rows in registers and rows read twice; the roundings are those of the sums, a product and the addition."""
+    from libmir_b200 import kernels
+    torch.manual_seed(hidden + count)
+    branches = [torch.randn(3, hidden) * (b + 1) for b in range(count)]
+    weights = [torch.rand(hidden) + 0.5 for _ in range(count)]
+    residual = torch.randn(3, hidden)
+    want = residual.double()
+    for branch, weight in zip(branches, weights):
+        want = want + 0.7 * branch.double() * torch.rsqrt((branch.double() ** 2).mean(-1, keepdim=True) + 1e-5) * weight.double()
+    got, half = residual.cuda(), torch.empty(3, hidden, dtype=torch.bfloat16, device="cuda")
+    kernels.add_normed_branches([b.cuda() for b in branches], [w.cuda() for w in weights], got, 1e-5, 0.7, half)
+    bound = 2e-6 * (1 + sum(b.abs().max() for b in branches))
+    assert float((got.double().cpu() - want).abs().max()) <= float(bound)
+    assert torch.equal(half, got.bfloat16())
