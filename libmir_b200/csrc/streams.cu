@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(512) add_layer_norm_kernel(
     }
   };
   // kEarly: both norms' weights are asked for ahead of the row, so that a few rows' chain of four sums does not wait for
-  // memory twice more (2 rows of 4,096: 5.1 us instead of 8.4); with many rows the registers serve more rows in flight
-  // (2,400 rows of 4,096: 35 us instead of 65)
+  // memory twice more (148 rows of 4,096: 4.0 us, 4.5 the other way); with more than a row for each SM the registers serve more
+  // rows in flight (296 rows of 4,096: 5.4 us, 6.9 this way; 2,400 rows 31 and 65)
   float early[kEarly ? 4 : 1][kEarly ? PIECES : 1][V];
   if constexpr (kEarly) {
 #pragma unroll
@@ -244,7 +244,7 @@ int launch_add_layer_norm(float* x, const float* y, const float* weight, const f
                           const float* next_weight, const float* next_bias, float next_eps, void* out, int tokens, int width,
                           cudaStream_t stream) {
 #define MIR_ADD_NORM(V, P)                                                                                               \
-  if (V * P <= 8 && tokens <= 2 * mir_sm_count())                                                                        \
+  if (V * P <= 8 && tokens <= mir_sm_count())                                                                            \
     return mir_launch("add_layer_norm", add_layer_norm_kernel<T, V, P, V * P <= 8>, dim3(tokens), dim3(threads), 0, stream, 0, x, \
                       y, weight, bias, eps, rows, next_weight, next_bias, next_eps, (T*)out, width);                    \
   return mir_launch("add_layer_norm", add_layer_norm_kernel<T, V, P, false>, dim3(tokens), dim3(threads), 0, stream, 0, x, y, weight, \

@@ -205,3 +205,21 @@ def test_normed_branches_of_every_count_and_width(count, hidden):
     bound = 2e-6 * (1 + sum(b.abs().max() for b in branches))
     assert float((got.double().cpu() - want).abs().max()) <= float(bound)
     assert torch.equal(half, got.bfloat16())
+
+
+@pytest.mark.parametrize("tokens", [1, 147, 148, 149])
+@pytest.mark.parametrize("width", [7, 2048, 4096, 4100])
+def test_addition_of_a_layer_norm_with_weights_asked_for_early_and_late(tokens, width):
+    from libmir_b200 import kernels
+    torch.manual_seed(tokens + width)
+    x, y, rows = torch.randn(tokens, width), torch.randn(tokens, width) * 2 + 1, torch.randn(tokens, width)
+    w, b, next_w, next_b = (torch.randn(width) for _ in range(4))
+
+    def norm(u, weight, bias):
+        mean = u.mean(-1, keepdim=True)
+        return (u - mean) / torch.sqrt(((u - mean) ** 2).mean(-1, keepdim=True) + 1e-5) * weight.double() + bias.double()
+    want = x.double() + norm(y.double(), w, b) + rows.double()
+    got, out = x.cuda(), torch.empty(tokens, width, device="cuda")
+    kernels.add_layer_norm(got, y.cuda(), w.cuda(), b.cuda(), 1e-5, rows.cuda(), next_w.cuda(), next_b.cuda(), 1e-5, out)
+    assert float((got.double().cpu() - want).abs().max()) <= 5e-6 * float(want.abs().max())
+    assert float((out.double().cpu() - norm(want, next_w, next_b)).abs().max()) <= 2e-5 * float(want.abs().max())
