@@ -298,9 +298,11 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
 }
 
 // One CTA per (token, head): the partitions' partial results into the normalised output.  The partitions' maxima and sums are
-// read side by side, and a thread takes four columns whose loads do not wait for one another (a column at a time, each
-// partition's numbers behind the other's: 8.5 us for 48 rows of 512 columns).
+// read side by side, and a thread takes V columns (four of 512, fewer of fewer, so that all threads have some) whose loads
+// do not wait for one another (a column at a time, each partition's numbers behind the other's: 8.5 us for 48 rows of 512
+// columns; 16 heads of 64 columns at 8,000 keys, 62 partitions: the whole attention 27 us with four columns a thread).
 constexpr int kMergeThreads = 128, kMergePartitions = 256;
+template <int V>
 __global__ void __launch_bounds__(kMergeThreads)
 latent_attention_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
                               __nv_bfloat16* __restrict__ out, int rank, int partitions) {
@@ -311,35 +313,41 @@ latent_attention_merge_kernel(const float* __restrict__ partial_o, const float* 
   float top = -INFINITY;                                         // (every warp for itself)
   for (int p = lane; p < partitions; p += 32) top = fmaxf(top, ml[p].x);
   top = warp_max(top);
-  for (int p = threadIdx.x; p < min(partitions, kMergePartitions); p += kMergeThreads) {
+  const int held = min(partitions, kMergePartitions);
+  for (int p = threadIdx.x; p < held; p += kMergeThreads) {
     const float2 both = ml[p];
     factor_s[p] = both.x != -INFINITY ? exp2f(both.x - top) : 0.0f;
     sum_s[p] = both.x != -INFINITY ? both.y : 0.0f;
   }
   __syncthreads();
-  auto factor_of = [&](int p) {                                  // (more partitions than are kept: formed again)
-    return p < kMergePartitions ? factor_s[p] : (ml[p].x != -INFINITY ? exp2f(ml[p].x - top) : 0.0f);
-  };
+  auto factor_of = [&](int p) { return ml[p].x != -INFINITY ? exp2f(ml[p].x - top) : 0.0f; };   // (of more than are held)
   float total = 0.0f;
-  for (int p = 0; p < partitions; ++p) {
-    const float factor = factor_of(p);
-    if (factor != 0.0f) total += (p < kMergePartitions ? sum_s[p] : ml[p].y) * factor;
-  }
+  auto add_part = [&](float factor, float part) { total = factor != 0.0f ? fmaf(part, factor, total) : total; };
+#pragma unroll 8
+  for (int p = 0; p < held; ++p) add_part(factor_s[p], sum_s[p]);
+  for (int p = held; p < partitions; ++p) add_part(factor_of(p), ml[p].y);
   const float inverse = total > 0.0f ? 1.0f / total : 0.0f;
-  for (int c = threadIdx.x * 4; c < rank; c += kMergeThreads * 4) {          // (rank is a multiple of 8)
-    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (int c = threadIdx.x * V; c < rank; c += kMergeThreads * V) {          // (rank is a multiple of 8)
+    float sum[V] = {};
     const float* from = partial_o + unit * partitions * rank + c;
-#pragma unroll 4
-    for (int p = 0; p < partitions; ++p) {
-      const float factor = factor_of(p);
-      if (factor == 0.0f) continue;                              // (a partition without keys)
-      const float4 v = *reinterpret_cast<const float4*>(from + (size_t)p * rank);
-      sum.x = fmaf(v.x, factor, sum.x); sum.y = fmaf(v.y, factor, sum.y);
-      sum.z = fmaf(v.z, factor, sum.z); sum.w = fmaf(v.w, factor, sum.w);
-    }
-    __nv_bfloat162* to = reinterpret_cast<__nv_bfloat162*>(out + unit * rank + c);
-    to[0] = __floats2bfloat162_rn(sum.x * inverse, sum.y * inverse);
-    to[1] = __floats2bfloat162_rn(sum.z * inverse, sum.w * inverse);
+    auto add_partition = [&](int p, float factor) {
+      float v[V];
+      if constexpr (V == 4) *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(from + (size_t)p * rank);
+      else if constexpr (V == 2) *reinterpret_cast<float2*>(v) = *reinterpret_cast<const float2*>(from + (size_t)p * rank);
+      else v[0] = from[(size_t)p * rank];
+#pragma unroll
+      for (int i = 0; i < V; ++i) sum[i] = factor != 0.0f ? fmaf(v[i], factor, sum[i]) : sum[i];   // (0: no keys)
+    };
+#pragma unroll 8
+    for (int p = 0; p < held; ++p) add_partition(p, factor_s[p]);
+    for (int p = held; p < partitions; ++p) add_partition(p, factor_of(p));
+#pragma unroll
+    for (int i = 0; i < V; ++i) sum[i] *= inverse;
+    __nv_bfloat16* to = out + unit * rank + c;
+    if constexpr (V == 1) to[0] = __float2bfloat16_rn(sum[0]);
+    else
+#pragma unroll
+      for (int i = 0; i < V; i += 2) *reinterpret_cast<__nv_bfloat162*>(to + i) = __floats2bfloat162_rn(sum[i], sum[i + 1]);
   }
 }
 
@@ -412,7 +420,12 @@ MIR_EXPORT int mir_latent_attention_bf16(const void* q, long long q_stride, void
   else MIR_LATENT(8);
 #undef MIR_LATENT
   if (status != MIR_OK || partitions == 1) return status;
-  latent_attention_merge_kernel<<<dim3(tokens * heads), dim3(kMergeThreads), 0, stream>>>(partial_o, partial_ml,
-                                                                               (__nv_bfloat16*)out, rank, partitions);
+  const dim3 merged(tokens * heads), merging(kMergeThreads);
+  if (rank > 256)
+    latent_attention_merge_kernel<4><<<merged, merging, 0, stream>>>(partial_o, partial_ml, (__nv_bfloat16*)out, rank, partitions);
+  else if (rank > 128)
+    latent_attention_merge_kernel<2><<<merged, merging, 0, stream>>>(partial_o, partial_ml, (__nv_bfloat16*)out, rank, partitions);
+  else
+    latent_attention_merge_kernel<1><<<merged, merging, 0, stream>>>(partial_o, partial_ml, (__nv_bfloat16*)out, rank, partitions);
   return mir_check_launch("latent_attention_merge");
 }

@@ -223,3 +223,30 @@ def test_addition_of_a_layer_norm_with_weights_asked_for_early_and_late(tokens, 
     kernels.add_layer_norm(got, y.cuda(), w.cuda(), b.cuda(), 1e-5, rows.cuda(), next_w.cuda(), next_b.cuda(), 1e-5, out)
     assert float((got.double().cpu() - want).abs().max()) <= 5e-6 * float(want.abs().max())
     assert float((out.double().cpu() - norm(want, next_w, next_b)).abs().max()) <= 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("partitions", [2, 5, 40])
+@pytest.mark.parametrize("rank,rotary", [(8, 8), (64, 32), (128, 0), (136, 8), (256, 64), (264, 8), (512, 64)])
+def test_merge_of_partitions_of_every_value_width(rank, rotary, partitions):
+    """One, two or four columns a thread; requests whose last partitions have no keys."""
+    from libmir_b200 import kernels
+    generator = torch.Generator().manual_seed(rank)
+    width, heads, page, contexts = rank + rotary, 3, 16, [1, 64, 65, 500, 40 * 64]
+    contexts = [min(c, partitions * 64) for c in contexts]
+    pages = [-(-c // page) for c in contexts]
+    table = torch.full((len(contexts), max(pages)), -1, dtype=torch.int32)
+    pool = torch.randn(sum(pages) * page, 1, width, generator=generator).to(torch.bfloat16)
+    q = (torch.randn(len(contexts), heads, width, generator=generator)).to(torch.bfloat16)
+    want, first = [], 0
+    for r, (context, count) in enumerate(zip(contexts, pages)):
+        table[r, :count] = torch.arange(first, first + count)
+        keys = pool[first * page:first * page + context, 0].double()
+        want.append(torch.softmax(q[r].double() @ keys.T * 0.1, -1) @ keys[:, :rank])
+        first += count
+    out = torch.full((len(contexts), heads * rank), float("nan"), dtype=torch.bfloat16, device="cuda")
+    alloc = lambda shape, kind: torch.full(shape, float("nan"), dtype=kind, device="cuda")
+    kernels.latent_attention(q.flatten(1).cuda(), out, pool.cuda(), table.cuda(), ints(range(len(contexts) + 1)), ints(contexts), page,
+                             heads, width, rank, 0.1, heads, 64, partitions, alloc)
+    want = torch.stack(want).view(len(contexts), -1)
+    # (weights rounded to 8 bits, then the result)
+    assert float((out.double().cpu() - want).abs().max()) <= 1e-2 * float(want.abs().max())
