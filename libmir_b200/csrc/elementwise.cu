@@ -23,11 +23,12 @@ __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict_
   for (int c = threadIdx.x; c < hidden; c += blockDim.x) dst[c] = ok ? to_float(src[c]) * scale : 0.0f;
 }
 
-// The same, eight neighbouring columns a thread (hidden a multiple of 8, rows on 16-byte boundaries): one load a thread for rows
-// of up to 4,096 (2 rows of 4,096: 8.5 us column by column).
+// The same, 16 bytes of the table a thread (hidden a multiple of 8, rows on 16-byte boundaries): one load a thread for bfloat16
+// rows of up to 4,096 (2 rows of 4,096: 8.5 us column by column).
 template <typename T>
 __global__ void __launch_bounds__(512) embed_wide_kernel(const T* __restrict__ table, const int* __restrict__ ids,
                                                          float* __restrict__ out, int hidden, int vocab, float scale) {
+  constexpr int V = 16 / sizeof(T);
   grid_launch_dependents();
   grid_dependency_wait();
   const int row = blockIdx.x;
@@ -35,13 +36,14 @@ __global__ void __launch_bounds__(512) embed_wide_kernel(const T* __restrict__ t
   const bool ok = id >= 0 && id < vocab;
   const T* src = table + (size_t)(ok ? id : 0) * hidden;
   float* dst = out + (size_t)row * hidden;
-  for (int c = threadIdx.x * 8; c < hidden; c += blockDim.x * 8) {
-    float v[8];
-    load8(src + c, v);
+  for (int c = threadIdx.x * V; c < hidden; c += blockDim.x * V) {
+    float v[V];
+    if constexpr (V == 8) load8(src + c, v);
+    else *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(src + c);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = ok ? v[i] * scale : 0.0f;
-    reinterpret_cast<float4*>(dst + c)[0] = make_float4(v[0], v[1], v[2], v[3]);
-    reinterpret_cast<float4*>(dst + c)[1] = make_float4(v[4], v[5], v[6], v[7]);
+    for (int i = 0; i < V; ++i) v[i] = ok ? v[i] * scale : 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; i += 4) reinterpret_cast<float4*>(dst + c)[i / 4] = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
   }
 }
 
@@ -524,7 +526,7 @@ MIR_EXPORT int mir_embed(int bf16, const void* table, const int* ids, float* out
   if (rows == 0) return MIR_OK;
   if (rows < 0 || hidden <= 0 || vocab <= 0) { mir_set_error("embed: bad sizes"); return MIR_BAD_ARGUMENT; }
   if (hidden % 8 == 0 && (((uintptr_t)table | (uintptr_t)out) & 15) == 0) {
-    const int threads = hidden >= 4096 ? 512 : (hidden / 8 + 31) / 32 * 32;
+    const int threads = row_threads(bf16 ? hidden / 8 : hidden / 4);
     if (bf16)
       return mir_launch("embed", embed_wide_kernel<__nv_bfloat16>, dim3(rows), dim3(threads), 0, stream, 0,
                         (const __nv_bfloat16*)table, ids, out, hidden, vocab, scale);

@@ -250,3 +250,16 @@ def test_merge_of_partitions_of_every_value_width(rank, rotary, partitions):
     want = torch.stack(want).view(len(contexts), -1)
     # (weights rounded to 8 bits, then the result)
     assert float((out.double().cpu() - want).abs().max()) <= 1e-2 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("hidden", [8, 100, 1000, 2048, 2056, 4096, 4104, 9000])
+def test_embedding_rows_of_every_width(dtype, hidden):
+    """Only moved and multiplied by a power of two: exact; ids outside the table give zeros."""
+    from libmir_b200 import kernels
+    torch.manual_seed(hidden)
+    table, ids = torch.randn(50, hidden).to(dtype), [49, 0, -1, 7, 50]
+    out = torch.full((5, hidden), float("nan"), device="cuda")
+    kernels.embed(table.cuda(), ints(ids), out, 2.0)
+    want = torch.stack([table[i].float() * 2.0 if 0 <= i < 50 else torch.zeros(hidden) for i in ids])
+    assert torch.equal(out.cpu(), want)
