@@ -300,7 +300,8 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
 // One CTA per (token, head): the partitions' partial results into the normalised output.  The partitions' maxima and sums are
 // read side by side, and a thread takes V columns (four of 512, fewer of fewer, so that all threads have some) whose loads
 // do not wait for one another (a column at a time, each partition's numbers behind the other's: 8.5 us for 48 rows of 512
-// columns; 16 heads of 64 columns at 8,000 keys, 62 partitions: the whole attention 27 us with four columns a thread).
+// columns; one row of 16 heads of 64 columns at 8,000 keys, 62 partitions: the whole attention 27 us with four columns a thread and
+// a branch beside each load, 15 this way; of 512 columns 38 and 29).
 constexpr int kMergeThreads = 128, kMergePartitions = 256;
 template <int V>
 __global__ void __launch_bounds__(kMergeThreads)
