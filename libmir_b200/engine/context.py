@@ -74,6 +74,20 @@ class Arena:
             self.chunk += 1
             self.offset = 0
 
+    def reserve(self, nbytes: int) -> None:
+        """Room for `nbytes` in a few tensors of one buffer: what is asked for next comes out of it.  A buffer that is added for
+        this has the size of the next power of two, so that a need which grows from step to step (the context of a long
+        prompt) adds a buffer for each doubling, and not one for each step."""
+        padding = 16 * self.ALIGN
+        while True:
+            if self.chunk >= len(self.chunks):
+                size = max(self.chunk_bytes, (1 << max(nbytes - 1, 0).bit_length()) + padding)
+                self.chunks.append(torch.empty(size, dtype=torch.uint8, device=self.device))
+            if self.offset + nbytes + padding <= self.chunks[self.chunk].numel():
+                return
+            self.chunk += 1
+            self.offset = 0
+
     def mark(self) -> tuple:
         """Where the next allocation goes: `rewind` to it gives back everything asked for since."""
         return self.chunk, self.offset
@@ -140,8 +154,10 @@ class StepContext(PartContext):
         return self.arena.alloc(shape, dtype)
 
     @contextlib.contextmanager
-    def temporary(self):
+    def temporary(self, nbytes: int = 0):
         mark = self.arena.mark()
+        if nbytes:
+            self.arena.reserve(nbytes)
         yield
         self.arena.rewind(mark)
 

@@ -50,9 +50,9 @@ class PartContext:
     `ScratchContext` as the smallest concrete form.
 
     alloc(shape, dtype)                   scratch memory that lives until the step ends.
-    temporary()                           a `with` block: what is asked for inside is given back when it ends, for large
-                                          scratch that only the kernels launched inside read (a step's kernels run in
-                                          order on one stream, so whoever gets it next writes behind them).
+    temporary(nbytes)                     a `with` block: what is asked for inside (about nbytes) is given back when it
+                                          ends, for large scratch that only the kernels launched inside read (a step's
+                                          kernels run in order on one stream, so whoever gets it next writes behind them).
     accumulate(x, weight, residual, bias) residual += x . weight^T (+ bias) on the 32-bit residual stream; every
                                           branch adds its result through this, so that the product can also
                                           prepare the norm named by `upcoming_norm` (see below).
@@ -111,7 +111,7 @@ class PartContext:
     def alloc(self, shape, dtype: torch.dtype) -> torch.Tensor:
         raise NotImplementedError
 
-    def temporary(self):
+    def temporary(self, nbytes: int = 0):
         return contextlib.nullcontext()
 
     def accumulate(self, x: torch.Tensor, weight: torch.Tensor, residual: torch.Tensor,

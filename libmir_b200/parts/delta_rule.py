@@ -161,9 +161,12 @@ class GatedDeltaRule(Mixer):
         read = ctx.alloc((tokens, self.v_width), torch.float32)
         # portions of prompts walk four tokens at a time, but for the 32-bit engine, whose results do not depend on the cut
         grouped = None
-        with ctx.temporary():
-            if self.env.dtype == torch.bfloat16 and not ctx.decode_only and s.key_dim <= kernels.DELTA_GROUPED_KEYS:
-                grouped = ctx.alloc((kernels.delta_rule_grouped_floats(tokens, ctx.num_rows, s.heads, s.key_dim),), torch.float32)
+        floats = 0
+        if self.env.dtype == torch.bfloat16 and not ctx.decode_only and s.key_dim <= kernels.DELTA_GROUPED_KEYS:
+            floats = kernels.delta_rule_grouped_floats(tokens, ctx.num_rows, s.heads, s.key_dim)
+        with ctx.temporary(4 * floats):
+            if floats:
+                grouped = ctx.alloc((floats,), torch.float32)
             kernels.delta_rule_scan(prepared, beta, decays, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,
                                     s.heads, s.kv_heads, s.key_dim, s.value_dim, grouped=grouped)
         mixed = ctx.alloc((tokens, self.v_width), self.env.dtype)

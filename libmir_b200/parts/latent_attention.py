@@ -26,7 +26,15 @@ from ..registry import build_part
 from .base import Mixer
 
 PORTION_QUERIES = 48        # queries of a portion for each key of context from which on keys and values are formed for it
-PORTION_SCRATCH = 512 << 20  # the most bytes that may take: 47,000 rows of 16 heads of 192 + 128, 24,800 of 32
+# The most bytes that may take (47,000 rows of 16 heads of 192 + 128, 24,800 of 32).  What is held is at most twice as much: as
+# the context grows, a buffer for each doubling.
+PORTION_SCRATCH = 512 << 20
+
+
+def _scratch_per_row(part) -> int:
+    """Bytes that a gathered row of latents takes with the keys and values formed from it."""
+    s = part.spec
+    return (part.key_width + s.heads * (s.head_dim + s.rotary_dim) + part.out_width) * 2
 
 
 def _pad8(n: int) -> int:
@@ -170,7 +178,7 @@ class LatentAttention(Mixer):
         contexts = [n + k for n, k in zip(before, portions)]
         s = self.spec
         rows = sum(-(-n // kernels.GATHER_ROWS) for n in contexts) * kernels.GATHER_ROWS
-        scratch = rows * (self.key_width + s.heads * (s.head_dim + s.rotary_dim) + self.out_width) * 2
+        scratch = rows * _scratch_per_row(self)
         return (min(portions, default=0) > 0 and scratch <= PORTION_SCRATCH
                 and sum(p * c for p, c in zip(portions, contexts)) >= PORTION_QUERIES * sum(contexts))
 
@@ -201,7 +209,7 @@ class LatentAttention(Mixer):
         tiles = [-(-n // kernels.GATHER_ROWS) for n in contexts]
         rows = sum(tiles) * kernels.GATHER_ROWS
         mixed = ctx.alloc((tokens, self.out_width), dtype)
-        with ctx.temporary():
+        with ctx.temporary(rows * _scratch_per_row(self)):
             gathered = ctx.alloc((rows, self.key_width), dtype)
             tile_table = ctx.alloc((len(contexts), max(tiles)), torch.int32)
             kernels.latent_gather(cache.k_pages, group.block_table, ctx.context_lens, cache.page_size, contexts, gathered, tile_table)

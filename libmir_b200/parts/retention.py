@@ -101,9 +101,9 @@ class Retention(Mixer):
         view = lambda name, width: packed[:, self.offsets[name]:self.offsets[name] + width]
         read = ctx.alloc((tokens, self.v_width), torch.float32)
         # a step with portions of prompts rotates once per token and head in a kernel of its own
-        with ctx.temporary():
-            prepared = None if ctx.decode_only else ctx.alloc(
-                (kernels.retention_prepared_floats(tokens, s.heads, s.key_dim),), torch.float32)
+        floats = 0 if ctx.decode_only else kernels.retention_prepared_floats(tokens, s.heads, s.key_dim)
+        with ctx.temporary(4 * floats):
+            prepared = ctx.alloc((floats,), torch.float32) if floats else None
             kernels.retention_scan(view("q", self.qk_width), view("k", self.qk_width), view("v", self.v_width),
                                    self.position.table if self.position is not None else None, self.decays,
                                    self.key_scale, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,

@@ -101,9 +101,9 @@ class Wkv(Mixer):
         kernels.linear(low, self.w_2, decay_raw, alloc=ctx.alloc)
         read = ctx.alloc((tokens, self.width), torch.float32)
         # a step with portions of prompts forms the decays once per token and head in a kernel of its own
-        with ctx.temporary():
-            prepared = None if ctx.decode_only else ctx.alloc(
-                (kernels.wkv_prepared_floats(tokens, s.heads, s.head_dim),), torch.float32)
+        floats = 0 if ctx.decode_only else kernels.wkv_prepared_floats(tokens, s.heads, s.head_dim)
+        with ctx.temporary(4 * floats):
+            prepared = ctx.alloc((floats,), torch.float32) if floats else None
             kernels.wkv_scan(projected[0], projected[1], projected[2], decay_raw, self.decay_bias, self.bonus, state,
                              ctx.query_starts, ctx.state_slots, ctx.positions, read, s.heads, s.head_dim, prepared=prepared)
         mixed = ctx.alloc((tokens, self.width), dtype)

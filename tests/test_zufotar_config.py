@@ -175,3 +175,36 @@ def test_when_keys_of_a_portion_are_formed(portion, before, expected):
     assert LatentAttention._takes_portions(part, ctx) is expected
     ctx.decode_only = True
     assert LatentAttention._takes_portions(part, ctx) is False
+
+
+@pytest.mark.parametrize("heads,portion", [(16, 512), (16, 2048), (32, 512), (32, 96)])
+def test_a_growing_context_does_not_add_a_buffer_a_step(heads, portion):
+    """One request's prompt in portions: what the arena holds stays within a small multiple of the largest step's need, layer after
+    layer, and the scratch of a layer lies in one buffer."""
+    import torch
+    from libmir_b200.engine.context import Arena, StepContext
+    from libmir_b200.kernels import GATHER_ROWS
+    from libmir_b200.parts.latent_attention import PORTION_SCRATCH
+    arena = Arena(torch.device("meta"))
+    ctx = StepContext(*[None] * 10, arena, torch.bfloat16)
+    largest, context = 0, 0
+    while True:
+        context += portion
+        rows = -(-context // GATHER_ROWS) * GATHER_ROWS
+        widths = (576, heads * 192, heads * 128)
+        need = rows * sum(widths) * 2
+        if need > PORTION_SCRATCH:
+            break
+        largest = need
+        arena.reset()
+        ctx.alloc((portion, 4096), torch.float32)
+        for _ in range(3):
+            mark = arena.mark()
+            with ctx.temporary(need):
+                places = []
+                for width in widths:
+                    ctx.alloc((rows, width), torch.bfloat16)
+                    places.append(arena.chunk)
+            assert len(set(places)) == 1 and arena.mark() == mark
+    assert largest > PORTION_SCRATCH // 2
+    assert arena.bytes() <= 2 * PORTION_SCRATCH + 2 * arena.chunk_bytes
