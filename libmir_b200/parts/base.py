@@ -44,6 +44,22 @@ class BuildEnv:
     device: torch.device
 
 
+# The most scratch that a recurrence's kernels take for a step's portions; a step that would need more is walked in runs of its tokens,
+# from state to state.  Half a gigabyte is 7,900 tokens of 64 heads of 64 (wkv) or 9,600 of 32 heads of 128 (the delta rule).
+RECURRENCE_SCRATCH = 512 << 20
+
+
+def scratch_runs(query_starts: torch.Tensor, tokens: int, nbytes: int):
+    """The runs of a step's tokens whose share of `nbytes` is within RECURRENCE_SCRATCH: pairs of a slice of the tokens and the
+    request rows' first tokens within it (query_starts itself where one run takes all)."""
+    count = max(1, -(-nbytes // RECURRENCE_SCRATCH))
+    if count == 1:
+        return [(slice(0, tokens), query_starts)]
+    size = -(-tokens // count)
+    return [(slice(first, min(first + size, tokens)), query_starts.clamp(first, min(first + size, tokens)) - first)
+            for first in range(0, tokens, size)]
+
+
 class PartContext:
     """What a step hands to every part.  The engine's StepContext (engine/context.py) derives from this and adds the
     packed rows' metadata; a part that needs nothing of the batch (a norm, a feed-forward) runs on this alone, with

@@ -25,7 +25,7 @@ import torch
 
 from .. import kernels
 from ..config.spec import CacheBundle, FixedState, ParamSpec
-from .base import Mixer
+from .base import Mixer, scratch_runs
 
 
 def _pad8(n: int) -> int:
@@ -160,15 +160,15 @@ class GatedDeltaRule(Mixer):
                                    prepared, beta, decays, s.heads, s.kv_heads, s.key_dim, s.value_dim)
         read = ctx.alloc((tokens, self.v_width), torch.float32)
         # portions of prompts walk four tokens at a time, but for the 32-bit engine, whose results do not depend on the cut
-        grouped = None
-        floats = 0
-        if self.env.dtype == torch.bfloat16 and not ctx.decode_only and s.key_dim <= kernels.DELTA_GROUPED_KEYS:
-            floats = kernels.delta_rule_grouped_floats(tokens, ctx.num_rows, s.heads, s.key_dim)
-        with ctx.temporary(4 * floats):
-            if floats:
-                grouped = ctx.alloc((floats,), torch.float32)
-            kernels.delta_rule_scan(prepared, beta, decays, state, ctx.query_starts, ctx.state_slots, ctx.positions, read,
-                                    s.heads, s.kv_heads, s.key_dim, s.value_dim, grouped=grouped)
+        grouping = self.env.dtype == torch.bfloat16 and not ctx.decode_only and s.key_dim <= kernels.DELTA_GROUPED_KEYS
+        floats = lambda count: kernels.delta_rule_grouped_floats(count, ctx.num_rows, s.heads, s.key_dim) if grouping else 0
+        for run, starts in scratch_runs(ctx.query_starts, tokens, 4 * floats(tokens)):
+            needed = floats(run.stop - run.start)
+            with ctx.temporary(4 * needed):
+                grouped = ctx.alloc((needed,), torch.float32) if grouping else None
+                kernels.delta_rule_scan(prepared[run], beta[run], decays[run], state, starts, ctx.state_slots,
+                                        ctx.positions[run], read[run], s.heads, s.kv_heads, s.key_dim, s.value_dim,
+                                        grouped=grouped)
         mixed = ctx.alloc((tokens, self.v_width), self.env.dtype)
         kernels.gated_head_norm(read, gate, self.norm, mixed, s.heads, s.value_dim, s.norm_eps, s.gate == "sigmoid")
         if overwrite:

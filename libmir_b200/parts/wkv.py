@@ -20,7 +20,7 @@ import torch
 
 from .. import kernels
 from ..config.spec import CacheBundle, FixedState, ParamSpec
-from .base import Mixer
+from .base import Mixer, scratch_runs
 
 MIXES = ("r", "k", "v", "g", "w")
 
@@ -102,10 +102,13 @@ class Wkv(Mixer):
         read = ctx.alloc((tokens, self.width), torch.float32)
         # a step with portions of prompts forms the decays once per token and head in a kernel of its own
         floats = 0 if ctx.decode_only else kernels.wkv_prepared_floats(tokens, s.heads, s.head_dim)
-        with ctx.temporary(4 * floats):
-            prepared = ctx.alloc((floats,), torch.float32) if floats else None
-            kernels.wkv_scan(projected[0], projected[1], projected[2], decay_raw, self.decay_bias, self.bonus, state,
-                             ctx.query_starts, ctx.state_slots, ctx.positions, read, s.heads, s.head_dim, prepared=prepared)
+        for run, starts in scratch_runs(ctx.query_starts, tokens, 4 * floats):
+            floats = 0 if ctx.decode_only else kernels.wkv_prepared_floats(run.stop - run.start, s.heads, s.head_dim)
+            with ctx.temporary(4 * floats):
+                prepared = ctx.alloc((floats,), torch.float32) if floats else None
+                kernels.wkv_scan(projected[0, run], projected[1, run], projected[2, run], decay_raw[run], self.decay_bias,
+                                 self.bonus, state, starts, ctx.state_slots, ctx.positions[run], read[run], s.heads,
+                                 s.head_dim, prepared=prepared)
         mixed = ctx.alloc((tokens, self.width), dtype)
         kernels.gated_head_norm(read, projected[3], self.norm, mixed, s.heads, s.head_dim, s.norm_eps, False)
         if overwrite:

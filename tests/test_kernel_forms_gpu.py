@@ -263,3 +263,43 @@ def test_embedding_rows_of_every_width(dtype, hidden):
     kernels.embed(table.cuda(), ints(ids), out, 2.0)
     want = torch.stack([table[i].float() * 2.0 if 0 <= i < 50 else torch.zeros(hidden) for i in ids])
     assert torch.equal(out.cpu(), want)
+
+
+@pytest.mark.parametrize("wkv", [True, False])
+@pytest.mark.parametrize("limit", [1 << 14, 1 << 16, 1 << 19])
+def test_a_recurrence_walked_in_runs_of_the_steps_tokens(monkeypatch, wkv, limit):
+    """Scratch beyond its bound: from one to many runs, single tokens and several requests in a run; wkv gives the bits of one walk,
+    the delta rule in groups of four the same sums from other group borders."""
+    from libmir_b200 import kernels
+    from libmir_b200.parts import base
+    monkeypatch.setattr(base, "RECURRENCE_SCRATCH", limit)
+    torch.manual_seed(limit)
+    counts, heads, dim = [1, 1, 130, 3, 61, 200], 3, 64
+    row_of, starts, slots, positions = batch(counts, [5, 0, 3, 1, 2, 4])
+    tokens, width = sum(counts), heads * dim
+    make = lambda *shape: torch.randn(*shape, device="cuda")
+    state0 = make(6, heads, dim, dim)
+    x, raw, bias, bonus = make(3, tokens, width).bfloat16(), make(tokens, width) - 3, make(width), make(width)
+    qkv, beta, decay = make(tokens, 3 * width) * 0.1, torch.rand(tokens, heads, device="cuda"), torch.rand(tokens, width, device="cuda")
+    qkv[:, width:2 * width] = torch.nn.functional.normalize(qkv[:, width:2 * width].view(tokens, heads, dim), dim=-1).view(tokens, width)
+
+    def walk(runs):
+        state, out = state0.clone(), torch.full((tokens, width), float("nan"), device="cuda")
+        for run, held in runs:
+            count = run.stop - run.start
+            if wkv:
+                kernels.wkv_scan(x[0, run], x[1, run], x[2, run], raw[run], bias, bonus, state, held, slots, positions[run], out[run],
+                                 heads, dim)
+            else:
+                grouped = torch.empty(kernels.delta_rule_grouped_floats(count, len(counts), heads, dim), device="cuda")
+                kernels.delta_rule_scan(qkv[run], beta[run], decay[run], state, held, slots, positions[run], out[run], heads, heads, dim,
+                                        dim, grouped=grouped)
+        return out, state
+    floats = kernels.wkv_prepared_floats(tokens, heads, dim) if wkv else kernels.delta_rule_grouped_floats(tokens, len(counts), heads, dim)
+    runs = base.scratch_runs(starts, tokens, 4 * floats)
+    assert len(runs) > 1 and runs[-1][0].stop == tokens
+    for got, want in zip(walk(runs), walk([(slice(0, tokens), starts)])):
+        if wkv:
+            assert torch.equal(got, want)
+        else:
+            assert float((got - want).norm() / want.norm()) <= 2e-6

@@ -208,3 +208,15 @@ def test_a_growing_context_does_not_add_a_buffer_a_step(heads, portion):
             assert len(set(places)) == 1 and arena.mark() == mark
     assert largest > PORTION_SCRATCH // 2
     assert arena.bytes() <= 2 * PORTION_SCRATCH + 2 * arena.chunk_bytes
+
+
+def test_a_step_is_walked_in_runs_once_the_scratch_passes_its_bound(monkeypatch):
+    import torch
+    from libmir_b200.parts import base
+    starts = torch.tensor([0, 1, 7, 7, 20], dtype=torch.int32)
+    assert [run for run, held in base.scratch_runs(starts, 20, base.RECURRENCE_SCRATCH)] == [slice(0, 20)]
+    monkeypatch.setattr(base, "RECURRENCE_SCRATCH", 100)
+    runs = base.scratch_runs(starts, 20, 250)
+    assert [run for run, _ in runs] == [slice(0, 7), slice(7, 14), slice(14, 20)]
+    assert [held.tolist() for _, held in runs] == [[0, 1, 7, 7, 7], [0, 0, 0, 0, 7], [0, 0, 0, 0, 6]]
+    assert all(held.dtype == torch.int32 and held.is_contiguous() for _, held in runs)
