@@ -105,6 +105,7 @@ class LatentAttention(Mixer):
         # products (the rotated part passes through rows of the identity).
         self.w_keys = self.w_values = None
         if (self.env.dtype == torch.bfloat16 and (s.head_dim, s.rotary_dim, s.value_dim) == (128, 64, 128)
+                and s.scale > 0                                  # (the tcgen05 kernel's running maximum is of scaled scores)
                 and self.position is not None and self.key_width % 8 == 0 and self.packed_width % 8 == 0 and (self.segments["g"] % 8 == 0 if s.gate else True)):
             w_keys = torch.zeros((s.heads, s.head_dim + s.rotary_dim, self.key_width), dtype=tensors["uk"].dtype,
                                  device=tensors["uk"].device)

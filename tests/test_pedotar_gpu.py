@@ -504,6 +504,18 @@ def test_far_tokens_decide_the_logits_in_prompt_and_in_decoding(tmp_path):
         close_logits(feed(model, "cut", ids, [15, 17, 300, 2, 31]), want, dtype, f"far tokens, portions, {dtype}")
 
 
+@pytest.mark.parametrize("scale", [-0.07, 0.0])
+def test_latent_attention_with_scores_that_are_turned_round_or_all_equal(tmp_path, scale):
+    """A scale of any sign at the head sizes whose prompts have their keys formed: prompt, portions and single tokens."""
+    config = {"architecture": "Pedotar", "vocab": 90, "width": 128, "norm": {"eps": 1e-5},
+              "layers": [dict(latent(16, 128, 64, 128, 72, scale), mlp=None)]}
+    ids = random_ids(np.random.default_rng(5), 90, 200)
+    folder = make_folder(tmp_path, config, seed=3, dtype="bfloat16")
+    model = load(folder, "bfloat16", 16, 50)
+    for label, cuts in (("whole", [200]), ("portions", [90, 100, 1, 9])):
+        close_logits(feed(model, label, ids, cuts), reference(folder, ids), "bfloat16", label)
+
+
 @pytest.mark.parametrize("dim,page", [(24, 8), (64, 4), (128, 16)])
 def test_the_edges_of_a_run_and_the_mixture_of_heads_show_in_the_logits(tmp_path, dim, page):
     """Two layers with runs of 37 and 21 positions: the plain implementation with runs one token longer or shorter, or
