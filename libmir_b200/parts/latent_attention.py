@@ -115,8 +115,8 @@ class LatentAttention(Mixer):
             self.w_values = tensors["uv"].contiguous()
 
     def weight_bytes(self):
-        return sum(t.numel() * t.element_size() for t in (self.w_in, self.w_uq, self.w_uk, self.w_uv, self.w_o)
-                   if t is not None)
+        tensors = (self.w_in, self.w_uq, self.w_uk, self.w_uv, self.w_o, self.w_keys, self.w_values)
+        return sum(t.numel() * t.element_size() for t in tensors if t is not None)
 
     def forward(self, ctx, cache, x, residual, overwrite=False):
         """residual += W_o (...) (or residual = with `overwrite`, for a mixer that combines several branches)."""

@@ -220,3 +220,14 @@ def test_a_step_is_walked_in_runs_once_the_scratch_passes_its_bound(monkeypatch)
     assert [run for run, _ in runs] == [slice(0, 7), slice(7, 14), slice(14, 20)]
     assert [held.tolist() for _, held in runs] == [[0, 1, 7, 7, 7], [0, 0, 0, 0, 7], [0, 0, 0, 0, 6]]
     assert all(held.dtype == torch.int32 and held.is_contiguous() for _, held in runs)
+
+
+def test_weights_laid_out_for_portions_are_counted():
+    import torch
+    from types import SimpleNamespace
+    from libmir_b200.parts.latent_attention import LatentAttention
+    part = SimpleNamespace(**{name: torch.empty(3, 5, dtype=torch.bfloat16, device="meta") for name in
+                              ("w_in", "w_uq", "w_uk", "w_uv", "w_o", "w_keys", "w_values")})
+    assert LatentAttention.weight_bytes(part) == 7 * 30
+    part.w_uq = part.w_keys = part.w_values = None
+    assert LatentAttention.weight_bytes(part) == 4 * 30
