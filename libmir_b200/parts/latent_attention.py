@@ -25,7 +25,12 @@ from ..config.spec import PagedKv, ParamSpec
 from ..registry import build_part
 from .base import Mixer
 
-PORTION_QUERIES = 48        # queries of a portion for each key of context from which on keys and values are formed for it
+# From how many queries on a portion's keys and values are formed: PORTION_PAIRS (query, head) pairs, between the two counts.  Below,
+# the folded kernel's one or two waves of CTAs are no longer than forming the context's keys.  Folded / formed, us: 16 heads,
+# 8,000 keys of context, 48 queries 136 / 160, 64 155 / 157, 96 218 / 160; 20,000 keys, 64 queries 317 / 296; 32 heads, 8,000
+# keys, 32 queries 156 / 199, 48 209 / 199, 64 290 / 198; up to 2,000 keys both are bound by their launches.
+PORTION_QUERIES = (48, 64)
+PORTION_PAIRS = 1024
 # The most bytes that may take (47,000 rows of 16 heads of 192 + 128, 24,800 of 32).  What is held is at most twice as much: as
 # the context grows, a buffer for each doubling.
 PORTION_SCRATCH = 512 << 20
@@ -168,24 +173,12 @@ class LatentAttention(Mixer):
             ctx.accumulate(mixed, self.w_o, residual)
 
     def _takes_portions(self, ctx) -> bool:
-        """Whether the step's rows attend over keys and values formed from the cached latents (`_portions`) instead of over
-        the latents themselves.  Forming them costs a pass over every request's whole context, and saves 768 of 1,088
-        multiply-adds for each query and key and the products that fold queries and unfold results, on a kernel that runs
-        at several times the rate: from about 48 queries for each key of context on it is less."""
-        if self.w_keys is None or ctx.decode_only or ctx.single_rows:
-            return False
-        starts, before = ctx.host_query_starts, ctx.host_start_positions
-        portions = [b - a for a, b in zip(starts, starts[1:])]
-        contexts = [n + k for n, k in zip(before, portions)]
-        s = self.spec
-        rows = sum(-(-n // kernels.GATHER_ROWS) for n in contexts) * kernels.GATHER_ROWS
-        scratch = rows * _scratch_per_row(self)
-        return (min(portions, default=0) > 0 and scratch <= PORTION_SCRATCH
-                and sum(p * c for p, c in zip(portions, contexts)) >= PORTION_QUERIES * sum(contexts))
+        """Whether any of the step's requests attends over keys and values formed from its cached latents."""
+        return any(formed for _, _, formed in portion_runs(self, ctx))
 
     def _portions(self, ctx, group, cache, packed, gate, table, magnitude, interleaved):
-        """The mixer's result before its output projection, for portions of prompts: queries of head_dim + rotary numbers
-        against keys and values of every head."""
+        """The mixer's result before its output projection for a step some of whose portions have their keys and values
+        formed: queries of head_dim + rotary numbers, rotated where they are; then every run of request rows its way."""
         s = self.spec
         tokens, dtype = packed.shape[0], self.env.dtype
         per_head = s.head_dim + s.rotary_dim
@@ -205,35 +198,95 @@ class LatentAttention(Mixer):
             kernels.linear(latent_q, self.w_uq, q, alloc=ctx.alloc)
             turned = q.view(tokens, s.heads, per_head)[:, :, s.head_dim:]
             kernels.rope_rows(turned, turned, ctx.positions, table, magnitude, interleaved)
-        starts, before = ctx.host_query_starts, ctx.host_start_positions
-        contexts = [n + b - a for n, a, b in zip(before, starts, starts[1:])]
-        tiles = [-(-n // kernels.GATHER_ROWS) for n in contexts]
-        rows = sum(tiles) * kernels.GATHER_ROWS
         mixed = ctx.alloc((tokens, self.out_width), dtype)
-        with ctx.temporary(rows * _scratch_per_row(self)):
-            gathered = ctx.alloc((rows, self.key_width), dtype)
-            tile_table = ctx.alloc((len(contexts), max(tiles)), torch.int32)
-            kernels.latent_gather(cache.k_pages, group.block_table, ctx.context_lens, cache.page_size, contexts, gathered, tile_table)
-            keys = ctx.alloc((rows, s.heads * per_head), dtype)
-            kernels.linear(gathered, self.w_keys, keys, alloc=ctx.alloc)
-            values = ctx.alloc((rows, self.out_width), dtype)
-            kernels.linear(gathered[:, :s.kv_rank], self.w_values, values, alloc=ctx.alloc)
-            kernels.prefill_attention_wide(q, mixed, keys, values, tile_table, ctx.query_starts, ctx.context_lens, s.heads,
-                                           s.scale, gate)
+        for first, last, formed in portion_runs(self, ctx):
+            if formed:
+                self._attend_formed(ctx, group, cache, q, mixed, gate, first, last)
+                continue
+            begin, end = ctx.host_query_starts[first], ctx.host_query_starts[last]
+            queries = q[begin:end].unflatten(1, (s.heads, per_head))
+            folded = ctx.alloc((end - begin, s.heads, self.key_width), dtype)
+            kernels.head_linear(queries[:, :, :s.head_dim], self.w_uk, folded[:, :, :s.kv_rank])
+            folded[:, :, s.kv_rank:].copy_(queries[:, :, s.head_dim:])
+            attended = ctx.alloc((end - begin, s.heads * s.kv_rank), dtype)
+            self.attend(ctx, group, cache, folded.view(end - begin, s.heads * self.key_width), attended, (first, last))
+            kernels.head_linear(attended.view(end - begin, s.heads, s.kv_rank), self.w_uv,
+                                mixed[begin:end].view(end - begin, s.heads, s.value_dim),
+                                gate[begin:end] if gate is not None else None)
         return mixed
 
-    def attend(self, ctx, group, cache, folded, out):
-        """Every packed row's folded query heads over its request's cached rows: one key head of kv_rank + rotary
-        dims whose first kv_rank dims are the value."""
+    def _attend_formed(self, ctx, group, cache, q, mixed, gate, first, last):
+        """Request rows [first, last): their cached rows in tiles, keys and values of every head by two products, and the
+        tcgen05 attention over them."""
         s = self.spec
+        starts, before = ctx.host_query_starts, ctx.host_start_positions
+        contexts = [before[r] + starts[r + 1] - starts[r] for r in range(first, last)]
+        tiles = [-(-n // kernels.GATHER_ROWS) for n in contexts]
+        rows = sum(tiles) * kernels.GATHER_ROWS
+        context_lens = ctx.context_lens[first:last]
+        with ctx.temporary(rows * _scratch_per_row(self)):
+            gathered = ctx.alloc((rows, self.key_width), self.env.dtype)
+            tile_table = ctx.alloc((len(contexts), max(tiles)), torch.int32)
+            kernels.latent_gather(cache.k_pages, group.block_table[first:last], context_lens, cache.page_size, contexts, gathered,
+                                  tile_table)
+            keys = ctx.alloc((rows, self.q_width), self.env.dtype)
+            kernels.linear(gathered, self.w_keys, keys, alloc=ctx.alloc)
+            values = ctx.alloc((rows, self.out_width), self.env.dtype)
+            kernels.linear(gathered[:, :s.kv_rank], self.w_values, values, alloc=ctx.alloc)
+            kernels.prefill_attention_wide(q, mixed, keys, values, tile_table, ctx.query_starts[first:last + 1], context_lens,
+                                           s.heads, s.scale, gate)
+
+    def attend(self, ctx, group, cache, folded, out, rows=None):
+        """Every packed row's folded query heads over its request's cached rows: one key head of kv_rank + rotary
+        dims whose first kv_rank dims are the value.  rows: the request rows whose tokens `folded` and `out` hold, if not all."""
+        s = self.spec
+        first, last = rows or (0, ctx.num_rows)
+        max_portion, max_context, starts, begin, end = ctx.max_portion, ctx.max_context, ctx.query_starts, 0, folded.shape[0]
+        if rows is not None:
+            begin, end = ctx.host_query_starts[first], ctx.host_query_starts[last]
+            if last <= ctx.single_rows:
+                max_portion, max_context = 1, ctx.single_context
+            else:
+                held = ctx.host_query_starts[first:last + 1]
+                portions = [b - a for a, b in zip(held, held[1:])]
+                max_portion = max(portions)
+                max_context = max(n + k for n, k in zip(portions, ctx.host_start_positions[first:last]))
+            starts = starts[first:last + 1]
+            if begin:
+                starts = starts - begin
         if self.env.dtype == torch.bfloat16 and kernels.latent_attention_takes(self.key_width, s.kv_rank):
             # tensor cores: the (token, head) pairs of a request are the rows of one query matrix over its keys
-            max_pairs = max(1, ctx.max_portion) * s.heads
-            per_partition, partitions = kernels.latent_attention_plan(ctx.num_rows, max_pairs, ctx.max_context)
-            kernels.latent_attention(folded, out, cache.k_pages, group.block_table, ctx.query_starts, ctx.context_lens,
-                                     cache.page_size, s.heads, self.key_width, s.kv_rank, s.scale, max_pairs,
-                                     per_partition, partitions, ctx.alloc)
+            max_pairs = max(1, max_portion) * s.heads
+            per_partition, partitions = kernels.latent_attention_plan(last - first, max_pairs, max_context)
+            kernels.latent_attention(folded, out, cache.k_pages, group.block_table[first:last], starts,
+                                     ctx.context_lens[first:last], cache.page_size, s.heads, self.key_width, s.kv_rank, s.scale,
+                                     max_pairs, per_partition, partitions, ctx.alloc)
             return
-        kernels.paged_attention_generic(folded, out, cache.k_pages, None, group.block_table, ctx.row_of_token,
-                                        ctx.positions, cache.page_size, s.heads, 1, self.key_width, s.scale, None,
+        kernels.paged_attention_generic(folded, out, cache.k_pages, None, group.block_table, ctx.row_of_token[begin:end],
+                                        ctx.positions[begin:end], cache.page_size, s.heads, 1, self.key_width, s.scale, None,
                                         value_dim=s.kv_rank, values_in_keys=True)
+
+
+def portion_runs(part, ctx) -> list:
+    """The step's request rows as runs (first, last + 1, formed) in their order: whether a request attends over keys and values
+    formed from its cached latents, or over the latents themselves, follows from its own portion and context and not from
+    what else is in the step.  Forming them costs a pass over the request's whole context, and saves 768 of 1,088 multiply-adds
+    for each query and key and the products that fold queries and unfold results, on a kernel that runs at several times
+    the rate.  The requests of a formed run take PORTION_SCRATCH together at most; one that takes more is not formed."""
+    if part.w_keys is None or ctx.decode_only:
+        return []
+    needed = min(PORTION_QUERIES[1], max(PORTION_QUERIES[0], -(-PORTION_PAIRS // part.spec.heads)))
+    runs, held = [(0, ctx.single_rows, False)] if ctx.single_rows else [], 0
+    starts = ctx.host_query_starts
+    for row in range(ctx.single_rows, len(starts) - 1):
+        before = ctx.host_start_positions[row]
+        portion = starts[row + 1] - starts[row]
+        scratch = -(-(before + portion) // kernels.GATHER_ROWS) * kernels.GATHER_ROWS * _scratch_per_row(part)
+        formed = portion >= needed and scratch <= PORTION_SCRATCH
+        if runs and runs[-1][2] == formed and not (formed and held + scratch > PORTION_SCRATCH):
+            runs[-1] = (runs[-1][0], row + 1, formed)
+            held += scratch
+        else:
+            runs.append((row, row + 1, formed))
+            held = scratch
+    return runs

@@ -231,3 +231,25 @@ def test_weights_laid_out_for_portions_are_counted():
     assert LatentAttention.weight_bytes(part) == 7 * 30
     part.w_uq = part.w_keys = part.w_values = None
     assert LatentAttention.weight_bytes(part) == 4 * 30
+
+
+def test_a_request_has_its_keys_formed_or_not_whatever_is_beside_it(monkeypatch):
+    from types import SimpleNamespace
+    from libmir_b200.parts import latent_attention
+
+    def runs(portions, befores, heads=16):
+        part = SimpleNamespace(w_keys=object(), key_width=576, out_width=heads * 128,
+                               spec=SimpleNamespace(heads=heads, head_dim=128, rotary_dim=64))
+        ctx = SimpleNamespace(decode_only=False, single_rows=portions.count(1),
+                              host_query_starts=[sum(portions[:i]) for i in range(len(portions) + 1)], host_start_positions=befores)
+        return latent_attention.portion_runs(part, ctx)
+    # decoding requests beside a portion, a short portion with a long context beside long ones
+    assert runs([1, 1, 512], [900, 3, 0]) == [(0, 2, False), (2, 3, True)]
+    assert runs([1, 64, 30, 200, 300], [900, 0, 20000, 0, 5]) == [(0, 1, False), (1, 2, True), (2, 3, False), (3, 5, True)]
+    assert runs([63, 64], [0, 0]) == [(0, 1, False), (1, 2, True)]           # 16 heads
+    assert runs([47, 48], [0, 0], heads=32) == [(0, 1, False), (1, 2, True)]
+    assert runs([60, 60], [0, 9]) == [(0, 2, False)]
+    # requests that take more than the scratch together go one run behind the other, one that takes more alone is not formed
+    row = (576 + 16 * 320) * 2
+    monkeypatch.setattr(latent_attention, "PORTION_SCRATCH", 3 * 128 * row)
+    assert runs([128, 130, 128, 100, 385], [0] * 5) == [(0, 2, True), (2, 4, True), (4, 5, False)]

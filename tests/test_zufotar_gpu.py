@@ -676,6 +676,40 @@ def test_portions_attend_over_keys_and_values_formed_from_latents(tmp_path):
     assert kernels.prefill_attention_error() == 0
 
 
+@pytest.mark.parametrize("scratch", [512 << 20, 3 << 20])
+def test_steps_that_form_keys_for_some_requests_and_not_for_others(tmp_path, monkeypatch, scratch):
+    """Single tokens, short and long portions in one step, in an order in which neither kind's rows lie together; and long ones
+    whose scratch does not fit together."""
+    from libmir_b200 import StepEntry, kernels
+    from libmir_b200.parts import latent_attention
+    monkeypatch.setattr(latent_attention, "PORTION_SCRATCH", scratch)
+    mixer = {"heads": 16, "dim": 128, "rot_dim": 64, "vdim": 128, "q_rank": 40, "kv_rank": 72, "scale": 0.07, "rot": {"dims": 64, "base": 1000.0}}
+    config = {"architecture": "Zufotar", "vocab": 101, "width": 128, "norm": {"eps": 1e-6}, "embedding": {"scale": 1.0},
+              "layers": [{"type": "latent_attention", "mlp": {"kind": "dense", "ff": 64}, "mixer": mixer}]}
+    folder = make_folder(tmp_path, config, seed=7, dtype="bfloat16")
+    rng = np.random.default_rng(4)
+    model = load(folder, "bfloat16", 16, 200)
+    lengths = {"a": 300, "b": 260, "c": 270, "d": 150}
+    ids = {name: random_ids(rng, config["vocab"], n) for name, n in lengths.items()}
+    cursor = dict.fromkeys(ids, 0)
+    got = {name: [] for name in ids}
+    for name in ids:
+        model.admit(name)
+    for counts in ({"a": 150, "b": 9, "c": 100}, {"a": 1, "b": 200, "c": 20, "d": 70}, {"a": 149, "b": 51, "c": 150, "d": 80}):
+        before = kernels.launch_counts().get("latent_gather", 0)
+        step = [StepEntry(name, ids[name][cursor[name]:cursor[name] + n], range(n)) for name, n in counts.items()]
+        logits = model.step(step).logits.cpu().numpy()
+        at = 0
+        for name, n in counts.items():
+            got[name].append(logits[at:at + n].copy())
+            cursor[name] += n
+            at += n
+        assert kernels.launch_counts().get("latent_gather", 0) > before
+    for name in ids:
+        close_logits(np.concatenate(got[name]), reference(folder, ids[name][:cursor[name]]), "bfloat16", name)
+    assert kernels.prefill_attention_error() == 0
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["A", "C", "D"])
 def test_batches_of_unequal_requests_with_pages_and_slots_that_change_hands(tmp_path, name, dtype):
