@@ -1174,10 +1174,11 @@ int launch_grouped_as(cudaStream_t stream, const float* qkv, const float* beta, 
                           dim3(tokens / kGroup + rows, (heads + 3) / 4), dim3(32, 4), 0, stream, 0, qkv, beta, decay,
                           query_starts, positions, grouped, rows, heads, kv_heads, key_dim, value_dim);
   if (status != MIR_OK) return status;
-  // Four columns a lane once their CTAs are enough for most SMs (1,400 and 874 tokens, 16 heads: 267 us, 310 with two), else
-  // two (2,048 tokens, 16 heads: 64 CTAs of four columns would leave most of the chip idle).
-  const long long ctas = (long long)rows * heads * ((value_dim + kScanWarps * 8 - 1) / (kScanWarps * 8));
-  if (ctas * 3 >= 2LL * mir_sm_count())
+  // Two columns a lane while their CTAs get an SM each, else four, half as many CTAs with twice the columns for a group's reads.
+  // 1,000 tokens, heads of 128, two / four columns: one request of 16 heads (128 CTAs of two columns) 134 / 187 us, of 20
+  // heads (160 CTAs) 211 / 188, of 24 216 / 192, of 32 220 / 196; two requests of 32 heads 426 / 323.
+  const long long ctas = (long long)rows * heads * ((value_dim + kScanWarps * 4 - 1) / (kScanWarps * 4));
+  if (ctas > mir_sm_count())
     return launch_grouped_walk<PER, 4>(stream, grouped, qkv, state, query_starts, state_slots, positions, out, rows, heads, kv_heads,
                                        key_dim, value_dim);
   return launch_grouped_walk<PER, 2>(stream, grouped, qkv, state, query_starts, state_slots, positions, out, rows, heads, kv_heads,
