@@ -306,8 +306,9 @@ constexpr int kFetchWarps = 4;          // that copy what the others will need
 constexpr int kScanThreads = (kScanWarps + kFetchWarps) * 32;
 constexpr int kScanChunk = 16;          // tokens whose inputs one stage of shared memory holds
 constexpr int kScanStages = 3;
+constexpr int kScanLanes = 16, kScanColumns = 2;   // lanes that share a column of the state, columns a lane holds
 
-// The recurrence.  LANES lanes share C columns of S (C value channels of one head): lane l holds the key channels
+// The recurrence.  LANES = 16 lanes share C = 2 columns of S (C value channels of one head): lane l holds the key channels
 // 4 (m LANES + l) .. + 3 for m < PER / 4 in registers, so a warp works on 32 / LANES * C columns at once, the two dot
 // products per token are log2(LANES) shuffle steps, and the state of a column (stored [head][value channel][key
 // channel]) is read and written in 16-byte pieces that lie side by side across the lanes.  The inputs of a token are
@@ -322,16 +323,21 @@ constexpr int kScanStages = 3;
 // lanes beside the next token's S^T k, a lane has C columns that share a token's inputs, and the arithmetic goes two
 // numbers an instruction.  Every number is formed by the same operations in the same order
 // whatever the step's shape, so a request's 32-bit results do not depend on how it was cut.
+// Sixteen lanes with two columns each read a token's inputs half as often as eight lanes with one: a prompt of 2,048 tokens at
+// 16 / 32 heads of 128 x 128 takes 375 / 520 us with a decay per channel (eight lanes: 476 / 707, thirty-two with four columns:
+// 413 / 570; before the fetching warps: 630 / 870) and 345 / 465 with one per head.  One choice for every shape of step, so
+// that a request's 32-bit results do not depend on how it was cut.
 //   qkv    [tokens, 2 G D + H V] 32-bit: unit q | unit k | v (delta_rule_prepare)
 //   beta   [tokens, H]; decay [tokens, H D] (PER_CHANNEL) or [tokens, H]
 //   state  [slots, H, V, D] 32-bit;  out [tokens, H V] 32-bit: o before the head norm
-template <int LANES, int PER, int C, bool PER_CHANNEL>
+template <int PER, bool PER_CHANNEL>
 __global__ void __launch_bounds__(kScanThreads, 2)
 delta_rule_scan_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
                        float* __restrict__ state, const int* __restrict__ query_starts,
                        const int* __restrict__ state_slots, const int* __restrict__ positions,
                        float* __restrict__ out, int heads, int kv_heads, int key_dim, int value_dim) {
   static_assert(PER % 4 == 0, "a lane holds whole 16-byte pieces");
+  constexpr int LANES = kScanLanes, C = kScanColumns;
   extern __shared__ __align__(16) float staged[];              // [kScanStages][kScanChunk tokens][row]
   grid_launch_dependents();
   grid_dependency_wait();
@@ -1063,20 +1069,17 @@ int launch_gated_wide_norm(const float* o, const TG* gate, long long ld_gate, co
 }
 constexpr int kWideNormColumns = 512, kWideNormLimit = 16384;   // rows of these widths take a CTA each
 
-// How many lanes share a column of the state: 0 lets the launcher choose, 8 / 16 / 32 fix it (for measurements).
-int g_scan_lanes = 0;
-
-template <int LANES, int PER, int C, bool PER_CHANNEL>
+template <int PER, bool PER_CHANNEL>
 int launch_scan_as(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
                    const int* query_starts, const int* state_slots, const int* positions, float* out, int rows,
                    int heads, int kv_heads, int key_dim, int value_dim) {
-  constexpr int columns = kScanWarps * (32 / LANES) * C;
-  constexpr int padded = LANES * PER;
+  constexpr int columns = kScanWarps * (32 / kScanLanes) * kScanColumns;
+  constexpr int padded = kScanLanes * PER;
   constexpr int row = 2 * padded + (PER_CHANNEL ? padded : 4) + 4 + columns;
   constexpr size_t smem = (size_t)kScanStages * kScanChunk * row * sizeof(float);
   static bool raised = false;                                    // more than 48 KB of shared memory needs the opt-in
   if (smem > 48 * 1024 && !raised) {
-    const cudaError_t err = cudaFuncSetAttribute(delta_rule_scan_kernel<LANES, PER, C, PER_CHANNEL>,
+    const cudaError_t err = cudaFuncSetAttribute(delta_rule_scan_kernel<PER, PER_CHANNEL>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) {
       mir_set_error("delta_rule_scan: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(err));
@@ -1084,7 +1087,7 @@ int launch_scan_as(cudaStream_t stream, const float* qkv, const float* beta, con
     }
     raised = true;
   }
-  return mir_launch("delta_rule_scan", delta_rule_scan_kernel<LANES, PER, C, PER_CHANNEL>,
+  return mir_launch("delta_rule_scan", delta_rule_scan_kernel<PER, PER_CHANNEL>,
                     dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps + kFetchWarps), smem, stream, 0, qkv,
                     beta, decay, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
 }
@@ -1119,34 +1122,21 @@ template <bool PER_CHANNEL>
 int launch_scan(cudaStream_t stream, const float* qkv, const float* beta, const float* decay, float* state,
                 const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
                 int kv_heads, int key_dim, int value_dim, bool single_tokens) {
-#define MIR_SCAN(L, P)                                                                                              \
-  return launch_scan_as<L, P, L / 8, PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, \
-                                           out, rows, heads, kv_heads, key_dim, value_dim);
-  // 0: chosen here.  Sixteen lanes with two columns each read a token's inputs half as often as eight lanes with one:
-  // a prompt of 2,048 tokens at 16 / 32 heads of 128 x 128 takes 375 / 520 us with a decay per channel (eight lanes: 476 / 707,
-  // thirty-two: 413 / 570; before the fetching warps: 630 / 870) and 345 / 465 with one per head.
-  // One choice for every shape of step, so that a request's 32-bit results do not depend on how it was cut.
-  const int lanes = g_scan_lanes ? g_scan_lanes : 16;
-  if (single_tokens && lanes == 16 && key_dim <= 256)
+  if (key_dim > 32 * kMaxPerLane) {
+    mir_set_error("delta_rule_scan: key_dim %d is larger than %d", key_dim, 32 * kMaxPerLane);
+    return MIR_BAD_ARGUMENT;
+  }
+  if (single_tokens)
     return launch_step<PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, rows, heads,
                                     kv_heads, key_dim, value_dim);
-  if (lanes == 8) {
-    if (key_dim <= 32) { MIR_SCAN(8, 4) }
-    if (key_dim <= 64) { MIR_SCAN(8, 8) }
-    if (key_dim <= 96) { MIR_SCAN(8, 12) }
-    if (key_dim <= 128) { MIR_SCAN(8, 16) }
-  }
-  if (lanes <= 16) {
-    if (key_dim <= 64) { MIR_SCAN(16, 4) }
-    if (key_dim <= 128) { MIR_SCAN(16, 8) }
-    if (key_dim <= 192) { MIR_SCAN(16, 12) }
-    if (key_dim <= 256) { MIR_SCAN(16, 16) }
-  }
-  if (key_dim <= 128) { MIR_SCAN(32, 4) }
-  if (key_dim <= 256) { MIR_SCAN(32, 8) }
+#define MIR_SCAN(P)                                                                                                  \
+  return launch_scan_as<P, PER_CHANNEL>(stream, qkv, beta, decay, state, query_starts, state_slots, positions, out, rows, \
+                                        heads, kv_heads, key_dim, value_dim)
+  if (key_dim <= 64) MIR_SCAN(4);
+  if (key_dim <= 128) MIR_SCAN(8);
+  if (key_dim <= 192) MIR_SCAN(12);
+  MIR_SCAN(16);
 #undef MIR_SCAN
-  mir_set_error("delta_rule_scan: key_dim %d is larger than %d", key_dim, 32 * kMaxPerLane);
-  return MIR_BAD_ARGUMENT;
 }
 
 template <int PER, int C>
@@ -1268,12 +1258,6 @@ MIR_EXPORT int mir_delta_rule_prepare(int bf16, int decay_f32, const void* x, lo
                       (const __nv_bfloat16*)x, ldx, tail, query_starts, state_slots, positions, channels, taps, 1);
   return mir_launch("short_conv_tail", short_conv_tail_kernel<float>, tail_grid, dim3(threads), 0, stream, 0,
                     (const float*)x, ldx, tail, query_starts, state_slots, positions, channels, taps, 1);
-}
-
-MIR_EXPORT int mir_delta_rule_set_lanes(int lanes) {
-  if (lanes != 0 && lanes != 8 && lanes != 16 && lanes != 32) { mir_set_error("delta_rule: lanes are 0, 8, 16 or 32"); return MIR_BAD_ARGUMENT; }
-  g_scan_lanes = lanes;
-  return MIR_OK;
 }
 
 // qkv, beta, decay as delta_rule_prepare leaves them; per_channel: decay is [tokens, heads * key_dim].  grouped: null, or

@@ -68,7 +68,6 @@ _SIGNATURES = {
                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
         "mir_delta_rule_scan": [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                 c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
-        "mir_delta_rule_set_lanes": [c_int],
         "mir_gated_head_norm": [c_int, c_int, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int,
                                 c_float, c_int, c_int, c_void_p],
         "mir_activation": [c_int, c_int, c_void_p, c_size_t, c_void_p],
@@ -647,17 +646,6 @@ def delta_rule_scan(qkv: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor, 
                                         state.data_ptr(), query_starts.data_ptr(), state_slots.data_ptr(),
                                         positions.data_ptr(), out.data_ptr(), _ptr(grouped), tokens, rows, heads, kv_heads,
                                         key_dim, value_dim, _stream()))
-
-
-def set_delta_rule_lanes(lanes: int) -> None:
-    """For measurements: how many lanes share one column of the delta rule's state (8, 16 or 32; 0: the launcher's
-    own choice)."""
-    for name in _LIBS or {"core": None}:
-        lib = library(name)
-        if hasattr(lib, "mir_delta_rule_set_lanes"):
-            lib.mir_delta_rule_set_lanes.argtypes = [c_int]
-            lib.mir_delta_rule_set_lanes.restype = c_int
-            _check(lib, lib.mir_delta_rule_set_lanes(int(lanes)))
 
 
 def gated_head_norm(o: torch.Tensor, gate: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, heads: int,
