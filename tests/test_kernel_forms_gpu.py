@@ -303,3 +303,81 @@ def test_a_recurrence_walked_in_runs_of_the_steps_tokens(monkeypatch, wkv, limit
             assert torch.equal(got, want)
         else:
             assert float((got - want).norm() / want.norm()) <= 2e-6
+
+
+def portions_alone(run, counts, *tokens):
+    """What `run` gives for each request in a step of its own: run(slot, tensors of its tokens) -> (out, state)."""
+    starts = np.concatenate([[0], np.cumsum(counts)])
+    return [run(r, *(t[..., starts[r]:starts[r + 1], :] for t in tokens)) for r in range(len(counts))]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim", [(2, 64), (24, 64), (32, 64), (64, 64), (64, 20), (150, 6), (40, 33), (70, 96)])
+def test_wkv_walks_with_one_two_and_four_columns_a_lane(dtype, heads, dim):
+    """Three requests (portions of every remainder of a run and a chunk) against the recurrence in 64 bits, and bit for bit against each
+    request alone, which takes fewer columns a lane."""
+    from libmir_b200 import kernels
+    torch.manual_seed(heads + dim)
+    counts, width = [37, 2, 50], heads * dim
+    tokens = sum(counts)
+    x = (torch.randn(3, tokens, width, device="cuda") * 0.5).to(dtype)
+    raw, bias, bonus = torch.randn(tokens, width, device="cuda") - 2, torch.randn(width, device="cuda"), torch.randn(width, device="cuda")
+    state0 = torch.randn(4, heads, dim, dim, device="cuda")
+    slots = [2, 0, 3]
+
+    def run(rows, x, raw, lengths):
+        _, starts, held, positions = batch(lengths, rows)
+        state, out = state0.clone(), torch.full((sum(lengths), width), float("nan"), device="cuda")
+        kernels.wkv_scan(x[0], x[1], x[2], raw, bias, bonus, state, starts, held, positions, out, heads, dim)
+        return out, state
+    out, state = run(slots, x, raw, counts)
+    assert torch.equal(state[1], state0[1])
+    begin = 0
+    per_head = lambda t: t.double().view(heads, dim)
+    for r, (alone, alone_state) in enumerate(portions_alone(lambda r, x, raw: run([slots[r]], x, raw.contiguous(), [raw.shape[0]]),
+                                                            counts, x, raw)):
+        assert torch.equal(alone, out[begin:begin + counts[r]]) and torch.equal(alone_state[slots[r]], state[slots[r]])
+        s = state0[slots[r]].double()                             # [head, value, key]
+        for t in range(begin, begin + counts[r]):
+            q, k, v = (per_head(x[i, t]) for i in range(3))
+            want = torch.einsum("hvk,hk->hv", s, q) + (q * per_head(bonus) * k).sum(-1, keepdim=True) * v
+            w = torch.exp(-torch.exp(per_head(raw[t]) + per_head(bias)))
+            s = s * w[:, None, :] + v[:, :, None] * k[:, None, :]
+            assert float((per_head(out[t]) - want).norm() / want.norm()) <= 2e-6
+        assert float((state[slots[r]].double() - s).norm() / s.norm()) <= 2e-6
+        begin += counts[r]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("heads,dim,value_dim", [(2, 64, 64), (24, 64, 65), (24, 30, 9), (24, 128, 130), (60, 32, 1), (24, 64, 128), (9, 200, 70)])
+def test_retention_walks_with_two_and_four_columns_a_lane(dtype, heads, dim, value_dim):
+    from libmir_b200 import kernels
+    torch.manual_seed(heads + value_dim)
+    counts = [37, 2, 50]
+    tokens, qk, width = sum(counts), heads * dim, heads * value_dim
+    packed = (torch.randn(tokens, 2 * qk + width, device="cuda") * 0.5).to(dtype)
+    decays = torch.rand(heads, device="cuda") * 0.2 + 0.8
+    state0 = torch.randn(4, heads, value_dim, dim, device="cuda")
+    slots = [2, 0, 3]
+
+    def run(rows, packed, lengths):
+        _, starts, held, positions = batch(lengths, rows)
+        state, out = state0.clone(), torch.full((sum(lengths), width), float("nan"), device="cuda")
+        prepared = torch.full((kernels.retention_prepared_floats(sum(lengths), heads, dim),), float("nan"), device="cuda")
+        kernels.retention_scan(packed[:, :qk], packed[:, qk:2 * qk], packed[:, 2 * qk:], None, decays, 0.25, state, starts, held, positions,
+                               out, heads, dim, value_dim, prepared=prepared)
+        return out, state
+    out, state = run(slots, packed, counts)
+    assert torch.equal(state[1], state0[1])
+    begin = 0
+    for r, (alone, alone_state) in enumerate(portions_alone(lambda r, packed: run([slots[r]], packed, [packed.shape[0]]), counts, packed)):
+        assert torch.equal(alone, out[begin:begin + counts[r]]) and torch.equal(alone_state[slots[r]], state[slots[r]])
+        s = state0[slots[r]].double()
+        for t in range(begin, begin + counts[r]):
+            q, k = (packed[t, i * qk:(i + 1) * qk].double().view(heads, dim) for i in range(2))
+            v = packed[t, 2 * qk:].double().view(heads, value_dim)
+            s = s * decays.double()[:, None, None] + 0.25 * v[:, :, None] * k[:, None, :]
+            want = torch.einsum("hvk,hk->hv", s, q)
+            assert float((out[t].double().view(heads, value_dim) - want).norm() / want.norm()) <= 2e-6
+        assert float((state[slots[r]].double() - s).norm() / s.norm()) <= 2e-6
+        begin += counts[r]
