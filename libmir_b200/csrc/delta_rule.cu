@@ -516,11 +516,13 @@ delta_rule_scan_kernel(const float* __restrict__ qkv, const float* __restrict__ 
 
 // A step of single tokens: the same operations on every number in the same order as delta_rule_scan_kernel (sixteen lanes a
 // column; C columns a lane, whose number changes no result), but a token's inputs go from global memory to registers and
-// nothing is staged: a step reads and writes the state once and has no next token to fetch for.
+// nothing is staged: a step reads and writes the state once and has no next token to fetch for.  WIDE (16-byte accesses, as
+// `wide` above) is known to the compiler, so that all loads are on their way before the first number is used: with a branch for
+// it between them one row of 16 heads of 128 took 3.4 us.
 // What bounds it: the bytes of the state.  64 rows of 32 heads of 128 x 128 61 us with a decay per channel (the walk's kernel 108), 49 with
 // one a head (105), 268 MB either way; eight rows of 16 heads 4.9 us (7.6), two rows 3.6 (3.3).
 // blockDim (32, kScanWarps), grid (rows, heads, ceil(value_dim / (kScanWarps * 2 C))).
-template <int PER, int C, bool PER_CHANNEL>
+template <int PER, int C, bool PER_CHANNEL, bool WIDE>
 __global__ void __launch_bounds__(kScanWarps * 32)
 delta_rule_step_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
                        float* __restrict__ state, const int* __restrict__ query_starts, const int* __restrict__ state_slots,
@@ -531,26 +533,25 @@ delta_rule_step_kernel(const float* __restrict__ qkv, const float* __restrict__ 
   grid_dependency_wait();
   const int lane = threadIdx.x, l = lane % LANES;
   const int row = blockIdx.x, head = blockIdx.y;
-  const int start = query_starts[row], end = query_starts[row + 1];
+  const int start = query_starts[row], end = query_starts[row + 1], slot = state_slots[row];
   if (end <= start || positions[start] < 0) return;             // the whole CTA: an empty or padding row
   const int column = blockIdx.z * (COLUMNS * kScanWarps) + threadIdx.y * COLUMNS + lane / LANES * C;
   const int width = 2 * kv_heads * key_dim + heads * value_dim, kv_head = head / (heads / kv_heads);
-  const bool wide = key_dim % 4 == 0 && width % 4 == 0;
-  float* column_state = state + (((size_t)state_slots[row] * heads + head) * value_dim + column) * key_dim;
+  float* column_state = state + (((size_t)slot * heads + head) * value_dim + column) * key_dim;
   Pair s[C][PER / 2];
 #pragma unroll
   for (int c = 0; c < C; ++c)
-    load_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, column + c < value_dim, wide);
+    load_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, column + c < value_dim, WIDE);
   const int my_column = lane_sum<C>(l);                          // of the C columns, the one whose read-out this lane writes
   for (int at = start; at < end; ++at) {                         // (one token, but for steps whose other rows are empty)
     const float* from = qkv + (size_t)at * width + (size_t)kv_head * key_dim;
     const float* value_of = qkv + (size_t)at * width + (size_t)2 * kv_heads * key_dim + (size_t)head * value_dim;
     const float* g_of = decay + ((size_t)at * heads + head) * (PER_CHANNEL ? key_dim : 1);
     Pair q[PER / 2], k[PER / 2], g[PER_CHANNEL ? PER / 2 : 1];
-    load_column<LANES, PER>(k, from + (size_t)kv_heads * key_dim, l, key_dim, true, wide);
-    if constexpr (PER_CHANNEL) load_column<LANES, PER>(g, g_of, l, key_dim, true, wide);
+    load_column<LANES, PER>(k, from + (size_t)kv_heads * key_dim, l, key_dim, true, WIDE);
+    if constexpr (PER_CHANNEL) load_column<LANES, PER>(g, g_of, l, key_dim, true, WIDE);
     else g[0] = pair_from(*g_of, *g_of);
-    load_column<LANES, PER>(q, from, l, key_dim, true, wide);
+    load_column<LANES, PER>(q, from, l, key_dim, true, WIDE);
     const float factor = beta[(size_t)at * heads + head];
     float value[C], total[C], parts[C];
 #pragma unroll
@@ -586,7 +587,7 @@ delta_rule_step_kernel(const float* __restrict__ qkv, const float* __restrict__ 
   }
 #pragma unroll
   for (int c = 0; c < C; ++c)
-    if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, wide);
+    if (column + c < value_dim) store_column<LANES, PER>(s[c], column_state + (size_t)c * key_dim, l, key_dim, WIDE);
 }
 
 // The recurrence four tokens at a time, for prompts whose results may be grouped by where the step begins (the bfloat16 engine;
@@ -1097,7 +1098,9 @@ int launch_step_as(cudaStream_t stream, const float* qkv, const float* beta, con
                    const int* query_starts, const int* state_slots, const int* positions, float* out, int rows, int heads,
                    int kv_heads, int key_dim, int value_dim) {
   constexpr int columns = kScanWarps * 2 * C;
-  return mir_launch("delta_rule_step", delta_rule_step_kernel<PER, C, PER_CHANNEL>,
+  const bool wide = key_dim % 4 == 0 && (2 * kv_heads * key_dim + heads * value_dim) % 4 == 0;
+  return mir_launch("delta_rule_step", wide ? delta_rule_step_kernel<PER, C, PER_CHANNEL, true>
+                                            : delta_rule_step_kernel<PER, C, PER_CHANNEL, false>,
                     dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps), 0, stream, 0, qkv, beta,
                     decay, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
 }
