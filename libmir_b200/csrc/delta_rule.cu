@@ -917,53 +917,68 @@ __global__ void gated_head_norm_kernel(const float* __restrict__ o, const TG* __
   }
 }
 
-// The same for heads of up to 128 numbers in whole 16-byte pieces: LANES lanes take a (token, head), four numbers each, and ask
-// for the gate and the weight with the head (the kernel above reads the head twice and the rest behind the sum: 2,274 tokens
-// of 16 heads of 128 18 us, here 12; two tokens 4.4, here 2.1).
-template <typename T, typename TG, int LANES>
-__global__ void __launch_bounds__(128) gated_quad_norm_kernel(const float* __restrict__ o, const TG* __restrict__ gate,
-                                                              long long ld_gate, const float* __restrict__ weight,
-                                                              T* __restrict__ out, int units, int heads, int value_dim, float eps,
-                                                              int sigmoid_gate, int weight_per_head) {
+// The same for heads of up to LANES * PIECES numbers, which LANES lanes hold in registers: the head is read once, and its gate and
+// weight asked for with it (the kernel above reads the head twice and the rest behind the sum: 2,274 tokens of 16 heads of 128
+// 13.1 us, here 11.2, of 64 heads of 64 40.8, here 20.8; two tokens of 16 heads of 128 3.0, here 2.0).  The sum is that of the
+// kernel above, bit for bit: there lane L has the numbers L, L + 32, ..., and the lanes' sums are added 16, 8, 4, 2 and 1
+// apart; with 16 or 8 lanes a lane has the numbers of two or four of those lanes, and the first steps are its own.
+template <typename T, typename TG, int LANES, int PIECES>
+__global__ void __launch_bounds__(128) gated_row_norm_kernel(const float* __restrict__ o, const TG* __restrict__ gate,
+                                                             long long ld_gate, const float* __restrict__ weight,
+                                                             T* __restrict__ out, int units, int heads, int value_dim, float eps,
+                                                             int sigmoid_gate, int weight_per_head) {
   grid_launch_dependents();
   const int unit = blockIdx.x * (128 / LANES) + threadIdx.x / LANES;       // token * heads + head
-  const int d = threadIdx.x % LANES * 4;
-  const bool live = unit < units && d < value_dim;
-  const int head = unit % heads;
-  float4 scale = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v = scale, z = scale;
-  if (live) scale = *reinterpret_cast<const float4*>(weight + (weight_per_head ? (size_t)head * value_dim : 0) + d);
+  const int l = threadIdx.x % LANES, head = unit % heads;
+  const int count = unit < units ? value_dim : 0;                          // (a warp's last heads may not be there)
+  const float* scale = weight + (weight_per_head ? (size_t)head * value_dim : 0);
+  const TG* gate_row = gate + (size_t)(unit / heads) * ld_gate + (size_t)head * value_dim;
+  const float* src = o + (size_t)unit * value_dim;
+  float w[PIECES], v[PIECES];
+  TG z[PIECES];
+#pragma unroll
+  for (int e = 0; e < PIECES; ++e) w[e] = l + LANES * e < count ? scale[l + LANES * e] : 0.0f;
   grid_dependency_wait();
-  if (live) {
-    v = *reinterpret_cast<const float4*>(o + (size_t)unit * value_dim + d);
-    z = quad_of(gate + (size_t)(unit / heads) * ld_gate + (size_t)head * value_dim + d);
-  }
-  float sum = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+#pragma unroll
+  for (int e = 0; e < PIECES; ++e) v[e] = l + LANES * e < count ? src[l + LANES * e] : 0.0f;
+#pragma unroll
+  for (int e = 0; e < PIECES; ++e) z[e] = l + LANES * e < count ? gate_row[l + LANES * e] : from_float<TG>(0.0f);
+  constexpr int OWN = 32 / LANES;                                // of the 32 sums, those of l, l + LANES, ...
+  float sums[OWN];
+#pragma unroll
+  for (int i = 0; i < OWN; ++i) sums[i] = 0.0f;
+#pragma unroll
+  for (int e = 0; e < PIECES; ++e) sums[e % OWN] = fmaf(v[e], v[e], sums[e % OWN]);
+#pragma unroll
+  for (int half = OWN / 2; half > 0; half >>= 1)
+#pragma unroll
+    for (int i = 0; i < half; ++i) sums[i] += sums[i + half];
+  float sum = sums[0];
 #pragma unroll
   for (int step = LANES / 2; step > 0; step >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, step);
-  if (!live) return;
   const float inverse = rsqrtf(sum / (float)value_dim + eps);
-  auto act = [&](float x) { return sigmoid_gate ? sigmoid(x) : silu(x); };
-  v = make_float4(v.x * inverse * scale.x * act(z.x), v.y * inverse * scale.y * act(z.y), v.z * inverse * scale.z * act(z.z),
-                  v.w * inverse * scale.w * act(z.w));
-  T* to = out + (size_t)unit * value_dim + d;
-  if constexpr (sizeof(T) == 4) {
-    *reinterpret_cast<float4*>(to) = v;
-  } else {
-    uint2 packed;
-    *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(v.x, v.y);
-    *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(v.z, v.w);
-    *reinterpret_cast<uint2*>(to) = packed;
+#pragma unroll
+  for (int e = 0; e < PIECES; ++e) {
+    const float gated = to_float(z[e]);
+    const float act = sigmoid_gate ? sigmoid(gated) : silu(gated);
+    if (l + LANES * e < count) out[(size_t)unit * value_dim + l + LANES * e] = from_float<T>(v[e] * inverse * w[e] * act);
   }
 }
 
 template <typename T, typename TG>
-int launch_gated_quad_norm(const float* o, const TG* gate, long long ld_gate, const float* weight, T* out, int units, int heads,
-                           int value_dim, float eps, int sigmoid_gate, int weight_per_head, cudaStream_t stream) {
-  if (value_dim <= 64)
-    return mir_launch("gated_head_norm", gated_quad_norm_kernel<T, TG, 16>, dim3((units + 7) / 8), dim3(128), 0, stream, 0, o, gate,
-                      ld_gate, weight, out, units, heads, value_dim, eps, sigmoid_gate, weight_per_head);
-  return mir_launch("gated_head_norm", gated_quad_norm_kernel<T, TG, 32>, dim3((units + 3) / 4), dim3(128), 0, stream, 0, o, gate,
+int launch_gated_norm(const float* o, const TG* gate, long long ld_gate, const float* weight, T* out, int units, int heads,
+                      int value_dim, float eps, int sigmoid_gate, int weight_per_head, cudaStream_t stream) {
+#define MIR_NORM(LANES, PIECES)                                                                                           \
+  return mir_launch("gated_head_norm", gated_row_norm_kernel<T, TG, LANES, PIECES>,                                      \
+                    dim3((units + 128 / LANES - 1) / (128 / LANES)), dim3(128), 0, stream, 0, o, gate, ld_gate, weight, out, units, \
+                    heads, value_dim, eps, sigmoid_gate, weight_per_head)
+  if (value_dim <= 32) MIR_NORM(8, 4);
+  if (value_dim <= 64) MIR_NORM(16, 4);
+  if (value_dim <= 128) MIR_NORM(32, 4);
+  if (value_dim <= 256) MIR_NORM(32, 8);
+  return mir_launch("gated_head_norm", gated_head_norm_kernel<T, TG>, dim3((units + 3) / 4), dim3(32, 4), 0, stream, 0, o, gate,
                     ld_gate, weight, out, units, heads, value_dim, eps, sigmoid_gate, weight_per_head);
+#undef MIR_NORM
 }
 
 // The same for wide rows (a norm over all heads at once): one CTA per (token, head), its sum by a fixed tree.  A thread keeps
@@ -1309,27 +1324,12 @@ MIR_EXPORT int mir_gated_head_norm(int bf16, int gate_f32, const float* o, const
     return launch_gated_wide_norm(o, (const float*)gate, ld_gate, weight, (float*)out, units, heads, value_dim, eps,
                                   sigmoid_gate, weight_per_head, stream);
   }
-  const size_t out_size = bf16 ? 2 : 4, gate_size = bf16 && !gate_f32 ? 2 : 4;
-  if (value_dim <= 128 && value_dim % 4 == 0 && ld_gate % 4 == 0 && (((uintptr_t)o | (uintptr_t)weight) & 15) == 0 &&
-      (uintptr_t)gate % (4 * gate_size) == 0 && (uintptr_t)out % (4 * out_size) == 0) {
-    if (bf16 && gate_f32)
-      return launch_gated_quad_norm(o, (const float*)gate, ld_gate, weight, (__nv_bfloat16*)out, units, heads, value_dim, eps,
-                                    sigmoid_gate, weight_per_head, stream);
-    if (bf16)
-      return launch_gated_quad_norm(o, (const __nv_bfloat16*)gate, ld_gate, weight, (__nv_bfloat16*)out, units, heads, value_dim,
-                                    eps, sigmoid_gate, weight_per_head, stream);
-    return launch_gated_quad_norm(o, (const float*)gate, ld_gate, weight, (float*)out, units, heads, value_dim, eps, sigmoid_gate,
-                                  weight_per_head, stream);
-  }
-  const dim3 grid((units + 3) / 4), block(32, 4);
   if (bf16 && gate_f32)
-    return mir_launch("gated_head_norm", gated_head_norm_kernel<__nv_bfloat16, float>, grid, block, 0, stream, 0, o,
-                      (const float*)gate, ld_gate, weight, (__nv_bfloat16*)out, units, heads, value_dim, eps, sigmoid_gate,
-                      weight_per_head);
+    return launch_gated_norm(o, (const float*)gate, ld_gate, weight, (__nv_bfloat16*)out, units, heads, value_dim, eps,
+                             sigmoid_gate, weight_per_head, stream);
   if (bf16)
-    return mir_launch("gated_head_norm", gated_head_norm_kernel<__nv_bfloat16, __nv_bfloat16>, grid, block, 0, stream, 0, o,
-                      (const __nv_bfloat16*)gate, ld_gate, weight, (__nv_bfloat16*)out, units, heads, value_dim, eps,
-                      sigmoid_gate, weight_per_head);
-  return mir_launch("gated_head_norm", gated_head_norm_kernel<float, float>, grid, block, 0, stream, 0, o, (const float*)gate,
-                    ld_gate, weight, (float*)out, units, heads, value_dim, eps, sigmoid_gate, weight_per_head);
+    return launch_gated_norm(o, (const __nv_bfloat16*)gate, ld_gate, weight, (__nv_bfloat16*)out, units, heads, value_dim, eps,
+                             sigmoid_gate, weight_per_head, stream);
+  return launch_gated_norm(o, (const float*)gate, ld_gate, weight, (float*)out, units, heads, value_dim, eps, sigmoid_gate,
+                           weight_per_head, stream);
 }

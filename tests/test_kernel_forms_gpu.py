@@ -381,3 +381,33 @@ def test_retention_walks_with_two_and_four_columns_a_lane(dtype, heads, dim, val
             assert float((out[t].double().view(heads, value_dim) - want).norm() / want.norm()) <= 2e-6
         assert float((state[slots[r]].double() - s).norm() / s.norm()) <= 2e-6
         begin += counts[r]
+
+
+@pytest.mark.parametrize("dtype,gate_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32), (torch.bfloat16, torch.bfloat16)])
+@pytest.mark.parametrize("value_dim,heads", [(1, 3), (32, 5), (33, 3), (64, 7), (65, 2), (128, 5), (200, 3), (256, 2), (257, 3)])
+@pytest.mark.parametrize("per_head", [False, True])
+def test_gated_norms_of_heads_sum_in_one_order_whatever_holds_them(dtype, gate_dtype, value_dim, heads, per_head):
+    """Eight, 16 and 32 lanes a head, and heads that are read twice: lane l of 32 sums the numbers l, l + 32, ... and
+    the lanes' sums are added by halves; gates off the 16-byte boundary."""
+    from libmir_b200 import kernels
+    torch.manual_seed(value_dim)
+    tokens = 5
+    o, gate = torch.randn(tokens, heads * value_dim), torch.randn(tokens, heads * value_dim + 3).to(gate_dtype)
+    weight = torch.rand(heads * value_dim if per_head else value_dim) + 0.5
+    rows = np.zeros((tokens * heads, -(-value_dim // 32) * 32))
+    rows[:, :value_dim] = o.double().numpy().reshape(tokens * heads, value_dim)
+    total = np.zeros((tokens * heads, 32))
+    for piece in np.split(rows, rows.shape[1] // 32, axis=1):
+        total = rounded(piece * piece + total)
+    for step in (16, 8, 4, 2, 1):
+        total = rounded(total + total[:, np.arange(32) ^ step])
+    mean = total[:, 0].astype(np.float32) / np.float32(value_dim) + np.float32(1e-5)
+    inverse = torch.rsqrt(torch.from_numpy(mean).cuda()).view(tokens, heads, 1)
+    out = torch.empty(tokens, heads * value_dim, dtype=dtype, device="cuda")
+    kernels.gated_head_norm(o.cuda(), gate.cuda()[:, 3:], weight.cuda(), out, heads, value_dim, 1e-5, False)
+    z = gate[:, 3:].double().view(tokens, heads, value_dim)
+    scaled = o.cuda().view(tokens, heads, value_dim) * inverse * weight.cuda().view(-1, value_dim)
+    want = scaled.double().cpu() * z * torch.sigmoid(z)
+    # the gate's own function is good to a few units in the last place; with the sum in another order a row would be off as a whole
+    error = (out.double().cpu().view_as(want) - want).abs()
+    assert bool((error <= (2 ** -8 if dtype == torch.bfloat16 else 4e-7) * want.abs() + 1e-30).all())
