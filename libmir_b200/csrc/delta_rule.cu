@@ -317,8 +317,7 @@ constexpr int kScanLanes = 16, kScanColumns = 2;   // lanes that share a column 
 // (rows, heads, ceil(value_dim / (kScanWarps * 32 / LANES * C))).
 //
 // What bounds it: the chain from one token's state to the next (a decay, a dot product of PER channels, the sum over the
-// lanes, the write's factor and a multiply-add) and the instructions of the one walking warp a scheduler has, which can
-// hide little of each other.  So what can be kept away from that warp is: the copies and their addresses belong to the
+// lanes, the write's factor and a multiply-add) on the one walking warp a scheduler has, which can hide little of it.  So what can be kept away from that warp is: the copies and their addresses belong to the
 // fetching warps, a token's inputs are in registers before the token before it ends, the read-out is summed over the
 // lanes beside the next token's S^T k, a lane has C columns that share a token's inputs, and the arithmetic goes two
 // numbers an instruction.  Every number is formed by the same operations in the same order
@@ -712,8 +711,9 @@ delta_rule_group_kernel(const float* __restrict__ qkv, const float* __restrict__
 // The walk over groups: lanes, columns, roles and stages as in delta_rule_scan_kernel, LANES = 16.  A group costs its chain one
 // sum over the lanes (4 C sums together, each in a lane of its own), one exchange and the four short sums, where four
 // tokens one after the other cost four of each.
-// What bounds it: shared memory.  A lane reads PER numbers of thirteen vectors a group whatever the columns it has, and a
-// warp's 16-byte read takes four cycles though its halves read the same: so C columns a lane cost 52 / C cycles a column.
+// What bounds it: one walking warp a scheduler, which issues in 0.38 (C = 2) and 0.49 (C = 4) of the cycles and otherwise waits
+// on shared memory, shuffles and the latency of the operation before; shared memory's data path is 0.60 and 0.49 busy: a lane
+// reads PER numbers of thirteen vectors a group whatever the columns it has, so C columns a lane cost 52 / C cycles a column.
 // 2,048 tokens with the group kernel, decay per channel / head: 16 heads 268 / 266 us (a token at a time 377 / 345), 32 heads
 // 392 / 388 (521 / 466); 1,400 and 874 tokens, 16 heads 267 / 264 (360 / 321), 32 heads 448 / 442 (598 / 537).
 template <int PER, int C>

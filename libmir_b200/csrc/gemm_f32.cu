@@ -13,7 +13,8 @@
 //                   each, 4.2 us for 2,048), which several CTAs on an SM, each with a ring of four
 //                   stages of 128 k that two warps of its own fill, hide behind the reads (3 rows, the products of
 //                   a layer of 2,048 with 5,504 inside: 27.6 us on average; all warps filling the ring: 29.5).
-//   gemm_f32_tile   more rows: bound by the multiply-adds.  A thread owns TM x TN outputs whose rows and columns lie
+//   gemm_f32_tile   more rows: bound by issue slots, 0.76 of them taken by 3.4 warps a scheduler (the multiply-adds' pipe 0.58
+//                   busy, shared memory's data path 0.61).  A thread owns TM x TN outputs whose rows and columns lie
 //                   (tile / threads) apart, and reads four k of each with one load.
 #include "common.cuh"
 

@@ -263,8 +263,9 @@ retention_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, long 
 // stages).  Several tokens' inputs are in registers at a time, their read-outs are summed over the lanes together, and the
 // arithmetic goes two numbers an instruction.
 // blockDim (32, kWarps + kFetchWarps), grid (rows, heads, ceil(value_dim / (kWarps * 32 / kLanes * C))).
-// What bounds it: the walking warps' instructions.  One column a lane spends four reads of shared memory on 24 operations of
-// the state; with C columns those reads are shared.
+// What bounds it: one walking warp a scheduler, which issues in 0.36 (C = 2) and 0.46 (C = 4) of the cycles and otherwise waits on
+// the latency of the operation before and on shared memory, whose data path is 0.46 and 0.41 busy.  One column a lane spends
+// four reads of shared memory on 24 operations of the state; with C columns those reads are shared.
 template <typename T, int PER, int kLanes, int C>
 __global__ void __launch_bounds__((kWarps + kFetchWarps) * 32, 2)
 retention_scan_prepared_kernel(const float* __restrict__ prepared, const T* __restrict__ v, long long ld,
@@ -450,7 +451,9 @@ int launch_prepared(cudaStream_t stream, const void* q, const void* k, const voi
 #define MIR_WALK(C)                                                                                                    \
   return launch_walk<T, PER, kLanes, C>(stream, prepared, v, ld, decays, state, query_starts, state_slots, positions, \
                                         out, rows, heads, dim, value_dim, activated)
-  // More columns a lane share a token's reads of shared memory; fewer fill the GPU with the heads of few requests.
+  // More columns a lane share a token's reads of shared memory; fewer fill the GPU with the heads of few requests: two until their
+  // CTAs have to share an SM (1,000 tokens, heads of 128, two / four columns: 16 heads, 128 CTAs, 113 / 133 us; 20 heads, 160
+  // CTAs, 152 / 136; heads of 64: 36 heads, 144 CTAs, 91 / 105, 40 heads, 160 CTAs, 116 / 106).
   const int narrow = kWarps * (32 / kLanes) * 2;                  // columns of a CTA with two a lane
   if constexpr (PER <= 8)
     if ((long long)rows * heads * ((value_dim + narrow - 1) / narrow) > mir_sm_count()) MIR_WALK(4);

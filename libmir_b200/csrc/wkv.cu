@@ -250,9 +250,10 @@ wkv_prepare_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __
 // state's arithmetic, two numbers an instruction; several tokens' inputs are in registers at a time and their read-outs
 // are summed over the lanes together.
 // blockDim (32, kScanWarps + kFetchWarps), grid (rows, heads, ceil(dim / (kScanWarps * 4 C))).
-// What bounds it: the walking warps' instructions, one warp on a scheduler.  C is chosen by the launcher.  A prompt of 2,048
-// tokens with 32 / 64 heads of 64 x 64, the preparation included: 224 / 257 us (640 / 693 when the walking warps also formed
-// the decays).
+// What bounds it: one walking warp a scheduler, which issues in 0.24 (C = 1) and 0.32 (C = 2) of the cycles and otherwise waits on
+// shared memory and on the latency of the operation before; shared memory's data path is 0.57 busy.  C is chosen by the
+// launcher.  A prompt of 2,048 tokens with 32 / 64 heads of 64 x 64, the preparation included: 224 / 257 us (640 / 693 when
+// the walking warps also formed the decays).
 constexpr int kFetchWarps = 4, kChunk = 16, kStages = 3;
 template <int PER, int C>
 __global__ void __launch_bounds__((kScanWarps + kFetchWarps) * 32, 2)
@@ -396,7 +397,9 @@ int launch_scan_for(cudaStream_t stream, const void* r, const void* k, const voi
   if (status != MIR_OK) return status;
 #define MIR_WKV(C)                                                                                                       \
   return launch_walk<PER, C>(stream, prepared, state, query_starts, state_slots, positions, out, rows, heads, dim)
-  // More columns a lane share a token's reads of shared memory; fewer fill the GPU with the heads of few requests.
+  // More columns a lane share a token's reads of shared memory; fewer fill the GPU with the heads of few requests: one, two or four
+  // as the CTAs of one column are up to an SM's worth, up to two, or more (1,000 tokens, heads of 64, one / two / four: 144
+  // CTAs 115 / 119 / 159 us, 160 170 / 122 / 160, 288 185 / 136 / 175, 320 328 / 190 / 178).
   if constexpr (PER <= 8) {
     const long long units = (long long)rows * heads * ((dim + 15) / 16);     // CTAs with one column a lane
     if (units > 2LL * mir_sm_count()) MIR_WKV(4);
