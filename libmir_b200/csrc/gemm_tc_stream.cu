@@ -63,15 +63,35 @@ struct StreamNorm {
   int activation;            // store epilogue: 0 none, 1 the tanh GELU of the result, 2 the exact (erf) GELU, 3 relu squared
 };
 
+// The products of routed experts on a few rows sorted by expert (csrc/moe.cu): tiles[2 i], tiles[2 i + 1] are the expert and
+// the first row of row tile i, which ends with its expert's rows, offsets[expert + 1], or after `tile_rows` of them;
+// tile_count[0] row tiles in all.  Expert e's weight rows start at row e * expert_rows; the result of sorted row r goes to
+// row scatter[r] of out (to row r without scatter).  list_ready: the lists were complete before any CTA of the kernel in
+// front could release this one, so weights may be asked for before that kernel is over.
+struct StreamGroups {
+  const int* tiles;
+  const int* tile_count;
+  const int* offsets;
+  const int* scatter;
+  int expert_rows, column_tiles, tile_rows, list_ready;
+};
+
 // (Shared memory lets three CTAs share an SM; the registers are capped as if six did: 56 instead of up to 95 per
 // thread, no spills, and the captured decode step at Qwen3-4B sizes takes 2.621 instead of 2.638 ms at batch 8,
 // 2.226 instead of 2.241 ms at batch 1.)
-template <int MODE>
+// GROUPED (routed experts; SWIGLU and F32 only): a CTA's row tile and its expert come from a list on the device.  The
+// weights then do depend on an earlier kernel; the gate-up product releases its dependents only behind its own wait, so that
+// the down product behind it finds the lists complete and fills its ring while the gate-up product drains (list_ready).
+// Bound by the experts' weights: three tokens of width 2,048, 6 of 64 experts of 1,024 each, 16 experts hit: gate-up 25 us and
+// down 11 us (134 and 67 MB, 20.5 and 10.3 us at the copy rate) where tiles of 128 pairs (csrc/gemm_tc.cu) took 32 and 19;
+// one token 13 and 6.5 us against 22 and 14.
+template <int MODE, bool GROUPED>
 __global__ void __launch_bounds__(kThreads, 6)
 tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
                  const void* __restrict__ bias, void* __restrict__ out, int ldo, int m, int n, int k, int up_offset,
-                 int tokens, int tile_rows, int stages, int stage_stride, uint32_t tmem_columns, StreamNorm norm) {
-  grid_launch_dependents();
+                 int tokens, int tile_rows, int stages, int stage_stride, uint32_t tmem_columns, StreamNorm norm,
+                 StreamGroups groups) {
+  if (!GROUPED || groups.list_ready) grid_launch_dependents();
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long barriers[2 * kMaxStages + 1];
   __shared__ uint32_t tmem_base_slot;
@@ -82,7 +102,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
   // tile_rows output features per CTA (128, 64 or 32; with the SwiGLU epilogue 64 gate and 64 up rows).  The A
   // operand always spans 128 rows of shared memory: rows beyond the tile hold whatever was there, and the
   // accumulator rows they produce are never read.
-  const int n0 = blockIdx.x * tile_rows;
+  const int n0 = (GROUPED ? (int)blockIdx.x % groups.column_tiles : (int)blockIdx.x) * tile_rows;
   const uint32_t weight_bytes = (MODE == SWIGLU ? 128u : (uint32_t)tile_rows) * 128u;
   const int total_steps = (k + kStepK - 1) / kStepK;
   const int per_split = (total_steps + splits - 1) / splits;
@@ -111,6 +131,29 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
   __syncthreads();
   tensor_fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  int x0 = 0, w0 = n0;                                        // first row of the activations and of the weights
+  if (GROUPED) {
+    if (!groups.list_ready) {
+      grid_dependency_wait();
+      grid_launch_dependents();
+    }
+    const int slot = blockIdx.x / groups.column_tiles;
+    m = 0;
+    // (volatile: the lists may be read before the wait, and then not through a line that this SM's L1 still holds)
+    const volatile int* list = groups.tiles;
+    if (slot < *(const volatile int*)groups.tile_count) {
+      const int expert = list[2 * slot];
+      x0 = list[2 * slot + 1];
+      w0 = expert * groups.expert_rows + n0;
+      m = min(groups.tile_rows, ((const volatile int*)groups.offsets)[expert + 1] - x0);
+    }
+    if (m <= 0) {                                             // fewer tiles than the launch allowed for: the whole cluster returns
+      if (warp == 1)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_columns) : "memory");
+      grid_dependency_wait();
+      return;
+    }
+  }
   MIR_TRACE_BEGIN(stream, (blockIdx.x == 0 && blockIdx.y == 0) || (blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1),
                   2 * MODE + (blockIdx.x == 0 && blockIdx.y == 0 ? 0 : 1))
   if (threadIdx.x == 0) MIR_TRACE_POINT(stream, 0);
@@ -122,8 +165,8 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
       auto load_weights = [&](int i, uint32_t barrier, uint32_t dst) {
         const int k0 = (step_begin + i) * kStepK;
         barrier_expect_bytes(barrier, stage_bytes);
-        tma_load_2d(dst, &w_map, barrier, k0, n0);
-        if (MODE == SWIGLU) tma_load_2d(dst + kWeightBytes / 2, &w_map, barrier, k0, up_offset + n0);
+        tma_load_2d(dst, &w_map, barrier, k0, w0);
+        if (MODE == SWIGLU) tma_load_2d(dst + kWeightBytes / 2, &w_map, barrier, k0, up_offset + w0);
       };
       // The weights belong to no kernel: the whole ring is filled with them before this kernel waits for the one
       // before it, whose results are only the activations.  Launched with programmatic stream serialization, the
@@ -137,7 +180,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
       MIR_TRACE_POINT(stream, 2);
       for (int i = 0; i < ahead; ++i)
         tma_load_2d(smem_base + (uint32_t)i * (uint32_t)stage_stride + weight_bytes, &x_map, full0 + 8 * i,
-                    (step_begin + i) * kStepK, 0);
+                    (step_begin + i) * kStepK, x0);
       MIR_TRACE_POINT(stream, 3);
       // (the stage and its parity are counted, not divided: `ahead` stages are filled, so step `ahead` takes stage
       // ahead % stages = 0 when the ring was filled, in its second turn)
@@ -148,7 +191,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         const uint32_t barrier = full0 + 8 * stage;
         const uint32_t dst = smem_base + (uint32_t)stage * (uint32_t)stage_stride;
         load_weights(i, barrier, dst);
-        tma_load_2d(dst + weight_bytes, &x_map, barrier, (step_begin + i) * kStepK, 0);
+        tma_load_2d(dst + weight_bytes, &x_map, barrier, (step_begin + i) * kStepK, x0);
         if (++stage == stages) { stage = 0; parity ^= 1u; }
       }
     }
@@ -192,9 +235,11 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
     // While the products run: what the epilogue needs from earlier kernels.  Per token 1, or the folded norm's
     // rsqrt(mean of squares + eps) (8 threads per token add the tiles' sums); and the old residual values.
     grid_dependency_wait();
-    if (tid < kNormStatStride) scale[tid] = 1.0f;
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (norm.sumsq != nullptr) {
+    if (!GROUPED) {
+      if (tid < kNormStatStride) scale[tid] = 1.0f;
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    }
+    if (!GROUPED && norm.sumsq != nullptr) {
       const int token = tid >> 2, part = tid & 3;              // 4 threads per token, 32 tokens
       float sum = 0.0f;
       if (token < m)
@@ -203,7 +248,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
       for (int o = 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
       if (part == 0) scale[token] = rsqrtf(sum / (float)k + norm.eps);
     }
-    if (MODE != SWIGLU && tid < tile_rows && n0 + tid < n) {
+    if (!GROUPED && MODE != SWIGLU && tid < tile_rows && n0 + tid < n) {
       if (bias != nullptr)
         extra = MODE == STORE ? __bfloat162float(reinterpret_cast<const bf16*>(bias)[n0 + tid])
                               : reinterpret_cast<const float*>(bias)[n0 + tid];
@@ -279,9 +324,9 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         for (int j = 0; j < BATCH; ++j) {
           const int token = token0 + j * stride;
           if (token < m && column < n) {
-            const float s = token < kNormStatStride ? scale[token] : 1.0f;
+            const float s = !GROUPED && token < kNormStatStride ? scale[token] : 1.0f;
             const float g = gate[j] * s;
-            reinterpret_cast<bf16*>(out)[(size_t)token * ldo + column] = __float2bfloat16_rn(g / (1.0f + __expf(-g)) * (up[j] * s));
+            reinterpret_cast<bf16*>(out)[(size_t)(x0 + token) * ldo + column] = __float2bfloat16_rn(g / (1.0f + __expf(-g)) * (up[j] * s));
           }
         }
       }
@@ -306,9 +351,12 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         for (int j = 0; j < BATCH; ++j) {
           const int token = token0 + j * splits;
           if (token >= m) break;                              // the same for every thread
-          const float result = value[j] * (token < kNormStatStride ? scale[token] : 1.0f) + extra + old[j];
+          const float result = GROUPED ? value[j] : value[j] * (token < kNormStatStride ? scale[token] : 1.0f) + extra + old[j];
           if (in_range) {
-            if (MODE == STORE) {
+            if (GROUPED) {
+              const int row = groups.scatter != nullptr ? groups.scatter[x0 + token] : x0 + token;
+              reinterpret_cast<float*>(out)[(size_t)row * ldo + column] = result;
+            } else if (MODE == STORE) {
               float stored = result;
               if (norm.activation == 1) {                     // 0.5 z (1 + tanh(sqrt(2 / pi) (z + 0.044715 z^3)))
                 float t;
@@ -326,7 +374,7 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
                 norm.weighted_out[(size_t)token * norm.ld_weighted + column] = __float2bfloat16_rn(result * next_weight);
             }
           }
-          if (MODE == F32 && norm.best_value != nullptr) {
+          if (!GROUPED && MODE == F32 && norm.best_value != nullptr) {
             // The head's logits: what a sampler asks first is each row's largest one.  Every warp leaves the best of
             // its 32 columns, so that the sampling kernel looks at V / 32 candidates instead of V logits.
             const bool counts = in_range && isfinite(result);
@@ -369,26 +417,29 @@ int g_forced_rows = 0;
 // beat 64- and 32-row tiles at every shape (QKV 9.0 / 15.5 / 18.1, output projection 7.7 / 10.5 / 11.5), and K is
 // best cut as far as one wave of CTAs allows (three fit on an SM): output projection 7.7 with 8 CTAs per tile,
 // 10.4 with 4, 16.8 with 2.
-void choose_shape(int n, int total_steps, bool swiglu, int* tile_rows, int* splits) {
+void choose_shape(int n, int total_steps, bool swiglu, int slots, int* tile_rows, int* splits) {
   const int rows = swiglu ? 64 : 128;
-  const int tiles = (n + rows - 1) / rows;
+  const long long tiles = (long long)((n + rows - 1) / rows) * slots;
   int s = 1;
   while (s < 8 && tiles * s * 2 <= 3 * 148 && total_steps / (s * 2) >= 4) s *= 2;
   *tile_rows = rows;
   *splits = s;
 }
 
-template <int MODE>
+// GROUPED: x [m, k] the sorted rows, w `weight_rows` rows, row tiles of at most groups.tile_rows rows from the device's list,
+// at most `slots` of them.
+template <int MODE, bool GROUPED = false>
 int launch(const void* x, int ldx, const void* w, const void* bias, void* out, int ldo, int m, int n, int k,
-           int up_offset, const StreamNorm& norm, cudaStream_t stream) {
-  const int tokens = (m + 15) / 16 * 16;
+           int up_offset, const StreamNorm& norm, cudaStream_t stream, StreamGroups groups = StreamGroups{}, int weight_rows = 0,
+           int slots = 1) {
+  const int tokens = GROUPED ? groups.tile_rows : (m + 15) / 16 * 16;
   const int total_steps = (k + kStepK - 1) / kStepK;
   int tile_rows, splits;
-  choose_shape(n, total_steps, MODE == SWIGLU, &tile_rows, &splits);
+  choose_shape(n, total_steps, MODE == SWIGLU, slots, &tile_rows, &splits);
   if (g_forced_splits > 0) splits = g_forced_splits;
-  if (g_forced_rows > 0 && MODE != SWIGLU) tile_rows = g_forced_rows;
+  if (g_forced_rows > 0 && MODE != SWIGLU && !GROUPED) tile_rows = g_forced_rows;
   CUtensorMap w_map, x_map;
-  int status = tensor_map_for(w, MODE == SWIGLU ? up_offset + n : n, k, k, tile_rows, &w_map);
+  int status = tensor_map_for(w, GROUPED ? weight_rows : MODE == SWIGLU ? up_offset + n : n, k, k, tile_rows, &w_map);
   if (status != MIR_OK) return status;
   status = tensor_map_for(x, m, k, ldx, tokens, &x_map);
   if (status != MIR_OK) return status;
@@ -401,7 +452,7 @@ int launch(const void* x, int ldx, const void* w, const void* bias, void* out, i
   const size_t smem = (size_t)stages * stage_stride + std::max(0, kWeightBytes - stage_stride) + 1024;
   static bool configured = false;
   if (!configured) {
-    const cudaError_t err = cudaFuncSetAttribute(tc_stream_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const cudaError_t err = cudaFuncSetAttribute(tc_stream_kernel<MODE, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  208 * 1024);
     if (err != cudaSuccess) {
       mir_set_error("tc_stream: cannot reserve shared memory: %s", cudaGetErrorString(err));
@@ -410,10 +461,13 @@ int launch(const void* x, int ldx, const void* w, const void* bias, void* out, i
     configured = true;
   }
   const int tiles = (n + tile_rows - 1) / tile_rows;
+  if (GROUPED) groups.column_tiles = tiles;
+  if ((long long)tiles * slots > 0x7fffffffll) { mir_set_error("tc_stream: too many tiles"); return MIR_BAD_ARGUMENT; }
   uint32_t tmem_columns = 32;
   while ((int)tmem_columns < tokens) tmem_columns *= 2;
-  return mir_launch_with(mir_pdl_for_streaming(), "tc_stream", tc_stream_kernel<MODE>, dim3(tiles, splits), dim3(kThreads), smem, stream, splits, w_map,
-                    x_map, bias, out, ldo, m, n, k, up_offset, tokens, tile_rows, stages, stage_stride, tmem_columns, norm);
+  return mir_launch_with(mir_pdl_for_streaming(), GROUPED ? "tc_stream_grouped" : "tc_stream", tc_stream_kernel<MODE, GROUPED>,
+                    dim3(tiles * slots, splits), dim3(kThreads), smem, stream, splits, w_map,
+                    x_map, bias, out, ldo, m, n, k, up_offset, tokens, tile_rows, stages, stage_stride, tmem_columns, norm, groups);
 }
 
 }  // namespace
@@ -498,6 +552,31 @@ MIR_EXPORT int mir_gemm_tc_stream_bf16(int mode, const void* x, int ldx, const v
   }
   mir_set_error("tc_stream: unknown mode %d", mode);
   return MIR_BAD_ARGUMENT;
+}
+
+// The products of routed experts on few rows sorted by expert.  mode 3 (SwiGLU): out bf16 [rows, n] = silu(x w_gate[e]^T) *
+// (x w_up[e]^T) with w = [experts * n gate rows; experts * n up rows]; mode 2: out float [*, n] = x w[e]^T, sorted row r's
+// result in row scatter[r].  tiles / tile_count / offsets: row tiles of tile_pairs (16 to 128, a multiple of 16) rows, their
+// number and the experts' row ranges, all on the device; at most max_tiles of them.  list_ready: these lists were complete
+// before the kernel in front of this one released its dependents (it was the gate-up product on the same lists).  k and ldx
+// multiples of 8, x and w 16-byte aligned.
+MIR_EXPORT int mir_gemm_tc_stream_grouped_bf16(int mode, const void* x, int ldx, int rows, const void* w, int experts,
+                                               void* out, int ldo, int n, int k, const int* tiles, const int* tile_count,
+                                               const int* offsets, const int* scatter, int tile_pairs, int max_tiles,
+                                               int list_ready, cudaStream_t stream) {
+  if (rows == 0 || n == 0) return MIR_OK;
+  if (rows < 0 || n < 0 || k <= 0 || (k % 8) || (ldx % 8) || ldx < k || ldo < n || ((uintptr_t)x & 15) ||
+      ((uintptr_t)w & 15) || experts <= 0 || max_tiles <= 0 || tiles == nullptr || tile_count == nullptr ||
+      offsets == nullptr || tile_pairs < 16 || tile_pairs > 128 || tile_pairs % 16 || (mode != SWIGLU && mode != F32)) {
+    mir_set_error("tc_stream_grouped: needs the SwiGLU or float epilogue, k and the row stride multiples of 8, 16-byte aligned "
+                  "operands and tiles of 16 to 128 rows (mode %d rows %d n %d k %d ldx %d ldo %d tiles of %d)", mode, rows, n, k,
+                  ldx, ldo, tile_pairs);
+    return MIR_BAD_ARGUMENT;
+  }
+  const StreamGroups groups{tiles, tile_count, offsets, scatter, n, 0, tile_pairs, list_ready};
+  if (mode == SWIGLU)
+    return launch<SWIGLU, true>(x, ldx, w, nullptr, out, ldo, rows, n, k, experts * n, StreamNorm{}, stream, groups, 2 * experts * n, max_tiles);
+  return launch<F32, true>(x, ldx, w, nullptr, out, ldo, rows, n, k, 0, StreamNorm{}, stream, groups, experts * n, max_tiles);
 }
 
 // Entries per row that mir_gemm_tc_stream_head_bf16 leaves for n output columns: four per tile of 128 columns.

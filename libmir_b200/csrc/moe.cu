@@ -12,7 +12,9 @@
 //                 from the tokens' rows, and the down projection of the hidden rows into one 32-bit row per pair, as
 //                 32-bit multiply-adds on tiles of 8 pairs (any type and size).  bfloat16 rows of 16-byte pieces run
 //                 the tcgen05 product of csrc/gemm_tc.cu instead, on tiles of 128 pairs of this file's list, after
-//                 moe_gather_rows has brought the tokens' rows into the pairs' order
+//                 moe_gather_rows has brought the tokens' rows into the pairs' order; steps of few tokens run the weight
+//                 streaming product of csrc/gemm_tc_stream.cu behind moe_plan_few, which is the route, the sort and the
+//                 gathering in one kernel
 //   moe_combine   residual[t] += sum over slots of weight * the pair's row (+ gate * the shared expert's row)
 // Everything the host needs to launch them is known before the step: no count is read back.
 #include <cfloat>
@@ -52,24 +54,20 @@ __device__ __forceinline__ void warp_best(float& value, int& index, bool want_ma
   }
 }
 
+// One token's choice by one warp.  z: its logits; score, choice [experts], group_score [groups], chosen [top] (RANKED): shared
+// memory of this warp.  ids_out, weights_out [top]: shared or global memory.
+struct RouteRule {
+  const float* correction;
+  int experts, top, groups, keep;
+  float scale;
+  int softmax_scores, group_by_max;
+};
 template <bool RANKED>
-__global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ correction,
-                                 int has_gate, int* __restrict__ ids, float* __restrict__ weights,
-                                 float* __restrict__ shared_gate, int tokens, int experts, int top, int groups, int keep,
-                                 float scale, int softmax_scores, int group_by_max) {
-  extern __shared__ float route_shared[];
-  grid_launch_dependents();
-  grid_dependency_wait();
-  const int lane = threadIdx.x, warp = threadIdx.y;
-  const int token = blockIdx.x * kRouteWarps + warp;
-  if (token >= tokens) return;
-  float* score = route_shared + (size_t)warp * (2 * experts + groups + (RANKED ? top : 0));
-  float* choice = score + experts;
-  float* group_score = choice + experts;
-  float* chosen = group_score + groups;
-  const float* z = logits + (size_t)token * ld;
+__device__ __forceinline__ void route_token(const float* __restrict__ z, const RouteRule& rule, float* score, float* choice,
+                                            float* group_score, float* chosen, int lane, int* ids_out, float* weights_out) {
+  const int experts = rule.experts, top = rule.top, groups = rule.groups, keep = rule.keep;
   float softmax_top = 0.0f, softmax_inverse = 1.0f;
-  if (softmax_scores) {                                          // over all the router's experts, in 32-bit
+  if (rule.softmax_scores) {                                     // over all the router's experts, in 32-bit
     float high = -FLT_MAX;
     for (int e = lane; e < experts; e += 32) high = fmaxf(high, z[e]);
     softmax_top = warp_max(high);
@@ -78,30 +76,31 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
     softmax_inverse = 1.0f / warp_sum(sum);
   }
   for (int e = lane; e < experts; e += 32) {
-    const float s = softmax_scores ? expf(z[e] - softmax_top) * softmax_inverse : sigmoid_of(z[e]);
+    const float s = rule.softmax_scores ? expf(z[e] - softmax_top) * softmax_inverse : sigmoid_of(z[e]);
     score[e] = s;
     // (plain softmax scores are in the logits' order: the choice then looks at the logits, which do not underflow)
-    choice[e] = correction != nullptr ? s + correction[e] : (softmax_scores && keep >= groups ? z[e] : s);
+    choice[e] = rule.correction != nullptr ? s + rule.correction[e] : (rule.softmax_scores && keep >= groups ? z[e] : s);
   }
-  if (has_gate && lane == 0) shared_gate[token] = sigmoid_of(z[experts]);
   __syncwarp();
   const int per_group = experts / groups;
   if (keep < groups) {
     // a group's score: the sum of its two largest choice scores (of its one score where a group is one expert)
     for (int g = lane; g < groups; g += 32) {
       float first = -FLT_MAX, second = -FLT_MAX;
+#pragma unroll 8
       for (int e = g * per_group; e < (g + 1) * per_group; ++e) {
         const float c = choice[e];
         if (c > first) { second = first; first = c; }
         else if (c > second) second = c;
       }
-      group_score[g] = (per_group > 1 && !group_by_max) ? first + second : first;
+      group_score[g] = (per_group > 1 && !rule.group_by_max) ? first + second : first;
     }
     __syncwarp();
     // experts of all but the `keep` best groups cannot be chosen: their choice scores count as minus infinity
     if (groups <= 32) {                                          // a group's rank: how many are better (or as good and before it)
       const float mine = lane < groups ? group_score[lane] : 0.0f;
       int rank = 0;
+#pragma unroll 8
       for (int g = 0; g < groups; ++g) {
         const float other = group_score[g];
         rank += other > mine || (other == mine && g < lane);
@@ -129,30 +128,29 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
   if constexpr (RANKED) {
     // An expert's rank among those that can be chosen is its slot: every lane counts for its own experts at once, instead
     // of one search over the warp for each slot (three tokens, 64 experts in 8 groups, 6 chosen: 9.2 us by searches).
-    int choosable = 0;
-    for (int first = 0; first < experts; first += 32) {
-      const int e = first + lane;
-      const float mine = e < experts ? choice[e] : -FLT_MAX;
-      const bool can = mine > -FLT_MAX;
-      int rank = 0;
-      for (int other = 0; other < experts; ++other) {
-        const float theirs = choice[other];
-        rank += theirs > mine || (theirs == mine && other < e);
-      }
-      if (can && rank < top) {
-        ids[(size_t)token * top + rank] = e;
-        chosen[rank] = score[e];
-      }
-      choosable += __popc(__ballot_sync(0xffffffffu, can));
+    // route_by_rank: at most 64 experts, two a lane.
+    const int e0 = lane, e1 = lane + 32;
+    const float mine0 = e0 < experts ? choice[e0] : -FLT_MAX, mine1 = e1 < experts ? choice[e1] : -FLT_MAX;
+    const bool can0 = mine0 > -FLT_MAX, can1 = mine1 > -FLT_MAX;
+    int rank0 = 0, rank1 = 0;
+#pragma unroll 16
+    for (int other = 0; other < experts; ++other) {
+      const float theirs = choice[other];
+      rank0 += theirs > mine0 || (theirs == mine0 && other < e0);
+      rank1 += theirs > mine1 || (theirs == mine1 && other < e1);
     }
+    if (can0 && rank0 < top) { ids_out[rank0] = e0; chosen[rank0] = score[e0]; }
+    if (can1 && rank1 < top) { ids_out[rank1] = e1; chosen[rank1] = score[e1]; }
+    const int choosable = __popc(__ballot_sync(0xffffffffu, can0)) + __popc(__ballot_sync(0xffffffffu, can1));
     for (int slot = choosable + lane; slot < top; slot += 32) {  // (fewer choosable experts than top: not a valid model)
-      ids[(size_t)token * top + slot] = 0;
+      ids_out[slot] = 0;
       chosen[slot] = score[0];
     }
     __syncwarp();
+#pragma unroll 8
     for (int slot = 0; slot < top; ++slot) total += chosen[slot];
-    const float factor = scale / (total + 1e-20f);
-    for (int slot = lane; slot < top; slot += 32) weights[(size_t)token * top + slot] = chosen[slot] * factor;
+    const float factor = rule.scale / (total + 1e-20f);
+    for (int slot = lane; slot < top; slot += 32) weights_out[slot] = chosen[slot] * factor;
   } else {
     for (int slot = 0; slot < top; ++slot) {
       float high = -FLT_MAX;
@@ -166,15 +164,32 @@ __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld,
       if (best < 0) best = 0;                                      // (fewer choosable experts than top: not a valid model)
       if (lane == 0) {
         choice[best] = -FLT_MAX;
-        ids[(size_t)token * top + slot] = best;
-        weights[(size_t)token * top + slot] = score[best];
+        ids_out[slot] = best;
+        weights_out[slot] = score[best];
       }
       total += score[best];
       __syncwarp();
     }
-    const float factor = scale / (total + 1e-20f);
-    for (int slot = lane; slot < top; slot += 32) weights[(size_t)token * top + slot] *= factor;
+    const float factor = rule.scale / (total + 1e-20f);
+    for (int slot = lane; slot < top; slot += 32) weights_out[slot] *= factor;
   }
+}
+
+template <bool RANKED>
+__global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, int has_gate, int* __restrict__ ids,
+                                 float* __restrict__ weights, float* __restrict__ shared_gate, int tokens, RouteRule rule) {
+  extern __shared__ float route_shared[];
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int lane = threadIdx.x, warp = threadIdx.y;
+  const int token = blockIdx.x * kRouteWarps + warp;
+  if (token >= tokens) return;
+  const int experts = rule.experts;
+  float* score = route_shared + (size_t)warp * (2 * experts + rule.groups + (RANKED ? rule.top : 0));
+  const float* z = logits + (size_t)token * ld;
+  if (has_gate && lane == 0) shared_gate[token] = sigmoid_of(z[experts]);
+  route_token<RANKED>(z, rule, score, score + experts, score + 2 * experts, score + 2 * experts + rule.groups, lane,
+                      ids + (size_t)token * rule.top, weights + (size_t)token * rule.top);
 }
 
 // The pairs ordered by expert, in three small kernels.  order[i] = the i-th pair when the pairs are sorted by expert
@@ -229,6 +244,134 @@ moe_sort_few_kernel(const int* __restrict__ ids, int pairs, int experts, int til
 #pragma unroll 8
   for (int p = 0; p < e; ++p) before += id_s[p] == id;
   order[base_s[id] + before] = e;
+}
+
+// Everything between the router's logits and the grouped products for a step of few tokens, in one kernel: a warp routes a
+// token, the pairs are ordered as moe_sort_few_kernel orders them, and the tokens' rows are brought into that order.  Every
+// CTA routes for itself (it takes the time of one token's chain of dependent steps, whoever does it).  The first one leaves
+// the results and the lists; the others hold 16 bytes of one token a thread, asked for beside the logits, and store them at
+// the places of the token's pairs.  A place is counted over all pairs, which needs no barrier but the one behind the routing.
+// It goes over its instructions twice: first, while the kernel in front still runs, on logits of zero, leaving nothing.  A
+// decoded token's weights have pushed this code out of the caches by the time a layer comes here, and a chain of
+// instruction fetches from memory takes longer than the routing.  Three tokens, 64 experts in 8 groups, 6 chosen, rows of
+// 2,048, inside a captured decode step: route, sort and gathering took 6.3 + 3.2 + 2.5 us one behind the other, this kernel
+// 8.1 without the first pass and 5.4 with it.
+// Shared memory: ids [pairs, a multiple of four, the rest INT_MAX] | weights, later the places [pairs] | zeros [experts] |
+// the warps' scratch of route_token.
+constexpr int kPlanThreads = 512;
+template <bool RANKED>
+__global__ void __launch_bounds__(kPlanThreads)
+moe_plan_few_kernel(const float* __restrict__ logits, long long ld, int has_gate, int* __restrict__ ids,
+                    float* __restrict__ weights, float* __restrict__ shared_gate, int tokens, RouteRule rule, int real_experts,
+                    int tile_pairs, int* __restrict__ order, int* __restrict__ offsets, int* __restrict__ tiles,
+                    int* __restrict__ tile_count, const uint4* __restrict__ h, long long ld_pieces, uint4* __restrict__ sorted_rows,
+                    int pieces) {
+  extern __shared__ __align__(16) float plan_shared[];
+  __shared__ int tile_sums[kPlanThreads / 32];
+  const int thread = threadIdx.x, lane = thread & 31, warp = thread >> 5;
+  const int top = rule.top, pairs = tokens * top, quads = (pairs + 3) / 4;
+  const int scratch = 2 * rule.experts + rule.groups + (RANKED ? top : 0);
+  int* id_s = reinterpret_cast<int*>(plan_shared);
+  float* weight_s = plan_shared + 4 * quads;
+  float* zeros = weight_s + pairs;
+  float* scratch_s = zeros + rule.experts;
+  grid_launch_dependents();
+  if (thread < 4) id_s[4 * quads - 1 - thread] = 0x7fffffff;
+  for (int e = thread; e < rule.experts; e += kPlanThreads) zeros[e] = 0.0f;
+  const long long copied = (long long)((int)blockIdx.x - 1) * kPlanThreads + thread;   // of the tokens' pieces
+  const int token = copied >= 0 && copied < (long long)tokens * pieces ? (int)(copied / pieces) : -1;
+  const int piece = (int)(copied - (long long)token * pieces);
+  __syncthreads();
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool real = pass == 1;
+    if (real) grid_dependency_wait();
+    uint4 held = make_uint4(0, 0, 0, 0);
+    if (real && token >= 0) held = h[(size_t)token * ld_pieces + piece];
+#pragma unroll 1
+    for (int t = warp; t < tokens; t += kPlanThreads / 32) {
+      const float* z = real ? logits + (size_t)t * ld : zeros;
+      float* score = scratch_s + (size_t)t * scratch;
+      if (real && has_gate && lane == 0 && blockIdx.x == 0) shared_gate[t] = sigmoid_of(z[rule.experts]);
+      route_token<RANKED>(z, rule, score, score + rule.experts, score + 2 * rule.experts, score + 2 * rule.experts + rule.groups,
+                          lane, id_s + t * top, weight_s + t * top);
+    }
+    __syncthreads();
+    // the place of pair p: the pairs of experts before its own, and those of its own ahead of it; -1 for an identity
+    // expert, whose pairs are left out
+    auto place_of = [&](int p) {
+      const int id = id_s[p];
+      int place = 0;
+#pragma unroll 4
+      for (int q = 0; q < quads; ++q) {
+        const int4 ids4 = reinterpret_cast<const int4*>(id_s)[q];
+        place += ids4.x < id || (ids4.x == id && 4 * q < p);
+        place += ids4.y < id || (ids4.y == id && 4 * q + 1 < p);
+        place += ids4.z < id || (ids4.z == id && 4 * q + 2 < p);
+        place += ids4.w < id || (ids4.w == id && 4 * q + 3 < p);
+      }
+      return id < real_experts ? place : -1;
+    };
+    if (blockIdx.x > 0) {
+      int* place_s = reinterpret_cast<int*>(weight_s);
+      for (int p = thread; p < pairs; p += kPlanThreads) place_s[p] = place_of(p);
+      __syncthreads();
+      if (token >= 0)
+        for (int slot = 0; slot < top; ++slot) {
+          const int place = place_s[token * top + slot];
+          if (real && place >= 0) sorted_rows[(size_t)place * pieces + piece] = held;
+        }
+    } else {
+      for (int p = thread; p < pairs; p += kPlanThreads) {
+        const int place = place_of(p);
+        if (real) {
+          ids[p] = id_s[p];
+          weights[p] = weight_s[p];
+          if (place >= 0) order[place] = p;
+        }
+      }
+      int tiles_before = 0;                                      // tiles of the experts of earlier rounds
+#pragma unroll 1
+      for (int first = 0; first < real_experts; first += kPlanThreads) {
+        const int e = first + thread;
+        int before = 0, mine = 0;                                // pairs of the experts before e, and of e
+#pragma unroll 4
+        for (int q = 0; q < quads; ++q) {
+          const int4 ids4 = reinterpret_cast<const int4*>(id_s)[q];
+          before += (ids4.x < e) + (ids4.y < e) + (ids4.z < e) + (ids4.w < e);
+          mine += (ids4.x == e) + (ids4.y == e) + (ids4.z == e) + (ids4.w == e);
+        }
+        const int my_tiles = e < real_experts ? (mine + tile_pairs - 1) / tile_pairs : 0;
+        int scan = my_tiles;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, scan, o);
+          if (lane >= o) scan += t;
+        }
+        if (lane == 31) tile_sums[warp] = scan;
+        __syncthreads();
+        int base = tiles_before + scan - my_tiles;
+#pragma unroll 4
+        for (int w = 0; w < kPlanThreads / 32; ++w) {
+          if (w < warp) base += tile_sums[w];
+          tiles_before += tile_sums[w];
+        }
+        if (real && e < real_experts) {
+          offsets[e] = before;
+          for (int t = 0; t < my_tiles; ++t) {
+            tiles[2 * (base + t)] = e;
+            tiles[2 * (base + t) + 1] = before + t * tile_pairs;
+          }
+          if (e == real_experts - 1) {
+            offsets[real_experts] = before + mine;
+            tile_count[0] = base + my_tiles;
+          }
+        }
+        __syncthreads();                                         // (tile_sums is written again in the next round)
+      }
+    }
+    __syncthreads();                                             // (the ids are written again in the next pass)
+  }
 }
 
 // One CTA per expert: how many pairs chose it.  (A prompt's 15,000 pairs are a few trips over the L2 for 1,024 threads.)
@@ -447,30 +590,47 @@ __global__ void moe_combine_kernel(float* __restrict__ residual, const float* __
   float total[V];
 #pragma unroll
   for (int v = 0; v < V; ++v) total[v] = 0.0f;
-  for (int s = 0; s < top; ++s) {
-    const size_t pair = (size_t)token * top + s;
-    const float weight = __ldg(weights + pair);
-    alignas(16) float row[V];
-    if (ids != nullptr && __ldg(ids + pair) >= real_experts) {
-      const T* src = identity_rows + (size_t)token * identity_stride + c;
+  const size_t at = (size_t)token * width + c;
+  // What does not depend on the slots, and the rows of kAhead slots, are asked for before the first sum: one trip to memory
+  // for them instead of one for every slot (three tokens, six slots, rows of 2,048: 4.2 us, now 2.4).
+  alignas(16) float old[V], shared[V];
 #pragma unroll
-      for (int v = 0; v < V; ++v) row[v] = to_float(src[v]);
-    } else if (V == 4) {
-      *reinterpret_cast<float4*>(row) = *reinterpret_cast<const float4*>(pair_rows + pair * width + c);
-    } else {
-      row[0] = pair_rows[pair * width + c];
+  for (int v = 0; v < V; ++v) old[v] = overwrite ? 0.0f : residual[at + v];
+#pragma unroll
+  for (int v = 0; v < V; ++v) shared[v] = shared_rows != nullptr ? shared_rows[at + v] : 0.0f;
+  const float gate = shared_rows != nullptr && shared_gate != nullptr ? shared_gate[token] : 1.0f;
+  constexpr int kAhead = 4;
+  for (int s0 = 0; s0 < top; s0 += kAhead) {
+    alignas(16) float row[kAhead][V];
+    float weight[kAhead];
+#pragma unroll
+    for (int j = 0; j < kAhead; ++j) {
+      if (s0 + j >= top) break;
+      const size_t pair = (size_t)token * top + s0 + j;
+      weight[j] = __ldg(weights + pair);
+      if (ids != nullptr && __ldg(ids + pair) >= real_experts) {
+        const T* src = identity_rows + (size_t)token * identity_stride + c;
+#pragma unroll
+        for (int v = 0; v < V; ++v) row[j][v] = to_float(src[v]);
+      } else if (V == 4) {
+        *reinterpret_cast<float4*>(row[j]) = *reinterpret_cast<const float4*>(pair_rows + pair * width + c);
+      } else {
+        row[j][0] = pair_rows[pair * width + c];
+      }
     }
 #pragma unroll
-    for (int v = 0; v < V; ++v) total[v] = fmaf(weight, row[v], total[v]);
+    for (int j = 0; j < kAhead; ++j) {
+      if (s0 + j >= top) break;
+#pragma unroll
+      for (int v = 0; v < V; ++v) total[v] = fmaf(weight[j], row[j][v], total[v]);
+    }
   }
-  const size_t at = (size_t)token * width + c;
   if (shared_rows != nullptr) {
-    const float gate = shared_gate != nullptr ? shared_gate[token] : 1.0f;
 #pragma unroll
-    for (int v = 0; v < V; ++v) total[v] = fmaf(gate, shared_rows[at + v], total[v]);
+    for (int v = 0; v < V; ++v) total[v] = fmaf(gate, shared[v], total[v]);
   }
 #pragma unroll
-  for (int v = 0; v < V; ++v) residual[at + v] = overwrite ? total[v] : residual[at + v] + total[v];
+  for (int v = 0; v < V; ++v) residual[at + v] = overwrite ? total[v] : old[v] + total[v];
 }
 
 template <typename T, typename TO, bool GATED>
@@ -503,8 +663,48 @@ MIR_EXPORT int mir_moe_route(const float* logits, long long ld, const float* cor
   const size_t smem = (size_t)kRouteWarps * (2 * experts + groups + (ranked ? top : 0)) * sizeof(float);
   return mir_launch("moe_route", ranked ? moe_route_kernel<true> : moe_route_kernel<false>,
                     dim3((tokens + kRouteWarps - 1) / kRouteWarps), dim3(32, kRouteWarps), smem, stream, 0, logits, ld,
-                    correction, has_gate, ids, weights, shared_gate, tokens, experts, top, groups, keep, scale,
-                    softmax_scores, group_by_max);
+                    has_gate, ids, weights, shared_gate, tokens,
+                    RouteRule{correction, experts, top, groups, keep, scale, softmax_scores, group_by_max});
+}
+
+// Whether mir_moe_plan_few takes a step of these sizes: places are counted over all pairs, and its shared memory needs no
+// opt-in.
+static size_t plan_few_shared(int tokens, int experts, int top, int groups) {
+  const size_t scratch = 2 * (size_t)experts + groups + (route_by_rank(experts, top) ? top : 0);
+  return (tokens * scratch + 2 * (size_t)tokens * top + 3 + experts) * sizeof(float);
+}
+MIR_EXPORT int mir_moe_plan_few_takes(int tokens, int experts, int real_experts, int top, int groups) {
+  return tokens > 0 && tokens <= 128 && real_experts > 0 && (long long)tokens * top <= kFewPairs && experts <= kMaxExperts &&
+         plan_few_shared(tokens, experts, top, groups) <= 47 * 1024;
+}
+
+// mir_moe_route, mir_moe_sort (tiles of tile_pairs pairs) and mir_moe_gather_rows in one kernel, for the sizes that
+// mir_moe_plan_few_takes says; the arguments are theirs.  `experts` counts the router's experts, `real_experts` those that
+// have weights; h [tokens, width] bfloat16, sorted_rows [tokens * top, width].
+MIR_EXPORT int mir_moe_plan_few(const float* logits, long long ld, const float* correction, int has_gate, int* ids,
+                                float* weights, float* shared_gate, int tokens, int experts, int real_experts, int top,
+                                int groups, int keep, float scale, int softmax_scores, int group_by_max, int tile_pairs,
+                                int* order, int* offsets, int* tiles, int* tile_count, const void* h, long long ld_h,
+                                void* sorted_rows, int width, cudaStream_t stream) {
+  if (tokens == 0) return MIR_OK;
+  if (tokens < 0 || experts <= 0 || experts > kMaxExperts || real_experts <= 0 || real_experts > experts || top <= 0 ||
+      top > experts || groups <= 0 || experts % groups || keep <= 0 || keep > groups ||
+      (long long)keep * (experts / groups) < top || (has_gate && shared_gate == nullptr) || tile_pairs <= 0 || width <= 0 ||
+      width % 8 || ld_h % 8 || ((uintptr_t)h & 15) || ((uintptr_t)sorted_rows & 15) ||
+      !mir_moe_plan_few_takes(tokens, experts, real_experts, top, groups)) {
+    mir_set_error("moe_plan_few: bad sizes (tokens %d, experts %d of which %d have weights, top %d, groups %d of which %d are "
+                  "kept, tiles of %d pairs, rows of %d with stride %lld)", tokens, experts, real_experts, top, groups, keep,
+                  tile_pairs, width, ld_h);
+    return MIR_BAD_ARGUMENT;
+  }
+  const bool ranked = route_by_rank(experts, top);
+  const int pieces = width / 8;
+  const long long copies = ((long long)tokens * pieces + kPlanThreads - 1) / kPlanThreads;
+  return mir_launch_with(mir_pdl_for_streaming(), "moe_plan_few", ranked ? moe_plan_few_kernel<true> : moe_plan_few_kernel<false>,
+                         dim3((unsigned)(1 + copies)), dim3(kPlanThreads), plan_few_shared(tokens, experts, top, groups), stream, 0,
+                         logits, ld, has_gate, ids, weights, shared_gate, tokens,
+                         RouteRule{correction, experts, top, groups, keep, scale, softmax_scores, group_by_max}, real_experts,
+                         tile_pairs, order, offsets, tiles, tile_count, (const uint4*)h, ld_h / 8, (uint4*)sorted_rows, pieces);
 }
 
 // How many tiles of tile_pairs pairs there can be at most for `pairs` pairs over `experts` experts (`tiles` holds two

@@ -94,6 +94,10 @@ _SIGNATURES = {
         "mir_moe_route": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_int, c_float, c_int, c_int, c_void_p],
         "mir_moe_tile_slots": [c_int, c_int, c_int],
+        "mir_moe_plan_few_takes": [c_int] * 5,
+        "mir_moe_plan_few": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+                             c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                             c_longlong, c_void_p, c_int, c_void_p],
         "mir_moe_sort": [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_void_p],
         "mir_moe_gate_up": [c_int, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -184,6 +188,8 @@ _SIGNATURES = {
         "mir_gemm_tc_stream_set_splits": [c_int, c_int, c_int],
         "mir_gemm_tc_bf16": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_void_p],
+        "mir_gemm_tc_stream_grouped_bf16": [c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+                                            c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
         "mir_gemm_tc_grouped_bf16": [c_int, c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p,
                                      c_void_p, c_void_p, c_void_p, c_int, c_void_p],
         "mir_gemm_tc_set_width": [c_int],
@@ -1071,6 +1077,11 @@ class ExpertOrder:
         self.tiles = alloc((2 * slots,), torch.int32)
         self.tile_count = alloc((1,), torch.int32)
         self.scratch = alloc((2, experts), torch.int32)            # counts and first tiles while sorting
+        self.rows = None                                           # the tokens' rows in this order, where they exist already
+
+    def max_tiles(self) -> int:
+        """No more tiles than this, whatever the routing: every tile holds a pair, and all but an expert's last are full."""
+        return min(self.pairs, self.pairs // self.tile_pairs + self.experts)
 
 
 EXPERT_TENSOR_CORES = True       # False: the grouped products of routed experts always run as 32-bit multiply-adds
@@ -1078,10 +1089,50 @@ EXPERT_TENSOR_CORES = True       # False: the grouped products of routed experts
 
 def expert_tile_pairs(dtype: torch.dtype, width: int, inter: int) -> int:
     """The tile the grouped products of routed experts work on.  bfloat16 rows of 16-byte pieces: tiles of 128 pairs
-    through the tcgen05 product (TMA, accumulators in tensor memory; it beats a kernel that streams an expert's weights
-    for a tile of few pairs at every size measured, 49 against 82 us at 8 tokens).  Everything else: tiles of 8 pairs
-    with 32-bit multiply-adds."""
+    through the tcgen05 product (TMA, accumulators in tensor memory).  Everything else: tiles of 8 pairs with 32-bit
+    multiply-adds.  (moe_plan_few orders the pairs of a step of few tokens for the streaming product instead.)"""
     return 128 if (EXPERT_TENSOR_CORES and dtype == torch.bfloat16 and width % 8 == 0 and inter % 8 == 0) else 8
+
+
+# Up to this many tokens a step's routed experts run as weight streams (0: never).  Router to sum, 64 experts of 1,024, width
+# 2,048, 6 chosen, tiles of 128 / streams (us): 1 token 46.6 / 29.2, 3 64 / 46, 8 111 / 93, 16 118 / 113; but 20 129 / 132, 32
+# 148 / 158: nearly all experts are hit then, both are bound by the weights, and places counted over all pairs cost more.
+EXPERT_FEW_TOKENS = 16
+
+
+def moe_plan_few_takes(dtype: torch.dtype, tokens: int, width: int, inter: int, experts: int, real_experts: int, top: int,
+                       groups: int) -> bool:
+    """Whether moe_plan_few and the streaming grouped products behind it take a step of these sizes."""
+    return (tokens <= EXPERT_FEW_TOKENS and expert_tile_pairs(dtype, width, inter) == 128
+            and bool(library("core").mir_moe_plan_few_takes(tokens, experts, real_experts, top, groups)))
+
+
+def moe_plan_few(h: torch.Tensor, logits: torch.Tensor, correction: Optional[torch.Tensor], has_gate: bool, ids: torch.Tensor,
+                 weights: torch.Tensor, shared_gate: Optional[torch.Tensor], experts: int, real_experts: int, top: int,
+                 groups: int, keep: int, scale: float, alloc, score: str = "sigmoid", group_score: str = "top2") -> ExpertOrder:
+    """moe_route, moe_sort and the gathering of the tokens' rows in one kernel, for the few tokens that
+    moe_plan_few_takes allows; an expert's pairs are one tile (a token chooses an expert once)."""
+    _require(score in ("sigmoid", "softmax") and group_score in ("top2", "max"), "moe_plan_few: unknown score rule")
+    _cuda(h, logits, correction, ids, weights, shared_gate)
+    tokens, width = h.shape
+    _require(logits.dtype == torch.float32 and logits.stride(1) == 1 and logits.shape[0] == tokens
+             and logits.shape[1] >= experts + int(has_gate)
+             and (correction is None or (correction.dtype == torch.float32 and correction.numel() == experts))
+             and ids.dtype == torch.int32 and ids.is_contiguous() and ids.shape == (tokens, top)
+             and weights.dtype == torch.float32 and weights.is_contiguous() and weights.shape == (tokens, top)
+             and (not has_gate or (shared_gate is not None and shared_gate.dtype == torch.float32
+                                   and shared_gate.numel() >= tokens))
+             and h.dtype == torch.bfloat16 and h.stride(1) == 1, "moe_plan_few: shapes or dtypes do not fit")
+    found = ExpertOrder(alloc, tokens * top, real_experts, -(-tokens // 16) * 16)
+    found.rows = alloc((found.pairs, width), torch.bfloat16)
+    lib = library("core")
+    _check(lib, lib.mir_moe_plan_few(logits.data_ptr(), logits.stride(0), _ptr(correction), int(has_gate), ids.data_ptr(),
+                                     weights.data_ptr(), _ptr(shared_gate), tokens, experts, real_experts, top, groups, keep,
+                                     float(scale), int(score == "softmax"), int(group_score == "max"), found.tile_pairs,
+                                     found.order.data_ptr(), found.offsets.data_ptr(), found.tiles.data_ptr(),
+                                     found.tile_count.data_ptr(), h.data_ptr(), h.stride(0), found.rows.data_ptr(), width,
+                                     _stream()))
+    return found
 
 
 def moe_sort(ids: torch.Tensor, experts: int, alloc, tile_pairs: int = 8) -> ExpertOrder:
@@ -1110,6 +1161,15 @@ def moe_gate_up(h: torch.Tensor, found: ExpertOrder, top: int, w_gate: torch.Ten
              and w_gate.is_contiguous() and w_up.is_contiguous() and hidden.is_contiguous()
              and hidden.shape == (found.pairs, inter) and found.pairs == tokens * top and found.experts == experts
              and h.dtype == w_gate.dtype == w_up.dtype == hidden.dtype, "moe_gate_up: shapes or dtypes do not fit")
+    if found.rows is not None:                                     # few tokens: their rows are in the pairs' order already
+        _require(found.rows.shape == (found.pairs, width) and w_up.data_ptr() == w_gate.data_ptr() + w_gate.numel() * 2,
+                 "moe_gate_up: the streaming product takes w_up right behind w_gate")
+        lib = library("bf16")
+        _check(lib, lib.mir_gemm_tc_stream_grouped_bf16(MODE_SWIGLU, found.rows.data_ptr(), width, found.pairs, w_gate.data_ptr(),
+                                                        experts, hidden.data_ptr(), inter, inter, width, found.tiles.data_ptr(),
+                                                        found.tile_count.data_ptr(), found.offsets.data_ptr(), None,
+                                                        found.tile_pairs, found.max_tiles(), 0, _stream()))
+        return
     if found.tile_pairs == 128:
         _require(h.dtype == torch.bfloat16 and alloc is not None
                  and w_up.data_ptr() == w_gate.data_ptr() + w_gate.numel() * 2,
@@ -1131,14 +1191,25 @@ def moe_gate_up(h: torch.Tensor, found: ExpertOrder, top: int, w_gate: torch.Ten
                                     inter, found.tile_pairs, _stream()))
 
 
-def moe_down(hidden: torch.Tensor, found: ExpertOrder, w_down: torch.Tensor, pair_rows: torch.Tensor) -> None:
-    """pair_rows[pair] = w_down[e] hidden[i] (32-bit [pairs, width]) for the i-th pair in expert order."""
+def moe_down(hidden: torch.Tensor, found: ExpertOrder, w_down: torch.Tensor, pair_rows: torch.Tensor,
+             behind_gate_up: bool = False) -> None:
+    """pair_rows[pair] = w_down[e] hidden[i] (32-bit [pairs, width]) for the i-th pair in expert order.  behind_gate_up: the
+    launch in front of this one on the stream was moe_gate_up of the same order (its kernel releases this one only when the
+    order is complete, so the first weights may be asked for while it still runs)."""
     _cuda(hidden, w_down, pair_rows)
     experts, width, inter = w_down.shape
     _require(hidden.is_contiguous() and hidden.shape == (found.pairs, inter) and w_down.is_contiguous()
              and hidden.dtype == w_down.dtype and pair_rows.dtype == torch.float32 and pair_rows.is_contiguous()
              and pair_rows.shape == (found.pairs, width) and found.experts == experts,
              "moe_down: shapes or dtypes do not fit")
+    if found.rows is not None:
+        lib = library("bf16")
+        _check(lib, lib.mir_gemm_tc_stream_grouped_bf16(MODE_F32, hidden.data_ptr(), inter, found.pairs, w_down.data_ptr(), experts,
+                                                        pair_rows.data_ptr(), width, width, inter, found.tiles.data_ptr(),
+                                                        found.tile_count.data_ptr(), found.offsets.data_ptr(),
+                                                        found.order.data_ptr(), found.tile_pairs, found.max_tiles(),
+                                                        int(behind_gate_up), _stream()))
+        return
     if found.tile_pairs == 128:
         _require(hidden.dtype == torch.bfloat16, "moe_down: the tcgen05 product takes bfloat16")
         lib = library("bf16")

@@ -17,7 +17,8 @@ Everything runs on the device without a count ever being read back (csrc/moe.cu)
 ordered by expert, two grouped products run over the ordered pairs with each pair's expert's weights (in bfloat16 on
 tensor cores: the tcgen05 product of csrc/gemm_tc.cu on row tiles from a list on the device; in float32 as 32-bit
 multiply-adds), and one kernel adds the weighted rows, and the shared
-expert's, into the 32-bit residual.
+expert's, into the 32-bit residual.  For a step of few tokens in bfloat16 one kernel routes, orders and gathers, and the two
+products stream the chosen experts' weights (csrc/gemm_tc_stream.cu).
 """
 
 from __future__ import annotations
@@ -100,13 +101,18 @@ class RoutedExperts(FeedForward):
         gate = ctx.alloc((tokens,), torch.float32) if self.shared_gate else None
         logits = ctx.alloc((tokens, self.router.shape[0]), torch.float32)
         kernels.linear(x, self.router, logits, alloc=ctx.alloc)       # 32-bit accumulation and result
-        kernels.moe_route(logits, self.correction, self.shared_gate, ids, weights, gate, self.routed, s.top, s.groups,
-                          s.keep_groups, s.scale, score=s.score, group_score=s.group_score)
-        found = kernels.moe_sort(ids, s.experts, ctx.alloc, kernels.expert_tile_pairs(dtype, s.hidden_size, s.expert_size))
+        if kernels.moe_plan_few_takes(dtype, tokens, s.hidden_size, s.expert_size, self.routed, s.experts, s.top, s.groups):
+            found = kernels.moe_plan_few(x, logits, self.correction, self.shared_gate, ids, weights, gate, self.routed,
+                                         s.experts, s.top, s.groups, s.keep_groups, s.scale, ctx.alloc, score=s.score,
+                                         group_score=s.group_score)
+        else:
+            kernels.moe_route(logits, self.correction, self.shared_gate, ids, weights, gate, self.routed, s.top, s.groups,
+                              s.keep_groups, s.scale, score=s.score, group_score=s.group_score)
+            found = kernels.moe_sort(ids, s.experts, ctx.alloc, kernels.expert_tile_pairs(dtype, s.hidden_size, s.expert_size))
         hidden = ctx.alloc((tokens * s.top, s.expert_size), dtype)
         kernels.moe_gate_up(x, found, s.top, self.w_gate, self.w_up, hidden, ctx.alloc)
         pair_rows = ctx.alloc((tokens * s.top, s.hidden_size), torch.float32)
-        kernels.moe_down(hidden, found, self.w_down, pair_rows)
+        kernels.moe_down(hidden, found, self.w_down, pair_rows, behind_gate_up=True)
         shared_rows = None
         if s.shared_size:
             shared_hidden = ctx.alloc((tokens, s.shared_size), dtype)
