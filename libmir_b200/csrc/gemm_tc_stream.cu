@@ -162,11 +162,15 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
       const uint32_t stage_bytes = weight_bytes + (uint32_t)tokens * 128u;
+      // A step reads every weight once: they leave the L2 first, so that what the step's small kernels come back to (their
+      // instructions above all, the activations, norms' weights) is still there.  Whole calls of 1 to 53 requests, mostly
+      // decoded tokens: 1.4 to 2.9 % faster (one prompt of 37 and 12 tokens at Qwen3-4B sizes 27.45 to 26.9 ms).
+      const uint64_t policy = l2_evict_first();
       auto load_weights = [&](int i, uint32_t barrier, uint32_t dst) {
         const int k0 = (step_begin + i) * kStepK;
         barrier_expect_bytes(barrier, stage_bytes);
-        tma_load_2d(dst, &w_map, barrier, k0, w0);
-        if (MODE == SWIGLU) tma_load_2d(dst + kWeightBytes / 2, &w_map, barrier, k0, up_offset + w0);
+        tma_load_2d_hint(dst, &w_map, barrier, k0, w0, policy);
+        if (MODE == SWIGLU) tma_load_2d_hint(dst + kWeightBytes / 2, &w_map, barrier, k0, up_offset + w0, policy);
       };
       // The weights belong to no kernel: the whole ring is filled with them before this kernel waits for the one
       // before it, whose results are only the activations.  Launched with programmatic stream serialization, the
