@@ -63,7 +63,7 @@ struct RouteRule {
   int softmax_scores, group_by_max;
 };
 template <bool RANKED>
-__device__ __forceinline__ void route_token(const float* __restrict__ z, const RouteRule& rule, float* score, float* choice,
+__device__ __forceinline__ void route_token(const float* z, const RouteRule& rule, float* score, float* choice,
                                             float* group_score, float* chosen, int lane, int* ids_out, float* weights_out) {
   const int experts = rule.experts, top = rule.top, groups = rule.groups, keep = rule.keep;
   float softmax_top = 0.0f, softmax_inverse = 1.0f;
@@ -261,11 +261,13 @@ moe_sort_few_kernel(const int* __restrict__ ids, int pairs, int experts, int til
 constexpr int kPlanThreads = 512;
 template <bool RANKED>
 __global__ void __launch_bounds__(kPlanThreads)
-moe_plan_few_kernel(const float* __restrict__ logits, long long ld, int has_gate, int* __restrict__ ids,
+moe_plan_few_kernel(const float* logits, long long ld, int has_gate, int* __restrict__ ids,
                     float* __restrict__ weights, float* __restrict__ shared_gate, int tokens, RouteRule rule, int real_experts,
                     int tile_pairs, int* __restrict__ order, int* __restrict__ offsets, int* __restrict__ tiles,
-                    int* __restrict__ tile_count, const uint4* __restrict__ h, long long ld_pieces, uint4* __restrict__ sorted_rows,
+                    int* __restrict__ tile_count, const uint4* h, long long ld_pieces, uint4* __restrict__ sorted_rows,
                     int pieces) {
+  // (logits and h carry no __restrict__: as invariant loads the compiler moves them in front of both passes, and so in front
+  // of the wait)
   extern __shared__ __align__(16) float plan_shared[];
   __shared__ int tile_sums[kPlanThreads / 32];
   const int thread = threadIdx.x, lane = thread & 31, warp = thread >> 5;

@@ -69,3 +69,32 @@ def test_few_tokens_through_their_experts(tokens, experts, real, top, groups, ke
         bound = inter * 2 ** -24 * (w_down[e].double().abs() @ hidden[place].abs()) + 1e-30
         assert ((pair_rows[pair] - want).abs() <= bound).all()
     assert kernels.tensor_core_linear_error() == 0
+
+
+def test_rows_of_a_kernel_that_still_runs():
+    """The tokens' rows and the router's logits come from products that are still running when the next kernels of a captured
+    step are released: what is gathered is what they leave, not what was there before."""
+    from libmir_b200 import kernels
+    generator = torch.Generator(device="cuda").manual_seed(1)
+    make = lambda *shape: (torch.randn(*shape, generator=generator, device="cuda") * 0.05).to(torch.bfloat16)
+    tokens, width, deep, experts, top = 3, 512, 65536, 64, 6
+    weight, router, x = make(width, deep), make(experts, width), make(tokens, deep)
+    h, logits = alloc((tokens, width), torch.bfloat16), alloc((tokens, experts), torch.float32)
+    ids, weights = alloc((tokens, top), torch.int32), alloc((tokens, top), torch.float32)
+
+    def step():
+        kernels.linear(x, weight, h)
+        kernels.linear(h, router, logits)
+        return kernels.moe_plan_few(h, logits, None, False, ids, weights, None, experts, experts, top, 8, 4, 1.0, alloc)
+    step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        found = step()
+    other_ids, other_weights = torch.zeros_like(ids), torch.zeros_like(weights)
+    for _ in range(3):
+        x.copy_(make(tokens, deep))
+        graph.replay()
+        kernels.moe_route(logits, None, False, other_ids, other_weights, None, experts, top, 8, 4, 1.0)
+        assert torch.equal(ids, other_ids) and torch.equal(weights, other_weights)
+        assert torch.equal(found.rows, h[found.order.long() // top])
