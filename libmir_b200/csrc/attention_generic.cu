@@ -48,6 +48,8 @@ __global__ void paged_attention_generic_kernel(
   const int warp = threadIdx.y;
   const int head = blockIdx.y * kWarpsPerBlock + warp;
   const int token = blockIdx.x;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (head >= heads) return;
   const int row = row_of_token[token];
   const int position = positions[token];
@@ -192,17 +194,15 @@ MIR_EXPORT int mir_paged_attention_generic(int bf16, const void* q, long long q_
   const dim3 grid(tokens, (heads + kWarpsPerBlock - 1) / kWarpsPerBlock);
   const dim3 block(32, kWarpsPerBlock);
 #define MIR_GENERIC(T, PIECES)                                                                                             \
-  paged_attention_generic_kernel<T, PIECES><<<grid, block, 0, stream>>>(                                                   \
+  return mir_launch("paged_attention_generic", paged_attention_generic_kernel<T, PIECES>, grid, block, 0, stream, 0,        \
       (const T*)q, (size_t)q_token_stride, (T*)out, (const T*)k_pages, (const T*)v_pages, block_table, table_width,        \
       row_of_token, positions, page_size, heads, kv_heads, head_dim, value_dim, value_row_width, scale, window,            \
       keep_first, sinks, (const T*)gate, (size_t)gate_stride, gate_per_head, softcap, rel_bias, rel_rows, chunk, slopes)
   if (bf16) {
     if (value_dim <= 128) MIR_GENERIC(__nv_bfloat16, 4);
-    else MIR_GENERIC(__nv_bfloat16, kMaxHeadDim / 32);
-  } else {
-    if (value_dim <= 128) MIR_GENERIC(float, 4);
-    else MIR_GENERIC(float, kMaxHeadDim / 32);
+    MIR_GENERIC(__nv_bfloat16, kMaxHeadDim / 32);
   }
+  if (value_dim <= 128) MIR_GENERIC(float, 4);
+  MIR_GENERIC(float, kMaxHeadDim / 32);
 #undef MIR_GENERIC
-  return mir_check_launch("paged_attention_generic");
 }

@@ -431,8 +431,8 @@ mixed_decode_scores_kernel(const bf16* __restrict__ q, long long q_stride, const
                            float* __restrict__ scores, float2* __restrict__ stats, int* __restrict__ arrived) {
   constexpr int PASSES = kKeys * LANES / 128, SUBS = 32 / LANES;
   __shared__ float s_s[R][kKeys];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int part = blockIdx.x, row = blockIdx.y;
   const int position = positions[row];
   if (position < 0) return;
@@ -532,8 +532,8 @@ mixed_decode_values_kernel(const bf16* __restrict__ v_pages, const int* __restri
   float* const weights = log_sums + (heads + 3) / 4 * 4;
   float* const mixed = weights + heads * kKeys;
   float* const sums = mixed + R * kKeys;
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int part = blockIdx.x, row = blockIdx.y;
   const int position = positions[row];
   if (position < 0) return;

@@ -311,11 +311,13 @@ decode_attention_kernel(const bf16* __restrict__ q, size_t q_stride, const bf16*
   const int head0 = kv_head * group + (blockIdx.y % group_tiles) * kDecodeHeads;
   const int valid_rows = min(kDecodeHeads, kv_head * group + group - head0);
   grid_launch_dependents();
-  // Launched with programmatic stream serialization, this kernel may start while the kernel before it (which
-  // writes the newest key and value and rotates q) still runs.  Positions and block tables are older than that
-  // kernel, and so is every key but the newest: the first copies of old keys start before the wait.
+  // Launched with programmatic stream serialization, this kernel may start while kernels of the step before it (one
+  // of which writes the newest key and value and rotates q) still run.  Positions and block tables are older than all of
+  // them (what writes those is not released early), and so is every key but the newest: the first copies of old keys
+  // start before the wait.  Nothing is written before it: an earlier layer may still read the same scratch.
   const int position = positions[row];
   if (position < 0) {                                         // padding row of a captured batch
+    grid_dependency_wait();
     if (keep_first > 0 && window > 0 && virtual_positions && part == 0 && blockIdx.y == 0 && threadIdx.x == 0)
       virtual_positions[row] = -1;
     return;
@@ -334,12 +336,15 @@ decode_attention_kernel(const bf16* __restrict__ q, size_t q_stride, const bf16*
   const bool renumbered = keep_first > 0 && window > 0;
   const int shift = renumbered ? first_tile - kept_tiles_end : 0;
   const int numbered_context = context - shift;
-  if (renumbered && virtual_positions && part == 0 && blockIdx.y == 0 && threadIdx.x == 0)
-    virtual_positions[row] = numbered_context - 1;
+  const bool names_last = renumbered && virtual_positions && part == 0 && blockIdx.y == 0 && threadIdx.x == 0;
   const int part_begin = part * partition;
   const int part_end = min(numbered_context, part_begin + partition);
   const int begin = renumbered ? part_begin : max(part_begin, first_tile);
-  if (begin >= part_end) return;                              // the merge skips this partition the same way
+  if (begin >= part_end) {                                    // the merge skips this partition the same way
+    grid_dependency_wait();
+    if (names_last) virtual_positions[row] = numbered_context - 1;
+    return;
+  }
   // the true first key of the tile numbered n, and the first true key beyond what may be read of it
   auto true_key = [&](int n) { return n < kept_tiles_end ? n : n + shift; };
   auto true_limit = [&](int n) { return n < kept_tiles_end ? kept_end : min(context, part_end + shift); };
@@ -366,6 +371,7 @@ decode_attention_kernel(const bf16* __restrict__ q, size_t q_stride, const bf16*
   }
 
   if (early) grid_dependency_wait();                          // q (and the newest key) come from the kernel before
+  if (names_last) virtual_positions[row] = numbered_context - 1;
   // Q fragments: rows 0..7 are the heads of the group, rows 8..15 are zero
   uint32_t qa[D / 16][4];
   {
@@ -531,11 +537,11 @@ decode_merge_kernel(const float* __restrict__ partial_o, const float* __restrict
   __shared__ float sums[kMergeWarps][D + 1];                   // [warp][elements, then the denominator]
   const int head = blockIdx.x, row = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  grid_launch_dependents();
   MIR_TRACE_BEGIN(merge, (blockIdx.x == 0 && blockIdx.y == 0) || (blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1),
                   300 + (blockIdx.x == 0 && blockIdx.y == 0 ? 0 : 1))
   if (threadIdx.x == 0) MIR_TRACE_POINT(merge, 0);
   grid_dependency_wait();
+  grid_launch_dependents();
   if (threadIdx.x == 0) MIR_TRACE_POINT(merge, 1);
   const int position = positions[row];
   const size_t index = (size_t)row * heads + head;
@@ -606,11 +612,11 @@ decode_merge_few_kernel(const float* __restrict__ partial_o, const float* __rest
   constexpr int PER = D / 32;                                  // elements per lane: 4, 2 or 1
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.x * kMergeWarps + warp, row = blockIdx.y;
-  grid_launch_dependents();
   MIR_TRACE_BEGIN(merge, (blockIdx.x == 0 && blockIdx.y == 0) || (blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1),
                   300 + (blockIdx.x == 0 && blockIdx.y == 0 ? 0 : 1))
   if (threadIdx.x == 0) MIR_TRACE_POINT(merge, 0);
   grid_dependency_wait();
+  grid_launch_dependents();
   if (threadIdx.x == 0) MIR_TRACE_POINT(merge, 1);
   if (head >= heads) return;
   const int position = positions[row];
@@ -694,8 +700,8 @@ prefill_attention_kernel(const bf16* __restrict__ q, size_t q_stride, bf16* __re
   const int head = blockIdx.x;                                // the fast index: all heads of the longest tile start first
   const int kv_head = head / (heads / kv_heads);
 
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   // which request row and which 64-token tile of its portion this CTA has
   int row = -1, local_tile = 0;
   {

@@ -396,8 +396,8 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = blockIdx.x, ctas = gridDim.x;
 
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   if (threadIdx.x == 0) {
     // how many query tiles the batch really has (the launch was sized for at most tile_slots)
     int total = 0;

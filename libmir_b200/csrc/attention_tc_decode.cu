@@ -150,9 +150,9 @@ tc_decode_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   const int head0 = kv_head * group + (blockIdx.y % group_tiles) * kHeads;
   const int valid_heads = min(kHeads, kv_head * group + group - head0);
   grid_launch_dependents();
-  // Launched with programmatic stream serialization, this kernel may start while the kernel before it (which
-  // writes the newest key and value and rotates q) still runs.  Positions and block tables are older than that
-  // kernel, and so is every key but the newest.
+  // Launched with programmatic stream serialization, this kernel may start while kernels of the step before it (one
+  // of which writes the newest key and value and rotates q) still run.  Positions and block tables are older than all of
+  // them (what writes those is not released early), and so is every key but the newest.
   const int position = positions[row];
   const int context = position + 1;
   const int first_key = (window > 0 && context > window) ? context - window : 0;

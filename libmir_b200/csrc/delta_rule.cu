@@ -55,8 +55,8 @@ __global__ void delta_rule_prepare_kernel(const T* __restrict__ x, long long ldx
                                           float* __restrict__ qkv, float* __restrict__ beta, float* __restrict__ decay,
                                           int heads, int kv_heads, int key_dim, int value_dim, int decay_width,
                                           int taps) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = blockIdx.x;
   if (positions[token] < 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -180,8 +180,8 @@ delta_rule_prepare_run_kernel(const T* __restrict__ x, long long ldx, const T* _
                               const int* __restrict__ state_slots, const int* __restrict__ positions,
                               float* __restrict__ qkv, float* __restrict__ beta, float* __restrict__ decay, int tokens,
                               int heads, int kv_heads, int key_dim, int value_dim, int decay_width, int taps) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x;
   const int first = blockIdx.x * RUN, last = min(first + RUN, tokens);
   const int keys = 2 * kv_heads, values = heads * value_dim;
@@ -338,8 +338,8 @@ delta_rule_scan_kernel(const float* __restrict__ qkv, const float* __restrict__ 
   static_assert(PER % 4 == 0, "a lane holds whole 16-byte pieces");
   constexpr int LANES = kScanLanes, C = kScanColumns;
   extern __shared__ __align__(16) float staged[];              // [kScanStages][kScanChunk tokens][row]
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   constexpr int COLUMNS = 32 / LANES * C;                       // per warp
   constexpr int BLOCK_COLUMNS = COLUMNS * kScanWarps;
   constexpr int PADDED = LANES * PER;                           // key channels with padding
@@ -528,8 +528,8 @@ delta_rule_step_kernel(const float* __restrict__ qkv, const float* __restrict__ 
                        const int* __restrict__ positions, float* __restrict__ out, int heads, int kv_heads, int key_dim,
                        int value_dim) {
   constexpr int LANES = 16, COLUMNS = 32 / LANES * C;            // of a warp
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x, l = lane % LANES;
   const int row = blockIdx.x, head = blockIdx.y;
   const int start = query_starts[row], end = query_starts[row + 1], slot = state_slots[row];
@@ -608,8 +608,8 @@ __global__ void __launch_bounds__(128)
 delta_rule_group_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
                         const int* __restrict__ query_starts, const int* __restrict__ positions, float* __restrict__ grouped,
                         int rows, int heads, int kv_heads, int key_dim, int value_dim) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x, group = blockIdx.x, head = blockIdx.y * 4 + threadIdx.y;
   if (head >= heads) return;
   int start = -1, end = 0, begin = 0;
@@ -728,8 +728,8 @@ delta_rule_grouped_scan_kernel(const float* __restrict__ grouped, const float* _
   constexpr int STAGE = CHUNK * ROW;
   constexpr int STAGES = 3;
   extern __shared__ __align__(16) float staged[];                // [STAGES][CHUNK groups][row]
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x;
   const int row = blockIdx.x, head = blockIdx.y;
   const int first_column = blockIdx.z * BLOCK_COLUMNS;
@@ -899,8 +899,8 @@ template <typename T, typename TG>
 __global__ void gated_head_norm_kernel(const float* __restrict__ o, const TG* __restrict__ gate, long long ld_gate,
                                        const float* __restrict__ weight, T* __restrict__ out, int units,
                                        int heads, int value_dim, float eps, int sigmoid_gate, int weight_per_head) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int unit = blockIdx.x * blockDim.y + threadIdx.y;       // token * heads + head
   if (unit >= units) return;
   const int lane = threadIdx.x;
@@ -927,7 +927,6 @@ __global__ void __launch_bounds__(128) gated_row_norm_kernel(const float* __rest
                                                              long long ld_gate, const float* __restrict__ weight,
                                                              T* __restrict__ out, int units, int heads, int value_dim, float eps,
                                                              int sigmoid_gate, int weight_per_head) {
-  grid_launch_dependents();
   const int unit = blockIdx.x * (128 / LANES) + threadIdx.x / LANES;       // token * heads + head
   const int l = threadIdx.x % LANES, head = unit % heads;
   const int count = unit < units ? value_dim : 0;                          // (a warp's last heads may not be there)
@@ -939,6 +938,7 @@ __global__ void __launch_bounds__(128) gated_row_norm_kernel(const float* __rest
 #pragma unroll
   for (int e = 0; e < PIECES; ++e) w[e] = l + LANES * e < count ? scale[l + LANES * e] : 0.0f;
   grid_dependency_wait();
+  grid_launch_dependents();
 #pragma unroll
   for (int e = 0; e < PIECES; ++e) v[e] = l + LANES * e < count ? src[l + LANES * e] : 0.0f;
 #pragma unroll
@@ -1004,7 +1004,6 @@ __global__ void __launch_bounds__(512) gated_wide_norm_kernel(const float* __res
                                                               T* __restrict__ out, int heads, int value_dim, float eps,
                                                               int sigmoid_gate, int weight_per_head) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   const int unit = blockIdx.x;                                  // token * heads + head
   const float* scale = weight + (weight_per_head ? (size_t)(unit % heads) * value_dim : 0);
   float w[PIECES][V], x[PIECES][V], g[PIECES][V];
@@ -1014,6 +1013,7 @@ __global__ void __launch_bounds__(512) gated_wide_norm_kernel(const float* __res
     if (d < value_dim) load_columns(w[p], scale + d);           // (older than the kernel before this one)
   }
   grid_dependency_wait();
+  grid_launch_dependents();
   const float* src = o + (size_t)unit * value_dim;
   const TG* gate_row = gate + (size_t)(unit / heads) * ld_gate + (size_t)(unit % heads) * value_dim;
   float sum = 0.0f;
@@ -1103,7 +1103,7 @@ int launch_scan_as(cudaStream_t stream, const float* qkv, const float* beta, con
     }
     raised = true;
   }
-  return mir_launch("delta_rule_scan", delta_rule_scan_kernel<PER, PER_CHANNEL>,
+  return mir_launch_alone("delta_rule_scan", delta_rule_scan_kernel<PER, PER_CHANNEL>,
                     dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps + kFetchWarps), smem, stream, 0, qkv,
                     beta, decay, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
 }
@@ -1168,7 +1168,7 @@ int launch_grouped_walk(cudaStream_t stream, const float* grouped, const float* 
     mir_set_error("delta_rule_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
     return MIR_CUDA_ERROR;
   }
-  return mir_launch("delta_rule_scan", delta_rule_grouped_scan_kernel<PER, C>,
+  return mir_launch_alone("delta_rule_scan", delta_rule_grouped_scan_kernel<PER, C>,
                     dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kScanWarps + kFetchWarps), smem, stream, 0,
                     grouped, qkv, state, query_starts, state_slots, positions, out, heads, kv_heads, key_dim, value_dim);
 }

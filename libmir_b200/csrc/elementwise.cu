@@ -13,8 +13,8 @@ using namespace mir;
 template <typename T>
 __global__ void embed_kernel(const T* __restrict__ table, const int* __restrict__ ids, float* __restrict__ out,
                              int hidden, int vocab, float scale) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const int id = ids[row];
   const bool ok = id >= 0 && id < vocab;
@@ -29,8 +29,8 @@ template <typename T>
 __global__ void __launch_bounds__(512) embed_wide_kernel(const T* __restrict__ table, const int* __restrict__ ids,
                                                          float* __restrict__ out, int hidden, int vocab, float scale) {
   constexpr int V = 16 / sizeof(T);
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const int id = ids[row];
   const bool ok = id >= 0 && id < vocab;
@@ -54,8 +54,8 @@ template <typename T>
 __global__ void embed_pairs_kernel(const T* __restrict__ table, const T* __restrict__ pairs, const int* __restrict__ ids,
                                    const int* __restrict__ previous, float* __restrict__ out, int hidden, int vocab,
                                    int buckets, long long mul_previous, long long mul_current, float scale) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const int id = ids[row];
   const int before = previous[row];
@@ -72,6 +72,8 @@ __global__ void embed_pairs_kernel(const T* __restrict__ table, const T* __restr
 // x <- 0.5 x (1 + tanh(sqrt(2 / pi) (x + 0.044715 x^3))), in place.
 template <typename T>
 __global__ void gelu_tanh_kernel(T* __restrict__ x, size_t total) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const float z = to_float(x[index]);
@@ -107,8 +109,8 @@ struct NormedBranches {
 __global__ void add_normed_branches_kernel(NormedBranches branches, float* __restrict__ residual,
                                            __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   float inverse[4];
   for (int b = 0; b < branches.count; ++b) {
@@ -134,8 +136,8 @@ __global__ void add_normed_branches_kernel(NormedBranches branches, float* __res
 __global__ void add_normed_branches_vec4_kernel(NormedBranches branches, float* __restrict__ residual,
                                                 __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const size_t base = (size_t)blockIdx.x * hidden;
   const int quads = hidden >> 2;
   float inverse[4];
@@ -171,7 +173,6 @@ template <int BRANCHES, int PIECES, bool EARLY>
 __global__ void __launch_bounds__(256) add_normed_branches_row_kernel(
     NormedBranches branches, float* __restrict__ residual, __nv_bfloat16* __restrict__ rounded, int hidden, float eps, float scale) {
   __shared__ float scratch[BRANCHES][32];
-  grid_launch_dependents();
   const int quads = hidden >> 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   float4 w[BRANCHES][PIECES], v[BRANCHES][PIECES], old[PIECES];
@@ -183,6 +184,7 @@ __global__ void __launch_bounds__(256) add_normed_branches_row_kernel(
       if (EARLY && c < quads) w[b][p] = __ldg(reinterpret_cast<const float4*>(branches.weight[b]) + c);
     }
   grid_dependency_wait();
+  grid_launch_dependents();
   const size_t base = (size_t)blockIdx.x * hidden;
 #pragma unroll
   for (int p = 0; p < PIECES; ++p) {
@@ -238,7 +240,6 @@ __global__ void __launch_bounds__(512) norm_scaled_sum_kernel(ScaledBranches bra
                                                               __nv_bfloat16* __restrict__ rounded, int hidden, float alpha,
                                                               float eps) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = (blockDim.x + 31) >> 5;
   const size_t base = (size_t)blockIdx.x * hidden;
   auto load = [](float (&v)[V], const float* from) {
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(512) norm_scaled_sum_kernel(ScaledBranches bra
   float early[V];
   if (kEarly && threadIdx.x * V < hidden) load(early, weight + threadIdx.x * V);
   grid_dependency_wait();
+  grid_launch_dependents();
   float u[PIECES][V];
   float sum = 0.0f;
 #pragma unroll
@@ -311,6 +313,8 @@ __global__ void __launch_bounds__(512) norm_scaled_sum_kernel(ScaledBranches bra
 
 // out[i] (+)= sum over branches b of scale_b * branch_b[i].
 __global__ void scaled_sum_kernel(ScaledBranches branches, float* __restrict__ out, size_t total, int accumulate) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   float sum = accumulate ? out[index] : 0.0f;
@@ -320,6 +324,8 @@ __global__ void scaled_sum_kernel(ScaledBranches branches, float* __restrict__ o
 
 // gelu_tanh on eight bfloat16 values per thread (16-byte accesses).
 __global__ void gelu_tanh_bf16x8_kernel(__nv_bfloat16* __restrict__ x, size_t total8) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total8) return;
   float z[8];
@@ -341,8 +347,8 @@ template <typename Tout>
 __global__ void rms_norm_kernel(const float* __restrict__ x, const float* __restrict__ weight,
                                 Tout* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
 
   const int row = blockIdx.x;
   const float* src = x + (size_t)(rows ? rows[row] : row) * hidden;
@@ -363,8 +369,8 @@ template <typename Tout>
 __global__ void rms_norm_vec4_kernel(const float* __restrict__ x, const float* __restrict__ weight,
                                      Tout* __restrict__ out, const int* __restrict__ rows, int hidden, float eps) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[row] : row) * hidden);
   const float4* w4 = reinterpret_cast<const float4*>(weight);
@@ -391,7 +397,6 @@ __global__ void __launch_bounds__(THREADS) rms_norm_row_kernel(const float* __re
                                                                Tout* __restrict__ out_b, const int* __restrict__ rows,
                                                                int hidden, float eps) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   const int quads = hidden >> 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   float4 w[PIECES], second[PAIR ? PIECES : 1], v[PIECES];
@@ -403,6 +408,7 @@ __global__ void __launch_bounds__(THREADS) rms_norm_row_kernel(const float* __re
     if (PAIR) second[p] = __ldg(reinterpret_cast<const float4*>(weight_b) + c);
   }
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const float4* src = reinterpret_cast<const float4*>(x + (size_t)(rows ? rows[row] : row) * hidden);
 #pragma unroll
@@ -470,6 +476,8 @@ int launch_rms_norm_pair(const float* x, const float* weight, const float* weigh
 // out[r, c] = silu(gu[r, c]) * gu[r, inter + c]; gu rows are [gate | up].
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, int inter, size_t total) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const size_t row = index / inter;
@@ -482,6 +490,8 @@ __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ out, i
 // The same, 8 columns per thread with 16-byte loads and stores (inter a multiple of 8, bf16).
 __global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
                                        int inter, size_t total8) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total8) return;
   const int per_row = inter / 8;
@@ -502,6 +512,8 @@ __global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ gu, __n
 // x[r, c] += bias[c]  (32-bit residual; used when a projection that accumulates into the residual has a bias).
 template <typename T>
 __global__ void add_bias_kernel(float* __restrict__ x, const T* __restrict__ bias, int cols, size_t total) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   x[index] += to_float(bias[index % cols]);
@@ -514,6 +526,14 @@ __global__ void cast_kernel(const Tin* __restrict__ src, Tout* __restrict__ dst,
   if (index < total) dst[index] = from_float<Tout>(to_float(src[index]));
 }
 
+// A thread for each of `total` elements.
+template <typename... KernelArgs, typename... Args>
+int launch_each(const char* what, void (*kernel)(KernelArgs...), size_t total, cudaStream_t stream, Args... args) {
+  if (total == 0) return MIR_OK;
+  return mir_launch(what, kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, stream, 0, args...);
+}
+
+// The same for what writes weights: not released early, since the kernels that stream weights ask for them before they wait.
 #define LAUNCH_1D(kernel, total, ...)                                                      \
   do {                                                                                     \
     const size_t n_ = (total);                                                             \
@@ -557,6 +577,8 @@ MIR_EXPORT int mir_embed_pairs(int bf16, const void* table, const void* pairs, c
 // computed in 32-bit.
 template <typename T>
 __global__ void activation_kernel(T* __restrict__ x, size_t total, int kind) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const float z = to_float(x[index]);
@@ -567,6 +589,8 @@ __global__ void activation_kernel(T* __restrict__ x, size_t total, int kind) {
 
 // x <- cap * tanh(x / cap) on 32-bit logits.
 __global__ void softcap_kernel(float* __restrict__ x, size_t total, float cap) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index < total) x[index] = cap * tanhf(x[index] / cap);
 }
@@ -574,6 +598,8 @@ __global__ void softcap_kernel(float* __restrict__ x, size_t total, float cap) {
 // residual[r, :] += rows[r, :] (if given) + vector (if given): what a pass of a looped run of layers starts with.
 __global__ void add_rows_kernel(float* __restrict__ residual, const float* __restrict__ rows,
                                 const float* __restrict__ vector, int hidden, size_t total) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   float v = residual[index];
@@ -588,8 +614,8 @@ __global__ void rms_norm_pair_kernel(const float* __restrict__ x, const float* _
                                      const float* __restrict__ weight_b, Tout* __restrict__ out_a,
                                      Tout* __restrict__ out_b, int hidden, float eps) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const float* src = x + (size_t)row * hidden;
   float sum = 0.0f;
@@ -607,10 +633,9 @@ __global__ void rms_norm_pair_kernel(const float* __restrict__ x, const float* _
 }
 
 MIR_EXPORT int mir_gelu_tanh(int bf16, void* x, size_t total, cudaStream_t stream) {
-  if (bf16 && total % 8 == 0 && ((uintptr_t)x & 15) == 0) LAUNCH_1D(gelu_tanh_bf16x8_kernel, total / 8, (__nv_bfloat16*)x, total / 8);
-  else if (bf16) LAUNCH_1D(gelu_tanh_kernel, total, (__nv_bfloat16*)x, total);
-  else LAUNCH_1D(gelu_tanh_kernel, total, (float*)x, total);
-  return mir_check_launch("gelu_tanh");
+  if (bf16 && total % 8 == 0 && ((uintptr_t)x & 15) == 0) return launch_each("gelu_tanh", gelu_tanh_bf16x8_kernel, total / 8, stream, x, total / 8);
+  if (bf16) return launch_each("gelu_tanh", gelu_tanh_kernel<__nv_bfloat16>, total, stream, x, total);
+  return launch_each("gelu_tanh", gelu_tanh_kernel<float>, total, stream, x, total);
 }
 
 // rows_b, weight_b: `count` (1 to 4) pointers each, to 32-bit [rows, hidden] and [hidden].  rounded: null, or bfloat16
@@ -708,8 +733,7 @@ MIR_EXPORT int mir_scaled_sum(const float* const* branch_rows, const float* scal
   ScaledBranches branches = {};
   branches.count = count;
   for (int b = 0; b < count; ++b) { branches.rows[b] = branch_rows[b]; branches.scale[b] = scales[b]; }
-  LAUNCH_1D(scaled_sum_kernel, total, branches, out, total, accumulate);
-  return mir_check_launch("scaled_sum");
+  return launch_each("scaled_sum", scaled_sum_kernel, total, stream, branches, out, total, accumulate);
 }
 
 MIR_EXPORT int mir_rms_norm(int bf16, const float* x, const float* weight, void* out, const int* rows, int n_rows,
@@ -730,23 +754,21 @@ MIR_EXPORT int mir_rms_norm(int bf16, const float* x, const float* weight, void*
 
 MIR_EXPORT int mir_activation(int kind, int bf16, void* x, size_t total, cudaStream_t stream) {
   if (kind < 1 || kind > 3) { mir_set_error("activation: unknown kind %d", kind); return MIR_BAD_ARGUMENT; }
-  if (bf16) LAUNCH_1D(activation_kernel, total, (__nv_bfloat16*)x, total, kind);
-  else LAUNCH_1D(activation_kernel, total, (float*)x, total, kind);
-  return mir_check_launch(kind == 1 ? "gelu_erf" : (kind == 2 ? "tanh" : "relu_squared"));
+  const char* name = kind == 1 ? "gelu_erf" : (kind == 2 ? "tanh" : "relu_squared");
+  return bf16 ? launch_each(name, activation_kernel<__nv_bfloat16>, total, stream, x, total, kind)
+              : launch_each(name, activation_kernel<float>, total, stream, x, total, kind);
 }
 
 MIR_EXPORT int mir_softcap(float* x, size_t total, float cap, cudaStream_t stream) {
   if (!(cap > 0.0f)) { mir_set_error("softcap: the cap must be greater than zero"); return MIR_BAD_ARGUMENT; }
-  LAUNCH_1D(softcap_kernel, total, x, total, cap);
-  return mir_check_launch("softcap");
+  return launch_each("softcap", softcap_kernel, total, stream, x, total, cap);
 }
 
 MIR_EXPORT int mir_add_rows(float* residual, const float* rows, const float* vector, int n_rows, int hidden,
                             cudaStream_t stream) {
   if (n_rows < 0 || hidden <= 0) { mir_set_error("add_rows: bad sizes"); return MIR_BAD_ARGUMENT; }
   const size_t total = (size_t)n_rows * hidden;
-  LAUNCH_1D(add_rows_kernel, total, residual, rows, vector, hidden, total);
-  return mir_check_launch("add_rows");
+  return launch_each("add_rows", add_rows_kernel, total, stream, residual, rows, vector, hidden, total);
 }
 
 MIR_EXPORT int mir_rms_norm_pair(int bf16, const float* x, const float* weight_a, const float* weight_b, void* out_a,
@@ -771,18 +793,16 @@ MIR_EXPORT int mir_silu_mul(int bf16, const void* gu, void* out, int rows, int i
   if (rows < 0 || inter <= 0) { mir_set_error("silu_mul: bad sizes"); return MIR_BAD_ARGUMENT; }
   const size_t total = (size_t)rows * inter;
   if (bf16 && inter % 8 == 0 && ((uintptr_t)gu & 15) == 0 && ((uintptr_t)out & 15) == 0)
-    LAUNCH_1D(silu_mul_bf16x8_kernel, total / 8, (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, inter, total / 8);
-  else if (bf16) LAUNCH_1D(silu_mul_kernel, total, (const __nv_bfloat16*)gu, (__nv_bfloat16*)out, inter, total);
-  else LAUNCH_1D(silu_mul_kernel, total, (const float*)gu, (float*)out, inter, total);
-  return mir_check_launch("silu_mul");
+    return launch_each("silu_mul", silu_mul_bf16x8_kernel, total / 8, stream, gu, out, inter, total / 8);
+  if (bf16) return launch_each("silu_mul", silu_mul_kernel<__nv_bfloat16>, total, stream, gu, out, inter, total);
+  return launch_each("silu_mul", silu_mul_kernel<float>, total, stream, gu, out, inter, total);
 }
 
 MIR_EXPORT int mir_add_bias(int bf16, float* x, const void* bias, int rows, int cols, cudaStream_t stream) {
   if (rows < 0 || cols <= 0) { mir_set_error("add_bias: bad sizes"); return MIR_BAD_ARGUMENT; }
   const size_t total = (size_t)rows * cols;
-  if (bf16) LAUNCH_1D(add_bias_kernel, total, x, (const __nv_bfloat16*)bias, cols, total);
-  else LAUNCH_1D(add_bias_kernel, total, x, (const float*)bias, cols, total);
-  return mir_check_launch("add_bias");
+  return bf16 ? launch_each("add_bias", add_bias_kernel<__nv_bfloat16>, total, stream, x, bias, cols, total)
+              : launch_each("add_bias", add_bias_kernel<float>, total, stream, x, bias, cols, total);
 }
 
 // kind: 0 f32->bf16, 1 bf16->f32, 2 f16->bf16, 3 f16->f32 (what a checkpoint may store, to what the engine keeps).
@@ -827,8 +847,8 @@ constexpr int kSlotsAtOnce = 64, kZeroPiece = 64 * 1024;
 struct ZeroSlots { int slot[kSlotsAtOnce]; };
 
 __global__ void __launch_bounds__(256) zero_slots_kernel(const long long* __restrict__ regions, ZeroSlots slots) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   char* base = reinterpret_cast<char*>(regions[2 * blockIdx.y]);
   const long long bytes = regions[2 * blockIdx.y + 1];
   char* record = base + (long long)slots.slot[blockIdx.z] * bytes;
@@ -846,8 +866,7 @@ __global__ void __launch_bounds__(256) zero_slots_kernel(const long long* __rest
 __global__ void decode_prepare_kernel(const int* __restrict__ positions, const int* __restrict__ block_table,
                                       int table_width, int page_size, int* __restrict__ slot_mapping,
                                       int* __restrict__ context_lens, int rows) {
-  grid_launch_dependents();
-  grid_dependency_wait();
+  grid_dependency_wait();                         // (no early release: what follows reads these numbers before it waits)
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= rows) return;
   const int position = positions[row];
@@ -866,8 +885,7 @@ __global__ void decode_prepare_kernel(const int* __restrict__ positions, const i
 __global__ void decode_advance_kernel(const int* __restrict__ sampled, int* __restrict__ tokens,
                                       int* __restrict__ positions, int* __restrict__ token_log, int log_steps,
                                       int* __restrict__ step_counter, int rows, int* __restrict__ previous) {
-  grid_launch_dependents();
-  grid_dependency_wait();
+  grid_dependency_wait();                         // (no early release: the next step reads the positions before it waits)
   const int step = *step_counter;
   __syncthreads();
   for (int row = threadIdx.x; row < rows; row += blockDim.x) {

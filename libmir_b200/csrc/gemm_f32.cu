@@ -74,6 +74,8 @@ gemm_f32_tile_kernel(const float* __restrict__ a, int lda, const float* __restri
 #pragma unroll
     for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
   const int steps = (k + DEPTH - 1) / DEPTH;
+  mir::grid_dependency_wait();
+  mir::grid_launch_dependents();
   auto fetch = [&](int step) {
     float* stage = shared + (step % STAGES) * (BM + BN) * ROW;
     load_tile<BM, DEPTH, THREADS, WIDE>(stage, a, lda, row0, m, step * DEPTH, k, threadIdx.x);
@@ -144,18 +146,33 @@ gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restri
 #pragma unroll
   for (int e = 0; e < EACH; ++e) acc[e] = 0.0f;
   const int steps = (k + kRowsDepth - 1) / kRowsDepth;
+  mir::grid_launch_dependents();
   if (threadIdx.x >= kRowsThreads) {               // two warps fetch: the others' chain of multiply-adds is not interrupted
     const int thread = threadIdx.x - kRowsThreads;
+    auto fetch_weights = [&](int step) {
+      if (step < steps)
+        load_tile<kRowsColumns, kRowsDepth, kRowsLoaders, WIDE>(shared + (step % kRowsStages) * STAGE, w, ldw, col0, n,
+                                                                step * kRowsDepth, k, thread);
+    };
+    auto fetch_rows = [&](int step) {
+      if (step < steps)
+        load_tile<MT, kRowsDepth, kRowsLoaders, WIDE>(shared + (step % kRowsStages) * STAGE + kRowsColumns * ROW, a, lda, 0, m,
+                                                      step * kRowsDepth, k, thread);
+    };
     auto fetch = [&](int step) {
-      if (step < steps) {
-        float* stage = shared + (step % kRowsStages) * STAGE;
-        load_tile<kRowsColumns, kRowsDepth, kRowsLoaders, WIDE>(stage, w, ldw, col0, n, step * kRowsDepth, k, thread);
-        load_tile<MT, kRowsDepth, kRowsLoaders, WIDE>(stage + kRowsColumns * ROW, a, lda, 0, m, step * kRowsDepth, k, thread);
-      }
+      fetch_weights(step);
+      fetch_rows(step);
       copy_commit();
     };
+    // the weights belong to no kernel: the ring's are on their way before the kernel in front is over
 #pragma unroll
-    for (int step = 0; step < kRowsStages - 1; ++step) fetch(step);
+    for (int step = 0; step < kRowsStages - 1; ++step) fetch_weights(step);
+    mir::grid_dependency_wait();
+#pragma unroll
+    for (int step = 0; step < kRowsStages - 1; ++step) {
+      fetch_rows(step);
+      copy_commit();
+    }
     copy_wait<kRowsStages - 2>();
     __syncthreads();                               // the first stage is there
     for (int step = 0; step < steps; ++step) {     // (into the stage that was multiplied last)
@@ -203,6 +220,7 @@ gemm_f32_rows_kernel(const float* __restrict__ a, int lda, const float* __restri
     }
     __syncthreads();
   }
+  mir::grid_dependency_wait();                     // (c may be what an earlier kernel left)
   if (!owner || col0 + tx >= n) return;
 #pragma unroll
   for (int e = 0; e < EACH; ++e)
@@ -219,22 +237,25 @@ struct Product {
   cudaStream_t stream;
 };
 
+// early: whether it may start beside the kernel in front.
 template <typename Kernel>
-int launch(Kernel kernel, dim3 grid, int threads, int smem, const Product& p) {
+int launch(bool early, Kernel kernel, dim3 grid, int threads, int smem, const Product& p) {
   const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (err != cudaSuccess) {
     mir_set_error("gemm_f32: %s", cudaGetErrorString(err));
     return MIR_CUDA_ERROR;
   }
-  kernel<<<grid, threads, smem, p.stream>>>(p.a, p.lda, p.w, p.ldw, p.bias, p.c, p.ldc, p.m, p.n, p.k, p.beta);
-  return mir_check_launch("gemm_f32");
+  return mir_launch_with(early && mir_pdl_enabled(), "gemm_f32", kernel, grid, dim3(threads), smem, p.stream, 0, p.a, p.lda, p.w, p.ldw, p.bias, p.c, p.ldc, p.m, p.n,
+                    p.k, p.beta);
 }
 
 template <int MT, bool WIDE>
 int launch_rows(const Product& p) {
   constexpr int smem = kRowsStages * (kRowsColumns + MT) * (kRowsDepth + 4) * (int)sizeof(float);
-  return launch(gemm_f32_rows_kernel<MT, WIDE>, dim3((p.n + kRowsColumns - 1) / kRowsColumns),
-                kRowsThreads + kRowsLoaders, smem, p);
+  // Started early, a grid that does not fill the GPU lands on the SMs that are left first, several CTAs on one (three rows,
+  // K 2,048: 128 CTAs 18.8 us plainly, 23.4 early; 192 12.0 and 15.2; 688 34.6 and 28.1).
+  const int ctas = (p.n + kRowsColumns - 1) / kRowsColumns;
+  return launch(ctas >= 3 * mir_sm_count(), gemm_f32_rows_kernel<MT, WIDE>, dim3(ctas), kRowsThreads + kRowsLoaders, smem, p);
 }
 
 template <int BM, int BN, int TM, int TN, bool WIDE>
@@ -245,7 +266,8 @@ int launch_tile(const Product& p) {
     mir_set_error("gemm_f32: %d rows exceed the grid limit", p.m);
     return MIR_BAD_ARGUMENT;
   }
-  return launch(gemm_f32_tile_kernel<BM, BN, TM, TN, DEPTH, STAGES, WIDE>, grid, (BM / TM) * (BN / TN), smem, p);
+  // (never early: 290 rows, tiles of two waves or less, 212 us plainly and 246 beside the kernel in front)
+  return launch(false, gemm_f32_tile_kernel<BM, BN, TM, TN, DEPTH, STAGES, WIDE>, grid, (BM / TM) * (BN / TN), smem, p);
 }
 
 template <bool WIDE>

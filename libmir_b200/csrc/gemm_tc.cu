@@ -113,8 +113,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_base_slot;
-  grid_launch_dependents();
   grid_dependency_wait();                                   // x (and out for ACCUM) come from earlier kernels
+  grid_launch_dependents();
   if (grouped.tiles != nullptr) {                           // the list of row tiles was written by an earlier kernel
     token_tiles = grouped.tile_count[0];
     tiles = token_tiles * column_tiles;

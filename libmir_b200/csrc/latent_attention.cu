@@ -43,8 +43,8 @@ __global__ void latent_prepare_kernel(const T* __restrict__ packed, long long ld
                                       const T* __restrict__ turn_src, long long src_token, long long src_head,
                                       T* __restrict__ turn_dst, long long dst_token, long long dst_head, int turn_heads) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = blockIdx.x;
   const int position = positions[token];
   if (position < 0) return;                                      // a padding row of a captured batch
@@ -103,6 +103,8 @@ __global__ void __launch_bounds__(256)
 latent_gather_kernel(const T* __restrict__ pages, int width, const int* __restrict__ block_table, int table_width,
                      const int* __restrict__ context_lens, int page_size, T* __restrict__ gathered,
                      int* __restrict__ tile_table, int tile_width) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.y, tile = blockIdx.x;
   const int context = context_lens[row], first_key = tile * kGatherRows;
   if (first_key >= context) return;
@@ -127,8 +129,8 @@ __global__ void rope_rows_kernel(const T* __restrict__ src, long long src_token,
                                  long long dst_token, long long dst_head, const int* __restrict__ positions,
                                  const float* __restrict__ inv_freq, float magnitude, int interleaved, int tokens,
                                  int heads, int rotary) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int half = rotary / 2;
   const long long index = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= (long long)tokens * heads * half) return;
@@ -156,8 +158,8 @@ __global__ void head_linear_kernel(const T* __restrict__ x, long long x_token, l
                                    const T* __restrict__ w, T* __restrict__ out, long long out_token, long long out_head,
                                    const T* __restrict__ gate, long long gate_token, int tokens, int in_dim, int out_dim) {
   __shared__ float rows[kHeadLinearTokens][kHeadLinearChunk];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int head = blockIdx.y;
   const int o = blockIdx.x * 32 + threadIdx.x;
   const int token = blockIdx.z * kHeadLinearTokens + threadIdx.y;
@@ -186,8 +188,8 @@ __global__ void head_linear_kernel(const T* __restrict__ x, long long x_token, l
 template <typename T>
 __global__ void sigmoid_gate_kernel(T* __restrict__ x, long long x_stride, const T* __restrict__ gate, long long gate_stride,
                                     int columns, size_t total) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const size_t row = index / columns;
@@ -248,12 +250,10 @@ MIR_EXPORT int mir_latent_gather(int bf16, const void* pages, int width, const i
   }
   const dim3 grid(tiles, rows);
   if (bf16)
-    latent_gather_kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)pages, width, block_table, table_width, context_lens,
-                                                   page_size, (__nv_bfloat16*)gathered, tile_table, tiles);
-  else
-    latent_gather_kernel<<<grid, 256, 0, stream>>>((const float*)pages, width, block_table, table_width, context_lens, page_size,
-                                                   (float*)gathered, tile_table, tiles);
-  return mir_check_launch("latent_gather");
+    return mir_launch("latent_gather", latent_gather_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, 0, pages, width,
+                      block_table, table_width, context_lens, page_size, gathered, tile_table, tiles);
+  return mir_launch("latent_gather", latent_gather_kernel<float>, grid, dim3(256), 0, stream, 0, pages, width, block_table,
+                    table_width, context_lens, page_size, gathered, tile_table, tiles);
 }
 
 MIR_EXPORT int mir_rope_rows(int bf16, const void* src, long long src_token, long long src_head, void* dst,

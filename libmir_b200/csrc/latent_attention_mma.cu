@@ -77,6 +77,8 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
   float* sum_s = correction_s + kRows;
   float* max_s = sum_s + kRows;
 
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int thread = threadIdx.x, lane = thread & 31, warp = thread >> 5;
   const int row = blockIdx.y;
   const int start = query_starts[row];
@@ -308,6 +310,8 @@ __global__ void __launch_bounds__(kMergeThreads)
 latent_attention_merge_kernel(const float* __restrict__ partial_o, const float* __restrict__ partial_ml,
                               __nv_bfloat16* __restrict__ out, int rank, int partitions) {
   __shared__ float factor_s[kMergePartitions], sum_s[kMergePartitions];
+  grid_dependency_wait();
+  grid_launch_dependents();
   const size_t unit = blockIdx.x;
   const int lane = threadIdx.x & 31;
   const float2* ml = reinterpret_cast<const float2*>(partial_ml) + unit * partitions;
@@ -374,11 +378,9 @@ int launch(cudaStream_t stream, dim3 grid, size_t smem, const void* q, long long
     }
     raised = smem;
   }
-  latent_attention_kernel<NT><<<grid, kThreads, smem, stream>>>(
-      (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)pages, block_table, table_width,
-      query_starts, context_lens, page_size, heads, width, rank, scale, partition_keys, partitions, partial_o, partial_ml,
-      query_rows, key_buffers);
-  return mir_check_launch("latent_attention");
+  return mir_launch("latent_attention", latent_attention_kernel<NT>, grid, dim3(kThreads), smem, stream, 0, q, q_stride, out, pages,
+                    block_table, table_width, query_starts, context_lens, page_size, heads, width, rank, scale, partition_keys,
+                    partitions, partial_o, partial_ml, query_rows, key_buffers);
 }
 
 }  // namespace
@@ -422,11 +424,7 @@ MIR_EXPORT int mir_latent_attention_bf16(const void* q, long long q_stride, void
 #undef MIR_LATENT
   if (status != MIR_OK || partitions == 1) return status;
   const dim3 merged(tokens * heads), merging(kMergeThreads);
-  if (rank > 256)
-    latent_attention_merge_kernel<4><<<merged, merging, 0, stream>>>(partial_o, partial_ml, (__nv_bfloat16*)out, rank, partitions);
-  else if (rank > 128)
-    latent_attention_merge_kernel<2><<<merged, merging, 0, stream>>>(partial_o, partial_ml, (__nv_bfloat16*)out, rank, partitions);
-  else
-    latent_attention_merge_kernel<1><<<merged, merging, 0, stream>>>(partial_o, partial_ml, (__nv_bfloat16*)out, rank, partitions);
-  return mir_check_launch("latent_attention_merge");
+  return mir_launch("latent_attention_merge", rank > 256 ? latent_attention_merge_kernel<4>
+                    : rank > 128 ? latent_attention_merge_kernel<2> : latent_attention_merge_kernel<1>, merged, merging, 0, stream, 0,
+                    partial_o, partial_ml, out, rank, partitions);
 }

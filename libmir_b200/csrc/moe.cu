@@ -179,8 +179,8 @@ template <bool RANKED>
 __global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, int has_gate, int* __restrict__ ids,
                                  float* __restrict__ weights, float* __restrict__ shared_gate, int tokens, RouteRule rule) {
   extern __shared__ float route_shared[];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int token = blockIdx.x * kRouteWarps + warp;
   if (token >= tokens) return;
@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(kMaxExperts)
 moe_sort_few_kernel(const int* __restrict__ ids, int pairs, int experts, int tile_pairs, int* __restrict__ order,
                     int* __restrict__ offsets, int* __restrict__ tiles, int* __restrict__ tile_count) {
   __shared__ int id_s[kFewPairs], count_s[kMaxExperts], base_s[kMaxExperts], pair_sums[32], tile_sums[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int e = threadIdx.x, lane = e & 31, warp = e >> 5;       // a thread: one expert, and one pair
   count_s[e] = 0;
   const int id = e < pairs ? ids[e] : -1;
@@ -277,7 +277,6 @@ moe_plan_few_kernel(const float* logits, long long ld, int has_gate, int* __rest
   float* weight_s = plan_shared + 4 * quads;
   float* zeros = weight_s + pairs;
   float* scratch_s = zeros + rule.experts;
-  grid_launch_dependents();
   if (thread < 4) id_s[4 * quads - 1 - thread] = 0x7fffffff;
   for (int e = thread; e < rule.experts; e += kPlanThreads) zeros[e] = 0.0f;
   const long long copied = (long long)((int)blockIdx.x - 1) * kPlanThreads + thread;   // of the tokens' pieces
@@ -287,7 +286,10 @@ moe_plan_few_kernel(const float* logits, long long ld, int has_gate, int* __rest
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     const bool real = pass == 1;
-    if (real) grid_dependency_wait();
+    if (real) {
+      grid_dependency_wait();
+      grid_launch_dependents();
+    }
     uint4 held = make_uint4(0, 0, 0, 0);
     if (real && token >= 0) held = h[(size_t)token * ld_pieces + piece];
 #pragma unroll 1
@@ -380,8 +382,8 @@ moe_plan_few_kernel(const float* logits, long long ld, int has_gate, int* __rest
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS) moe_count_kernel(const int* __restrict__ ids, int pairs, int* __restrict__ counts) {
   __shared__ float scratch[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int expert = blockIdx.x;
   int n = 0;
 #pragma unroll 4
@@ -394,8 +396,8 @@ __global__ void __launch_bounds__(THREADS) moe_count_kernel(const int* __restric
 __global__ void moe_offsets_kernel(const int* __restrict__ counts, int experts, int tile_pairs, int* __restrict__ offsets,
                                    int* __restrict__ first_tile, int* __restrict__ tile_count) {
   __shared__ int pair_sums[32], tile_sums[32];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;    // 1024 threads: one expert each
   const int e = threadIdx.x;
   const int mine = e < experts ? counts[e] : 0;
@@ -439,8 +441,8 @@ moe_place_kernel(const int* __restrict__ ids, int pairs, int tile_pairs, const i
                  const int* __restrict__ first_tile, int* __restrict__ order, int* __restrict__ tiles) {
   constexpr int WARPS = THREADS / 32;
   __shared__ int warp_counts[WARPS];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int expert = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int begin = offsets[expert], total = offsets[expert + 1] - begin;
@@ -498,8 +500,8 @@ moe_grouped_kernel(const T* __restrict__ x, long long ldx, const int* __restrict
                    const int* __restrict__ offsets, int K, int N) {
   __shared__ __align__(16) float rows[kExpertTile][kGroupedChunk];
   __shared__ int source[kExpertTile];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   if ((int)blockIdx.x >= tile_count[0]) return;
   const int lane = threadIdx.x, warp = threadIdx.y, thread = warp * 32 + lane;
   const int expert = tiles[2 * blockIdx.x], start = tiles[2 * blockIdx.x + 1];
@@ -584,8 +586,8 @@ __global__ void moe_combine_kernel(float* __restrict__ residual, const float* __
                                    const float* __restrict__ shared_gate, int width, int top, int overwrite,
                                    const int* __restrict__ ids, int real_experts, const T* __restrict__ identity_rows,
                                    long long identity_stride) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = blockIdx.x;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
   if (c >= width) return;
@@ -774,8 +776,8 @@ MIR_EXPORT int mir_moe_down(int bf16, const void* hidden, const int* order, cons
 __global__ void moe_gather_rows_kernel(const uint4* __restrict__ h, long long ld_pieces, const int* __restrict__ order, int top,
                                        uint4* __restrict__ sorted, int pieces, size_t total,
                                        const int* __restrict__ sorted_count) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const size_t row = index / pieces;

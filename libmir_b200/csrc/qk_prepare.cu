@@ -28,7 +28,6 @@ qk_prepare_kernel(T* __restrict__ qkv, long long row_stride, const int* __restri
                   int span, int after, int write_kv) {
   extern __shared__ float prepare_shared[];          // [rotary_dim] cosines, sines | [warps][head_dim]
   __shared__ float scratch[32];
-  grid_launch_dependents();
   const int token = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kThreads / 32;
   const int half = rotary_dim / 2;
@@ -40,6 +39,7 @@ qk_prepare_kernel(T* __restrict__ qkv, long long row_stride, const int* __restri
   for (int pair = threadIdx.x; pair < half; pair += kThreads)
     sincosf(position * inv_freq[pair], &sines[pair], &cosines[pair]);
   grid_dependency_wait();
+  grid_launch_dependents();
   T* row = qkv + (size_t)token * (size_t)row_stride;
   const int q_width = heads * head_dim, k_width = kv_heads * head_dim;
   float inverse_q = 1.0f, inverse_k = 1.0f;

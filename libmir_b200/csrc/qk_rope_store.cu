@@ -57,8 +57,8 @@ __global__ void qk_rope_store_kernel(T* __restrict__ qkv, const int* __restrict_
                                      int head_dim, int value_dim, int rotary_dim, float eps, int write_kv,
                                      int units_per_cta, int interleaved, long long row_stride, int queries_only, QkForms forms) {
   extern __shared__ float angles[];                 // [half] cosines then [half] sines of this token
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = blockIdx.x;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;

@@ -108,8 +108,8 @@ retention_scan_kernel(const T* __restrict__ q, const T* __restrict__ k, const T*
   constexpr int ROW = 2 * PADDED + 4 + BLOCK_COLUMNS;             // q | k | q . k | v of this CTA's columns
   constexpr int CHUNK = SHORT ? kWarps : (PADDED <= 64 ? 32 : (PADDED <= 128 ? 16 : 8));
   __shared__ __align__(16) float staged[CHUNK * ROW];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int thread = warp * 32 + lane;
   const int l = lane % kLanes;
@@ -241,8 +241,8 @@ retention_prepare_kernel(const T* __restrict__ q, const T* __restrict__ k, long 
                          int activated) {
   constexpr int PADDED = 32 * PER_LANE;
   using Inputs = TokenInputs<T, PER_LANE>;
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x;
   const long long unit = (long long)blockIdx.x * kWarps + threadIdx.y;
   if (unit >= (long long)tokens * heads) return;
@@ -279,8 +279,8 @@ retention_scan_prepared_kernel(const float* __restrict__ prepared, const T* __re
   constexpr int ROW = PREPARED + BLOCK_COLUMNS;                   // and v of this CTA's columns
   constexpr int CHUNK = PADDED <= 128 ? 16 : 8, STAGES = 3, STAGE = CHUNK * ROW;
   extern __shared__ __align__(16) float staged[];                 // [STAGES][CHUNK][ROW]
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x;
   const int row = blockIdx.x, head = blockIdx.y;
   const int first_column = blockIdx.z * BLOCK_COLUMNS;
@@ -431,7 +431,7 @@ int launch_walk(cudaStream_t stream, const float* prepared, const void* v, long 
     mir_set_error("retention_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
     return MIR_CUDA_ERROR;
   }
-  return mir_launch("retention_scan", retention_scan_prepared_kernel<T, PER, kLanes, C>,
+  return mir_launch_alone("retention_scan", retention_scan_prepared_kernel<T, PER, kLanes, C>,
                     dim3(rows, heads, (value_dim + columns - 1) / columns), dim3(32, kWarps + kFetchWarps), smem, stream, 0,
                     prepared, (const T*)v, ld, decays, state, query_starts, state_slots, positions, out, heads, dim,
                     value_dim, activated);

@@ -360,8 +360,8 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float* __restric
   __shared__ int candidate_count;                  // slice 0: candidates gathered
   __shared__ int search_mode;                      // slice 0: 0 the candidates decided, 1 the nucleus must be searched
   __shared__ Crossing crossing;                    // slice 0: result of a pass of find_crossing
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   cg::cluster_group cluster = cg::this_cluster();
   const int row = blockIdx.x, slice = blockIdx.y;
   const SampleOptions opt = options[row];
@@ -708,6 +708,8 @@ __global__ void __launch_bounds__(kThreads) sample_kernel(const float* __restric
 // multiplied (runtime/src/sampling/candidate.rs:92-107).  `ids` holds each row's DISTINCT history tokens.
 __global__ void penalty_kernel(float* __restrict__ logits, size_t ld, int vocab, const int* __restrict__ ids,
                                const int* __restrict__ id_rows, const float* __restrict__ penalties, int count) {
+  grid_dependency_wait();
+  grid_launch_dependents();
   const int index = blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= count) return;
   const int row = id_rows[index], id = ids[index];
@@ -741,6 +743,6 @@ MIR_EXPORT int mir_sample(const float* logits, long long ld, int rows, int vocab
 MIR_EXPORT int mir_repetition_penalty(float* logits, long long ld, int vocab, const int* ids, const int* id_rows,
                                       const float* penalties, int count, cudaStream_t stream) {
   if (count == 0) return MIR_OK;
-  penalty_kernel<<<(count + 255) / 256, 256, 0, stream>>>(logits, (size_t)ld, vocab, ids, id_rows, penalties, count);
-  return mir_check_launch("repetition_penalty");
+  return mir_launch("repetition_penalty", penalty_kernel, dim3((count + 255) / 256), dim3(256), 0, stream, 0, logits, (size_t)ld, vocab,
+                    ids, id_rows, penalties, count);
 }

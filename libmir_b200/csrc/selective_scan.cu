@@ -201,8 +201,8 @@ selective_scan_kernel(const T* __restrict__ x, long long ldx, const float* __res
   T* const raw_c = reinterpret_cast<T*>(shared + at.raw_c);
   float* const sums = reinterpret_cast<float*>(shared + at.sums);
   const int first_channel = blockIdx.y * kChannels;
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const int start = query_starts[row], end = query_starts[row + 1];
   if (end <= start || positions[start] < 0) return;              // the whole CTA: an empty or padding row
@@ -374,7 +374,6 @@ selective_scan_single_kernel(const T* __restrict__ x, long long ldx, const float
                              const int* __restrict__ state_slots, const int* __restrict__ positions, T* __restrict__ out,
                              int channels, int n) {
   constexpr int PAIRS = Channel<PER>::PAIRS;
-  grid_launch_dependents();
   const int l = threadIdx.x % kLanes;
   const int channel = blockIdx.y * kChannels + threadIdx.x / kLanes;
   const bool active = channel < channels;
@@ -385,6 +384,7 @@ selective_scan_single_kernel(const T* __restrict__ x, long long ldx, const float
   held.load(held.rate, rates + own, numbers, wide);
   const float bias = active ? step_bias[channel] : 0.0f, skip_factor = active ? skip[channel] : 0.0f;
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = query_starts[blockIdx.x];
   if (query_starts[blockIdx.x + 1] <= token || positions[token] < 0) return;    // the whole CTA: an empty or padding row
   float* const own_state = state + (size_t)state_slots[blockIdx.x] * channels * n + own;
@@ -427,7 +427,7 @@ int launch(const void* x, long long ldx, const float* raw_step, const float* ste
       return MIR_CUDA_ERROR;
     }
   }
-  return mir_launch("selective_scan", selective_scan_kernel<T, PER>, grid, dim3(kWalkers + kHelpers), smem, stream, 0,
+  return mir_launch_alone("selective_scan", selective_scan_kernel<T, PER>, grid, dim3(kWalkers + kHelpers), smem, stream, 0,
                     (const T*)x, ldx, raw_step, step_bias, (const T*)b, (const T*)c, ldb, (const T*)z, ldz, rates, skip, state,
                     query_starts, state_slots, positions, (T*)out, channels, n, columns, chunk);
 }

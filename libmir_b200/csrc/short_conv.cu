@@ -23,8 +23,8 @@ __global__ void short_conv_silu_kernel(const T* __restrict__ x, long long ldx, c
                                        const int* __restrict__ row_of_token, const int* __restrict__ query_starts,
                                        const int* __restrict__ state_slots, const int* __restrict__ positions,
                                        TO* __restrict__ out, int channels, int taps) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   if (c >= channels || positions[token] < 0) return;
@@ -79,8 +79,8 @@ short_conv_silu_wide_kernel(const T* __restrict__ x, long long ldx, const T* __r
                             const int* __restrict__ query_starts, const int* __restrict__ state_slots,
                             const int* __restrict__ positions, TO* __restrict__ out, int tokens, int channels) {
   constexpr int V = Piece<T>::kCount;
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
   if (c >= channels) return;
   const int first = blockIdx.x * RUN, count = min(RUN, tokens - first);

@@ -12,8 +12,8 @@ template <typename T>
 __global__ void short_conv_tail_kernel(const T* __restrict__ x, long long ldx, float* __restrict__ tail,
                                        const int* __restrict__ query_starts, const int* __restrict__ state_slots,
                                        const int* __restrict__ positions, int channels, int taps, int skip_single) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   const int start = query_starts[row], count = query_starts[row + 1] - start;

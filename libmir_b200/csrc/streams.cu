@@ -91,8 +91,8 @@ __global__ void __launch_bounds__(512, 3) layer_norm_kernel(const float* __restr
                                   const int* __restrict__ rows, int width, float eps) {
   extern __shared__ float row_values[];            // [width]
   __shared__ float scratch[64];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = rows != nullptr ? rows[blockIdx.x] : blockIdx.x;
   const int count = read != nullptr ? streams : 1;
   const float* base = x + (size_t)token * count * width;
@@ -128,7 +128,6 @@ __global__ void __launch_bounds__(512) add_layer_norm_kernel(
     float eps, const float* __restrict__ rows, const float* __restrict__ next_weight, const float* __restrict__ next_bias,
     float next_eps, T* __restrict__ out, int width) {
   __shared__ float scratch[128];
-  grid_launch_dependents();
   const size_t base = (size_t)blockIdx.x * width;
   auto load = [](float (&v)[V], const float* from) {
     if constexpr (V == 4) {
@@ -156,6 +155,7 @@ __global__ void __launch_bounds__(512) add_layer_norm_kernel(
     }
   }
   grid_dependency_wait();
+  grid_launch_dependents();
   float branch[PIECES][V], old[PIECES][V];
   float sum = 0.0f;
 #pragma unroll
@@ -272,8 +272,8 @@ int launch_add_layer_norm(float* x, const float* y, const float* weight, const f
 __global__ void streams_write_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ mix,
                                      const float* __restrict__ write, int streams, int width, size_t total) {
   __shared__ float m[kMaxStreams * kMaxStreams + kMaxStreams];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   for (int i = threadIdx.x; i < streams * streams; i += blockDim.x) m[i] = mix[i];
   for (int i = threadIdx.x; i < streams; i += blockDim.x) m[kMaxStreams * kMaxStreams + i] = write[i];
   __syncthreads();
@@ -299,8 +299,8 @@ __global__ void streams_write_kernel(float* __restrict__ x, const float* __restr
 
 __global__ void streams_spread_kernel(const float* __restrict__ x, float* __restrict__ out, int streams, int width,
                                       size_t total) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const size_t token = index / width;
@@ -311,8 +311,8 @@ __global__ void streams_spread_kernel(const float* __restrict__ x, float* __rest
 
 __global__ void streams_sum_kernel(const float* __restrict__ x, float* __restrict__ out, int streams, int width,
                                    size_t total) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const size_t index = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (index >= total) return;
   const size_t token = index / width;
@@ -336,8 +336,8 @@ __global__ void streams_write_norm_kernel(float* __restrict__ x, const float* __
   __shared__ float m[kMaxStreams * kMaxStreams + 2 * kMaxStreams];
   constexpr int kCount = S > 0 ? S : kMaxStreams;
   const int streams = S > 0 ? S : streams_given;
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   for (int i = threadIdx.x; i < streams * streams; i += blockDim.x) m[i] = mix[i];
   for (int i = threadIdx.x; i < streams; i += blockDim.x) {
     m[kMaxStreams * kMaxStreams + i] = write[i];

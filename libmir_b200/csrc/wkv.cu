@@ -22,8 +22,8 @@ __global__ void wkv_mix_kernel(const T* __restrict__ h, long long ld, float* __r
                                const float* __restrict__ mu, const int* __restrict__ row_of_token,
                                const int* __restrict__ query_starts, const int* __restrict__ state_slots,
                                const int* __restrict__ positions, T* __restrict__ out, int tokens, int width) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int token = blockIdx.x;
   if (positions[token] < 0) return;                              // a padding row of a captured batch
   const int row = row_of_token[token];
@@ -49,8 +49,8 @@ template <typename T>
 __global__ void wkv_tail_kernel(const T* __restrict__ h, long long ld, float* __restrict__ tail,
                                 const int* __restrict__ query_starts, const int* __restrict__ state_slots,
                                 const int* __restrict__ positions, int width) {
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int row = blockIdx.x;
   const int start = query_starts[row], end = query_starts[row + 1];
   if (end - start < 2 || positions[start] < 0) return;
@@ -179,8 +179,8 @@ wkv_step_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __res
   constexpr int BLOCK_COLUMNS = 32 / kLanes * kScanWarps;
   using Stage = Stager<T, kLanes * PER, kScanWarps, BLOCK_COLUMNS>;
   __shared__ __align__(16) float staged[kScanWarps * Stage::ROW];
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x, warp = threadIdx.y, l = lane % kLanes;
   const int row = blockIdx.x, head = blockIdx.y;
   const int first_column = blockIdx.z * BLOCK_COLUMNS;
@@ -218,8 +218,8 @@ wkv_prepare_kernel(const T* __restrict__ r, const T* __restrict__ k, const T* __
                    const float* __restrict__ decay_raw, const float* __restrict__ decay_bias, const float* __restrict__ bonus,
                    const int* __restrict__ positions, float* __restrict__ prepared, int tokens, int heads, int dim) {
   constexpr int PADDED = 32 * PER_LANE;
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x;
   const long long unit = (long long)blockIdx.x * kScanWarps + threadIdx.y;
   if (unit >= (long long)tokens * heads) return;
@@ -266,8 +266,8 @@ wkv_scan_kernel(const float* __restrict__ prepared, float* __restrict__ state, c
   constexpr int ROW = 3 * PADDED + 4 + BLOCK_COLUMNS;            // r | k | decay | bonus term | v of this CTA's columns
   constexpr int STAGE = kChunk * ROW;
   extern __shared__ __align__(16) float staged[];                // [kStages][kChunk][ROW]
-  grid_launch_dependents();
   grid_dependency_wait();
+  grid_launch_dependents();
   const int lane = threadIdx.x;
   const int row = blockIdx.x, head = blockIdx.y;
   const int first_column = blockIdx.z * BLOCK_COLUMNS;
@@ -373,7 +373,7 @@ int launch_walk(cudaStream_t stream, const float* prepared, float* state, const 
     mir_set_error("wkv_scan: cannot reserve %d bytes of shared memory: %s", smem, cudaGetErrorString(err));
     return MIR_CUDA_ERROR;
   }
-  return mir_launch("wkv_scan", wkv_scan_kernel<PER, C>, dim3(rows, heads, (dim + columns - 1) / columns),
+  return mir_launch_alone("wkv_scan", wkv_scan_kernel<PER, C>, dim3(rows, heads, (dim + columns - 1) / columns),
                     dim3(32, kScanWarps + kFetchWarps), smem, stream, 0, prepared, state, query_starts, state_slots, positions,
                     out, heads, dim);
 }

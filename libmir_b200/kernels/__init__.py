@@ -300,10 +300,10 @@ def library(name: str) -> ctypes.CDLL:
 
 
 def set_programmatic_launch(mode) -> None:
-    """How kernels are launched: 0 / False plainly; 1 / True all with programmatic stream serialization (a
+    """How kernels are launched: 0 / False plainly; 1 / True (the default) with programmatic stream serialization (a
     kernel's start overlaps the previous kernel's end; every kernel waits for its predecessor before it touches
-    activations); 2 only the weight-streaming products, whose first weights are then on their way while the
-    kernel before them drains."""
+    activations), but for the few whose CTAs each want an SM of their own; 2 only the weight-streaming products, whose
+    first weights are then on their way while the kernel before them drains."""
     for name in ("core", "bf16"):
         lib = library(name)
         lib.mir_set_pdl.argtypes = [c_int]
