@@ -68,18 +68,19 @@ struct StreamNorm {
 // tile_count[0] row tiles in all.  Expert e's weight rows start at row e * expert_rows; the result of sorted row r goes to
 // row scatter[r] of out (to row r without scatter).  list_ready: the lists were complete before any CTA of the kernel in
 // front could release this one, so weights may be asked for before that kernel is over.
+// tiles == nullptr: products of one shape side by side, every one with its own weights and its own `rows_each` rows.
 struct StreamGroups {
   const int* tiles;
   const int* tile_count;
   const int* offsets;
   const int* scatter;
-  int expert_rows, column_tiles, tile_rows, list_ready;
+  int expert_rows, column_tiles, tile_rows, list_ready, rows_each;
 };
 
 // (Shared memory lets three CTAs share an SM; the registers are capped as if six did: 56 instead of up to 95 per
 // thread, no spills, and the captured decode step at Qwen3-4B sizes takes 2.621 instead of 2.638 ms at batch 8,
 // 2.226 instead of 2.241 ms at batch 1.)
-// GROUPED (routed experts; SWIGLU and F32 only): a CTA's row tile and its expert come from a list on the device.  The
+// GROUPED (routed experts, SWIGLU and F32; products side by side, STORE): a CTA's row tile and its expert come from a list on the device.  The
 // weights then do depend on an earlier kernel; the gate-up product releases its dependents only behind its own wait, so that
 // the down product behind it finds the lists complete and fills its ring while the gate-up product drains (list_ready).
 // Bound by the experts' weights: three tokens of width 2,048, 6 of 64 experts of 1,024 each, 16 experts hit: gate-up 25 us and
@@ -139,9 +140,13 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
     }
     const int slot = blockIdx.x / groups.column_tiles;
     m = 0;
-    // (volatile: the lists may be read before the wait, and then not through a line that this SM's L1 still holds)
-    const volatile int* list = groups.tiles;
-    if (slot < *(const volatile int*)groups.tile_count) {
+    if (groups.tiles == nullptr) {
+      x0 = slot * groups.rows_each;
+      w0 = slot * groups.expert_rows + n0;
+      m = groups.rows_each;
+    } else if (slot < *(const volatile int*)groups.tile_count) {
+      // (volatile: the lists may be read before the wait, and then not through a line that this SM's L1 still holds)
+      const volatile int* list = groups.tiles;
       const int expert = list[2 * slot];
       x0 = list[2 * slot + 1];
       w0 = expert * groups.expert_rows + n0;
@@ -357,7 +362,9 @@ tc_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
           if (token >= m) break;                              // the same for every thread
           const float result = GROUPED ? value[j] : value[j] * (token < kNormStatStride ? scale[token] : 1.0f) + extra + old[j];
           if (in_range) {
-            if (GROUPED) {
+            if (GROUPED && MODE == STORE) {
+              reinterpret_cast<bf16*>(out)[(size_t)(x0 + token) * ldo + column] = __float2bfloat16_rn(result);
+            } else if (GROUPED) {
               const int row = groups.scatter != nullptr ? groups.scatter[x0 + token] : x0 + token;
               reinterpret_cast<float*>(out)[(size_t)row * ldo + column] = result;
             } else if (MODE == STORE) {
@@ -577,10 +584,25 @@ MIR_EXPORT int mir_gemm_tc_stream_grouped_bf16(int mode, const void* x, int ldx,
                   ldx, ldo, tile_pairs);
     return MIR_BAD_ARGUMENT;
   }
-  const StreamGroups groups{tiles, tile_count, offsets, scatter, n, 0, tile_pairs, list_ready};
+  const StreamGroups groups{tiles, tile_count, offsets, scatter, n, 0, tile_pairs, list_ready, 0};
   if (mode == SWIGLU)
     return launch<SWIGLU, true>(x, ldx, w, nullptr, out, ldo, rows, n, k, experts * n, StreamNorm{}, stream, groups, 2 * experts * n, max_tiles);
   return launch<F32, true>(x, ldx, w, nullptr, out, ldo, rows, n, k, 0, StreamNorm{}, stream, groups, experts * n, max_tiles);
+}
+
+// `count` products of one shape side by side: out[g] = x[g] . w[g]^T, x [count, m, k], w [count, n, k], out [count, m, n]
+// bfloat16, all contiguous.  1 <= m <= 128, k a multiple of 8, x and w 16-byte aligned.
+MIR_EXPORT int mir_gemm_tc_stream_side_by_side_bf16(const void* x, const void* w, void* out, int count, int m, int n, int k,
+                                                    cudaStream_t stream) {
+  if (m == 0 || n == 0 || count == 0) return MIR_OK;
+  if (count < 0 || m < 0 || m > 128 || n < 0 || k <= 0 || (k % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) ||
+      (long long)count * n > 0x7fffffffll) {
+    mir_set_error("tc_stream_side_by_side: needs 1..128 rows, k a multiple of 8 and 16-byte aligned operands (%d products, m %d n %d "
+                  "k %d)", count, m, n, k);
+    return MIR_BAD_ARGUMENT;
+  }
+  const StreamGroups groups{nullptr, nullptr, nullptr, nullptr, n, 0, (m + 15) / 16 * 16, 1, m};
+  return launch<STORE, true>(x, k, w, nullptr, out, n, count * m, n, k, 0, StreamNorm{}, stream, groups, count * n, count);
 }
 
 // Entries per row that mir_gemm_tc_stream_head_bf16 leaves for n output columns: four per tile of 128 columns.

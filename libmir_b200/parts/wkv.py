@@ -40,7 +40,7 @@ class Wkv(Mixer):
         if s.head_dim > 256:
             raise ValueError("the recurrence kernel takes heads up to 256 wide")
         self.width = s.heads * s.head_dim
-        self.mu = self.w_r = self.w_k = self.w_v = self.w_g = self.w_1 = self.w_2 = self.w_o = None
+        self.mu = self.w_rkvg = self.w_1 = self.w_2 = self.w_o = None
         self.decay_bias = self.bonus = self.norm = None
 
     def cache_requirement(self):
@@ -65,7 +65,7 @@ class Wkv(Mixer):
     def bind(self, tensors):
         s = self.spec
         self.mu = torch.stack([tensors[f"mu.{name}"] for name in MIXES]).contiguous()
-        self.w_r, self.w_k, self.w_v, self.w_g = (tensors[name].contiguous() for name in ("r", "k", "v", "g"))
+        self.w_rkvg = torch.stack([tensors[name] for name in ("r", "k", "v", "g")]).contiguous()
         rank = _pad8(s.decay_rank)
         w_1 = torch.zeros((rank, s.hidden_size), dtype=tensors["w1"].dtype, device=tensors["w1"].device)
         w_1[:s.decay_rank] = tensors["w1"]
@@ -78,7 +78,7 @@ class Wkv(Mixer):
         self.norm = tensors["norm"].contiguous()
 
     def weight_bytes(self):
-        tensors = (self.mu, self.w_r, self.w_k, self.w_v, self.w_g, self.w_1, self.w_2, self.w_o, self.decay_bias,
+        tensors = (self.mu, self.w_rkvg, self.w_1, self.w_2, self.w_o, self.decay_bias,
                    self.bonus, self.norm)
         return sum(t.numel() * t.element_size() for t in tensors)
 
@@ -92,8 +92,7 @@ class Wkv(Mixer):
         kernels.wkv_mix(x, tail, self.mu, ctx.row_of_token, ctx.query_starts, ctx.state_slots, ctx.positions, mixes,
                         single_tokens_only=ctx.decode_only)
         projected = ctx.alloc((4, tokens, self.width), dtype)
-        for index, weight in enumerate((self.w_r, self.w_k, self.w_v, self.w_g)):
-            kernels.linear(mixes[index], weight, projected[index], alloc=ctx.alloc)
+        kernels.linear_side_by_side(mixes[:4], self.w_rkvg, projected, alloc=ctx.alloc)
         low = ctx.alloc((tokens, self.w_1.shape[0]), dtype)
         kernels.linear(mixes[4], self.w_1, low, alloc=ctx.alloc)
         kernels.tanh(low)

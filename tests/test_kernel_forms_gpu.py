@@ -411,3 +411,18 @@ def test_gated_norms_of_heads_sum_in_one_order_whatever_holds_them(dtype, gate_d
     # the gate's own function is good to a few units in the last place; with the sum in another order a row would be off as a whole
     error = (out.double().cpu().view_as(want) - want).abs()
     assert bool((error <= (2 ** -8 if dtype == torch.bfloat16 else 4e-7) * want.abs() + 1e-30).all())
+
+
+@pytest.mark.parametrize("groups,rows,n,k", [(4, 1, 128, 64), (4, 3, 200, 136), (5, 16, 40, 72), (2, 17, 256, 512), (3, 32, 130, 64), (4, 33, 64, 64), (2, 5, 64, 60)])
+def test_products_side_by_side(groups, rows, n, k):
+    """Products of one shape in one launch (up to 32 rows; a row more and a k that is no multiple of eight go one by one): columns and steps that end inside a tile,
+    neighbouring groups' rows inside a tile."""
+    from libmir_b200 import kernels
+    torch.manual_seed(rows)
+    x, w = torch.randn(groups, rows, k).bfloat16(), torch.randn(groups, n, k).bfloat16()
+    out = torch.full((groups, rows, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    kernels.linear_side_by_side(x.cuda(), w.cuda(), out, alloc=lambda shape, kind: torch.empty(shape, dtype=kind, device="cuda"))
+    want = x.double() @ w.double().transpose(1, 2)
+    # rounded to 8 bits of mantissa; the 32-bit sums are off by far less than one of its units unless they cancel
+    bound = 2 ** -8 * want.abs() + k * 2 ** -24 * (x.double().abs() @ w.double().abs().transpose(1, 2))
+    assert ((out.cpu().double() - want).abs() <= bound).all()
