@@ -57,7 +57,10 @@ __device__ __forceinline__ void copy_wait_all() {
 //   q [tokens, heads * width] (row stride q_stride): the folded queries; out [tokens, heads * rank]
 //   pages [cache rows, width]; block_table [request rows, table_width]; query_starts [rows + 1]; context_lens [rows]
 //   partial_o [tokens * heads, partitions, rank], partial_ml [tokens * heads, partitions, 2]: only with partitions > 1
-template <int NT>
+// MT: tiles of 16 query rows a CTA has at most (decoded tokens bring heads / 16 of the four): what no row needs is in neither
+// the registers nor the instructions, which a decoded token's layer fetches anew (three rows of 16 heads at 1,100 keys, 512
+// of 576 columns the value: 17.3 us with four tiles and two key tiles a CTA, 10.4 with one of each).
+template <int NT, int MT>
 __global__ void __launch_bounds__(kThreads)
 latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride, __nv_bfloat16* __restrict__ out,
                         const __nv_bfloat16* __restrict__ pages, const int* __restrict__ block_table, int table_width,
@@ -115,9 +118,9 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
   float running_max = -INFINITY, running_sum = 0.0f;
   const float scale2 = scale * kLog2e;
 
-  float o[4][NT][4];
+  float o[MT][NT][4];
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
+  for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
@@ -155,9 +158,9 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
     }
     // S = Q K^T: this warp's 8 keys against all 64 query rows
     {
-      float s[4][4];
+      float s[MT][4];
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) s[mt][e] = 0.0f;
       const __nv_bfloat16* b_at = k_s + (size_t)(warp * 8 + (lane & 7)) * ld + ((lane >> 3) & 1) * 8;
@@ -167,7 +170,7 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
         unsigned b[2];
         ldmatrix_x2(b, b_at + k);
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt) {
+        for (int mt = 0; mt < MT; ++mt) {
           if (mt < row_tiles) {                                   // (decoded tokens: heads / 16 of the four)
             unsigned a[4];
             ldmatrix_x4(a, a_at + (size_t)mt * 16 * ld + k);
@@ -177,7 +180,7 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
       }
       const int g = lane >> 2, c = warp * 8 + (lane & 3) * 2;
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         s_s[(mt * 16 + g) * lds + c] = s[mt][0];
         s_s[(mt * 16 + g) * lds + c + 1] = s[mt][1];
         s_s[(mt * 16 + g + 8) * lds + c] = s[mt][2];
@@ -221,7 +224,7 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
     if (first_column < rank) {
       const int g = lane >> 2;
 #pragma unroll
-      for (int mt = 0; mt < 4; ++mt) {
+      for (int mt = 0; mt < MT; ++mt) {
         const float low = correction_s[mt * 16 + g], high = correction_s[mt * 16 + g + 8];
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -232,9 +235,9 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
       const __nv_bfloat16* b_at = k_s + (size_t)(lane & 15) * ld + first_column;
 #pragma unroll
       for (int k = 0; k < kKeys; k += 16) {
-        unsigned a[4][4];
+        unsigned a[MT][4];
 #pragma unroll
-        for (int mt = 0; mt < 4; ++mt)
+        for (int mt = 0; mt < MT; ++mt)
           if (mt < row_tiles) ldmatrix_x4(a[mt], a_at + mt * 16 * ldp + k);
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -242,7 +245,7 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
             unsigned b[2];
             ldmatrix_x2_trans(b, b_at + (size_t)k * ld + nt * 8);
 #pragma unroll
-            for (int mt = 0; mt < 4; ++mt)
+            for (int mt = 0; mt < MT; ++mt)
               if (mt < row_tiles) mma_bf16(o[mt][nt], a[mt], b);
           }
         }
@@ -258,7 +261,7 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
   const int g = lane >> 2, c2 = (lane & 3) * 2;
   if (partitions == 1) {
 #pragma unroll
-    for (int mt = 0; mt < 4; ++mt) {
+    for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         const int r = mt * 16 + g + half * 8;
@@ -278,7 +281,7 @@ latent_attention_kernel(const __nv_bfloat16* __restrict__ q, long long q_stride,
     return;
   }
 #pragma unroll
-  for (int mt = 0; mt < 4; ++mt) {
+  for (int mt = 0; mt < MT; ++mt) {
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const int r = mt * 16 + g + half * 8;
@@ -363,14 +366,14 @@ size_t shared_bytes(int width, int query_rows = kRows, int key_buffers = 1) {
          (size_t)kRows * (kKeys + 8) * 2 + 3 * kRows * 4;
 }
 
-template <int NT>
+template <int NT, int MT>
 int launch(cudaStream_t stream, dim3 grid, size_t smem, const void* q, long long q_stride, void* out, const void* pages,
            const int* block_table, int table_width, const int* query_starts, const int* context_lens, int page_size,
            int heads, int width, int rank, float scale, int partition_keys, int partitions, float* partial_o,
            float* partial_ml, int query_rows, int key_buffers) {
   static size_t raised = 0;
   if (smem > raised) {
-    const cudaError_t err = cudaFuncSetAttribute(latent_attention_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const cudaError_t err = cudaFuncSetAttribute(latent_attention_kernel<NT, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem);
     if (err != cudaSuccess) {
       mir_set_error("latent_attention: cannot reserve %zu bytes of shared memory: %s", smem, cudaGetErrorString(err));
@@ -378,7 +381,7 @@ int launch(cudaStream_t stream, dim3 grid, size_t smem, const void* q, long long
     }
     raised = smem;
   }
-  return mir_launch("latent_attention", latent_attention_kernel<NT>, grid, dim3(kThreads), smem, stream, 0, q, q_stride, out, pages,
+  return mir_launch("latent_attention", latent_attention_kernel<NT, MT>, grid, dim3(kThreads), smem, stream, 0, q, q_stride, out, pages,
                     block_table, table_width, query_starts, context_lens, page_size, heads, width, rank, scale, partition_keys,
                     partitions, partial_o, partial_ml, query_rows, key_buffers);
 }
@@ -414,7 +417,7 @@ MIR_EXPORT int mir_latent_attention_bf16(const void* q, long long q_stride, void
   const size_t smem = shared_bytes(width, query_rows, key_buffers);
   int status;
 #define MIR_LATENT(N)                                                                                              \
-  status = launch<N>(stream, grid, smem, q, q_stride, out, pages, block_table, table_width, query_starts,         \
+  status = (query_rows <= 16 ? launch<N, 1> : query_rows <= 32 ? launch<N, 2> : launch<N, 4>)(stream, grid, smem, q, q_stride, out, pages, block_table, table_width, query_starts,         \
                      context_lens, page_size, heads, width, rank, scale, partition_keys, partitions, partial_o, \
                      partial_ml, query_rows, key_buffers)
   if (rank <= 64) MIR_LATENT(1);

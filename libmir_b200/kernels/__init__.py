@@ -897,8 +897,8 @@ def latent_attention_plan(num_rows: int, max_pairs: int, max_context: int) -> tu
     tiles = max(1, -(-max_context // 64))
     sms = 148
     # one wave of CTAs, two tiles or more a partition (measured at 8 rows x 2,049 keys: 31 us with 17 partitions, 43
-    # with 33, 65 with 4; at 64 rows 123 us with 2, 133 with 4)
-    partitions = max(1, min(max(1, tiles // 2), sms // blocks, 64))
+    # with 33, 65 with 4; at 64 rows 123 us with 2, 133 with 4), a tile each where that is less than a wave
+    partitions = max(1, min(tiles if blocks * tiles <= sms else max(1, tiles // 2), sms // blocks, 64))
     per_partition = -(-tiles // partitions) * 64
     return per_partition, -(-max_context // per_partition) if max_context > 0 else 1
 
