@@ -50,6 +50,7 @@ constexpr int kStages = 4;                  // shared-memory ring
 constexpr int kStageStride = (kTileM + 256) * 128;   // 48 KB: 128 token rows and up to 256 weight rows of 128 bytes
 constexpr int kEpilogueWarps = 8;          // two per quarter of the accumulator lanes; they share its columns
 constexpr int kThreads = (2 + kEpilogueWarps) * 32;  // producer warp, issuer warp, epilogue warps
+constexpr int kPlaces = 64;                 // tiles of a CTA whose places are looked up before the first of them
 constexpr uint32_t kTmemColumns = 512;      // two accumulators of up to 256 columns
 // GELU: STORE of gelu_tanh(acc), no bias; GELU_ERF: the same with the exact form 0.5 z (1 + erf(z / sqrt 2)); RELU2: the
 // same with the square of relu
@@ -70,8 +71,28 @@ struct GroupedRows {
   int group_rows;
 };
 
-// One CTA per SM walks over output tiles (token tile fastest, so CTAs that run together share weight rows in
-// L2).  A tile is 128 tokens x `width` accumulator columns (width a multiple of 16, at most 256; with the SwiGLU
+// Where a tile of the output lies: its tile of rows, its tile of columns.  Plain products: token tile fastest, so CTAs that
+// run together share weight rows in L2.  Grouped ones: one group behind the other, a group's row tiles fastest, so that its
+// weights are read once and its rows stay in L2 for all its column tiles (14,800 pairs of 64 experts, 2 x 1,024 columns, K
+// 2,048: 131 us; with the row tiles of all groups fastest, which goes over all rows for every column tile, 172).  The weights'
+// boxes brought into the L2 ten steps ahead: 155 us.
+// A grouped tile's place takes four reads behind one another, which the producer would wait for at every tile: the threads of
+// a CTA look its first kPlaces up side by side before the first tile.
+struct Place { int m0, row_end, n0, w0; };                   // first row, end of the rows, first column, first row of the weights
+__device__ __forceinline__ Place place_of(int tile, int token_tiles, int column_tiles, int out_width, int m, const GroupedRows& grouped) {
+  if (grouped.tiles == nullptr) {
+    const int n0 = tile / token_tiles * out_width;
+    return Place{tile % token_tiles * kTileM, m, n0, n0};
+  }
+  const int inside = tile / column_tiles;                    // some row tile of the group: its tiles lie one behind the other
+  const int group = grouped.tiles[2 * inside], begin = grouped.offsets[group];
+  const int first = inside - (grouped.tiles[2 * inside + 1] - begin) / kTileM;
+  const int end = grouped.offsets[group + 1], count = (end - begin + kTileM - 1) / kTileM, local = tile - first * column_tiles;
+  const int n0 = local / count * out_width;
+  return Place{begin + local % count * kTileM, end, n0, group * grouped.group_rows + n0};
+}
+
+// One CTA per SM walks over output tiles (their order: place_of).  A tile is 128 tokens x `width` accumulator columns (width a multiple of 16, at most 256; with the SwiGLU
 // epilogue width / 2 gate columns followed by width / 2 up columns).  Two accumulators of 256 columns alternate,
 // so the epilogue of one tile overlaps the products of the next.
 template <int MODE>
@@ -82,6 +103,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long barriers[2 * kStages + 4];   // full, empty, accumulator full[2], free[2]
   __shared__ uint32_t tmem_base_slot;
+  __shared__ Place places[kPlaces];
   if (*reinterpret_cast<volatile int*>(&g_tc_gemm_error) != 0) return;   // an earlier wait ran out: do not queue up more
   // the swizzle pattern repeats every 1024 bytes; the stages start on such a boundary
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -118,7 +140,14 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
   if (grouped.tiles != nullptr) {                           // the list of row tiles was written by an earlier kernel
     token_tiles = grouped.tile_count[0];
     tiles = token_tiles * column_tiles;
+    const int tile = blockIdx.x + threadIdx.x * gridDim.x;
+    if (threadIdx.x < kPlaces && tile < tiles) places[threadIdx.x] = place_of(tile, token_tiles, column_tiles, out_width, m, grouped);
+    __syncthreads();
   }
+  auto place_at = [&](int tile, int number) {                // of this CTA's number-th tile
+    return grouped.tiles != nullptr && number < kPlaces ? places[number]
+                                                        : place_of(tile, token_tiles, column_tiles, out_width, m, grouped);
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
@@ -126,10 +155,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
       const uint64_t xm = reinterpret_cast<uint64_t>(&x_map), wm = reinterpret_cast<uint64_t>(&w_map);
       uint32_t count = 0;                                    // stages filled so far, over all tiles
       bool alive = true;
-      for (int tile = blockIdx.x; tile < tiles && alive; tile += gridDim.x) {
-        const int row_tile = tile % token_tiles, n0 = (tile / token_tiles) * out_width;
-        const int m0 = grouped.tiles != nullptr ? grouped.tiles[2 * row_tile + 1] : row_tile * kTileM;
-        const int w0 = n0 + (grouped.tiles != nullptr ? grouped.tiles[2 * row_tile] * grouped.group_rows : 0);
+      int number = 0;
+      for (int tile = blockIdx.x; tile < tiles && alive; tile += gridDim.x, ++number) {
+        const Place place = place_at(tile, number);
+        const int m0 = place.m0, w0 = place.w0;
         for (int step = 0; step < steps; ++step, ++count) {
           const uint32_t stage = count % kStages, parity = (count / kStages) & 1u;
           if (!wait_barrier(empty0 + 8 * stage, parity ^ 1u)) { g_tc_gemm_error = 1; alive = false; break; }
@@ -192,9 +221,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
     bool alive = true;
     for (int tile = blockIdx.x; tile < tiles && alive; tile += gridDim.x, ++local) {
       const uint32_t buffer = local & 1u, use = (local >> 1) & 1u;
-      const int row_tile = tile % token_tiles, n0 = (tile / token_tiles) * out_width;
-      const int m0 = grouped.tiles != nullptr ? grouped.tiles[2 * row_tile + 1] : row_tile * kTileM;
-      const int row_end = grouped.tiles != nullptr ? grouped.offsets[grouped.tiles[2 * row_tile] + 1] : m;
+      const Place place = place_at(tile, (int)local);
+      const int n0 = place.n0, m0 = place.m0, row_end = place.row_end;
       const int source_row = m0 + quarter * 32 + lane;
       // where this thread's row of results goes: its own row, or the place the sorted row came from
       const int row = (grouped.tiles != nullptr && grouped.scatter != nullptr && source_row < row_end)
