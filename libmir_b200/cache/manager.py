@@ -67,6 +67,13 @@ class GroupInfo:
             dead = max(dead, length // self.chunk * self.chunk)
         return max(0, dead)
 
+    def length_of(self, dead: int) -> int:
+        """The least length at which `dead` (> 0) keys are dead."""
+        reached = [dead + self.window - 1] if self.window is not None else []
+        if self.chunk is not None:
+            reached.append(-(-dead // self.chunk) * self.chunk)
+        return min(reached)
+
     @property
     def keep_first(self) -> int:
         """With a window: the request's first tokens that every later query still sees (their pages stay)."""
@@ -238,6 +245,17 @@ class CacheManager:
             pool.forget(page)
             dropped += 1
         return dropped
+
+    def untouched_until(self, sequence: Sequence_) -> int:
+        """The length up to which the request's pages stay as they are when its next token (not committed yet) and those
+        behind it are fed one by one: nothing is taken below this length and nothing given back."""
+        page = self.page_size
+        until = min((len(table) * page for table in sequence.tables), default=1 << 62)
+        for index, group in enumerate(self.groups):
+            if group.releases:                                 # the first step that leaves block `first` without a reader
+                first = max(sequence.first_live[index], self._blocks_for(group.keep_first))
+                until = min(until, group.length_of(first * page + page) - 1)
+        return until
 
     def commit(self, sequence: Sequence_, new_length: int, tokens: Optional[Sequence[int]] = None) -> None:
         """The tokens up to new_length are now cached; release what windows have passed.  `tokens`: the ids that were

@@ -78,6 +78,21 @@ int mir_sm_count() {
 
 MIR_EXPORT int mir_abi_version() { return 1; }
 
+// What a decode step uploads: once `event` says that the last upload has left the pinned block, `bytes` of `from` go into that
+// block and on to the device in stream order, and the event is recorded behind the copy.  One call from Python: a tensor's
+// copy_ and an event's synchronize and record took 18 us of a step's 60 on the host, this takes 5.
+MIR_EXPORT int mir_upload(cudaEvent_t event, void* pinned, const void* from, size_t bytes, void* device, cudaStream_t stream) {
+  cudaError_t err = cudaEventSynchronize(event);
+  if (err == cudaSuccess) {
+    memcpy(pinned, from, bytes);
+    err = cudaMemcpyAsync(device, pinned, bytes, cudaMemcpyHostToDevice, stream);
+  }
+  if (err == cudaSuccess) err = cudaEventRecord(event, stream);
+  if (err == cudaSuccess) return MIR_OK;
+  mir_set_error("upload: %s", cudaGetErrorString(err));
+  return MIR_CUDA_ERROR;
+}
+
 // 0 off, 1 every kernel but the ones that are launched alone, 2 only the kernels that stream weights before they wait.
 // Whole calls by streaming ones / every kernel (ms), the gaps between the small kernels of a decoded token being what goes:
 // Zufotar 16.5 / 15.9, Biravik 13.8 / 13.4, Doderax 13.0 / 12.7, Qwen3-4B sizes, one prompt of 37 and 12 tokens, 27.3 / 27.0.

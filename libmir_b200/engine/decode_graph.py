@@ -84,7 +84,7 @@ class DecodeGraph:
         self.meta = torch.zeros(upload + groups * rows + rows + rows + (rows + 1) + rows, dtype=torch.int32,
                                 device=device)
         self.staging = torch.zeros(upload, dtype=torch.int32, pin_memory=True)
-        self._host = self.staging.numpy()
+        self._host = np.zeros(upload, dtype=np.int32)         # what goes into the staging block when the last upload has left it
         self._upload = upload
         cut = lambda index: self.meta[int(self._offsets[index]):int(self._offsets[index + 1])]
         self.options = cut(0).view(torch.uint8)
@@ -117,8 +117,11 @@ class DecodeGraph:
         self.host_tokens = torch.zeros(rows, dtype=torch.int32, pin_memory=True)
         self.launches_per_replay = 0
         self.replays = 0
-        self._copied = None
+        self._copied = torch.cuda.Event()
+        self._copied.record()
         self._fast_tokens, self._fast_positions = self._host_part(1), self._host_part(2)
+        self._fast_previous = self._host_part(4 + groups) if self.pairs else None
+        self._results: Dict[int, tuple] = {}       # rows -> the views of a step's logits and sampled tokens
         self._live_rows = -1                       # rows the upload block was last filled for
         self._greedy_options = False               # whether its sampling records are the greedy defaults
         self.graph: Optional[torch.cuda.CUDAGraph] = None
@@ -162,7 +165,7 @@ class DecodeGraph:
         greedy = np.zeros(self.rows, dtype=kernels.SAMPLE_OPTIONS)
         greedy["top_p"] = 1.0
         self._host_part(0)[:] = greedy.view(np.int32)
-        self.meta[:self._upload].copy_(self.staging)
+        self.meta[:self._upload].copy_(torch.from_numpy(self._host))
         stream = torch.cuda.Stream(device=self.runner.device)
         stream.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(stream):
@@ -190,8 +193,6 @@ class DecodeGraph:
     def load(self, tokens: Sequence[int], sequences, options: Optional[np.ndarray]) -> None:
         """Fill the upload block for the live rows (the rest is padding) and copy it to the device."""
         n = len(tokens)
-        if self._copied is not None:
-            self._copied.synchronize()             # the previous copy has read the pinned block
         host_tokens, host_positions, host_slots = self._host_part(1), self._host_part(2), self._host_part(3)
         host_tokens[:n] = tokens
         host_positions[:n] = [seq.length for seq in sequences]
@@ -233,22 +234,26 @@ class DecodeGraph:
                 if written[r] is not None:
                     table[r] = 0
                     written[r] = None
-        self.meta[:self._upload].copy_(self.staging, non_blocking=True)
-        if self._copied is None:
-            self._copied = torch.cuda.Event()
-        self._copied.record()
+        kernels.upload(self._copied, self.staging, self._host, self.meta)
 
     def load_again(self, tokens: Sequence[int], sequences, draws: Optional[Sequence[float]] = None) -> None:
-        """The upload for the same rows with the same sampling settings as the last `load`, none of which got a page
-        since: only the tokens, the positions and (for samplers that draw) the draws differ."""
+        """The upload for the same rows with the same sampling settings as the last `load`, whose pages are what they were
+        then: only the tokens, the positions, the tokens before them and (for samplers that draw) the draws differ."""
         n = len(tokens)
-        self._copied.synchronize()                 # the previous copy has read the pinned block
         self._fast_tokens[:n] = tokens
         self._fast_positions[:n] = [seq.length for seq in sequences]
+        if self.pairs:
+            self._fast_previous[:n] = [seq.last_token for seq in sequences]
         if draws is not None:
             self._host_part(0).view(kernels.SAMPLE_OPTIONS)["draw"][:n] = draws
-        self.meta[:self._upload].copy_(self.staging, non_blocking=True)
-        self._copied.record()
+        kernels.upload(self._copied, self.staging, self._host, self.meta)
+
+    def results(self, rows: int) -> tuple:
+        """The logits and the sampled tokens of the first `rows` rows (views of the graph's buffers)."""
+        views = self._results.get(rows)
+        if views is None:
+            views = self._results[rows] = (self.logits[:rows], self.sampled[:rows])
+        return views
 
     def replay(self) -> None:
         self.graph.replay()

@@ -94,6 +94,7 @@ _SIGNATURES = {
         "mir_moe_route": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_int, c_float, c_int, c_int, c_void_p],
         "mir_moe_tile_slots": [c_int, c_int, c_int],
+        "mir_upload": [c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p],
         "mir_moe_plan_few_takes": [c_int] * 5,
         "mir_moe_plan_few": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_int, c_int, c_float, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -298,6 +299,13 @@ def library(name: str) -> ctypes.CDLL:
         function.restype = c_int
     _LIBS[name] = lib
     return lib
+
+
+def upload(event: torch.cuda.Event, pinned: torch.Tensor, block: np.ndarray, device: torch.Tensor) -> None:
+    """`block` through the pinned tensor into `device` (all int32 of one size), in the order of the current stream, once
+    `event` (recorded before) says that the last upload has left the pinned tensor; records `event` behind the copy."""
+    lib = library("core")
+    _check(lib, lib.mir_upload(event.cuda_event, pinned.data_ptr(), block.ctypes.data, block.nbytes, device.data_ptr(), _stream()))
 
 
 def set_programmatic_launch(mode) -> None:

@@ -333,3 +333,32 @@ def test_random_orders_with_a_prefix_cache_share_only_what_is_the_same(seed, pag
     manager.check()
     assert pool.available == pool.count and manager.free_slots == 4
     assert pool.free + len(manager.prefix) == pool.count
+
+
+@given(st.lists(st.tuples(st.one_of(st.none(), st.integers(1, 23)), st.one_of(st.none(), st.integers(1, 19)), st.integers(0, 9)), max_size=3),
+       st.integers(1, 8), st.integers(0, 40))
+@settings(max_examples=150, deadline=None)
+def test_the_length_up_to_which_pages_stay_as_they_are(groups, page, start):
+    """Token by token: below the length that is promised tables change at no step, and at it they do (a page is taken, or one is
+    given back that still held keys of readers)."""
+    plan = [CacheEntryPlan(i, PagedKv(1, 8 + i, window=w, keep_first=k, chunk=c), i, True) for i, (w, c, k) in enumerate(groups)]
+    manager = CacheManager(plan, page_size=page, num_pages=90, max_requests=1)
+    seq = manager.admit("r")
+    manager.grow(seq, start); manager.commit(seq, start)
+    promised = None
+    for length in range(start, start + 45):
+        before = ([list(table) for table in seq.tables], list(seq.first_live))
+        manager.grow(seq, length + 1)
+        grown = [list(table) for table in seq.tables]
+        if promised is not None and length < promised:
+            assert grown == before[0]
+        until = manager.untouched_until(seq)                 # what a step asks before it commits
+        manager.commit(seq, length + 1)
+        released = [list(table) for table in seq.tables] != grown
+        if promised is not None and length < promised:
+            assert not released
+        elif promised is not None and groups:
+            assert released or grown != before[0]
+        assert (until <= length) == released
+        promised = until if length + 1 <= until else None
+    manager.check()
