@@ -245,13 +245,21 @@ delta_rule_prepare_run_kernel(const T* __restrict__ x, long long ldx, const T* _
   const int my_row = row_of_token[mine];
   const int my_start = query_starts[my_row], my_end = query_starts[my_row + 1], my_position = positions[mine];
   float taps_of[4][kRunTaps];                                    // [channel][tap], right-aligned: the last is the token's own
+  if (taps == kRunTaps && (uintptr_t)w % (kRunTaps * sizeof(T)) == 0) {      // a channel's taps in one load (2,274 tokens, below: 75 to 70 us)
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < kRunTaps; ++j) {
-      const int tap = j - (kRunTaps - taps);
-      taps_of[i][j] = tap >= 0 ? to_float(w[(size_t)(c + i) * taps + tap]) : 0.0f;
+    for (int i = 0; i < 4; ++i) {
+      const float4 own = quad_of(w + (size_t)(c + i) * kRunTaps);
+      taps_of[i][0] = own.x; taps_of[i][1] = own.y; taps_of[i][2] = own.z; taps_of[i][3] = own.w;
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < kRunTaps; ++j) {
+        const int tap = j - (kRunTaps - taps);
+        taps_of[i][j] = tap >= 0 ? to_float(w[(size_t)(c + i) * taps + tap]) : 0.0f;
+      }
+  }
   const float q_scale = rsqrtf((float)key_dim);
   float4 before[kRunTaps - 1] = {};                              // the inputs before the token, right-aligned
   int row = -1;
