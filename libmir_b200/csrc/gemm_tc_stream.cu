@@ -39,6 +39,11 @@ constexpr int kWeightBytes = 128 * 128;     // a stage's weights: 128 rows of 12
 constexpr int kMaxStages = 8;
 constexpr int kThreads = 6 * 32;            // producer warp, issuer warp, four epilogue warps
 constexpr int kRingBytes = 72 * 1024;       // per CTA, so that three CTAs fit on an SM
+// A product of few CTAs has too little on its way with three small rings' worth of SMs (160 CTAs: 11.5 MB): six stages, so that
+// two CTAs fit on an SM.  Whole calls, ring of 72 / 90 / 108 / 126 KB for up to 222 CTAs: Qwen3-4B sizes, one prompt of 37 and
+// 12 tokens 25.9 / 25.2 / 25.0 / 28.4 ms, 8 prompts of 320 and 24 tokens 62.7 / 60.7 / 60.2 / 66.9 (the kernels around it no longer
+// fit beside it); for up to 160 or 256 CTAs the same to 0.5 %.
+constexpr int kLargeRingBytes = 108 * 1024, kLargeRingCtas = 222;
 int g_ring_bytes = kRingBytes;               // for measurements
 enum Epilogue : int { STORE = 0, ACCUM = 1, F32 = 2, SWIGLU = 3 };
 
@@ -427,12 +432,14 @@ int g_forced_rows = 0;
 // Tile height and how many CTAs share K.  Measured on B200 (8 rows, inside a CUDA graph, us): whole 128-row tiles
 // beat 64- and 32-row tiles at every shape (QKV 9.0 / 15.5 / 18.1, output projection 7.7 / 10.5 / 11.5), and K is
 // best cut as far as one wave of CTAs allows (three fit on an SM): output projection 7.7 with 8 CTAs per tile,
-// 10.4 with 4, 16.8 with 2.
+// 10.4 with 4, 16.8 with 2.  A wave that is nearly full (385 to 444 CTAs) leaves no room for the next kernel's: Doderax, whose
+// mixers' inputs are 50 tiles, whole call 12.32 ms with 400 CTAs, 12.18 with 200; up to 300 CTAs only, Qwen3-4B sizes 25.0 to 25.8.
+constexpr int kMostCtas = 384;
 void choose_shape(int n, int total_steps, bool swiglu, int slots, int* tile_rows, int* splits) {
   const int rows = swiglu ? 64 : 128;
   const long long tiles = (long long)((n + rows - 1) / rows) * slots;
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= 3 * 148 && total_steps / (s * 2) >= 4) s *= 2;
+  while (s < 8 && tiles * s * 2 <= kMostCtas && total_steps / (s * 2) >= 4) s *= 2;
   *tile_rows = rows;
   *splits = s;
 }
@@ -457,7 +464,9 @@ int launch(const void* x, int ldx, const void* w, const void* bias, void* out, i
   const int weight_bytes = (MODE == SWIGLU ? 128 : tile_rows) * 128;
   const int stage_stride = (weight_bytes + tokens * 128 + 1023) / 1024 * 1024;
   const int tile_bytes = tokens * 128 * 4;                    // the transposed tile reuses the ring
-  int stages = std::max(2, std::min(kMaxStages, g_ring_bytes / stage_stride));
+  const long long ctas = (long long)((n + tile_rows - 1) / tile_rows) * slots * splits;
+  const int ring = g_ring_bytes == kRingBytes && ctas <= kLargeRingCtas ? kLargeRingBytes : g_ring_bytes;
+  int stages = std::max(2, std::min(kMaxStages, ring / stage_stride));
   while (stages * stage_stride < tile_bytes) ++stages;
   // the A operand of the last stage reads 128 rows whatever the tile's height: room for that behind the ring
   const size_t smem = (size_t)stages * stage_stride + std::max(0, kWeightBytes - stage_stride) + 1024;
