@@ -426,3 +426,40 @@ def test_products_side_by_side(groups, rows, n, k):
     # rounded to 8 bits of mantissa; the 32-bit sums are off by far less than one of its units unless they cancel
     bound = 2 ** -8 * want.abs() + k * 2 ** -24 * (x.double().abs() @ w.double().abs().transpose(1, 2))
     assert ((out.cpu().double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("n,k", [(14208, 520), (14209, 512), (24576, 512), (24577, 520), (28416, 256), (28417, 264)])
+@pytest.mark.parametrize("rows", [1, 32])
+def test_weight_streams_on_both_sides_of_the_rings_and_the_cuts(rows, n, k):
+    """111 and 112 tiles of columns cut in two (222 and 224 blocks), 192 and 193 (384 blocks, or no cut), 222 and 223 that are not
+    cut: the large ring and the small one, with steps that do not fill it."""
+    from libmir_b200 import kernels
+    torch.manual_seed(n + rows)
+    x, w = torch.randn(rows, k).bfloat16(), torch.randn(n, k).bfloat16()
+    out = torch.full((rows, n), float("nan"), device="cuda")
+    kernels.linear(x.cuda(), w.cuda(), out)
+    # sums of k products in 32 bits: each partial sum off by at most 2^-24 of the sum of the products' sizes
+    bound = k * 2 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert ((out.cpu().double() - x.double() @ w.double().T).abs() <= bound).all()
+    assert kernels.tensor_core_linear_error() == 0
+
+
+@pytest.mark.parametrize("experts,width,full", [(640, 2560, 0), (1024, 2560, 0), (1024, 2568, 300)])
+def test_grouped_products_of_more_tiles_than_are_looked_up_at_once(experts, width, full):
+    """43, 69 and 76 tiles a block: one expert's tiles behind another's, with an expert of several tiles of rows among them."""
+    from libmir_b200 import kernels
+    torch.manual_seed(experts)
+    inter, alloc = 8, lambda shape, kind: torch.zeros(shape, dtype=kind, device="cuda")
+    ids = torch.cat([torch.arange(experts), torch.full((full,), experts // 2)]).int()[:, None].contiguous()
+    found = kernels.moe_sort(ids.cuda(), experts, alloc, 128)
+    hidden, w = torch.randn(len(ids), inter).bfloat16().cuda(), torch.randn(experts, width, inter).bfloat16().cuda()
+    out = torch.full((len(ids), width), float("nan"), device="cuda")
+    kernels.moe_down(hidden, found, w, out)
+    order = found.order.long()
+    for first in range(0, len(ids), 64):
+        pairs = order[first:first + 64]
+        x, rows = hidden[first:first + 64].double(), w[ids[:, 0].cuda().long()[pairs]].double()
+        error = (out[pairs].double() - torch.einsum("pi,pwi->pw", x, rows)).abs()
+        # eight products in 32 bits, each partial sum off by at most 2^-24 of the sum of their sizes
+        assert (error <= inter * 2 ** -24 * torch.einsum("pi,pwi->pw", x.abs(), rows.abs())).all()
+    assert kernels.tensor_core_linear_error() == 0
