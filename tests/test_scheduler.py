@@ -1,9 +1,13 @@
 """The scheduler's decisions with the real cache manager and a step function that runs nothing (no GPU)."""
 
+from array import array
+from types import SimpleNamespace
+
+import numpy as np
 import pytest
 import torch
 
-from libmir_b200 import KvCapacity, SchedulerError, build_spec
+from libmir_b200 import KvCapacity, SchedulerError, StepEntry, build_spec
 from libmir_b200.cache import CacheManager
 from libmir_b200.config import GenerationSettings, SchedulerConfig
 from libmir_b200.engine.scheduler import Request, Scheduler
@@ -341,3 +345,23 @@ def test_random_traffic_with_a_prefix_cache_feeds_every_token_once_in_order(seed
             assert item.finish_reason == "out_of_pages"
     pool = manager.groups[0].pool
     assert pool.available == pool.count and manager.free_slots == 4 and not manager.live
+
+
+@pytest.mark.parametrize("kind", [list, tuple, bytearray, lambda ids: memoryview(bytes(ids)), lambda ids: np.array(ids, np.uint8),
+                                  lambda ids: np.array(ids, np.int64), lambda ids: array("q", ids), lambda ids: array("i", ids),
+                                  lambda ids: torch.tensor(ids), lambda ids: [np.int64(i) for i in ids]])
+def test_token_ids_are_whole_numbers_whatever_holds_them(kind):
+    """A step's tokens packed on the host: one id an element, also where the elements are narrower or wider than the ids that
+    go to the device; an id outside the vocabulary is named with its request."""
+    _, runner, manager = build()
+    runner.storage = SimpleNamespace(views=None)
+    runner._stage = lambda arrays: [torch.from_numpy(np.array(a).reshape(-1)) for a in arrays]
+    for name in ("a", "b"):
+        manager.admit(name)
+    first, second = [5, 0, 96, 17, 33, 2, 1, 8], [9, 11, 3, 4]
+    entries, sequences = runner.reserve([StepEntry("a", kind(first), [7]), StepEntry("b", kind(second), [3])])
+    ctx, _, _ = runner.build_context(entries, sequences)
+    assert ctx.tokens.tolist() == first + second and ctx.tokens.dtype == torch.int32
+    for outside in (-1, TINY_A["vocab_size"], 2 ** 31 + 9, -2 ** 40):
+        with pytest.raises(SchedulerError, match="'b'.*outside"):
+            runner.build_context([entries[0], StepEntry("b", [9, outside], [0])], sequences)
