@@ -1087,6 +1087,7 @@ class ExpertOrder:
         self.tile_count = alloc((1,), torch.int32)
         self.scratch = alloc((2, experts), torch.int32)            # counts and first tiles while sorting
         self.rows = None                                           # the tokens' rows in this order, where they exist already
+        self.streamed_on = None                                    # the stream on which moe_gate_up streamed weights by this order
 
     def max_tiles(self) -> int:
         """No more tiles than this, whatever the routing: every tile holds a pair, and all but an expert's last are full."""
@@ -1178,6 +1179,7 @@ def moe_gate_up(h: torch.Tensor, found: ExpertOrder, top: int, w_gate: torch.Ten
                                                         experts, hidden.data_ptr(), inter, inter, width, found.tiles.data_ptr(),
                                                         found.tile_count.data_ptr(), found.offsets.data_ptr(), None,
                                                         found.tile_pairs, found.max_tiles(), 0, _stream()))
+        found.streamed_on = _stream()
         return
     if found.tile_pairs == 128:
         _require(h.dtype == torch.bfloat16 and alloc is not None
@@ -1200,11 +1202,8 @@ def moe_gate_up(h: torch.Tensor, found: ExpertOrder, top: int, w_gate: torch.Ten
                                     inter, found.tile_pairs, _stream()))
 
 
-def moe_down(hidden: torch.Tensor, found: ExpertOrder, w_down: torch.Tensor, pair_rows: torch.Tensor,
-             behind_gate_up: bool = False) -> None:
-    """pair_rows[pair] = w_down[e] hidden[i] (32-bit [pairs, width]) for the i-th pair in expert order.  behind_gate_up: the
-    launch in front of this one on the stream was moe_gate_up of the same order (its kernel releases this one only when the
-    order is complete, so the first weights may be asked for while it still runs)."""
+def moe_down(hidden: torch.Tensor, found: ExpertOrder, w_down: torch.Tensor, pair_rows: torch.Tensor) -> None:
+    """pair_rows[pair] = w_down[e] hidden[i] (32-bit [pairs, width]) for the i-th pair in expert order."""
     _cuda(hidden, w_down, pair_rows)
     experts, width, inter = w_down.shape
     _require(hidden.is_contiguous() and hidden.shape == (found.pairs, inter) and w_down.is_contiguous()
@@ -1212,12 +1211,14 @@ def moe_down(hidden: torch.Tensor, found: ExpertOrder, w_down: torch.Tensor, pai
              and pair_rows.shape == (found.pairs, width) and found.experts == experts,
              "moe_down: shapes or dtypes do not fit")
     if found.rows is not None:
+        # Behind moe_gate_up of the same order on the same stream the first weights may be asked for ahead of the wait: its
+        # kernel releases what follows only when the order is complete.
         lib = library("bf16")
         _check(lib, lib.mir_gemm_tc_stream_grouped_bf16(MODE_F32, hidden.data_ptr(), inter, found.pairs, w_down.data_ptr(), experts,
                                                         pair_rows.data_ptr(), width, width, inter, found.tiles.data_ptr(),
                                                         found.tile_count.data_ptr(), found.offsets.data_ptr(),
                                                         found.order.data_ptr(), found.tile_pairs, found.max_tiles(),
-                                                        int(behind_gate_up), _stream()))
+                                                        int(found.streamed_on == _stream()), _stream()))
         return
     if found.tile_pairs == 128:
         _require(hidden.dtype == torch.bfloat16, "moe_down: the tcgen05 product takes bfloat16")

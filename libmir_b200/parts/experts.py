@@ -112,7 +112,7 @@ class RoutedExperts(FeedForward):
         hidden = ctx.alloc((tokens * s.top, s.expert_size), dtype)
         kernels.moe_gate_up(x, found, s.top, self.w_gate, self.w_up, hidden, ctx.alloc)
         pair_rows = ctx.alloc((tokens * s.top, s.hidden_size), torch.float32)
-        kernels.moe_down(hidden, found, self.w_down, pair_rows, behind_gate_up=True)
+        kernels.moe_down(hidden, found, self.w_down, pair_rows)
         shared_rows = None
         if s.shared_size:
             shared_hidden = ctx.alloc((tokens, s.shared_size), dtype)

@@ -56,7 +56,7 @@ def test_few_tokens_through_their_experts(tokens, experts, real, top, groups, ke
 
     both_d, hidden, pair_rows = both.cuda(), alloc((tokens * top, inter), bf16), alloc((tokens * top, width), torch.float32)
     kernels.moe_gate_up(h_d, found, top, both_d[:real], both_d[real:], hidden, alloc)
-    kernels.moe_down(hidden, found, w_down.cuda(), pair_rows, behind_gate_up=True)
+    kernels.moe_down(hidden, found, w_down.cuda(), pair_rows)
     pair_rows, hidden = pair_rows.cpu().double(), hidden.cpu().double()
     for place, pair in enumerate(order.tolist()):
         e, x = int(ids.reshape(-1)[pair]), h[pair // top].double()
