@@ -2194,8 +2194,8 @@ def linear_side_by_side(x: torch.Tensor, weights: torch.Tensor, out: torch.Tenso
     groups, m, k = x.shape
     n = weights.shape[1]
     _require(weights.shape == (groups, n, k) and out.shape == (groups, m, n), "linear_side_by_side: shapes do not fit")
-    if x.dtype == weights.dtype == out.dtype == torch.bfloat16 and 0 < m <= get_option("few_rows_max") and k % 8 == 0 \
-            and get_option("few_rows_modes") & 1 and x.is_contiguous() and weights.is_contiguous() and out.is_contiguous() \
+    if x.dtype == weights.dtype == out.dtype == torch.bfloat16 and 0 < m <= min(get_option("few_rows_max"), STREAM_MAX_ROWS) \
+            and k % 8 == 0 and get_option("few_rows_modes") & 1 and x.is_contiguous() and weights.is_contiguous() and out.is_contiguous() \
             and x.data_ptr() % 16 == 0 and weights.data_ptr() % 16 == 0:
         _cuda(x, weights, out)
         lib = library("bf16")

@@ -63,3 +63,15 @@ def test_a_down_product_looks_ahead_only_behind_its_own_gate_up(recorder):
     assert looks_ahead(first) == 0
     gate_up(second)
     assert looks_ahead(second) == 1 and looks_ahead(first) == 0
+
+
+@pytest.mark.parametrize("rows, allowed, together", [(128, 201, True), (129, 201, False), (32, 33, True), (33, 33, True), (34, 33, False)])
+def test_products_side_by_side_keep_to_the_rows_the_weight_stream_takes(recorder, monkeypatch, rows, allowed, together):
+    """few_rows_max may be raised beyond the 128 rows of the streaming kernel: more rows go one product behind the other."""
+    recorder.answers["mir_get_option"] = allowed                 # (an odd number: also few_rows_modes with the store epilogue)
+    alone = []
+    monkeypatch.setattr(kernels, "linear", lambda x, w, out, alloc=None: alone.append(x.shape))
+    x, w = torch.zeros(4, rows, 16, dtype=torch.bfloat16), torch.zeros(4, 24, 16, dtype=torch.bfloat16)
+    kernels.linear_side_by_side(x, w, torch.zeros(4, rows, 24, dtype=torch.bfloat16))
+    streamed = [args for name, args in recorder.calls if name == "mir_gemm_tc_stream_side_by_side_bf16"]
+    assert (len(streamed), len(alone)) == ((1, 0) if together else (0, 4))
