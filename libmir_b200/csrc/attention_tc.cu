@@ -392,7 +392,10 @@ tc_prefill_attention_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   __shared__ float references[2][kStreams][kRows];
   __shared__ float handed[2][kRows];                          // kShared: a row's reference after the CTA's tile g, by g & 1
   __shared__ int query_tiles_slot;
-  if (*reinterpret_cast<volatile int*>(&g_tc_attention_error) != 0) return;
+  if (*reinterpret_cast<volatile int*>(&g_tc_attention_error) != 0) {       // an earlier wait ran out: do not queue up more
+    grid_dependency_wait();                                   // (what follows takes the kernels in front of this one for over)
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int cta = blockIdx.x, ctas = gridDim.x;
 

@@ -104,7 +104,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant_
   __shared__ __align__(8) unsigned long long barriers[2 * kStages + 4];   // full, empty, accumulator full[2], free[2]
   __shared__ uint32_t tmem_base_slot;
   __shared__ Place places[kPlaces];
-  if (*reinterpret_cast<volatile int*>(&g_tc_gemm_error) != 0) return;   // an earlier wait ran out: do not queue up more
+  if (*reinterpret_cast<volatile int*>(&g_tc_gemm_error) != 0) {            // an earlier wait ran out: do not queue up more
+    grid_dependency_wait();                                 // (what follows takes the kernels in front of this one for over)
+    return;
+  }
   // the swizzle pattern repeats every 1024 bytes; the stages start on such a boundary
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

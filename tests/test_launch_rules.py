@@ -1,5 +1,8 @@
 """What the host decides about a launch, and what every kernel's source has to keep, without a GPU."""
 
+import re
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -75,3 +78,68 @@ def test_products_side_by_side_keep_to_the_rows_the_weight_stream_takes(recorder
     kernels.linear_side_by_side(x, w, torch.zeros(4, rows, 24, dtype=torch.bfloat16))
     streamed = [args for name, args in recorder.calls if name == "mir_gemm_tc_stream_side_by_side_bf16"]
     assert (len(streamed), len(alone)) == ((1, 0) if together else (0, 4))
+
+
+def kernels_of(source):
+    """(name, body) of every kernel in a CUDA source, comments left out."""
+    source = re.sub(r"//[^\n]*", "", source)
+    for match in re.finditer(r"\b__global__\b", source):
+        opened = source.index("{", match.end())
+        if ";" in source[match.end():opened]:
+            continue                                             # a declaration
+        depth, at = 1, opened + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(source[at], 0)
+            at += 1
+        head = re.sub(r"__launch_bounds__\s*\((?:[^()]|\([^()]*\))*\)", "", source[match.end():opened])
+        yield re.search(r"(\w+)\s*\(", head).group(1), source[opened + 1:at - 1]
+
+
+def leaves_before_it_waits(body):
+    """Whether some return of a kernel is not behind a wait that every thread coming there has been through: one in the same
+    block or in a block around it, under no condition of its own."""
+    blocks, waited = [False], [False]                            # of each open block: a function of its own; waited in it
+    token = re.compile(r"\{|\}|grid_dependency_wait\(\)|\breturn\b")
+    for match in token.finditer(body):
+        statement = re.split(r"[;{}]", body[:match.start()])[-1]
+        if match.group() == "{":
+            blocks.append(blocks[-1] or re.search(r"\]\s*\([^()]*\)\s*(mutable\s*)?(->\s*\w+\s*)?$", statement) is not None)
+            waited.append(waited[-1])
+        elif match.group() == "}":
+            blocks.pop()
+            waited.pop()
+        elif match.group() == "return":
+            if not blocks[-1] and not waited[-1]:
+                return True
+        elif not re.search(r"\b(if|else|for|while)\b", statement):
+            waited[-1] = True
+    return False
+
+
+def test_kernels_wait_for_the_one_in_front_on_every_way_out():
+    """A kernel that is over before the one in front of it lets the next kernel run beside that one.  So every kernel that may be
+    released early waits, also where it has nothing to do; only what is always launched plainly need not."""
+    plain = {"cast_kernel", "random_normal_kernel", "paged_attention_mixed_kernel", "mixed_row_sums_kernel", "mixed_weights_kernel",
+             "mixed_values_kernel", "mixed_row_sums_tc_kernel", "mixed_weights_tc_kernel", "mixed_values_tc_kernel"}
+    folder = Path(kernels.__file__).parent.parent / "csrc"
+    sources = {path.name: path.read_text() for path in sorted(folder.glob("*.cu*"))}
+    found = [(file, name, body) for file, source in sources.items() for name, body in kernels_of(source)]
+    assert len(found) > 60
+    launched_plainly = {re.sub(r"<.*", "", name) for source in sources.values() for name in re.findall(r"(\w+(?:<[\w, ]*>)?)<<<", source)}
+    assert launched_plainly - {"kernel"} <= plain                # ("kernel": the macro for what writes weights)
+    for file, name, body in found:
+        if name in plain:
+            assert "grid_launch_dependents" not in body, (file, name)
+            continue
+        assert "grid_dependency_wait()" in body, (file, name)
+        assert not leaves_before_it_waits(body), (file, name)
+
+
+def test_the_check_of_waits_sees_a_way_out_without_one():
+    wait = "mir::grid_dependency_wait();"
+    fine = ("int a = 0; " + wait + " if (a) return;", "if (a) { " + wait + " return; }", "auto f = [&](int x) { return x; }; " + wait,
+            "auto f = [&](int x) -> int { if (x) { return 1; } return x; }; " + wait, "if (!a) " + wait + " if (a) " + wait)
+    wrong = ("if (a) return; " + wait, "if (a) { b(); return; } " + wait, "if (a) " + wait + " if (b) return; " + wait,
+             "if (a) { " + wait + " } if (b) return;", "for (;;) { " + wait + " } return;")
+    assert not any(leaves_before_it_waits(body) for body in fine)
+    assert all(leaves_before_it_waits(body) for body in wrong)
