@@ -44,7 +44,7 @@ constexpr int kRingBytes = 72 * 1024;       // per CTA, so that three CTAs fit o
 // 12 tokens 25.9 / 25.2 / 25.0 / 28.4 ms, 8 prompts of 320 and 24 tokens 62.7 / 60.7 / 60.2 / 66.9 (the kernels around it no longer
 // fit beside it); for up to 160 or 256 CTAs the same to 0.5 %.
 constexpr int kLargeRingBytes = 108 * 1024, kLargeRingCtas = 222;
-int g_ring_bytes = kRingBytes;               // for measurements
+int g_forced_ring = 0;                       // for measurements (0: the launcher chooses)
 enum Epilogue : int { STORE = 0, ACCUM = 1, F32 = 2, SWIGLU = 3 };
 
 __device__ int g_tc_stream_error = 0;
@@ -71,8 +71,8 @@ struct StreamNorm {
 // The products of routed experts on a few rows sorted by expert (csrc/moe.cu): tiles[2 i], tiles[2 i + 1] are the expert and
 // the first row of row tile i, which ends with its expert's rows, offsets[expert + 1], or after `tile_rows` of them;
 // tile_count[0] row tiles in all.  Expert e's weight rows start at row e * expert_rows; the result of sorted row r goes to
-// row scatter[r] of out (to row r without scatter).  list_ready: the lists were complete before any CTA of the kernel in
-// front could release this one, so weights may be asked for before that kernel is over.
+// row scatter[r] of out (to row r without scatter).  list_ready: the gate-up product on the same lists went over the
+// stream before; it releases what follows only when they are complete, so weights may be asked for ahead of the wait.
 // tiles == nullptr: products of one shape side by side, every one with its own weights and its own `rows_each` rows.
 struct StreamGroups {
   const int* tiles;
@@ -444,6 +444,15 @@ void choose_shape(int n, int total_steps, bool swiglu, int slots, int* tile_rows
   *splits = s;
 }
 
+}  // namespace
+
+// Bytes of the ring of a product of `ctas` CTAs.
+MIR_EXPORT int mir_gemm_tc_stream_ring(long long ctas) {
+  return g_forced_ring > 0 ? g_forced_ring : ctas <= kLargeRingCtas ? kLargeRingBytes : kRingBytes;
+}
+
+namespace {
+
 // GROUPED: x [m, k] the sorted rows, w `weight_rows` rows, row tiles of at most groups.tile_rows rows from the device's list,
 // at most `slots` of them.
 template <int MODE, bool GROUPED = false>
@@ -465,8 +474,7 @@ int launch(const void* x, int ldx, const void* w, const void* bias, void* out, i
   const int stage_stride = (weight_bytes + tokens * 128 + 1023) / 1024 * 1024;
   const int tile_bytes = tokens * 128 * 4;                    // the transposed tile reuses the ring
   const long long ctas = (long long)((n + tile_rows - 1) / tile_rows) * slots * splits;
-  const int ring = g_ring_bytes == kRingBytes && ctas <= kLargeRingCtas ? kLargeRingBytes : g_ring_bytes;
-  int stages = std::max(2, std::min(kMaxStages, ring / stage_stride));
+  int stages = std::max(2, std::min(kMaxStages, mir_gemm_tc_stream_ring(ctas) / stage_stride));
   while (stages * stage_stride < tile_bytes) ++stages;
   // the A operand of the last stage reads 128 rows whatever the tile's height: room for that behind the ring
   const size_t smem = (size_t)stages * stage_stride + std::max(0, kWeightBytes - stage_stride) + 1024;
@@ -500,16 +508,16 @@ MIR_EXPORT int mir_gemm_tc_stream_error() {
 
 MIR_EXPORT int mir_gemm_tc_stream_max_rows() { return 128; }
 
-// For measurements: 1, 2, 4 or 8 CTAs per cluster, the ring's size in KB, the tile's height (0: the launcher chooses).
+// For measurements: 1, 2, 4 or 8 CTAs per cluster, the ring's size in KB, the tile's height (0: the launcher chooses each).
 MIR_EXPORT int mir_gemm_tc_stream_set_splits(int splits, int ring_kb, int tile_rows) {
-  if ((splits != 0 && splits != 1 && splits != 2 && splits != 4 && splits != 8) || ring_kb < 32 || ring_kb > 200 ||
+  if ((splits != 0 && splits != 1 && splits != 2 && splits != 4 && splits != 8) || (ring_kb != 0 && (ring_kb < 32 || ring_kb > 200)) ||
       (tile_rows != 0 && tile_rows != 32 && tile_rows != 64 && tile_rows != 128)) {
-    mir_set_error("tc_stream: splits must be 0, 1, 2, 4 or 8, the ring 32..200 KB, the tile 0, 32, 64 or 128 rows");
+    mir_set_error("tc_stream: splits must be 0, 1, 2, 4 or 8, the ring 0 or 32..200 KB, the tile 0, 32, 64 or 128 rows");
     return MIR_BAD_ARGUMENT;
   }
   g_forced_splits = splits;
   g_forced_rows = tile_rows;
-  g_ring_bytes = ring_kb * 1024;
+  g_forced_ring = ring_kb * 1024;
   return MIR_OK;
 }
 
@@ -577,9 +585,8 @@ MIR_EXPORT int mir_gemm_tc_stream_bf16(int mode, const void* x, int ldx, const v
 // The products of routed experts on few rows sorted by expert.  mode 3 (SwiGLU): out bf16 [rows, n] = silu(x w_gate[e]^T) *
 // (x w_up[e]^T) with w = [experts * n gate rows; experts * n up rows]; mode 2: out float [*, n] = x w[e]^T, sorted row r's
 // result in row scatter[r].  tiles / tile_count / offsets: row tiles of tile_pairs (16 to 128, a multiple of 16) rows, their
-// number and the experts' row ranges, all on the device; at most max_tiles of them.  list_ready: these lists were complete
-// before the kernel in front of this one released its dependents (it was the gate-up product on the same lists).  k and ldx
-// multiples of 8, x and w 16-byte aligned.
+// number and the experts' row ranges, all on the device; at most max_tiles of them.  list_ready: the gate-up product (mode 3) on
+// these lists went over `stream` before.  k and ldx multiples of 8, x and w 16-byte aligned.
 MIR_EXPORT int mir_gemm_tc_stream_grouped_bf16(int mode, const void* x, int ldx, int rows, const void* w, int experts,
                                                void* out, int ldo, int n, int k, const int* tiles, const int* tile_count,
                                                const int* offsets, const int* scatter, int tile_pairs, int max_tiles,

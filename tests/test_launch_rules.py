@@ -143,3 +143,15 @@ def test_the_check_of_waits_sees_a_way_out_without_one():
              "if (a) { " + wait + " } if (b) return;", "for (;;) { " + wait + " } return;")
     assert not any(leaves_before_it_waits(body) for body in fine)
     assert all(leaves_before_it_waits(body) for body in wrong)
+
+
+def test_a_weight_streams_ring_is_the_one_asked_for():
+    lib = kernels.library("bf16")
+    try:
+        for forced in (72, 108, 40, 0):
+            assert lib.mir_gemm_tc_stream_set_splits(0, forced, 0) == 0
+            assert [lib.mir_gemm_tc_stream_ring(ctas) for ctas in (1, 222, 223, 10000)] == \
+                ([forced * 1024] * 4 if forced else [108 * 1024] * 2 + [72 * 1024] * 2)
+        assert lib.mir_gemm_tc_stream_set_splits(0, 201, 0) != 0 and lib.mir_gemm_tc_stream_set_splits(0, 31, 0) != 0
+    finally:
+        lib.mir_gemm_tc_stream_set_splits(0, 0, 0)
