@@ -469,28 +469,41 @@ def test_repeated_greedy_decode_steps_take_the_short_path_and_stay_right(tmp_pat
     model.unload()
 
 
-@pytest.mark.parametrize("requests, prompt", [(1, 125), (3, 126), (96, 20), (97, 20)])
-def test_decoded_tokens_on_both_sides_of_the_short_context_rule(tmp_path, requests, prompt):
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("requests, prompt, page", [(1, 125, 16), (3, 126, 16), (96, 20, 16), (97, 20, 16), (2, 126, 32)])
+def test_decoded_tokens_on_both_sides_of_the_short_context_rule(tmp_path, requests, prompt, page, captured):
     """Up to 128 keys and 192 pairs of request and KV head run the mma.sync kernel, more the tcgen05 kernel: contexts that
-    pass 128 keys, and 192 and 194 pairs of short ones; every request's logits are the plain implementation's."""
+    pass 128 keys, and 192 and 194 pairs of short ones; every request's logits are the plain implementation's.  A captured
+    step goes by its table, which is 8 pages wide or more: 128 keys with pages of 16, 256 with pages of 32."""
     from libmir_b200 import StepEntry, kernels
+    from libmir_b200.engine.decode_graph import row_bucket
+    from libmir_b200.sampling import RequestSampler
     config = ALL["E"]
     folder = make_folder(tmp_path, config, seed=8, dtype="bfloat16", sharpen=4.0)
     rng = np.random.default_rng(8)
     texts = [random_ids(rng, config["vocab_size"], prompt + 5) for _ in range(min(requests, 4))]
-    model = load(folder, "bfloat16", pages=256, page_size=16, max_batch_requests=128)
+    model = load(folder, "bfloat16", pages=256, page_size=page, max_batch_requests=128)
     reference = [plain_logits(folder, ids) for ids in texts]
     ids_of = lambda r: texts[r % len(texts)]
+    samplers = [RequestSampler() for _ in range(requests)] if captured else None
     for r in range(requests):
         model.admit(str(r))
         model.step([StepEntry(str(r), ids_of(r)[:prompt - r % 2], [])])          # lengths that differ by one
+    seen = None
     for step in range(5):
         starts = [prompt - r % 2 + step for r in range(requests)]
         counts = kernels.launch_counts()
-        got = model.step([StepEntry(str(r), [ids_of(r)[starts[r]]], [0]) for r in range(requests)]).logits.cpu().numpy()
-        short = max(starts) + 1 <= 128 and requests * config["num_key_value_heads"] <= 192
+        got = model.step([StepEntry(str(r), [ids_of(r)[starts[r]]], [0]) for r in range(requests)], samplers).logits.cpu().numpy()
+        short = max(starts) + 1 <= 128 and (row_bucket(requests) if captured else requests) * config["num_key_value_heads"] <= 192
+        if captured:
+            short = short and page <= 16
         now = kernels.launch_counts()
         ran = [now.get(name, 0) - counts.get(name, 0) for name in ("decode_attention", "decode_attention_tc")]
-        assert (ran[1] == 0) == short and (ran[0] > 0) == short, (step, ran)
+        if captured and short == seen:
+            assert ran == [0, 0], (step, ran)                                    # a replay: counted when it was captured
+        else:
+            assert (ran[1] == 0) == short and (ran[0] > 0) == short, (step, ran)
+        seen = short
         for r in range(requests):
             check(got[r], reference[r % len(texts)][starts[r]], TOL["bfloat16"], f"request {r} step {step}")
+    model.unload()

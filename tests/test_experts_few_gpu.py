@@ -54,9 +54,10 @@ def test_few_tokens_through_their_experts(tokens, experts, real, top, groups, ke
     assert tiles[:, 0].tolist() == counts.nonzero().reshape(-1).tolist()   # one tile for every expert that has a pair
     assert tiles[:, 1].tolist() == found.offsets.cpu()[:-1][counts > 0].tolist()
 
-    both_d, hidden, pair_rows = both.cuda(), alloc((tokens * top, inter), bf16), alloc((tokens * top, width), torch.float32)
+    both_d, w_down_d = both.cuda(), w_down.cuda()
+    hidden, pair_rows = alloc((tokens * top, inter), bf16), alloc((tokens * top, width), torch.float32)
     kernels.moe_gate_up(h_d, found, top, both_d[:real], both_d[real:], hidden, alloc)
-    kernels.moe_down(hidden, found, w_down.cuda(), pair_rows)
+    kernels.moe_down(hidden, found, w_down_d, pair_rows)
     pair_rows, hidden = pair_rows.cpu().double(), hidden.cpu().double()
     for place, pair in enumerate(order.tolist()):
         e, x = int(ids.reshape(-1)[pair]), h[pair // top].double()
@@ -71,30 +72,47 @@ def test_few_tokens_through_their_experts(tokens, experts, real, top, groups, ke
     assert kernels.tensor_core_linear_error() == 0
 
 
-def test_rows_of_a_kernel_that_still_runs():
+def test_experts_behind_kernels_that_still_run():
     """The tokens' rows and the router's logits come from products that are still running when the next kernels of a captured
-    step are released: what is gathered is what they leave, not what was there before."""
+    step are released, and the down product asks for weights by lists that the plan left a kernel before: every replay with
+    other tokens leaves what the same kernels leave when each starts behind the end of the one in front."""
     from libmir_b200 import kernels
     generator = torch.Generator(device="cuda").manual_seed(1)
     make = lambda *shape: (torch.randn(*shape, generator=generator, device="cuda") * 0.05).to(torch.bfloat16)
-    tokens, width, deep, experts, top = 3, 512, 65536, 64, 6
+    tokens, width, deep, experts, top, inter = 3, 512, 65536, 64, 6, 256
     weight, router, x = make(width, deep), make(experts, width), make(tokens, deep)
-    h, logits = alloc((tokens, width), torch.bfloat16), alloc((tokens, experts), torch.float32)
-    ids, weights = alloc((tokens, top), torch.int32), alloc((tokens, top), torch.float32)
+    both, w_down = make(2 * experts, inter, width), make(experts, width, inter)
 
-    def step():
+    def step(buffers):
+        h, logits, ids, weights, hidden, pair_rows = buffers
         kernels.linear(x, weight, h)
         kernels.linear(h, router, logits)
-        return kernels.moe_plan_few(h, logits, None, False, ids, weights, None, experts, experts, top, 8, 4, 1.0, alloc)
-    step()
+        found = kernels.moe_plan_few(h, logits, None, False, ids, weights, None, experts, experts, top, 8, 4, 1.0, alloc)
+        kernels.moe_gate_up(h, found, top, both[:experts], both[experts:], hidden, alloc)
+        kernels.moe_down(hidden, found, w_down, pair_rows)
+        return found
+
+    buffers, others = ([alloc((tokens, width), torch.bfloat16), alloc((tokens, experts), torch.float32),
+                        alloc((tokens, top), torch.int32), alloc((tokens, top), torch.float32),
+                        alloc((tokens * top, inter), torch.bfloat16), alloc((tokens * top, width), torch.float32)] for _ in range(2))
+    step(buffers)
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        found = step()
-    other_ids, other_weights = torch.zeros_like(ids), torch.zeros_like(weights)
-    for _ in range(3):
+        found = step(buffers)
+    chosen = set()
+    for _ in range(6):
         x.copy_(make(tokens, deep))
         graph.replay()
-        kernels.moe_route(logits, None, False, other_ids, other_weights, None, experts, top, 8, 4, 1.0)
-        assert torch.equal(ids, other_ids) and torch.equal(weights, other_weights)
-        assert torch.equal(found.rows, h[found.order.long() // top])
+        torch.cuda.synchronize()
+        kernels.set_programmatic_launch(0)
+        try:
+            plain = step(others)
+        finally:
+            kernels.set_programmatic_launch(1)
+        for one, other in zip(buffers, others):
+            assert torch.equal(one, other)
+        assert torch.equal(found.order, plain.order) and torch.equal(found.rows, buffers[0][found.order.long() // top])
+        chosen.add(tuple(buffers[2].flatten().tolist()))
+    assert len(chosen) == 6                                                # another routing every time
+    assert kernels.tensor_core_linear_error() == 0
