@@ -89,8 +89,6 @@ struct MirStepDesc {
 
 namespace {
 
-constexpr int kShortKeys = 128, kShortUnits = 192;            // see attend(): keys; requests x KV heads
-
 #define MIR_TRY(call)                    \
   do {                                   \
     const int status_ = (call);          \
@@ -170,14 +168,10 @@ struct Run {
       const int singles = step.decode_only ? step.rows : step.singles;
       if (singles > 0) {
         const int longest = step.decode_only ? step.max_context : step.single_context;
-        // Decoded tokens of few requests whose contexts all fit into one tile of keys run the mma.sync kernel, one CTA for a
-        // request and KV head: the tcgen05 kernel's chain (two products through tensor memory, four barriers) is longer than
-        // the work.  Decode steps at Qwen3-4B sizes, 12 layers, tcgen05 / mma.sync (us): up to 128 keys 1 request 706 / 686,
-        // 4 722 / 707, 8 737 / 728, 24 886 / 878, but 53 1,045 / 1,075; up to 256 keys 1 request 720 / 740, 24 907 / 918.
-        if (step.decode_only && longest <= kShortKeys && singles * layer.kv_heads <= kShortUnits) {
+        if (step.decode_only && mir_decode_attention_short(singles, layer.kv_heads, longest)) {
           MIR_TRY(mir_decode_attention_bf16(step.qkv, width, step.mixed, layer.k_pages, layer.v_pages, group.block_table,
                                             group.table_width, step.positions, singles, layer.page_size, layer.heads,
-                                            layer.kv_heads, layer.head_dim, layer.scale, layer.window, kShortKeys, 1,
+                                            layer.kv_heads, layer.head_dim, layer.scale, layer.window, MIR_SHORT_KEYS, 1,
                                             step.attention_scratch, step.attention_scratch_floats, step.stream));
           return MIR_OK;
         }

@@ -112,6 +112,8 @@ int mir_decode_attention_paged_bf16(const void* q, long long q_stride, void* out
                                     const int* positions, int rows, int page_size, int heads, int kv_heads,
                                     int head_dim, float scale, int window, int partition, int num_partitions,
                                     float* scratch, long long scratch_floats, cudaStream_t stream);
+#define MIR_SHORT_KEYS 128              // most keys of a context that mir_decode_attention_short takes
+int mir_decode_attention_short(int rows, int kv_heads, int longest);
 int mir_decode_partition_keys(int rows, int heads, int kv_heads, int head_dim, int page_size, int longest);
 int mir_decode_attention_plan(int rows, int heads, int kv_heads, int head_dim, int page_size, int longest,
                               int* partition, int* partitions, long long* scratch_floats);

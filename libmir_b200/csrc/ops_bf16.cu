@@ -145,6 +145,16 @@ MIR_EXPORT int mir_decode_partition_keys(int rows, int heads, int kv_heads, int 
   return best;
 }
 
+// Whether the decoded tokens of a step without portions, in a layer that the executor knows (csrc/executor.cu; the same from
+// Python), run the mma.sync kernel on one partition, one CTA for a request and KV head: few requests whose contexts all fit
+// into one tile of keys.  The tcgen05 kernel's chain (two products through tensor memory, four barriers) is longer than the
+// work there.  Decode steps at Qwen3-4B sizes (8 KV heads), 12 layers, tcgen05 / mma.sync (us): up to 128 keys 1 request 706 /
+// 686, 4 722 / 707, 8 737 / 728, 24 886 / 878, but 53 1,045 / 1,075; up to 256 keys 1 request 720 / 740, 24 907 / 918.
+constexpr int kShortUnits = 192;                              // requests x KV heads: the last pair of figures that gained
+MIR_EXPORT int mir_decode_attention_short(int rows, int kv_heads, int longest) {
+  return longest <= MIR_SHORT_KEYS && (long long)rows * kv_heads <= kShortUnits;
+}
+
 // Attention of single decoded tokens over the pages: the tcgen05 kernel where it takes the sizes, else the mma.sync
 // kernel.  Arguments as mir_decode_attention_bf16, and how many token rows the cache tensors have.
 // sinks (32-bit, one per query head: its exponential joins the softmax's denominator) and gate (rows [token][heads *

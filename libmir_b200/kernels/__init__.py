@@ -165,6 +165,7 @@ _SIGNATURES = {
         "mir_head_logits_bf16": [c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
                                  c_int, c_void_p, c_size_t, c_void_p, c_void_p],
         "mir_gemm_tc_stream_head_candidates": [c_int],
+        "mir_decode_attention_short": [c_int, c_int, c_int],
         "mir_decode_partition_keys": [c_int, c_int, c_int, c_int, c_int, c_int],
         "mir_decode_attention_plan": [c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p],
         "mir_decode_attention_tc_error": [],
@@ -1786,6 +1787,15 @@ def decode_attention_kept_plan(rows: int, heads: int, head_dim: int, max_context
     return partition, count, decode_attention_scratch_floats(rows, heads, head_dim, count)
 
 
+SHORT_KEYS = 128             # most keys of a context that decode_attention_short takes (MIR_SHORT_KEYS)
+
+
+def decode_attention_short(rows: int, kv_heads: int, max_context: int) -> bool:
+    """Whether `rows` decoded tokens (a step without portions) of a layer that the native executor knows run the mma.sync
+    kernel on one partition of SHORT_KEYS keys; the rule is native, the executor's own."""
+    return bool(library("bf16").mir_decode_attention_short(rows, kv_heads, max_context))
+
+
 def decode_attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tensor,
                      block_table: torch.Tensor, positions: torch.Tensor, page_size: int, heads: int, kv_heads: int,
                      head_dim: int, scale: float, window: Optional[int], partition: int, num_partitions: int,
@@ -1793,7 +1803,7 @@ def decode_attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor
                      numbering: Optional[torch.Tensor] = None, sinks: Optional[torch.Tensor] = None,
                      gate: Optional[torch.Tensor] = None, gate_per_head: bool = False, softcap: Optional[float] = None,
                      distance_bias: Optional[torch.Tensor] = None, slopes: Optional[torch.Tensor] = None,
-                     value_dim: Optional[int] = None) -> None:
+                     value_dim: Optional[int] = None, short: bool = False) -> None:
     """bf16 split-KV attention for a batch of single tokens (row r of qkv belongs to request row r).  `keep_first`:
     with a window, the request's first keys that stay visible; the mma.sync kernel then walks over the kept keys and
     the window's as one run, and `numbering` (int32 [rows]) is scratch for the merge.  `sinks`, `gate`: as
@@ -1801,7 +1811,8 @@ def decode_attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor
     merge of its partitions, adds the sink's term and applies the gate).  `gate_per_head`, `softcap`, `distance_bias`:
     as paged_attention_generic takes them: the scores are capped and biased in 32-bit before the softmax, by the
     tcgen05 kernel where it takes the sizes and the partition (decode_attention_plan), else by the mma.sync kernel.
-    `slopes` likewise; `value_dim`: width of a value head where it differs from a key head's."""
+    `slopes` likewise; `value_dim`: width of a value head where it differs from a key head's.  `short`: the mma.sync kernel, none
+    of these options (decode_attention_short)."""
     _cuda(qkv, out, k_pages, v_pages, block_table, positions, scratch, sinks, gate, distance_bias, slopes)
     rows = out.shape[0]
     value_dim = head_dim if value_dim is None else value_dim
@@ -1816,6 +1827,14 @@ def decode_attention(qkv: torch.Tensor, out: torch.Tensor, k_pages: torch.Tensor
     lib = library("bf16")
     _require(k_pages.is_contiguous() and v_pages.is_contiguous() and k_pages.shape[0] == v_pages.shape[0],
              "decode_attention: the cache tensors must be contiguous [token rows, kv_heads, head_dim]")
+    if short:
+        _require(not (keep_first and window) and sinks is None and gate is None and not softcap and distance_bias is None
+                 and slopes is None and value_dim == head_dim, "decode_attention: a short context goes with none of the options")
+        _check(lib, lib.mir_decode_attention_bf16(
+            qkv.data_ptr(), qkv.stride(0), out.data_ptr(), k_pages.data_ptr(), v_pages.data_ptr(), block_table.data_ptr(),
+            block_table.shape[1], positions.data_ptr(), rows, page_size, heads, kv_heads, head_dim, scale, int(window or 0),
+            partition, num_partitions, _ptr(scratch), 0 if scratch is None else scratch.numel(), _stream()))
+        return
     if gate_per_head or softcap or distance_bias is not None or slopes is not None or value_dim != head_dim:
         _require(not (keep_first and window), "decode_attention: capped or biased scores do not go with kept first keys")
         _check(lib, lib.mir_decode_attention_paged_scored_bf16(

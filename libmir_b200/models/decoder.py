@@ -258,10 +258,12 @@ class DecoderModel:
             return self._runs_list
         from ..kernels.executor import LayerRun
         self._native = {}
-        if kernels.NATIVE_LAYERS:
-            for index, entry in enumerate(self.spec.schedule):
-                self._native[index] = self.blocks[entry.layer].native_descriptor(ctx.cache_view(index)) \
-                    if entry.opens_pass is None else None        # (a pass opens from Python, before its first block)
+        for index, entry in enumerate(self.spec.schedule):
+            described = self.blocks[entry.layer].native_descriptor(ctx.cache_view(index))
+            if described is not None:
+                self.blocks[entry.layer].mixer.in_native_layer = True
+            # (a pass opens from Python, before its first block)
+            self._native[index] = described if kernels.NATIVE_LAYERS and entry.opens_pass is None else None
         runs, index = [], 0
         while index < len(self.spec.schedule):
             if self._native.get(index) is None:

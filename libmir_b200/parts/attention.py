@@ -85,6 +85,9 @@ class SoftmaxAttention(Mixer):
         if s.fixed_sink is not None:
             self.sinks = torch.full((s.heads,), float(s.fixed_sink), dtype=torch.float32, device=env.device)
 
+    # whether the layer is of the kind that the native executor runs: the same kernels then, whoever launches them
+    in_native_layer = False
+
     @property
     def graph_safe(self):
         return self.position is None or self.position.graph_safe
@@ -345,13 +348,14 @@ class SoftmaxAttention(Mixer):
             singles = ctx.num_rows if ctx.decode_only else ctx.single_rows
             if singles:
                 longest = ctx.max_context if ctx.decode_only else ctx.single_context
-                partition, count, floats = kernels.decode_attention_plan(singles, s.heads, s.kv_heads, s.head_dim,
-                                                                         cache.page_size, longest)
+                short = ctx.decode_only and self.in_native_layer and kernels.decode_attention_short(singles, s.kv_heads, longest)
+                partition, count, floats = (kernels.SHORT_KEYS, 1, 0) if short else \
+                    kernels.decode_attention_plan(singles, s.heads, s.kv_heads, s.head_dim, cache.page_size, longest)
                 scratch = ctx.alloc((floats,), torch.float32) if floats else None
                 kernels.decode_attention(qkv[:singles], out[:singles], cache.k_pages, cache.v_pages,
                                          group.block_table[:singles], ctx.positions, cache.page_size, s.heads,
                                          s.kv_heads, s.head_dim, s.scale, s.window, partition, count, scratch,
-                                         sinks=self.sinks, gate=gate[:singles] if gate is not None else None)
+                                         sinks=self.sinks, gate=gate[:singles] if gate is not None else None, short=short)
             if singles < ctx.num_rows:
                 kernels.prefill_attention(qkv, out, cache.k_pages, cache.v_pages, group.block_table[singles:],
                                           ctx.query_starts[singles:], ctx.context_lens[singles:], cache.page_size,

@@ -401,6 +401,35 @@ def test_native_executor_and_python_parts_launch_the_same_work(tmp_path, name, d
     check(results[0][-1].numpy(), reference[329], TOL[dtype], "against the plain implementation")
 
 
+@pytest.mark.parametrize("captured", [False, True])
+@pytest.mark.parametrize("name, page", [("E", 16), ("E", 8), ("F", 8)])
+def test_native_executor_and_python_parts_agree_on_short_contexts(tmp_path, name, page, captured, monkeypatch):
+    """Decoded tokens whose contexts grow past 128 keys: the executor and the parts choose the same attention kernel at every
+    step, so the logits are the same bits."""
+    from libmir_b200 import StepEntry, kernels
+    from libmir_b200.sampling import RequestSampler
+    config = ALL[name]
+    folder = make_folder(tmp_path, config, seed=31, dtype="bfloat16", sharpen=4.0)
+    rng = np.random.default_rng(31)
+    first, second = random_ids(rng, config["vocab_size"], 140), random_ids(rng, config["vocab_size"], 60)
+    results, ran = [], []
+    for native in (True, False):
+        monkeypatch.setattr(kernels, "NATIVE_LAYERS", native)
+        model = load(folder, "bfloat16", page_size=page, pages=128)
+        model.admit("a"); model.admit("b")
+        logits = [model.step([StepEntry("a", first[:120], [119]), StepEntry("b", second[:31], [30])]).logits.clone()]
+        before = kernels.launch_counts()
+        for offset in range(14):
+            logits.append(model.step([StepEntry("a", [first[120 + offset]], [0]), StepEntry("b", [second[31 + offset]], [0])],
+                                     [RequestSampler(), RequestSampler()] if captured else None).logits.clone())
+        after = kernels.launch_counts()
+        ran.append([after.get(kind, 0) - before.get(kind, 0) for kind in ("decode_attention", "decode_attention_tc")])
+        results.append(torch.cat(logits).cpu())
+        model.unload()
+    assert torch.equal(results[0], results[1]) and ran[0] == ran[1], ran
+    assert ran[0][0] > 0 and (ran[0][1] > 0) == (name == "E"), ran           # (heads of 64 know the mma.sync kernel only)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_repeated_greedy_decode_steps_take_the_short_path_and_stay_right(tmp_path, dtype):
     """Captured greedy decode steps of the same requests skip what cannot have changed (StepRunner._step_again) until
