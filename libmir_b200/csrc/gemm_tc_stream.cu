@@ -432,19 +432,30 @@ int g_forced_rows = 0;
 // Tile height and how many CTAs share K.  Measured on B200 (8 rows, inside a CUDA graph, us): whole 128-row tiles
 // beat 64- and 32-row tiles at every shape (QKV 9.0 / 15.5 / 18.1, output projection 7.7 / 10.5 / 11.5), and K is
 // best cut as far as one wave of CTAs allows (three fit on an SM): output projection 7.7 with 8 CTAs per tile,
-// 10.4 with 4, 16.8 with 2.  A wave that is nearly full (385 to 444 CTAs) leaves no room for the next kernel's: Doderax, whose
-// mixers' inputs are 50 tiles, whole call 12.32 ms with 400 CTAs, 12.18 with 200; up to 300 CTAs only, Qwen3-4B sizes 25.0 to 25.8.
-constexpr int kMostCtas = 384;
+// 10.4 with 4, 16.8 with 2.
+// One wave is what the GPU holds of whole clusters: a cluster lies within a GPC, so three CTAs an SM make 444 CTAs in clusters
+// of two, 416 in clusters of four and 384 in clusters of eight (cudaOccupancyMaxActiveClusters); what is left over runs behind
+// all others.  Decode steps of 12 layers, one row (us): clusters of eight 400 CTAs (QKV of 50 tiles, K 2,560) 650, cut in four
+// 617; outputs of 50 tiles 1,855 and 1,771; 384 CTAs 421, cut in four 436.  Clusters of four 400 CTAs (QKV of 100 tiles, K 2,048)
+// 514, cut in two 551; gate-up of 100 tiles 502 and 513; but 432 CTAs 706 and 673.  Clusters of two 444 CTAs 997, not cut 1,023.
+int most_ctas(int splits) { return splits >= 8 ? 384 : splits == 4 ? 416 : 444; }
 void choose_shape(int n, int total_steps, bool swiglu, int slots, int* tile_rows, int* splits) {
   const int rows = swiglu ? 64 : 128;
   const long long tiles = (long long)((n + rows - 1) / rows) * slots;
   int s = 1;
-  while (s < 8 && tiles * s * 2 <= kMostCtas && total_steps / (s * 2) >= 4) s *= 2;
+  while (s < 8 && tiles * s * 2 <= most_ctas(s * 2) && total_steps / (s * 2) >= 4) s *= 2;
   *tile_rows = rows;
   *splits = s;
 }
 
 }  // namespace
+
+// How many CTAs share K in a product of n columns (SwiGLU: of each half), `slots` of them side by side.
+MIR_EXPORT int mir_gemm_tc_stream_splits(int n, int k, int swiglu, int slots) {
+  int tile_rows, splits;
+  choose_shape(n, (k + kStepK - 1) / kStepK, swiglu != 0, slots, &tile_rows, &splits);
+  return splits;
+}
 
 // Bytes of the ring of a product of `ctas` CTAs.
 MIR_EXPORT int mir_gemm_tc_stream_ring(long long ctas) {

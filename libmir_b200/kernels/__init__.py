@@ -189,6 +189,7 @@ _SIGNATURES = {
         "mir_gemm_tc_stream_error": [],
         "mir_gemm_tc_stream_set_splits": [c_int, c_int, c_int],
         "mir_gemm_tc_stream_ring": [c_longlong],
+        "mir_gemm_tc_stream_splits": [c_int, c_int, c_int, c_int],
         "mir_gemm_tc_bf16": [c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                              c_void_p],
         "mir_gemm_tc_stream_side_by_side_bf16": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p],

@@ -428,11 +428,13 @@ def test_products_side_by_side(groups, rows, n, k):
     assert ((out.cpu().double() - want).abs() <= bound).all()
 
 
-@pytest.mark.parametrize("n,k", [(14208, 520), (14209, 512), (24576, 512), (24577, 520), (28416, 256), (28417, 264)])
+@pytest.mark.parametrize("n,k", [(14208, 520), (14209, 512), (24576, 512), (24577, 520), (28416, 256), (28417, 264),
+                                 (28416, 512), (28417, 512), (6144, 2048), (6145, 2056), (13312, 1024), (13313, 1032)])
 @pytest.mark.parametrize("rows", [1, 32])
 def test_weight_streams_on_both_sides_of_the_rings_and_the_cuts(rows, n, k):
-    """111 and 112 tiles of columns cut in two (222 and 224 blocks), 192 and 193 (384 blocks, or no cut), 222 and 223 that are not
-    cut: the large ring and the small one, with steps that do not fill it."""
+    """111 and 112 tiles of columns cut in two (222 and 224 blocks), 192, 193 and 222 cut in two, 222 and 223 that are not; 48
+    cut in eight and 49 in four, 104 cut in four and 105 in two: the large ring and the small one, with steps that do not fill
+    it."""
     from libmir_b200 import kernels
     torch.manual_seed(n + rows)
     x, w = torch.randn(rows, k).bfloat16(), torch.randn(n, k).bfloat16()

@@ -155,3 +155,17 @@ def test_a_weight_streams_ring_is_the_one_asked_for():
         assert lib.mir_gemm_tc_stream_set_splits(0, 201, 0) != 0 and lib.mir_gemm_tc_stream_set_splits(0, 31, 0) != 0
     finally:
         lib.mir_gemm_tc_stream_set_splits(0, 0, 0)
+
+
+@pytest.mark.parametrize("tiles, splits", [(1, 8), (48, 8), (49, 4), (50, 4), (55, 4), (100, 4), (104, 4), (105, 2), (192, 2), (193, 2), (222, 2),
+                                           (223, 1), (1000, 1)])
+@pytest.mark.parametrize("swiglu", [0, 1])
+def test_weight_streams_are_cut_as_far_as_whole_clusters_fit_at_once(tiles, splits, swiglu):
+    """384 blocks in clusters of eight, 416 in clusters of four, 444 in clusters of two; a block has four steps of 64 or more."""
+    lib, width = kernels.library("bf16"), 64 if swiglu else 128
+    for n in (tiles * width, tiles * width - width + 1):
+        assert lib.mir_gemm_tc_stream_splits(n, 4096, swiglu, 1) == splits
+        assert lib.mir_gemm_tc_stream_splits(n, 511, swiglu, 1) == min(splits, 2)
+        assert lib.mir_gemm_tc_stream_splits(n, 448, swiglu, 1) == 1
+    if tiles % 2 == 0:
+        assert lib.mir_gemm_tc_stream_splits(tiles // 2 * width, 4096, swiglu, 2) == splits
