@@ -88,6 +88,7 @@ constexpr int kStreamThreads = kRows * kParts;
 // handed out to four warps at a time, so the twentieth warp costs the others nothing
 __host__ __device__ constexpr int threads_for(int streams) { return (4 + 8 * streams) * 32; }
 constexpr int kFirstSoftmaxWarp = 2;
+static_assert(Layout<kDim>::kSmemBytes + kLeastSharedBeside > kSharedOfSm, "no other kernel with tensor memory beside this one");
 constexpr uint32_t kTmemColumns = 512;      // S0 at 0, S1 at 128, O of stream 0 at 256, of stream 1 at 384
 constexpr float kRescaleThreshold = 8.0f;   // log2 of how far a tile's maximum may exceed the running one
 

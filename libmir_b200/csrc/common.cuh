@@ -25,10 +25,16 @@ void mir_count_launch(const char* what);   // launches that do not end in mir_ch
 // the stream is still draining.  Its CTAs run up to mir::grid_dependency_wait() (prefetching what does not
 // depend on the earlier kernel, e.g. weights) and block there until the earlier kernel has completed and
 // its writes are visible.  Every kernel launched through mir_launch calls grid_dependency_wait() before it
-// reads an activation or writes anything, so the order of memory effects is the order of the stream.  What a kernel may
+// reads an activation or writes anything, so the order of memory effects is the order of the stream; one that has nothing to do
+// waits as well, or what follows would run beside the kernels in front of it.  What a kernel may
 // read before it waits (weights, a step's positions, slots and block tables, keys of earlier steps) is written by copies
 // and by kernels without grid_launch_dependents(): a run of kernels that release one another early may all be resident
-// together, but none of them starts before the last kernel that does not.
+// together, but none of them starts before the last kernel that does not.  Only the wait promises that such a kernel's stores
+// are visible, its end alone does not: between it and the reader lies one more kernel that waits (in a step the embedding).  A
+// weight or slot written by a kernel that is released early, or by the launch directly in front, is not covered.
+// Kernels that take all 512 columns of tensor memory (csrc/gemm_tc.cu, csrc/attention_tc.cu) take so much shared memory that no
+// other kernel with tensor memory fits beside them on an SM: one of those that had its columns already, and waits here for the
+// kernel in front to end, would keep it from ever getting its own.
 bool mir_pdl_enabled();
 bool mir_pdl_for_streaming();   // also true in the mode that launches only the weight-streaming kernels this way
 

@@ -252,8 +252,9 @@ int launch(bool early, Kernel kernel, dim3 grid, int threads, int smem, const Pr
 template <int MT, bool WIDE>
 int launch_rows(const Product& p) {
   constexpr int smem = kRowsStages * (kRowsColumns + MT) * (kRowsDepth + 4) * (int)sizeof(float);
-  // Started early, a grid that does not fill the GPU lands on the SMs that are left first, several CTAs on one (three rows,
-  // K 2,048: 128 CTAs 18.8 us plainly, 23.4 early; 192 12.0 and 15.2; 688 34.6 and 28.1).
+  // Started early, a grid that does not fill the GPU lands on the SMs that are left first, several CTAs on one.  Within decode
+  // steps of three rows, plainly / early (us): 128 CTAs, K 2,048 and 5,504 together, 18.8 / 23.4; 192, K 2,048, 12.0 / 15.2; 688
+  // 34.6 / 28.1.  One such product behind the other: 128 CTAs, K 2,048 11.9 / 11.9, K 5,504 27.3 / 26.7; 192 13.0 / 14.2; 688 35 / 32.
   const int ctas = (p.n + kRowsColumns - 1) / kRowsColumns;
   return launch(ctas >= 3 * mir_sm_count(), gemm_f32_rows_kernel<MT, WIDE>, dim3(ctas), kRowsThreads + kRowsLoaders, smem, p);
 }

@@ -52,6 +52,7 @@ constexpr int kEpilogueWarps = 8;          // two per quarter of the accumulator
 constexpr int kThreads = (2 + kEpilogueWarps) * 32;  // producer warp, issuer warp, epilogue warps
 constexpr int kPlaces = 64;                 // tiles of a CTA whose places are looked up before the first of them
 constexpr uint32_t kTmemColumns = 512;      // two accumulators of up to 256 columns
+static_assert(kStages * kStageStride + 1024 + kLeastSharedBeside > kSharedOfSm, "no other kernel with tensor memory beside this one");
 // GELU: STORE of gelu_tanh(acc), no bias; GELU_ERF: the same with the exact form 0.5 z (1 + erf(z / sqrt 2)); RELU2: the
 // same with the square of relu
 enum Epilogue : int { STORE = 0, ACCUM = 1, F32 = 2, SWIGLU = 3, GELU = 4, GELU_ERF = 5, RELU2 = 6 };

@@ -149,8 +149,10 @@ MIR_EXPORT int mir_decode_partition_keys(int rows, int heads, int kv_heads, int 
 // Python), run the mma.sync kernel on one partition, one CTA for a request and KV head: few requests whose contexts all fit
 // into one tile of keys.  The tcgen05 kernel's chain (two products through tensor memory, four barriers) is longer than the
 // work there.  Decode steps at Qwen3-4B sizes (8 KV heads), 12 layers, tcgen05 / mma.sync (us): up to 128 keys 1 request 706 /
-// 686, 4 722 / 707, 8 737 / 728, 24 886 / 878, but 53 1,045 / 1,075; up to 256 keys 1 request 720 / 740, 24 907 / 918.
-constexpr int kShortUnits = 192;                              // requests x KV heads: the last pair of figures that gained
+// 686, 4 722 / 707, 8 737 / 728, 24 886 / 878, but 53 1,045 / 1,075; up to 256 keys 1 request 720 / 740, 24 907 / 918.  Other
+// groupings of heads, width 4,096, up to 80 keys (from one request to the rule's last): 32 heads on 2 KV heads 1 662 / 577, 64
+// 900 / 809; 48 on 4 1 737 / 657, 48 938 / 918; 64 on 8 1 757 / 725, 24 885 / 851; 32 on 32 1 663 / 659, 6 702 / 686.
+constexpr int kShortUnits = 192;                              // requests x KV heads: 24 requests above; 256 still gain, 512 lose
 MIR_EXPORT int mir_decode_attention_short(int rows, int kv_heads, int longest) {
   return longest <= MIR_SHORT_KEYS && (long long)rows * kv_heads <= kShortUnits;
 }

@@ -76,6 +76,8 @@ int mir_sm_count() {
   return count;
 }
 
+MIR_EXPORT int mir_multiprocessors() { return mir_sm_count(); }
+
 MIR_EXPORT int mir_abi_version() { return 1; }
 
 // What a decode step uploads: once `event` says that the last upload has left the pinned block, `bytes` of `from` go into that

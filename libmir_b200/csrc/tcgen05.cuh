@@ -13,6 +13,10 @@ namespace tc {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// A kernel that takes all columns of tensor memory keeps every other kernel with tensor memory off its SM by shared memory (see
+// common.cuh): the least such a kernel's CTA takes (csrc/gemm_tc_stream.cu, two stages), and what an SM has.
+constexpr int kLeastSharedBeside = 36 * 1024, kSharedOfSm = 228 * 1024;
+
 constexpr unsigned long long kWaitNanoseconds = 500ull * 1000ull * 1000ull;
 
 __device__ __forceinline__ unsigned long long global_nanoseconds() {

@@ -94,6 +94,7 @@ _SIGNATURES = {
         "mir_moe_route": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                           c_int, c_float, c_int, c_int, c_void_p],
         "mir_moe_tile_slots": [c_int, c_int, c_int],
+        "mir_multiprocessors": [],
         "mir_upload": [c_void_p, c_void_p, c_void_p, c_size_t, c_void_p, c_void_p],
         "mir_moe_plan_few_takes": [c_int] * 5,
         "mir_moe_plan_few": [c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -315,7 +316,9 @@ def set_programmatic_launch(mode) -> None:
     """How kernels are launched: 0 / False plainly; 1 / True (the default) with programmatic stream serialization (a
     kernel's start overlaps the previous kernel's end; every kernel waits for its predecessor before it touches
     activations), but for the few whose CTAs each want an SM of their own; 2 only the weight-streaming products, whose
-    first weights are then on their way while the kernel before them drains."""
+    first weights are then on their way while the kernel before them drains.  What is read ahead of that wait (weights of
+    products and norms, slots, positions, block tables) must not come from the launches in front of it: between the kernel
+    that writes it and the one that reads it lies a copy, a library's kernel or decode_prepare, and one launch more."""
     for name in ("core", "bf16"):
         lib = library(name)
         lib.mir_set_pdl.argtypes = [c_int]
@@ -906,7 +909,7 @@ def latent_attention_plan(num_rows: int, max_pairs: int, max_context: int) -> tu
     most of the GPU idle (decoded tokens)."""
     blocks = max(1, num_rows * (-(-max_pairs // 64)))
     tiles = max(1, -(-max_context // 64))
-    sms = 148
+    sms = library("core").mir_multiprocessors()
     # one wave of CTAs, two tiles or more a partition (measured at 8 rows x 2,049 keys: 31 us with 17 partitions, 43
     # with 33, 65 with 4; at 64 rows 123 us with 2, 133 with 4), a tile each where that is less than a wave
     partitions = max(1, min(tiles if blocks * tiles <= sms else max(1, tiles // 2), sms // blocks, 64))
@@ -1107,9 +1110,12 @@ def expert_tile_pairs(dtype: torch.dtype, width: int, inter: int) -> int:
     return 128 if (EXPERT_TENSOR_CORES and dtype == torch.bfloat16 and width % 8 == 0 and inter % 8 == 0) else 8
 
 
-# Up to this many tokens a step's routed experts run as weight streams (0: never).  Router to sum, 64 experts of 1,024, width
-# 2,048, 6 chosen, tiles of 128 / streams (us): 1 token 46.6 / 29.2, 3 64 / 46, 8 111 / 93, 16 118 / 113; but 20 129 / 132, 32
-# 148 / 158: nearly all experts are hit then, both are bound by the weights, and places counted over all pairs cost more.
+# Up to this many tokens a step's routed experts run as weight streams (0: never).  Router to sum, tiles of 128 / streams (us), at
+# 1, 8, 16, 20 and 32 tokens: 64 experts of 1,024, width 2,048, 6 chosen 46.6 / 28.0, 101 / 85, 119 / 112, 137 / 133, 150 / 154;
+# 128 of 768, 8 chosen 51 / 35, 114 / 99, 151 / 140, 165 / 173, 190 / 205; 256 of 512, 8 chosen 44 / 33, 90 / 87, 128 / 124, 152 /
+# 158, 187 / 189; 16 of 1,024, 1 chosen 37 / 17, 47 / 28, 55 / 37, 58 / 43, 56 / 48; 8 of 14,336, width 4,096, 2 chosen 208 / 129,
+# 434 / 398, 462 / 425, 465 / 439, 466 / 439.  Beyond 16 the places counted over all pairs cost more where many are chosen, and
+# nearly all experts are hit, so that both are bound by the weights.
 EXPERT_FEW_TOKENS = 16
 
 
