@@ -306,8 +306,10 @@ def library(name: str) -> ctypes.CDLL:
 
 
 def upload(event: torch.cuda.Event, pinned: torch.Tensor, block: np.ndarray, device: torch.Tensor) -> None:
-    """`block` through the pinned tensor into `device` (all int32 of one size), in the order of the current stream, once
+    """`block` through the pinned tensor into the front of `device` (all int32), in the order of the current stream, once
     `event` (recorded before) says that the last upload has left the pinned tensor; records `event` behind the copy."""
+    _require(block.dtype == np.int32 and block.flags.c_contiguous and block.size <= pinned.numel() and block.size <= device.numel(),
+             "upload: a contiguous int32 block that fits both buffers is needed")
     lib = library("core")
     _check(lib, lib.mir_upload(event.cuda_event, pinned.data_ptr(), block.ctypes.data, block.nbytes, device.data_ptr(), _stream()))
 

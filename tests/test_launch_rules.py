@@ -2,11 +2,13 @@
 
 import re
 from pathlib import Path
+from types import SimpleNamespace
 
+import numpy as np
 import pytest
 import torch
 
-from libmir_b200 import kernels
+from libmir_b200 import KernelError, kernels
 
 
 class Recorder:
@@ -169,3 +171,23 @@ def test_weight_streams_are_cut_as_far_as_whole_clusters_fit_at_once(tiles, spli
         assert lib.mir_gemm_tc_stream_splits(n, 448, swiglu, 1) == 1
     if tiles % 2 == 0:
         assert lib.mir_gemm_tc_stream_splits(tiles // 2 * width, 4096, swiglu, 2) == splits
+
+
+@pytest.mark.parametrize("block, pinned, device, fits", [(8, 8, 8, True), (8, 8, 20, True), (8, 7, 20, False), (8, 20, 7, False)])
+def test_an_upload_stays_within_its_buffers(recorder, block, pinned, device, fits):
+    event = SimpleNamespace(cuda_event=0)
+    buffers = torch.zeros(pinned, dtype=torch.int32), np.zeros(block, np.int32), torch.zeros(device, dtype=torch.int32)
+    if fits:
+        kernels.upload(event, *buffers)
+        assert recorder.last("mir_upload")[3] == 4 * block
+        return
+    with pytest.raises(KernelError, match="upload"):
+        kernels.upload(event, *buffers)
+    assert not recorder.calls
+
+
+@pytest.mark.parametrize("block", [np.zeros(4, np.int64), np.zeros(16, np.int32)[::2]])
+def test_an_upload_takes_words_that_lie_side_by_side(recorder, block):
+    with pytest.raises(KernelError, match="upload"):
+        kernels.upload(SimpleNamespace(cuda_event=0), torch.zeros(64, dtype=torch.int32), block, torch.zeros(64, dtype=torch.int32))
+    assert not recorder.calls
