@@ -347,7 +347,9 @@ decode_attention_kernel(const bf16* __restrict__ q, size_t q_stride, const bf16*
   }
   // the true first key of the tile numbered n, and the first true key beyond what may be read of it
   auto true_key = [&](int n) { return n < kept_tiles_end ? n : n + shift; };
-  auto true_limit = [&](int n) { return n < kept_tiles_end ? kept_end : min(context, part_end + shift); };
+  // (a position beyond what the table holds reads no entry: its keys count as released)
+  const int held = table_width * page_size;
+  auto true_limit = [&](int n) { return min(held, n < kept_tiles_end ? kept_end : min(context, part_end + shift)); };
 
   // this warp's buffers: [stage][16 rows of K, 16 rows of V]
   bf16* stage_base = reinterpret_cast<bf16*>(smem_raw) + (size_t)warp * kDecodeStages * STAGE_ELEMS;

@@ -465,3 +465,27 @@ def test_grouped_products_of_more_tiles_than_are_looked_up_at_once(experts, widt
         # eight products in 32 bits, each partial sum off by at most 2^-24 of the sum of their sizes
         assert (error <= inter * 2 ** -24 * torch.einsum("pi,pwi->pw", x.abs(), rows.abs())).all()
     assert kernels.tensor_core_linear_error() == 0
+
+
+@pytest.mark.parametrize("position, keep_first, window", [(40, 0, None), (33, 0, None), (70, 0, 30), (52, 4, 25), (127, 20, 100)])
+def test_decoded_tokens_read_no_page_beyond_their_table(position, keep_first, window):
+    """A position beyond what the block table holds: the mma.sync kernel takes the keys there as released, as the tcgen05 kernel
+    does.  What lies behind the table in memory are pages whose keys and values would show."""
+    from libmir_b200 import kernels
+    torch.manual_seed(position)
+    rows, width, wide, page, heads, dim = 2, 2, 8, 16, 4, 128
+    qkv = torch.randn(rows, 3 * heads * dim).bfloat16().cuda()
+    pages = torch.randn(2, 32 * page, heads, dim).bfloat16().cuda()
+    pages[:, 16 * page:] = float("nan")
+    memory = torch.arange(16, 32, dtype=torch.int32, device="cuda")
+    memory[:rows * width] = torch.arange(rows * width)
+    narrow, same = memory[:rows * width].view(rows, width), torch.full((rows, wide), -1, dtype=torch.int32, device="cuda")
+    same[:, :width] = narrow
+    positions = torch.full((rows,), position, dtype=torch.int32, device="cuda")
+    outputs = []
+    for table in (narrow, same):
+        outputs.append(torch.full((rows, heads * dim), float("nan"), dtype=torch.bfloat16, device="cuda"))
+        numbering = torch.zeros(rows, dtype=torch.int32, device="cuda")
+        kernels.decode_attention(qkv, outputs[-1], pages[0], pages[1], table, positions, page, heads, heads, dim, dim ** -0.5, window,
+                                 128, 1, None, keep_first=keep_first, numbering=numbering, short=keep_first == 0)
+    assert torch.isfinite(outputs[0]).all() and torch.equal(*outputs)
